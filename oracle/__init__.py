@@ -30,11 +30,11 @@ def _dp(a):
 
 def build(reference=None):
     """Compile the restatement, and oracle/_ref when a reference tree is given
-    (the argument, else $SCP3_REFERENCE) and exists."""
+    (the argument, else $SCP3_REFERENCE) and holds the sources."""
     import subprocess
     subprocess.run(["make", "-s", "-C", HERE, "all"], check=True)
     ref = reference or os.environ.get("SCP3_REFERENCE")
-    if ref and os.path.isdir(ref):
+    if ref and os.path.exists(os.path.join(ref, "sobol.cpp")):
         subprocess.run(["make", "-s", "-C", HERE, "ref", "REF=" + ref], check=True)
 
 
