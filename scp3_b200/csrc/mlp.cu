@@ -12,9 +12,9 @@
 //              activations stored BF16 for the next layer and FP32
 //              pre-activations kept for training;
 //              head_kernel: y = h3 . w4 + b4, one warp per sample
-//   backward   FP32 register-tiled GEMMs for dX = dZ W and dW = dZ^T X,
-//              gelu_backward for dZ = dH * GELU'(Z), a per-column reduction for
-//              the bias gradients
+//   backward   FP32 register-tiled GEMMs for dX = dZ W (GELU' and the bias
+//              gradients' row sums in its epilogue) and dW = dZ^T X (samples split
+//              over CTAs)
 //   update     adam_kernel on FP32 master weights, refreshing the BF16 copies
 //
 // Layout: weights W_l row-major [out][in] (in padded to a multiple of 32);
@@ -252,60 +252,213 @@ __global__ void input_kernel(const float* __restrict__ q, int M, int nin, int ki
     X[e] = __float2bfloat16_rn(k < nin ? q[(size_t)m * nin + k] : 0.0f);
 }
 
-// Generic FP32 GEMM C[M][N] = sum_k A(m,k) B(k,n) with strided operands (A(m,k)
-// at A[m*sam + k*sak], B(k,n) at B[k*sbk + n*sbn]), 64x64 tiles, 4x4 per thread.
-template <typename TA, typename TB>
-__global__ void __launch_bounds__(256) gemm_f32(const TA* __restrict__ A, int64_t sam, int64_t sak,
-                                                 const TB* __restrict__ B, int64_t sbk, int64_t sbn, int M, int N, int K,
-                                                 float* __restrict__ C, int64_t ldc, float beta)
+// ---------------------------------------------------------------- backward
+// FP32 throughout.  One 64 x 64 tile per CTA of 64 threads, an 8 x 8 block per
+// thread (rows 4 ty + {0..3} and 32 + 4 ty + {0..3}, columns likewise in tx), 16-deep
+// K slices double-buffered in shared memory: four 16-byte shared loads per 64
+// FMAs, ten CTAs per SM.
+//   dz_gemm   dZ_{l-1} = (dZ_l W_l) * GELU'(Z_{l-1}); tiles over (samples, inputs),
+//             the 64-row column sums of its result (bias gradient) beside it
+//   dw_gemm   gW_l = dZ_l^T X_l, the samples split over up to kDwSplits CTAs per
+//             tile, each with its own partial
+//   head_backward  dZ_2 = dy w_3 * GELU'(Z_2) and the 64-row sums of dy H_2 and dZ_2
+//   sum_parts adds partials and row sums in order (deterministic)
+// What bounds it: FP32 FMA issue (9 GFLOP per 2^14-sample batch of the 48-256-256-256-1
+// network).  A batch of 2^14: 10.7 ms per loss_and_grad call before, 0.83 ms now, of
+// which dw_gemm 174 us and dz_gemm 174 us, 25-29 TFLOP/s (before, each dW tile was
+// one CTA over all samples, 16 CTAs, 2.5 ms each, and the column sums one thread each,
+// 0.9 ms each).
+constexpr int kBT = 64, kBKs = 16, kBThreads = 64;
+constexpr int kDwSplits = 64;      // most partials of a weight gradient
+constexpr int kDwRows = 256;       // samples per partial until kDwSplits are reached
+
+struct TileAcc {
+    float v[8][8];
+};
+
+__device__ __forceinline__ void tile_fma(const float (*As)[kBT + 4], const float (*Bs)[kBT + 4], int tx, int ty,
+                                         TileAcc& c)
 {
-    __shared__ float As[16][65], Bs[16][65];
-    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-    const int m0 = blockIdx.x * 64, n0 = blockIdx.y * 64;
-    float acc[4][4] = {};
-    for (int k0 = 0; k0 < K; k0 += 16) {
-        for (int e = tid; e < 64 * 16; e += 256) {
-            const int r = e >> 4, k = e & 15;
-            const int m = m0 + r, n = n0 + r, kk = k0 + k;
-            As[k][r] = (m < M && kk < K) ? (float)A[m * sam + kk * sak] : 0.0f;
-            Bs[k][r] = (n < N && kk < K) ? (float)B[kk * sbk + n * sbn] : 0.0f;
+#pragma unroll
+    for (int k = 0; k < kBKs; k++) {
+        float a[8], b[8];
+        *reinterpret_cast<float4*>(a) = *reinterpret_cast<const float4*>(&As[k][4 * ty]);
+        *reinterpret_cast<float4*>(a + 4) = *reinterpret_cast<const float4*>(&As[k][32 + 4 * ty]);
+        *reinterpret_cast<float4*>(b) = *reinterpret_cast<const float4*>(&Bs[k][4 * tx]);
+        *reinterpret_cast<float4*>(b + 4) = *reinterpret_cast<const float4*>(&Bs[k][32 + 4 * tx]);
+#pragma unroll
+        for (int i = 0; i < 8; i++)
+#pragma unroll
+            for (int j = 0; j < 8; j++) c.v[i][j] = fmaf(a[i], b[j], c.v[i][j]);
+    }
+}
+
+__device__ __forceinline__ int tile_pos(int q, int i) { return (i < 4 ? 0 : 32) + 4 * q + (i & 3); }
+
+// grid (M / 64, nin / 64); hid and nin multiples of 64 (layers 1 and 2).
+__global__ void __launch_bounds__(kBThreads) dz_gemm(const float* __restrict__ dZ, const float* __restrict__ W,
+                                                     const float* __restrict__ Zin, int hid, int nin,
+                                                     float* __restrict__ out, float* __restrict__ rowsum)
+{
+    __shared__ __align__(16) float As[2][kBKs][kBT + 4], Bs[2][kBKs][kBT + 4];
+    const int tid = threadIdx.x, tx = tid & 7, ty = tid >> 3;
+    const int m0 = blockIdx.x * kBT, n0 = blockIdx.y * kBT;
+    float4 ra[4], rb[4];
+    auto fetch = [&](int k0) {
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int e = tid + 64 * i;
+            ra[i] = *reinterpret_cast<const float4*>(dZ + (size_t)(m0 + (e >> 2)) * hid + k0 + 4 * (e & 3));
+            rb[i] = *reinterpret_cast<const float4*>(W + (size_t)(k0 + (e >> 4)) * nin + n0 + 4 * (e & 15));
         }
-        __syncthreads();
+    };
+    auto stash = [&](int buf) {
 #pragma unroll
-        for (int k = 0; k < 16; k++) {
-            float av[4], bv[4];
-#pragma unroll
-            for (int i = 0; i < 4; i++) av[i] = As[k][ty + 16 * i], bv[i] = Bs[k][tx + 16 * i];
-#pragma unroll
-            for (int i = 0; i < 4; i++)
-#pragma unroll
-                for (int j = 0; j < 4; j++) acc[i][j] += av[i] * bv[j];
+        for (int i = 0; i < 4; i++) {
+            const int e = tid + 64 * i, r = e >> 2, k = 4 * (e & 3);
+            As[buf][k][r] = ra[i].x, As[buf][k + 1][r] = ra[i].y, As[buf][k + 2][r] = ra[i].z, As[buf][k + 3][r] = ra[i].w;
+            *reinterpret_cast<float4*>(&Bs[buf][e >> 4][4 * (e & 15)]) = rb[i];
         }
+    };
+    TileAcc c{};
+    fetch(0);
+    stash(0);
+    __syncthreads();
+    for (int k0 = 0, cur = 0; k0 < hid; k0 += kBKs, cur ^= 1) {
+        const bool more = k0 + kBKs < hid;
+        if (more) fetch(k0 + kBKs);
+        tile_fma(As[cur], Bs[cur], tx, ty, c);
+        if (more) stash(cur ^ 1);
         __syncthreads();
     }
+    float cs[8] = {};
 #pragma unroll
-    for (int i = 0; i < 4; i++)
+    for (int i = 0; i < 8; i++) {
+        const size_t row = (size_t)(m0 + tile_pos(ty, i)) * nin + n0;
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const int m = m0 + ty + 16 * i, n = n0 + tx + 16 * j;
-            if (m < M && n < N) C[(size_t)m * ldc + n] = acc[i][j] + (beta != 0.0f ? beta * C[(size_t)m * ldc + n] : 0.0f);
+        for (int h = 0; h < 2; h++) {
+            const float4 z = *reinterpret_cast<const float4*>(Zin + row + 32 * h + 4 * tx);
+            float4 d;
+            d.x = c.v[i][4 * h] * gelu_grad(z.x), d.y = c.v[i][4 * h + 1] * gelu_grad(z.y);
+            d.z = c.v[i][4 * h + 2] * gelu_grad(z.z), d.w = c.v[i][4 * h + 3] * gelu_grad(z.w);
+            *reinterpret_cast<float4*>(out + row + 32 * h + 4 * tx) = d;
+            cs[4 * h] += d.x, cs[4 * h + 1] += d.y, cs[4 * h + 2] += d.z, cs[4 * h + 3] += d.w;
+        }
+    }
+    float* red = &As[0][0][0];                         // [8 ty][64 columns]; the loop ended on a barrier
+#pragma unroll
+    for (int j = 0; j < 8; j++) red[ty * kBT + tile_pos(tx, j)] = cs[j];
+    __syncthreads();
+    float t = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 8; i++) t += red[i * kBT + tid];
+    rowsum[(size_t)blockIdx.x * nin + n0 + tid] = t;
+}
+
+// grid (hid / 64, ceil(nin / 64), splits); ldx (X's row length) is a multiple of 32.
+__global__ void __launch_bounds__(kBThreads) dw_gemm(const float* __restrict__ dZ, const __nv_bfloat16* __restrict__ X,
+                                                     int M, int hid, int nin, int ldx, float* __restrict__ part)
+{
+    __shared__ __align__(16) float As[2][kBKs][kBT + 4], Bs[2][kBKs][kBT + 4];
+    const int tid = threadIdx.x, tx = tid & 7, ty = tid >> 3;
+    const int o0 = blockIdx.x * kBT, i0 = blockIdx.y * kBT;
+    // samples [mb, me) in 16-row steps (M is a multiple of 64)
+    const int steps = M / kBKs, mb = (int)((long long)steps * blockIdx.z / gridDim.z) * kBKs,
+              me = (int)((long long)steps * (blockIdx.z + 1) / gridDim.z) * kBKs;
+    float4 ra[4];
+    uint4 rb[2];
+    auto fetch = [&](int m) {
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int e = tid + 64 * i;
+            ra[i] = *reinterpret_cast<const float4*>(dZ + (size_t)(m + (e >> 4)) * hid + o0 + 4 * (e & 15));
+        }
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            const int e = tid + 64 * i, col = i0 + 8 * (e & 7);
+            rb[i] = col < ldx ? *reinterpret_cast<const uint4*>(X + (size_t)(m + (e >> 3)) * ldx + col)
+                              : make_uint4(0, 0, 0, 0);
+        }
+    };
+    auto stash = [&](int buf) {
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int e = tid + 64 * i;
+            *reinterpret_cast<float4*>(&As[buf][e >> 4][4 * (e & 15)]) = ra[i];
+        }
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            const int e = tid + 64 * i;
+            const uint32_t w[4] = {rb[i].x, rb[i].y, rb[i].z, rb[i].w};
+            float f[8];
+#pragma unroll
+            for (int j = 0; j < 4; j++) f[2 * j] = __uint_as_float(w[j] << 16), f[2 * j + 1] = __uint_as_float(w[j] & 0xffff0000u);
+            float* d = &Bs[buf][e >> 3][8 * (e & 7)];
+            *reinterpret_cast<float4*>(d) = *reinterpret_cast<const float4*>(f);
+            *reinterpret_cast<float4*>(d + 4) = *reinterpret_cast<const float4*>(f + 4);
+        }
+    };
+    TileAcc c{};
+    if (mb < me) {
+        fetch(mb);
+        stash(0);
+    }
+    __syncthreads();
+    for (int m = mb, cur = 0; m < me; m += kBKs, cur ^= 1) {
+        const bool more = m + kBKs < me;
+        if (more) fetch(m + kBKs);
+        tile_fma(As[cur], Bs[cur], tx, ty, c);
+        if (more) stash(cur ^ 1);
+        __syncthreads();
+    }
+    float* P = part + (size_t)blockIdx.z * hid * nin;
+#pragma unroll
+    for (int i = 0; i < 8; i++)
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            const int col = i0 + tile_pos(tx, j);
+            if (col < nin) P[(size_t)(o0 + tile_pos(ty, i)) * nin + col] = c.v[i][j];
         }
 }
 
-__global__ void gelu_backward(const float* __restrict__ Z, float* __restrict__ dH, int64_t n)
+// One CTA of hid threads per 64 samples, thread k on feature k.
+__global__ void head_backward(const float* __restrict__ dy, const float* __restrict__ w3, const float* __restrict__ Z,
+                              const __nv_bfloat16* __restrict__ H, float* __restrict__ dZ, float* __restrict__ sum_w,
+                              float* __restrict__ sum_z, float* __restrict__ sum_y)
 {
-    const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e < n) dH[e] *= gelu_grad(Z[e]);
+    const int hid = blockDim.x, k = threadIdx.x;
+    const float w = w3[k];
+    float sw = 0.0f, sz = 0.0f, sy = 0.0f;
+#pragma unroll 8
+    for (int r = 0; r < 64; r++) {
+        const size_t m = (size_t)blockIdx.x * 64 + r, e = m * hid + k;
+        const float d = dy[m], g = d * w * gelu_grad(Z[e]);
+        dZ[e] = g;
+        sw = fmaf(d, __bfloat162float(H[e]), sw);
+        sz += g;
+        sy += d;
+    }
+    sum_w[(size_t)blockIdx.x * hid + k] = sw;
+    sum_z[(size_t)blockIdx.x * hid + k] = sz;
+    if (k == 0) sum_y[blockIdx.x] = sy;
 }
 
-// Column sums (bias gradient): out[n] = sum_m D[m][n].
-__global__ void colsum(const float* __restrict__ D, int M, int N, float* __restrict__ out)
+// out[e] = sum over p of part[p * n + e], in order within each of 8 interleaved
+// chains (warp w of the CTA takes p = w, w + 8, ...), the chains then added in order.
+// grid ceil(n / 32), 256 threads.
+__global__ void __launch_bounds__(256) sum_parts(const float* __restrict__ part, int np, int n, float* __restrict__ out)
 {
-    const int n = blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= N) return;
-    float s = 0.0f;
-    for (int m = 0; m < M; m++) s += D[(size_t)m * N + n];
-    out[n] = s;
+    __shared__ float s[8][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, e = blockIdx.x * 32 + lane;
+    float t = 0.0f;
+    if (e < n)
+        for (int p = w; p < np; p += 8) t += part[(size_t)p * n + e];
+    s[w][lane] = t;
+    __syncthreads();
+    if (w || e >= n) return;
+#pragma unroll
+    for (int i = 1; i < 8; i++) t += s[i][lane];
+    out[e] = t;
 }
 
 // MSE loss on normalised targets: d = (y - t)/M ... dy = 2 (y - t) / M, loss accumulated.
@@ -361,6 +514,10 @@ int Net::alloc(int n_in_, int hidden_, int max_batch_)
     kin = (n_in + 31) / 32 * 32;
     max_batch = (max_batch_ + 63) / 64 * 64;
     const int ins[4] = {n_in, hid, hid, hid}, outs[4] = {hid, hid, hid, 1};
+    size_t off = 0;
+    for (int l = 0; l < 4; l++) off += (size_t)outs[l] * ins[l] + outs[l];
+    SCP3_CUDA(cudaMalloc(&gflat, sizeof(float) * off));
+    off = 0;
     for (int l = 0; l < 4; l++) {
         in[l] = ins[l];
         out[l] = outs[l];
@@ -368,8 +525,9 @@ int Net::alloc(int n_in_, int hidden_, int max_batch_)
         const size_t nw = (size_t)out[l] * in[l];
         SCP3_CUDA(cudaMalloc(&w[l], sizeof(float) * nw));
         SCP3_CUDA(cudaMalloc(&b[l], sizeof(float) * out[l]));
-        SCP3_CUDA(cudaMalloc(&gw[l], sizeof(float) * nw));
-        SCP3_CUDA(cudaMalloc(&gb[l], sizeof(float) * out[l]));
+        gw[l] = gflat + off;             // gradients in the flat parameter order, one copy out
+        gb[l] = gw[l] + nw;
+        off += nw + out[l];
         SCP3_CUDA(cudaMalloc(&mw[l], sizeof(float) * nw * 2));
         SCP3_CUDA(cudaMalloc(&mb[l], sizeof(float) * out[l] * 2));
         SCP3_CUDA(cudaMemset(mw[l], 0, sizeof(float) * nw * 2));
@@ -387,17 +545,22 @@ int Net::alloc(int n_in_, int hidden_, int max_batch_)
     SCP3_CUDA(cudaMalloc(&ybuf, sizeof(float) * max_batch));
     SCP3_CUDA(cudaMalloc(&dy, sizeof(float) * max_batch));
     SCP3_CUDA(cudaMalloc(&loss, sizeof(float)));
+    const size_t rb = max_batch / 64, nsplit = std::max<size_t>(1, std::min<size_t>(kDwSplits, max_batch / kDwRows));
+    SCP3_CUDA(cudaMalloc(&part, sizeof(float) * nsplit * hid * std::max(hid, n_in)));
+    for (int k = 0; k < 2; k++) SCP3_CUDA(cudaMalloc(&rsum[k], sizeof(float) * rb * hid));
+    SCP3_CUDA(cudaMalloc(&ysum, sizeof(float) * rb));
     return SCP3GPU_OK;
 }
 
 void Net::free_all()
 {
     for (int l = 0; l < 4; l++) {
-        void* ps[] = {w[l], b[l], gw[l], gb[l], mw[l], mb[l], wb[l]};
+        void* ps[] = {w[l], b[l], mw[l], mb[l], wb[l]};
         for (void* p : ps)
             if (p) cudaFree(p);
     }
-    void* ps[] = {X, Z[0], Z[1], Z[2], H[0], H[1], H[2], dA, dB, ybuf, dy, loss};
+    void* ps[] = {X, Z[0], Z[1], Z[2], H[0], H[1], H[2], dA, dB, ybuf, dy, loss,
+                  gflat, part, rsum[0], rsum[1], ysum};
     for (void* p : ps)
         if (p) cudaFree(p);
 }
@@ -496,23 +659,20 @@ int Net::backward(const float* q, const float* t, int M, cudaStream_t s, float* 
         normalise_kernel<<<blocks(M, 256), 256, 0, s>>>(ybuf, t, M, out_scale, out_shift, dA, dB);
         mse_grad<<<blocks(M, 256), 256, 0, s>>>(dA, dB, M, dy, loss);
     }
-    // head: gw3[k] = sum_m dy[m] H2[m][k]; gb3 = sum dy; dH2 = dy w3^T
-    gemm_f32<float, __nv_bfloat16><<<dim3(1, blocks(hid, 64)), 256, 0, s>>>(dy, 0, 1, H[2], hid, 1, 1, hid, M,
-                                                                              gw[3], hid, 0.0f);
-    colsum<<<1, 32, 0, s>>>(dy, M, 1, gb[3]);
-    gemm_f32<float, float><<<dim3(blocks(M, 64), blocks(hid, 64)), 256, 0, s>>>(dy, 1, 0, w[3], 0, 1, M, hid, 1,
-                                                                              dA, hid, 0.0f);
-    for (int l = 2; l >= 0; l--) {
-        gelu_backward<<<blocks((int64_t)M * hid, 256), 256, 0, s>>>(Z[l], dA, (int64_t)M * hid);   // dZ_l
+    // head: gw3[k] = sum_m dy[m] H2[m][k]; gb3 = sum dy; dZ2 = dy w3 * GELU'(Z2)
+    const int rb = M / 64;
+    head_backward<<<rb, hid, 0, s>>>(dy, w[3], Z[2], H[2], dA, rsum[0], rsum[1], ysum);
+    sum_parts<<<blocks(hid, 32), 256, 0, s>>>(rsum[0], rb, hid, gw[3]);
+    sum_parts<<<1, 256, 0, s>>>(ysum, rb, 1, gb[3]);
+    const int splits = std::max(1, std::min(kDwSplits, M / kDwRows));
+    for (int l = 2; l >= 0; l--) {     // dA = dZ_l, rsum[1] = its 64-row sums
+        sum_parts<<<blocks(hid, 32), 256, 0, s>>>(rsum[1], rb, hid, gb[l]);
         // gw_l[o][i] = sum_m dZ[m][o] Xin[m][i]
-        const __nv_bfloat16* Xin = l == 0 ? X : H[l - 1];
-        const int ld_in = inpad[l];
-        gemm_f32<float, __nv_bfloat16><<<dim3(blocks(hid, 64), blocks(in[l], 64)), 256, 0, s>>>(
-            dA, 1, hid, Xin, ld_in, 1, hid, in[l], M, gw[l], in[l], 0.0f);
-        colsum<<<blocks(hid, 128), 128, 0, s>>>(dA, M, hid, gb[l]);
-        if (l > 0) {   // dH_{l-1}[m][i] = sum_o dZ[m][o] W_l[o][i]
-            gemm_f32<float, float><<<dim3(blocks(M, 64), blocks(hid, 64)), 256, 0, s>>>(dA, hid, 1, w[l], in[l], 1, M,
-                                                                                      hid, hid, dB, hid, 0.0f);
+        dw_gemm<<<dim3(hid / kBT, blocks(in[l], kBT), splits), kBThreads, 0, s>>>(dA, l == 0 ? X : H[l - 1], M, hid,
+                                                                                 in[l], inpad[l], part);
+        sum_parts<<<blocks((int64_t)hid * in[l], 32), 256, 0, s>>>(part, splits, hid * in[l], gw[l]);
+        if (l > 0) {   // dZ_{l-1}[m][i] = (sum_o dZ[m][o] W_l[o][i]) GELU'(Z_{l-1}[m][i])
+            dz_gemm<<<dim3(rb, hid / kBT), kBThreads, 0, s>>>(dA, w[l], Z[l - 1], hid, hid, dB, rsum[1]);
             std::swap(dA, dB);
         }
     }
@@ -719,21 +879,14 @@ int scp3gpu_mlp_grad(scp3gpu_mlp* m, const float* q, const float* t, int n, floa
     if (!m || !q || !t || n < 64 || n % 64 != 0 || n > m->net.max_batch)
         return fail(SCP3GPU_ERR_ARG, "mlp_grad: n must be a multiple of 64 within the batch size");
     Dev g(m->dev);
-    float* td = nullptr;
-    SCP3_CUDA(cudaMalloc(&td, sizeof(float) * n));
     SCP3_CUDA(cudaMemcpyAsync(m->qbuf, q, sizeof(float) * (size_t)n * m->net.n_in, cudaMemcpyHostToDevice, m->s));
-    SCP3_CUDA(cudaMemcpyAsync(td, t, sizeof(float) * n, cudaMemcpyHostToDevice, m->s));
-    int rc = m->net.backward(m->qbuf, td, n, m->s, loss);
-    cudaFree(td);
+    SCP3_CUDA(cudaMemcpyAsync(m->tbuf, t, sizeof(float) * n, cudaMemcpyHostToDevice, m->s));
+    int rc = m->net.backward(m->qbuf, m->tbuf, n, m->s, loss);
     if (rc) return rc;
     if (grad)
-        for (int l = 0; l < 4; l++) {
-            const size_t nw = (size_t)m->net.out[l] * m->net.in[l];
-            SCP3_CUDA(cudaMemcpy(grad, m->net.gw[l], sizeof(float) * nw, cudaMemcpyDeviceToHost));
-            grad += nw;
-            SCP3_CUDA(cudaMemcpy(grad, m->net.gb[l], sizeof(float) * m->net.out[l], cudaMemcpyDeviceToHost));
-            grad += m->net.out[l];
-        }
+        SCP3_CUDA(cudaMemcpyAsync(grad, m->net.gflat, sizeof(float) * (size_t)scp3gpu_mlp_num_params(m),
+                                  cudaMemcpyDeviceToHost, m->s));
+    SCP3_CUDA(cudaStreamSynchronize(m->s));
     return SCP3GPU_OK;
 }
 

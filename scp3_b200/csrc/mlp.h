@@ -18,6 +18,8 @@ struct Net {
     float* Z[3] = {};
     __nv_bfloat16* H[3] = {};
     float *dA = nullptr, *dB = nullptr, *ybuf = nullptr, *dy = nullptr, *loss = nullptr;
+    // backward: all gradients (gw, gb point into it), weight-gradient partials, sums over 64 rows
+    float *gflat = nullptr, *part = nullptr, *rsum[2] = {}, *ysum = nullptr;
     float out_scale = 1.0f, out_shift = 0.0f;   // y = raw * scale + shift
     int64_t step = 0;
 

@@ -133,3 +133,25 @@ def test_builds_sharing_a_network_run_concurrently(sur):
     b.accumulate(0, 1 << 18)
     assert np.array_equal(a.read(0), seq[0])
     assert np.array_equal(b.read(0), seq[1])
+
+
+@pytest.mark.parametrize("n_in,hidden,n", [(48, 256, 64), (21, 192, 320), (65, 64, 16448), (66, 128, 4096)])
+def test_gradient_tile_edges(sur, n_in, hidden, n):
+    """Weight-gradient tiles past the input width, one sample split and many, row
+    blocks that do not divide the splits.  A BF16 activation may round the other way
+    where the FP32 sums land within ~1e-6 of a tie: ~5e-4 of the activations, each by
+    2^-8 of itself, so ~9e-5 of the gradient's norm at most; 3e-4 allows for it."""
+    from oracle import mlp_oracle as mo
+    rng = np.random.default_rng(n)
+    net = sur.MLP(n_in, hidden=hidden, max_batch=n, seed=2)
+    q = rng.normal(scale=np.sqrt(0.5), size=(n, n_in)).astype(np.float32)
+    t = rng.normal(size=n).astype(np.float32)
+    loss, g = net.loss_and_grad(q, t)
+    loss_or, g_or = mo.loss_and_grad(net.get_params(), q, t, n_in, hidden)
+    assert loss == pytest.approx(loss_or, rel=1e-4)
+    k = 0
+    for o, i in ((hidden, n_in), (hidden, hidden), (hidden, hidden), (1, hidden)):
+        for m in (o * i, o):
+            seg = slice(k, k + m)
+            assert np.linalg.norm(g[seg] - g_or[seg]) <= 3e-4 * np.linalg.norm(g_or[seg]), (o, i, m)
+            k += m
