@@ -1,0 +1,754 @@
+// Sums over samples of products of FP64 values, as exact integer products on the
+// tensor cores: sum_s A_i(s) B_j(s) for the plain FP64 form of both estimators
+// (ScaledMatrixElements.cpp:951-971 and :102-725).
+//
+// Why.  The FP64 pipe does 64 FMA per clock and SM, the tensor cores 65536 8-bit
+// ones: a product of two 56-bit fixed-point numbers in 34 products of 8-bit digits
+// is worth 4 FP64 pipes or so (the clock is lower under this load).  The DFMA kernel this replaces ran at 0.72 of that pipe:
+// 8.9 ms per 2^17 samples of the hexamer doubles basis.
+//
+// Digits.  Within a pass every operand row has one power-of-two scale, 2^e above
+// its largest |value|; a value is rounded to the integer x 2^(54 - e) (|.| <= 2^54,
+// the rounding is half a unit of FP64's last place for values near the largest) and
+// written as seven balanced base-256 digits, each -128..127, most significant first.
+// The product of two rows is sum over digit pairs (i, j) of 2^(8 (14 - i - j)) D_ij;
+// the 34 pairs with i + j <= 9 are formed.  Measured against compensated sums of the
+// same values, 2^13 samples: norm-wise error 1.6e-16 (dimer), 7.7e-17 (hexamer) and
+// 4.9e-16 (trimer, |V| up to 34 times its rms), against 4.2e-16, 4.9e-16 and 7.2e-16 of
+// an FP64 product; with i + j <= 8 only (28 pairs) 4.8e-15, 1.4e-15 and 1.5e-14.  D_ij is accumulated in 32-bit integers,
+// exactly: a run is at most 18432 samples, so a group of equal i + j (up to 7 pairs of
+// 2^14) stays below 2^31.  A row whose values are not all finite reads NaN in every
+// element it enters.
+//
+// Operand layout: [row block of 128][k-block of 64 samples][digit][128 rows x 64 B],
+// each 8 KB box in the 64-byte-swizzled order the MMA descriptors read (16-byte chunk
+// c of row r at c ^ ((r >> 1) & 3)).
+//
+// contract_i8_kernel: a work unit is (sample range, 128 x 256 tile); four sweeps
+// over the unit's k-blocks, for the digit sums 9 and 8, 7 and 6, 5 and 4, 3 and 2; a
+// sweep's two sums own the two 256-column TMEM accumulators.  In one k-block of a sweep
+// the digits come in a chain (1, 7, 2, 6, 3, 5, 4 for the sums 9 and 8; n, 1, n-1, 2,
+// ... with n = 6, 4, 2 for the others) whose neighbours add up to the one and the other
+// sum in turn, and whose last pairs with itself, so every digit (A box and two B boxes,
+// 24 KB) is loaded once and is free again two steps later: 53 bytes loaded per clock
+// and SM, 8 or 9 steps in flight in a ring of 9.  After a sweep eight warps add the two
+// accumulators, joined in 64 bits, into the unit's own FP64 partial, by reductions
+// that need no read (a read-modify-write took 10 us a drain).
+// What bounds it: the tensor pipe under the power limit (one M = 128, N = 256, K = 32
+// product takes 128 clocks alone on an SM, like a K = 16 product of kind::f16).
+// Bounded waits as in contract_tc.cu.
+#include <algorithm>
+#include <cstring>
+
+#include "common.cuh"
+#include "contract_i8.h"
+#include "hermite.cuh"
+
+namespace scp3 {
+namespace i8 {
+
+namespace {
+
+constexpr unsigned long long kWaitNs = 4000000000ull;
+#include "tc_ptx.cuh"
+
+constexpr int kDigits = 7, kSweeps = 4, kTile = 128, kN = 256;
+constexpr int kBox = kTile * kKB;                  // 8 KB: one digit of 128 rows x 64 samples
+constexpr int kSlot = 3 * kBox, kRing = 9;         // A box, two B boxes
+constexpr int kRunKB = 288;                        // k-blocks per run: 7 * 2^14 * 18432 < 2^31
+constexpr int kSmem = kRing * kSlot + 1024 + 256;
+constexpr int kThreads = 320, kEpiWarps = 8;
+// kind::i8: D S32, A and B signed 8-bit, K-major
+constexpr uint32_t kIdesc = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kN >> 3) << 17) |
+                            ((uint32_t)(kTile >> 4) << 24);
+
+__device__ __forceinline__ void mma_i8(uint32_t d, uint64_t a, uint64_t b, uint32_t acc)
+{
+    asm volatile(
+        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n}\n" ::"r"(d),
+        "l"(a), "l"(b), "r"(kIdesc), "r"(acc));
+}
+
+// 16 columns of each of two accumulators
+__device__ __forceinline__ void tmem_ld16x2(uint32_t ta, uint32_t tb, int* a, int* b)
+{
+    uint32_t r[32];
+#define SCP3_LD16(k, t)                                                                                               \
+    asm volatile(                                                                                                     \
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"      \
+        : "=r"(r[k]), "=r"(r[k + 1]), "=r"(r[k + 2]), "=r"(r[k + 3]), "=r"(r[k + 4]), "=r"(r[k + 5]), "=r"(r[k + 6]), \
+          "=r"(r[k + 7]), "=r"(r[k + 8]), "=r"(r[k + 9]), "=r"(r[k + 10]), "=r"(r[k + 11]), "=r"(r[k + 12]),          \
+          "=r"(r[k + 13]), "=r"(r[k + 14]), "=r"(r[k + 15])                                                           \
+        : "r"(t))
+    SCP3_LD16(0, ta);
+    SCP3_LD16(16, tb);
+#undef SCP3_LD16
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int j = 0; j < 16; j++) a[j] = (int)r[j], b[j] = (int)r[16 + j];
+}
+
+// One thread owns an element of the partials, so its reductions keep their order
+__device__ __forceinline__ void add_f64(double* p, double x)
+{
+    asm volatile("red.relaxed.gpu.global.add.f64 [%0], %1;" ::"l"(p), "d"(x) : "memory");
+}
+
+// Sweeps t = 0..3 take digits 1..sweep_digits(t); digit (1 = most significant) of step e
+// of sweep t's chain.  Steps e - 1 and e add up to the sweep's larger sum, 9 - 2t, where
+// in_large, else to the smaller, 8 - 2t, as the last digit and itself do.
+__host__ __device__ __forceinline__ int sweep_digits(int t) { return t ? 8 - 2 * t : 7; }
+__host__ __device__ __forceinline__ int chain_digit(int t, int e)
+{
+    if (t == 0) return (e & 1) ? 7 - (e >> 1) : 1 + (e >> 1);
+    return (e & 1) ? (e + 1) >> 1 : 8 - 2 * t - (e >> 1);
+}
+__host__ __device__ __forceinline__ bool in_large(int t, int e) { return ((e & 1) != 0) == (t != 0); }
+
+__device__ __forceinline__ double pow2(int e) { return __hiloint2double((1023 + e) << 20, 0); }
+
+// Exponent e with every |value| of the row below 2^e, from the high word of the largest
+__device__ __forceinline__ int row_exp(int hi) { return max((hi >> 20) - 1022, -960); }
+__device__ __forceinline__ double row_unit(int hi)     // value of one unit of the row's integers
+{
+    return hi >= 0x7ff00000 ? __longlong_as_double(0x7ff8000000000000ll) : pow2(row_exp(hi) - 54);
+}
+
+__global__ void __launch_bounds__(kThreads, 1)
+    contract_i8_kernel(const uint8_t* __restrict__ x, long long nkb_alloc, const int* __restrict__ rowmax,
+                       const int4* __restrict__ tiles, int ntiles, int nsplit, int nkb_pass, int units,
+                       double* __restrict__ partial, int* __restrict__ err_flag)
+{
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    uint64_t* full = reinterpret_cast<uint64_t*>(smem + kRing * kSlot);
+    uint64_t* empty = full + kRing;
+    uint64_t* acc_full = empty + kRing;
+    uint64_t* acc_empty = acc_full + 1;
+    uint64_t* drain = acc_empty + 1;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain + 1);
+    volatile int* abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    auto krange = [&](int u, int& lo, int& hi) {
+        const int split = u / ntiles;
+        lo = (int)((long long)split * nkb_pass / nsplit);
+        hi = (int)((long long)(split + 1) * nkb_pass / nsplit);
+    };
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < kRing; s++) {
+            mbar_init(full + s, 1);
+            mbar_init(empty + s, 1);
+        }
+        mbar_init(acc_full, 1);
+        mbar_init(acc_empty, kEpiWarps);
+        mbar_init(drain, 1);
+        *abort = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(tmem_slot)));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *tmem_slot;
+
+    if (warp == 0) {
+        if (lane == 0) {
+            int slot = 0;
+            uint32_t phase = 0, issued = 0, issued_phase = 0;   // bit per slot
+            bool ok = true;
+            for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
+                int lo, hi;
+                krange(u, lo, hi);
+                const int4 ti = tiles[u % ntiles];
+                const size_t rb = (size_t)nkb_alloc * (kDigits * kBox);
+                const uint8_t* pa = x + (ti.x / kTile) * rb;
+                const uint8_t* pb0 = x + (ti.y / kTile) * rb;
+                const uint8_t* pb1 = x + (ti.w / kTile) * rb;
+                for (int r0 = lo; r0 < hi && ok; r0 += kRunKB)
+                    for (int t = 0; t < kSweeps && ok; t++)
+                        for (int kb = r0; kb < min(hi, r0 + kRunKB) && ok; kb++)
+                            for (int e = 0; e < sweep_digits(t); e++) {
+                                if (!mbar_wait(empty + slot, phase ^ 1, abort)) {
+                                    ok = false;
+                                    break;
+                                }
+                                uint8_t* st = smem + slot * kSlot;
+                                mbar_expect_tx(full + slot, kSlot);
+                                const size_t o = ((size_t)kb * kDigits + chain_digit(t, e) - 1) * kBox;
+                                bulk_load(st, pa + o, kBox, full + slot);
+                                bulk_load(st + kBox, pb0 + o, kBox, full + slot);
+                                bulk_load(st + 2 * kBox, pb1 + o, kBox, full + slot);
+                                issued |= 1u << slot;
+                                issued_phase = (issued_phase & ~(1u << slot)) | phase << slot;
+                                if (++slot == kRing) {
+                                    slot = 0;
+                                    phase ^= 1;
+                                }
+                            }
+            }
+            if (*abort) {
+                for (int s = 0; s < kRing; s++)
+                    if ((issued >> s) & 1) {
+                        volatile int never = 0;
+                        mbar_wait(full + s, (issued_phase >> s) & 1, &never);
+                    }
+            }
+        }
+    } else if (warp == 1) {
+        if (lane == 0) {
+            int slot = 0, use = 0;
+            uint32_t phase = 0;
+            bool ok = true;
+            for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
+                int lo, hi;
+                krange(u, lo, hi);
+                for (int r0 = lo; r0 < hi && ok; r0 += kRunKB)
+                    for (int t = 0; t < kSweeps && ok; t++, use++) {
+                        const int n = sweep_digits(t);
+                        if (!mbar_wait(acc_empty, (use & 1) ^ 1, abort)) {
+                            ok = false;
+                            break;
+                        }
+                        tc_fence_after();
+                        for (int kb = r0; kb < min(hi, r0 + kRunKB) && ok; kb++) {
+                            uint64_t pa = 0, pb = 0;
+                            int prev = 0;
+                            for (int e = 0; e < n; e++) {
+                                if (!mbar_wait(full + slot, phase, abort)) {
+                                    ok = false;
+                                    break;
+                                }
+                                tc_fence_after();
+                                uint8_t* st = smem + slot * kSlot;
+                                const uint64_t ca = smem_desc64(st), cb = smem_desc64(st + kBox);
+                                if (e) {
+                                    const uint32_t d = tmem + (in_large(t, e) ? 0u : (uint32_t)kN);
+                                    const uint32_t acc = kb != r0 || e > 2;
+                                    mma_i8(d, pa, cb, acc);
+                                    mma_i8(d, pa + 2, cb + 2, 1);
+                                    mma_i8(d, ca, pb, 1);
+                                    mma_i8(d, ca + 2, pb + 2, 1);
+                                    mma_commit(empty + prev);
+                                }
+                                if (e == n - 1) {      // in sweep 3 the smaller sum's first
+                                    mma_i8(tmem + kN, ca, cb, kb != r0 || n > 2);
+                                    mma_i8(tmem + kN, ca + 2, cb + 2, 1);
+                                    mma_commit(empty + slot);
+                                }
+                                pa = ca, pb = cb, prev = slot;
+                                if (++slot == kRing) {
+                                    slot = 0;
+                                    phase ^= 1;
+                                }
+                            }
+                        }
+                        if (ok) mma_commit(acc_full);
+                    }
+            }
+            mma_commit(drain);
+            volatile int never = 0;
+            mbar_wait(drain, 0, &never);
+        }
+    } else {
+        // warp w reads TMEM lane quadrant w % 4 and column half (w - 2) / 4
+        const int quad = warp & 3, half = (warp - 2) >> 2;
+        const int row = quad * 32 + lane;
+        int use = 0;
+        bool ok = true;
+        for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
+            int lo, hi;
+            krange(u, lo, hi);
+            const int4 ti = tiles[u % ntiles];
+            const double ra = row_unit(rowmax[ti.x + row]);
+            const int* cmax = rowmax + (half ? ti.w : ti.y);
+            double* P = partial + (size_t)u * (size_t)(kTile * kN) + (size_t)half * kTile * kTile + row;
+            for (int r0 = lo; r0 < hi && ok; r0 += kRunKB)
+                for (int t = 0; t < kSweeps; t++, use++) {
+                    if (!mbar_wait(acc_full, use & 1, abort)) {
+                        ok = false;
+                        break;
+                    }
+                    tc_fence_after();
+                    const double w = ra * pow2(8 * (5 + 2 * t));     // the larger digit sum: 2^(8 (14 - (9 - 2t)))
+                    const uint32_t base = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(half * kTile);
+#pragma unroll 1
+                    for (int c0 = 0; c0 < kTile; c0 += 16) {
+                        int a0[16], a1[16];
+                        tmem_ld16x2(base + c0, base + kN + c0, a0, a1);
+#pragma unroll
+                        for (int j = 0; j < 16; j++) {
+                            // |.| < 2^40: exact through the bits of 1.5 * 2^52
+                            const long long d = ((long long)a1[j] << 8) + a0[j] + 0x4338000000000000ll;
+                            add_f64(P + (size_t)(c0 + j) * kTile,
+                                    (__longlong_as_double(d) - 6755399441055744.0) * w * row_unit(cmax[c0 + j]));
+                        }
+                    }
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(acc_empty);
+                }
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (threadIdx.x == 0 && *abort) atomicExch(err_flag, 1);
+    if (warp == 1) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem));
+    }
+}
+
+// ---------------------------------------------------------------- the operand
+// A CTA tabulates the entries the rows use for 32 samples in FP64, one (mode, sample)
+// per thread at a time; thread (g, r) then takes 16 of the samples (half g; the scan 8)
+// of rows
+// 4r .. 4r+3 and on in steps of the CTA: consecutive rows mostly share their first factor, read
+// once.  Table entry i, 16-byte chunk c (0..7) of half g lies at chunk 8 g + (c ^ (i &
+// 7)), and half 1 reads its chunks in the order c ^ 4, so that four rows with
+// consecutive entries read without bank conflicts (the eight lanes of a 16-byte phase).
+constexpr int kS = 32, kScanThreads = 512, kDigitThreads = 256;
+constexpr int kModeKinds = 12;     // h1 h2 h3 K10 K20 K30 K11 K12 K13 K22 K23 K33
+
+__device__ __forceinline__ void put_entry(double* tab, int r, int l, double val)
+{
+    if (r >= 0) tab[r * kS + ((((l >> 4) << 3) + (((l >> 1) & 7) ^ (r & 7))) << 1) + (l & 1)] = val;
+}
+
+// entries[m][kind]: table entry or -1; v_entry: V's, or -1
+template <int kThreadsPerCta>
+__device__ __forceinline__ void build_table(const int16_t* __restrict__ entries, int v_entry, int nm,
+                                            const double* __restrict__ q, const double* __restrict__ v,
+                                            const double* __restrict__ vq, int64_t s0, double* tab)
+{
+    const int l = threadIdx.x & 31;
+    const int64_t s = s0 + l;
+    const double V = v[s];
+    if (threadIdx.x < kS) put_entry(tab, 0, l, 1.0);
+    else if (threadIdx.x < 2 * kS) put_entry(tab, v_entry, l, V);
+    for (int m = threadIdx.x >> 5; m < nm; m += kThreadsPerCta / 32) {
+        const double x = __ldg(q + s * nm + m);
+        const int16_t* e = entries + m * kModeKinds;
+#pragma unroll
+        for (int a = 1; a <= 3; a++) put_entry(tab, e[a - 1], l, ho(a, x));
+        if (!vq) continue;
+        const double Vm = __ldg(vq + s * nm + m);
+#pragma unroll
+        for (int a = 1; a <= 3; a++) {
+            put_entry(tab, e[2 + a], l, stein_weight(a, 0, x, V, Vm));
+#pragma unroll
+            for (int b = a; b <= 3; b++) {
+                const int k = a == 1 ? 5 + b : a == 2 ? 7 + b : 11;      // K1b at 6.., K2b at 9.., K33 at 11
+                if (e[k] >= 0) put_entry(tab, e[k], l, stein_weight(a, b, x, V, Vm));
+            }
+        }
+    }
+}
+
+// the 16 values of half g of entry i; register pair k holds samples 2 (k ^ 4 g), + 1
+__device__ __forceinline__ void read16(const double* tab, uint32_t i, int g, double* o)
+{
+    const double2* t = reinterpret_cast<const double2*>(tab + (size_t)i * kS) + 8 * g;
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+        const double2 d = t[(k ^ (g << 2)) ^ (i & 7)];
+        o[2 * k] = d.x, o[2 * k + 1] = d.y;
+    }
+}
+
+__device__ __forceinline__ void mul16(const double* tab, uint32_t i, int g, double* o)
+{
+    const double2* t = reinterpret_cast<const double2*>(tab + (size_t)i * kS) + 8 * g;
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+        const double2 d = t[(k ^ (g << 2)) ^ (i & 7)];
+        o[2 * k] *= d.x, o[2 * k + 1] *= d.y;
+    }
+}
+
+// the scan's share: the 8 samples of quarter g (half g / 2); the second half reads its
+// chunks in another order, so that two rows' four quarters meet no bank conflict
+template <bool kMul>
+__device__ __forceinline__ void read8(const double* tab, uint32_t i, int g, double* o)
+{
+    const double2* t = reinterpret_cast<const double2*>(tab + (size_t)i * kS) + 8 * (g >> 1);
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const double2 d = t[(4 * (g & 1) + (k ^ (g & 2))) ^ (i & 7)];
+        if (kMul) o[2 * k] *= d.x, o[2 * k + 1] *= d.y;
+        else o[2 * k] = d.x, o[2 * k + 1] = d.y;
+    }
+}
+
+// Row values of `d` (entry indices); `fa` caches the first factor of entry `pia`.
+__device__ __forceinline__ void row16(const double* tab, uint32_t d, int g, uint32_t& pia, double* fa, double* o)
+{
+    const uint32_t ia = d & 1023u, ib = (d >> 10) & 1023u, ic = d >> 20;
+    if (ia != pia) {
+        read16(tab, ia, g, fa);
+        pia = ia;
+    }
+#pragma unroll
+    for (int k = 0; k < 16; k++) o[k] = fa[k];
+    if (ib) mul16(tab, ib, g, o);
+    if (ic) mul16(tab, ic, g, o);
+}
+
+__device__ __forceinline__ int max_hi8(const double* o)
+{
+    int m = 0;
+#pragma unroll
+    for (int k = 0; k < 8; k++) m = max(m, __double2hiint(o[k]) & 0x7fffffff);
+    return m;
+}
+
+// Largest |value| of every row over the pass (its high word), and the sums of the
+// summed rows.  CTA (x, y): sample blocks x, x + gridDim.x, ..., rows of chunk y.
+// dual: row dual + r is V times row r; the summed rows follow the described ones, and
+// xdesc ends on a multiple of four rows.
+__global__ void __launch_bounds__(kScanThreads, 1)
+    scan_kernel(const int16_t* __restrict__ entries, int v_entry, int trows, const uint32_t* __restrict__ xdesc,
+                int ndesc, int dual, int nsum, int per, int nm, const double* __restrict__ q,
+                const double* __restrict__ v, const double* __restrict__ vq, int nblk, int* __restrict__ rowmax,
+                double* __restrict__ spart)
+{
+    extern __shared__ __align__(16) double tab[];      // [trows][32], then [per] doubles
+    double* keep = tab + (size_t)trows * kS;           // (max, max of V times the row) or the sum
+    int2* mx = reinterpret_cast<int2*>(keep);
+    const int r0 = blockIdx.y * per, r1 = min(ndesc + nsum, r0 + per);
+    for (int r = threadIdx.x; r < r1 - r0; r += kScanThreads) keep[r] = 0.0;
+    const int g = threadIdx.x & 3, rl = threadIdx.x >> 2, w0 = 4 * (rl & 7);     // w0: rows below in the warp
+    for (int b = blockIdx.x; b < nblk; b += gridDim.x) {
+        __syncthreads();
+        build_table<kScanThreads>(entries, v_entry, nm, q, v, vq, (int64_t)b * kS, tab);
+        __syncthreads();
+        double vv[8], fa[8];
+        if (dual) read8<false>(tab, v_entry, g, vv);
+        // whole warps take the same number of rounds: the quarters meet in shuffles
+        for (int rb = r0 + 4 * rl; rb - w0 < r1; rb += kScanThreads) {
+            uint32_t pia = kZeroRow;
+            uint32_t d4[4] = {kZeroRow, kZeroRow, kZeroRow, kZeroRow};
+            if (rb < r1) *reinterpret_cast<uint4*>(d4) = __ldg(reinterpret_cast<const uint4*>(xdesc + rb));
+            const bool sum = rb - w0 + 32 > ndesc;     // the warp holds summed rows
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                const int row = rb + u;
+                const uint32_t d = d4[u];
+                double o[8];
+                int m = 0, mv = 0;
+                double t = 0.0;
+                if (d != kZeroRow) {
+                    const uint32_t ia = d & 1023u, ib = (d >> 10) & 1023u, ic = d >> 20;
+                    if (ia != pia) {
+                        read8<false>(tab, ia, g, fa);
+                        pia = ia;
+                    }
+#pragma unroll
+                    for (int k = 0; k < 8; k++) o[k] = fa[k];
+                    if (ib) read8<true>(tab, ib, g, o);
+                    if (ic) read8<true>(tab, ic, g, o);
+                    if (row < ndesc) {
+                        m = max_hi8(o);
+                        if (dual) {
+#pragma unroll
+                            for (int k = 0; k < 8; k++) o[k] *= vv[k];
+                            mv = max_hi8(o);
+                        }
+                    } else {
+                        t = ((o[0] + o[1]) + (o[2] + o[3])) + ((o[4] + o[5]) + (o[6] + o[7]));
+                    }
+                }
+                if (sum) {
+                    t += __shfl_xor_sync(0xffffffffu, t, 1);
+                    t += __shfl_xor_sync(0xffffffffu, t, 2);
+                    if (g == 0 && row >= ndesc && d != kZeroRow) keep[row - r0] += t;
+                    if (rb - w0 >= ndesc) continue;
+                }
+                m = max(m, __shfl_xor_sync(0xffffffffu, m, 1));
+                m = max(m, __shfl_xor_sync(0xffffffffu, m, 2));
+                if (dual) {
+                    mv = max(mv, __shfl_xor_sync(0xffffffffu, mv, 1));
+                    mv = max(mv, __shfl_xor_sync(0xffffffffu, mv, 2));
+                }
+                if (g == 0 && row < ndesc && d != kZeroRow)
+                    mx[row - r0] = make_int2(max(mx[row - r0].x, m), max(mx[row - r0].y, mv));
+            }
+        }
+    }
+    __syncthreads();
+    for (int r = r0 + threadIdx.x; r < r1; r += kScanThreads) {
+        if (r >= ndesc) {
+            spart[(size_t)blockIdx.x * nsum + (r - ndesc)] = keep[r - r0];
+        } else {
+            if (mx[r - r0].x) atomicMax(rowmax + r, mx[r - r0].x);
+            if (dual && mx[r - r0].y) atomicMax(rowmax + dual + r, mx[r - r0].y);
+        }
+    }
+}
+
+// sums[i] += the scan blocks' partials: warp w of a CTA adds the blocks w, w + 8, ...
+// of 32 sums in order, the eight warp sums are then added in order
+__global__ void __launch_bounds__(256) add_sums_kernel(const double* __restrict__ spart, int nsum, int nblocks,
+                                                       double* __restrict__ sums)
+{
+    __shared__ double ws[8][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, i = blockIdx.x * 32 + lane;
+    double t = 0.0;
+    if (i < nsum)
+        for (int b = w; b < nblocks; b += 8) t += spart[(size_t)b * nsum + i];
+    ws[w][lane] = t;
+    __syncthreads();
+    if (w || i >= nsum) return;
+#pragma unroll
+    for (int k = 1; k < 8; k++) t += ws[k][lane];
+    sums[i] += t;
+}
+
+// The seven digits of 16 values (register order of read16) into a row's 16-byte
+// chunk of each digit's box: the bytes of x + sum 128 256^b, each xor 0x80.
+__device__ __forceinline__ void put_digits(const double* o, int hi, int g, uint8_t* p)
+{
+    const double inv = hi >= 0x7ff00000 ? 0.0 : pow2(54 - row_exp(hi));
+    uint32_t w[kDigits][4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        uint32_t lo[4], h[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const long long t = __double2ll_rn(o[4 * j + k] * inv) + 0x0080808080808080ll;
+            lo[k] = (uint32_t)t ^ 0x80808080u;
+            h[k] = (uint32_t)(t >> 32) ^ 0x00808080u;
+        }
+        // 4 x 4 byte transposes: byte b of the four values becomes one word
+        const uint32_t l01 = __byte_perm(lo[0], lo[1], 0x5140), l23 = __byte_perm(lo[2], lo[3], 0x5140);
+        const uint32_t m01 = __byte_perm(lo[0], lo[1], 0x7362), m23 = __byte_perm(lo[2], lo[3], 0x7362);
+        w[6][j] = __byte_perm(l01, l23, 0x5410);
+        w[5][j] = __byte_perm(l01, l23, 0x7632);
+        w[4][j] = __byte_perm(m01, m23, 0x5410);
+        w[3][j] = __byte_perm(m01, m23, 0x7632);
+        const uint32_t h01 = __byte_perm(h[0], h[1], 0x5140), h23 = __byte_perm(h[2], h[3], 0x5140);
+        const uint32_t n01 = __byte_perm(h[0], h[1], 0x7362), n23 = __byte_perm(h[2], h[3], 0x7362);
+        w[2][j] = __byte_perm(h01, h23, 0x5410);
+        w[1][j] = __byte_perm(h01, h23, 0x7632);
+        w[0][j] = __byte_perm(n01, n23, 0x5410);
+    }
+#pragma unroll
+    for (int i = 0; i < kDigits; i++)     // half 1 holds its samples as 8..15, 0..7
+        *reinterpret_cast<uint4*>(p + i * kBox) =
+            g ? make_uint4(w[i][2], w[i][3], w[i][0], w[i][1]) : make_uint4(w[i][0], w[i][1], w[i][2], w[i][3]);
+}
+
+// CTA (x, y): the 32 samples of block x, rows of chunk y (`per` rows, a multiple of 4).
+__global__ void __launch_bounds__(kDigitThreads, 2)
+    digits_kernel(const int16_t* __restrict__ entries, int v_entry, const uint32_t* __restrict__ xdesc, int ndesc,
+                  int dual, int per, int nm, const double* __restrict__ q, const double* __restrict__ v,
+                  const double* __restrict__ vq, const int* __restrict__ rowmax, int64_t nkb_alloc,
+                  uint8_t* __restrict__ x)
+{
+    extern __shared__ __align__(16) double tab[];
+    build_table<kDigitThreads>(entries, v_entry, nm, q, v, vq, (int64_t)blockIdx.x * kS, tab);
+    __syncthreads();
+    const int g = threadIdx.x & 1, rl = threadIdx.x >> 1;
+    const int64_t kb = blockIdx.x >> 1;
+    const int c = ((blockIdx.x & 1) << 1) | g;          // 16-byte chunk of the box rows
+    auto box = [&](int row) {
+        const int rin = row & (kTile - 1);
+        return x + ((size_t)(row / kTile) * nkb_alloc + kb) * (kDigits * kBox) + rin * kKB +
+               ((c ^ ((rin >> 1) & 3)) << 4);
+    };
+    double vv[16], fa[16];
+    if (dual) read16(tab, v_entry, g, vv);
+    const int r0 = blockIdx.y * per, r1 = min(ndesc, r0 + per);
+    for (int rb = r0 + 4 * rl; rb < r1; rb += 2 * kDigitThreads) {
+        uint32_t pia = kZeroRow;
+        uint4 d4 = __ldg(reinterpret_cast<const uint4*>(xdesc + rb));
+#pragma unroll 1
+        for (int u = 0; u < 4; u++) {
+            const int row = rb + u;
+            const uint32_t d = d4.x;
+            d4 = make_uint4(d4.y, d4.z, d4.w, kZeroRow);
+            if (d == kZeroRow) continue;
+            double o[16];
+            row16(tab, d, g, pia, fa, o);
+            put_digits(o, __ldg(rowmax + row), g, box(row));
+            if (dual) {
+#pragma unroll
+                for (int k = 0; k < 16; k++) o[k] *= vv[k];
+                put_digits(o, __ldg(rowmax + dual + row), g, box(dual + row));
+            }
+        }
+    }
+}
+
+size_t digits_smem(const Plan& p) { return sizeof(double) * (size_t)p.trows * kS; }
+size_t scan_smem(const Plan& p) { return digits_smem(p) + sizeof(double) * (size_t)p.scan_per; }
+int described(const Plan& p) { return p.dual ? p.dual : p.rows; }
+int scan_chunks(const Plan& p) { return (described(p) + p.nsum + p.scan_per - 1) / p.scan_per; }
+int scan_blocks(const Plan& p, int64_t k)
+{
+    return (int)std::max<int64_t>(1, std::min<int64_t>(k / kS, p.sms / scan_chunks(p)));
+}
+
+}  // namespace
+
+void direct_rows(const std::vector<uint32_t>& desc, int nm, int nb_pad, std::vector<uint32_t>& tspec,
+                 std::vector<uint32_t>& xdesc)
+{
+    std::vector<uint32_t> at((size_t)4 * nm, 0);      // entry of level l of mode m
+    tspec = {kOne, kV};
+    xdesc.assign(nb_pad, kZeroRow);
+    for (size_t r = 0; r < desc.size(); r++) {
+        int mm[3], ll[3];
+        const int k = decode(desc[r], mm, ll);
+        uint32_t d = 0;
+        for (int a = 0; a < k; a++) {
+            uint32_t& e = at[(size_t)4 * mm[a] + ll[a]];
+            if (!e) {
+                e = (uint32_t)tspec.size();
+                tspec.push_back(kHo | (uint32_t)ll[a] << 4 | (uint32_t)mm[a] << 8);
+            }
+            d |= e << (10 * a);
+        }
+        xdesc[r] = d;
+    }
+}
+
+constexpr int kScanStep = kScanThreads, kMinScanRows = 2048;     // rows a scan CTA keeps a value of, at least
+int table_room() { return (int)((227 * 1024 - sizeof(double) * kMinScanRows) / (sizeof(double) * kS)); }
+
+// Clocks of a pass: waves of units, each 136 per sample (34 products of 128 clocks per
+// 32 samples) and four drains, and the 256 KB partials' clearing and read-out.
+int plan_splits(int ntiles, int64_t chunk, int sms)
+{
+    int best_m = 1;
+    double best = 1e300;
+    for (int m = 1; m <= sms; m++) {
+        const int64_t units = (int64_t)ntiles * m;
+        if (m > 1 && units * kTile * kN * 8 > (4ll << 30)) break;
+        const double cost = (double)((units + sms - 1) / sms) * (136.0 * chunk / m + 40000.0) + 150.0 * units;
+        if (cost < best) best = cost, best_m = m;
+    }
+    return best_m;
+}
+
+int create(Plan& p, const std::vector<uint32_t>& tspec, const std::vector<uint32_t>& xdesc, int rows, int dual,
+           int nsum, int nm, const std::vector<int4>& tiles, int nsplit, int64_t chunk, int sms)
+{
+    p = Plan{};
+    p.rows = rows, p.dual = dual, p.nsum = nsum, p.nm = nm, p.trows = (int)tspec.size();
+    p.ntiles = (int)tiles.size(), p.nsplit = nsplit, p.sms = sms;
+    p.chunk = chunk, p.nkb = chunk / kKB;
+    if (rows % kTile || chunk % kKB || (int)xdesc.size() != described(p) + nsum || p.trows > kMaxTable)
+        return fail(SCP3GPU_ERR_ARG, "contract_i8: operand not tiled");
+    if (p.trows > table_room()) return fail(SCP3GPU_ERR_ARG, "contract_i8: too many modes for the expansion's table");
+    // entry of each kind of each mode
+    std::vector<int16_t> entries((size_t)nm * kModeKinds, -1);
+    p.v_entry = -1;
+    for (int i = 0; i < p.trows; i++) {
+        const int kind = tspec[i] & 15, a = (tspec[i] >> 4) & 3, b = (tspec[i] >> 6) & 3, m = tspec[i] >> 8;
+        if (kind == kV) p.v_entry = i;
+        else if (kind != kOne)
+            entries[(size_t)m * kModeKinds + (kind == kHo ? a - 1 : kind == kKa0 ? 2 + a : a == 1 ? 5 + b : a == 2 ? 7 + b : 11)] =
+                (int16_t)i;
+    }
+    std::vector<uint32_t> desc4 = xdesc;
+    desc4.resize((xdesc.size() + 3) / 4 * 4, kZeroRow);
+    // rows per scan CTA: what fits beside the table, in whole trips of the CTA
+    const int room = (int)((227 * 1024 - digits_smem(p)) / sizeof(double)) / kScanStep * kScanStep;
+    p.scan_per = std::min(room, ((int)xdesc.size() + kScanStep - 1) / kScanStep * kScanStep);
+    const size_t xbytes = (size_t)rows * chunk * kDigits;
+    int rc;
+    if ((rc = upload(&p.entries, entries.data(), entries.size())) || (rc = upload(&p.xdesc, desc4.data(), desc4.size())) ||
+        (rc = upload(&p.tiles, tiles.data(), tiles.size())) || (rc = dalloc(&p.x, xbytes)) ||
+        (rc = dalloc(&p.rowmax, (size_t)rows)) || (rc = dalloc(&p.err, (size_t)1)) ||
+        (rc = dalloc(&p.partial, (size_t)p.nsplit * p.ntiles * kTile * kN)) ||
+        (nsum && ((rc = dalloc(&p.spart, (size_t)scan_blocks(p, chunk) * nsum)) || (rc = dalloc(&p.sums, (size_t)nsum))))) {
+        destroy(p);
+        return rc;
+    }
+    // padding rows are never written: zero the row blocks that hold any
+    const size_t block = (size_t)p.nkb * kDigits * kBox;
+    for (int rb = 0; rb < described(p) / kTile; rb++)
+        if (std::find(xdesc.begin() + rb * kTile, xdesc.begin() + (rb + 1) * kTile, kZeroRow) != xdesc.begin() + (rb + 1) * kTile) {
+            SCP3_CUDA(cudaMemset(p.x + rb * block, 0, block));
+            if (dual) SCP3_CUDA(cudaMemset(p.x + (rb + dual / kTile) * block, 0, block));
+        }
+    SCP3_CUDA(cudaMemset(p.err, 0, sizeof(int)));
+    return SCP3GPU_OK;
+}
+
+void destroy(Plan& p)
+{
+    void* ptrs[] = {p.x, p.rowmax, p.entries, p.xdesc, p.tiles, p.partial, p.spart, p.sums, p.err};
+    for (void* q : ptrs)
+        if (q) cudaFree(q);
+    p = Plan{};
+}
+
+int zero(const Plan& p, cudaStream_t s)
+{
+    SCP3_CUDA(cudaMemsetAsync(p.partial, 0, sizeof(double) * (size_t)p.nsplit * p.ntiles * kTile * kN, s));
+    if (p.nsum) SCP3_CUDA(cudaMemsetAsync(p.sums, 0, sizeof(double) * (size_t)p.nsum, s));
+    SCP3_CUDA(cudaMemsetAsync(p.err, 0, sizeof(int), s));
+    return SCP3GPU_OK;
+}
+
+int prepare(const Plan& p, const double* q, const double* v, const double* vq, int64_t k, cudaStream_t s)
+{
+    if (k <= 0) return SCP3GPU_OK;
+    if (k > p.chunk || k % kKB) return fail(SCP3GPU_ERR_ARG, "contract_i8: pass not in k-blocks");
+    const int ndesc = described(p), nblk = (int)(k / kS), nx = scan_blocks(p, k);
+    SCP3_CUDA(cudaMemsetAsync(p.rowmax, 0, sizeof(int) * (size_t)p.rows, s));
+    SCP3_CUDA(cudaFuncSetAttribute(scan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scan_smem(p)));
+    SCP3_CUDA(cudaFuncSetAttribute(digits_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)digits_smem(p)));
+    scan_kernel<<<dim3(nx, scan_chunks(p)), kScanThreads, scan_smem(p), s>>>(p.entries, p.v_entry, p.trows, p.xdesc,
+                                                                            ndesc, p.dual, p.nsum, p.scan_per, p.nm, q,
+                                                                            v, vq, nblk, p.rowmax, p.spart);
+    SCP3_CUDA(cudaGetLastError());
+    if (p.nsum) add_sums_kernel<<<(p.nsum + 31) / 32, 256, 0, s>>>(p.spart, p.nsum, nx, p.sums);
+    SCP3_CUDA(cudaGetLastError());
+    // all rows of a block in one CTA (the table is built once) where there are blocks enough
+    const int want = std::max(1, 4 * p.sms / nblk);
+    const int per = std::max(kDigitThreads, ((ndesc + want - 1) / want + 3) / 4 * 4);
+    digits_kernel<<<dim3(nblk, (ndesc + per - 1) / per), kDigitThreads, digits_smem(p), s>>>(
+        p.entries, p.v_entry, p.xdesc, ndesc, p.dual, per, p.nm, q, v, vq, p.rowmax, p.nkb, p.x);
+    SCP3_CUDA(cudaGetLastError());
+    return SCP3GPU_OK;
+}
+
+int contract(const Plan& p, int64_t k, cudaStream_t s)
+{
+    if (k <= 0) return SCP3GPU_OK;
+    const int units = p.ntiles * p.nsplit;
+    SCP3_CUDA(cudaFuncSetAttribute(contract_i8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
+    contract_i8_kernel<<<std::min(units, p.sms), kThreads, kSmem, s>>>(p.x, (long long)p.nkb, p.rowmax, p.tiles, p.ntiles,
+                                                                       p.nsplit, (int)(k / kKB), units, p.partial, p.err);
+    SCP3_CUDA(cudaGetLastError());
+    return SCP3GPU_OK;
+}
+
+int check(const Plan& p, cudaStream_t s)
+{
+    int err = 0;
+    SCP3_CUDA(cudaMemcpyAsync(&err, p.err, sizeof(int), cudaMemcpyDeviceToHost, s));
+    SCP3_CUDA(cudaStreamSynchronize(s));
+    return err ? fail(SCP3GPU_ERR_TIMEOUT, "integer contraction: a bounded pipeline wait expired") : SCP3GPU_OK;
+}
+
+}  // namespace i8
+}  // namespace scp3
+
+// Host-only view of the contraction's digit sweeps, for tests: the digit of step e of
+// sweep t (0..3) and whether its sum with step e - 1 is the sweep's larger one; returns
+// the digits of the sweep, negative on bad arguments.
+extern "C" int scp3gpu_internal_digit_chain(int t, int e, int* digit, int* large)
+{
+    using namespace scp3::i8;
+    if (t < 0 || t > 3 || e < 0 || e >= sweep_digits(t) || !digit || !large) return -1;
+    *digit = chain_digit(t, e);
+    *large = in_large(t, e);
+    return sweep_digits(t);
+}

@@ -306,23 +306,48 @@ __global__ void __launch_bounds__(kThreads, 1)
 // the sum over the splits, in order, of unit (split * ntiles + t) at row
 // r % 128 and column 128 h + c % 128 (transposed: row c % 128, column
 // 128 h + r % 128).
-__global__ void unpack_n256_kernel(const double* __restrict__ partial, const int* __restrict__ block_owner, int nt,
-                                   int ntiles, int nsplit, int nb, double divisor, const double* __restrict__ diag,
-                                   double zpe, double* __restrict__ M, int64_t ld)
+// `err` (may be null): a non-zero flag makes every element NaN.  kGroups > 1: that
+// many threads per element, each summing a contiguous share of the splits, the
+// shares then added in order (bases of a few tiles have up to one split per SM, and
+// one thread's chain of 148 loads took 35 us).
+template <int kGroups>
+__global__ void __launch_bounds__(256) unpack_n256_kernel(const double* __restrict__ partial,
+                                                          const int* __restrict__ block_owner, int nt, int ntiles,
+                                                          int nsplit, int nb, double divisor,
+                                                          const double* __restrict__ diag, double zpe,
+                                                          double* __restrict__ M, int64_t ld,
+                                                          const int* __restrict__ err)
 {
-    const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= (int64_t)nb * nb) return;
-    const int j = (int)(e / nb), i = (int)(e - (int64_t)j * nb);
-    const int r = min(i, j), c = max(i, j);
-    const int ti = r / kTile, tj = c / kTile;
-    const int own = block_owner[ti * nt + tj];
-    const int t = own >> 2, h = own & 1;
-    const int rr = r - ti * kTile, cc = c - tj * kTile;
-    const size_t off = (own & 2) ? (size_t)(h * kTile + rr) * kTile + cc : (size_t)(h * kTile + cc) * kTile + rr;
+    constexpr int kPer = 256 / kGroups;                 // elements per CTA
+    const int x = threadIdx.x % kPer, g = threadIdx.x / kPer;
+    const int64_t e = (int64_t)blockIdx.x * kPer + x;
+    const bool in = e < (int64_t)nb * nb;
+    const int j = in ? (int)(e / nb) : 0, i = in ? (int)(e - (int64_t)j * nb) : 0;
     double val = 0.0;
-    for (int s = 0; s < nsplit; s++) val += partial[((size_t)s * ntiles + t) * (size_t)(kTile * kN2) + off];
+    if (in) {
+        const int r = min(i, j), c = max(i, j);
+        const int ti = r / kTile, tj = c / kTile;
+        const int own = block_owner[ti * nt + tj];
+        const int t = own >> 2, h = own & 1;
+        const int rr = r - ti * kTile, cc = c - tj * kTile;
+        const size_t off = (own & 2) ? (size_t)(h * kTile + rr) * kTile + cc : (size_t)(h * kTile + cc) * kTile + rr;
+        const int s1 = nsplit * (g + 1) / kGroups;
+#pragma unroll 4
+        for (int s = nsplit * g / kGroups; s < s1; s++)
+            val += partial[((size_t)s * ntiles + t) * (size_t)(kTile * kN2) + off];
+    }
+    if (kGroups > 1) {
+        __shared__ double part[kGroups][kPer];
+        part[g][x] = val;
+        __syncthreads();
+        if (g) return;
+#pragma unroll
+        for (int k = 1; k < kGroups; k++) val += part[k][x];
+    }
+    if (!in) return;
     val = val / divisor;
     if (diag && i == j) val = (val + diag[i]) + zpe;
+    if (err && *err) val = __longlong_as_double(0x7ff8000000000000ll);
     M[(size_t)j * ld + i] = val;
 }
 
@@ -786,12 +811,16 @@ int launch_contract(const uint16_t* x, int64_t nkb_alloc, const int4* tiles, int
 }
 
 int launch_unpack(const double* partial, const int* owner, int nt, int ntiles, int nsplit, int nb, double divisor,
-                   const double* diag, double zpe, double* M, int64_t ld, cudaStream_t s)
+                   const double* diag, double zpe, double* M, int64_t ld, cudaStream_t s, const int* err)
 {
     const int64_t total = (int64_t)nb * nb;
     if (total <= 0) return SCP3GPU_OK;
-    unpack_n256_kernel<<<(unsigned)((total + 255) / 256), 256, 0, s>>>(partial, owner, nt, ntiles, nsplit, nb, divisor,
-                                                                      diag, zpe, M, ld);
+    if (nsplit < 16)
+        unpack_n256_kernel<1><<<(unsigned)((total + 255) / 256), 256, 0, s>>>(partial, owner, nt, ntiles, nsplit, nb,
+                                                                              divisor, diag, zpe, M, ld, err);
+    else
+        unpack_n256_kernel<8><<<(unsigned)((total + 31) / 32), 256, 0, s>>>(partial, owner, nt, ntiles, nsplit, nb,
+                                                                            divisor, diag, zpe, M, ld, err);
     SCP3_CUDA(cudaGetLastError());
     return SCP3GPU_OK;
 }

@@ -46,9 +46,11 @@ struct scp3gpu_hbuild {
     cudaEvent_t prepared[2] = {nullptr, nullptr}, contracted[2] = {nullptr, nullptr};
     cudaEvent_t head_done[2] = {nullptr, nullptr};   // a pass's whole waves of contraction units done
     int64_t pass = 0;                 // split form: passes launched (buffer = pass & 1)
-    int nb = 0, nb_pad = 0, ntasks = 0, nsplit = 1;
+    int nb = 0, ntasks = 0;
     int64_t chunk = 0;
-    TileMap tm{};
+    i8::Plan ip{};                    // plain form, direct estimator: operand, tiles, partials
+    int nt = 0;                       // its 128-row panels
+    int* owner = nullptr;             // [nt * nt] which tile holds block (ti <= tj), as tc::Plan::tile_index
     bool split_form = false;
     bool pes_fp32 = false;
     // tables
@@ -64,11 +66,9 @@ struct scp3gpu_hbuild {
     float* q32b[2] = {nullptr, nullptr};
     double* vb[2] = {nullptr, nullptr};
     double* normals[2] = {nullptr, nullptr};
-    double *phi = nullptr, *w = nullptr;
     double* vq = nullptr;             // gradient path: dV_anh/dq of the selected modes, [chunk][nmodes]
     bool gradient = false;
     SteinPlan sp{};                   // gradient path: tables, operands and sums
-    double* partial = nullptr;
     tc::Plan tcp{};
     // read-out
     double* dense = nullptr;
@@ -112,33 +112,35 @@ struct Timed {
     }
 };
 
-// Samples per device pass and the split of each pass over CTAs of a tile, plain
-// FP64 form with the direct estimator: 128 x 128 tiles with one CTA per SM
-// (contract_fp64_t128_kernel), in passes of 2^16 samples by default (fewer where
-// Phi and W of a pass would pass ~4 GB), so a unit's partial write-back is spread
-// over at least 8192 samples at the usual split.  Sample ranges per tile (nsplit, a
-// power of two, each range at least 2048 samples) minimise the waves of units
-// per unit of work: the units of a pass run in ceil(units / sms) waves.  (The
-// gradient estimator plans its own passes: stein_create.)
-void plan_fp64(scp3gpu_hbuild* h, int sms)
+// The plain FP64 form with the direct estimator: Phi and V Phi as one operand of the
+// integer contraction (contract_i8.cu), the 128 x 256 tiles of the split form's
+// cover with Phi rows against V Phi rows, passes of 2^16 samples (fewer while a
+// pass's digits would pass ~4 GB).
+int plan_fp64(scp3gpu_hbuild* h, const std::vector<uint32_t>& desc, int sms)
 {
-    const int T = 128;
-    h->tm.tile = T;
-    h->tm.nt = (h->nb + T - 1) / T;
-    h->tm.ntiles = h->tm.nt * (h->tm.nt + 1) / 2;
-    h->nb_pad = h->tm.nt * T;
+    h->nt = (h->nb + tc::kTile - 1) / tc::kTile;
+    const int nb_pad = h->nt * tc::kTile;
     int64_t chunk = h->cfg.chunk > 0 ? h->cfg.chunk : 65536;
-    // keep Phi and W of one pass under ~4 GB
-    while (chunk > 4096 && (int64_t)h->nb_pad * chunk * 16 > (4ll << 30)) chunk /= 2;
+    while (chunk > 4096 && (int64_t)2 * nb_pad * chunk * 7 > (4ll << 30)) chunk /= 2;
     h->chunk = chunk;
-    int nsplit = 1;
-    double best = 1e300;
-    for (int ns = 1; chunk / ns >= 2048 && chunk % (16ll * ns) == 0; ns *= 2) {
-        const int64_t units = (int64_t)h->tm.ntiles * ns;
-        const double cost = (double)((units + sms - 1) / sms) / ns;   // waves per unit of work
-        if (cost < best - 1e-9) best = cost, nsplit = ns;
+    std::vector<uint32_t> tspec, xdesc;
+    i8::direct_rows(desc, h->cfg.nmodes, nb_pad, tspec, xdesc);
+    std::vector<tc::BaseTile> base;
+    tc::add_cluster_tiles(base, 0, h->nt, h->nt, 0, 0);
+    std::vector<int4> tiles;
+    std::vector<int> owner((size_t)h->nt * h->nt, -1);
+    for (const tc::BaseTile& t : base) {
+        for (int k = 0; k < 2; k++)
+            if (t.halves & (1 << k)) {
+                const int s = k ? t.s1 : t.s0, tr = (t.tr >> k) & 1;
+                owner[(size_t)(tr ? s : t.ti) * h->nt + (tr ? t.ti : s)] = 4 * (int)tiles.size() + 2 * tr + k;
+            }
+        tiles.push_back(make_int4(t.ti * tc::kTile, nb_pad + t.s0 * tc::kTile, 0, nb_pad + t.s1 * tc::kTile));
     }
-    h->nsplit = nsplit;
+    int rc = upload(&h->owner, owner.data(), owner.size());
+    if (rc) return rc;
+    return i8::create(h->ip, tspec, xdesc, 2 * nb_pad, nb_pad, 0, h->cfg.nmodes, tiles,
+                      i8::plan_splits((int)tiles.size(), chunk, sms), chunk, sms);
 }
 
 }  // namespace
@@ -176,7 +178,7 @@ int launch_chunk(scp3gpu_hbuild* h, int64_t index0, int64_t nvalid, const double
     a.normals32 = normals32_dev;
     a.index0 = index0;
     a.n = h->split_form ? tc::pass_samples(h->tcp, nvalid)
-                        : h->gradient ? stein_pass_samples(h->sp, nvalid) : round_up(nvalid, 16ll * h->nsplit);
+                        : h->gradient ? stein_pass_samples(h->sp, nvalid) : i8::pass_samples(nvalid);
     a.nvalid = nvalid;
     a.q64 = h->split_form ? nullptr : h->q64;
     a.q32 = h->split_form ? h->q32b[b] : nullptr;
@@ -236,12 +238,11 @@ int launch_chunk(scp3gpu_hbuild* h, int64_t index0, int64_t nvalid, const double
     }
     {
         Timed t(h, 1);
-        rc = launch_expand_fp64_sm(h->desc, h->nb, h->cfg.nmodes, h->q64, h->v, a.n, h->nb_pad, h->phi, h->w,
-                                   h->stream);
+        rc = i8::prepare(h->ip, h->q64, h->v, nullptr, a.n, h->stream);
     }
     if (rc) return rc;
     Timed t(h, 2);
-    return launch_contract_fp64_t128(h->phi, h->w, h->nb_pad, a.n, h->tm, h->nsplit, h->partial, h->stream);
+    return i8::contract(h->ip, a.n, h->stream);
 }
 
 }  // namespace
@@ -278,9 +279,7 @@ int zero_sums(scp3gpu_hbuild* h)
 {
     if (h->split_form) return tc::zero(h->tcp, h->stream);
     if (h->gradient) return stein_zero(h->sp, h->stream);
-    SCP3_CUDA(cudaMemsetAsync(h->partial, 0, sizeof(double) * (size_t)h->nsplit * h->tm.ntiles * h->tm.tile *
-                                                 h->tm.tile, h->stream));
-    return SCP3GPU_OK;
+    return i8::zero(h->ip, h->stream);
 }
 
 
@@ -488,11 +487,12 @@ int scp3gpu_hbuild_destroy(scp3gpu_hbuild* h)
     if (h->prep_stream) cudaStreamSynchronize(h->prep_stream);
     void* ptrs[] = {h->sur_ws, h->vq, h->ybuf, h->vdir, h->shift, h->x0, h->MUa, h->omega, h->modes, h->tasks, h->desc, h->q64, h->q32b[0],
                     h->q32b[1], h->vb[0], h->vb[1],
-                    h->v, h->normals[0], h->normals[1], h->phi, h->w, h->partial, h->dense, h->hodiag,
+                    h->v, h->normals[0], h->normals[1], h->owner, h->dense, h->hodiag,
                     h->counters};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     tc::destroy(h->tcp);
+    i8::destroy(h->ip);
     stein_destroy(h->sp);
     for (int b = 0; b < 2; b++) {
         if (h->copied[b]) cudaEventDestroy(h->copied[b]);
@@ -601,7 +601,6 @@ int scp3gpu_hbuild_create(const scp3gpu_config* c, scp3gpu_hbuild** out)
         if ((rc = tc::create(h->tcp, h->nb, c->nmodes, c->n2, c->n3, c->chunk, sms, f16)))
             return bail(rc);
         h->chunk = h->tcp.chunk;
-        h->nb_pad = h->tcp.nb_pad;
         for (int b = 0; b < 2; b++)
             if ((rc = dalloc(&h->q32b[b], (size_t)h->chunk * c->nmodes)) || (rc = dalloc(&h->vb[b], (size_t)h->chunk)))
                 return bail(rc);
@@ -613,16 +612,12 @@ int scp3gpu_hbuild_create(const scp3gpu_config* c, scp3gpu_hbuild** out)
             if ((rc = stein_create(h->sp, desc, c->nmodes, c->chunk, sms, c->precision != SCP3GPU_PREC_FP64)))
                 return bail(rc);
             h->chunk = h->sp.chunk;
-            h->nsplit = h->sp.nsplit;
-            h->nb_pad = h->sp.nb_pad;
             if ((rc = dalloc(&h->q64, (size_t)h->chunk * c->nmodes)) || (rc = dalloc(&h->v, (size_t)h->chunk)) ||
                 (rc = dalloc(&h->vq, (size_t)h->chunk * c->nmodes)))
                 return bail(rc);
         } else {
-            plan_fp64(h, sms);
-            if ((rc = dalloc(&h->q64, (size_t)h->chunk * c->nmodes)) || (rc = dalloc(&h->v, (size_t)h->chunk)) ||
-                (rc = dalloc(&h->partial, (size_t)h->nsplit * h->tm.ntiles * h->tm.tile * h->tm.tile)) ||
-                (rc = dalloc(&h->phi, (size_t)h->nb_pad * h->chunk)) || (rc = dalloc(&h->w, (size_t)h->nb_pad * h->chunk)))
+            if ((rc = plan_fp64(h, desc, sms)) || (rc = dalloc(&h->q64, (size_t)h->chunk * c->nmodes)) ||
+                (rc = dalloc(&h->v, (size_t)h->chunk)))
                 return bail(rc);
         }
     }
@@ -685,7 +680,7 @@ int scp3gpu_hbuild_add_epot(scp3gpu_hbuild* h, const double* q, const double* V,
     SCP3_CUDA(cudaStreamSynchronize(h->stream));
     for (int64_t off = 0; off < n; off += h->chunk) {
         const int64_t c = std::min(h->chunk, n - off);
-        const int64_t kn = h->split_form ? tc::pass_samples(h->tcp, c) : round_up(c, 16ll * h->nsplit);
+        const int64_t kn = h->split_form ? tc::pass_samples(h->tcp, c) : i8::pass_samples(c);
         SCP3_CUDA(cudaMemsetAsync(h->v, 0, sizeof(double) * kn, h->stream));
         SCP3_CUDA(cudaMemcpyAsync(h->v, V + off, sizeof(double) * c, cudaMemcpyHostToDevice, h->stream));
         int rc;
@@ -698,9 +693,8 @@ int scp3gpu_hbuild_add_epot(scp3gpu_hbuild* h, const double* q, const double* V,
         } else {
             SCP3_CUDA(cudaMemsetAsync(h->q64, 0, sizeof(double) * kn * nm, h->stream));
             SCP3_CUDA(cudaMemcpyAsync(h->q64, q + off * nm, sizeof(double) * c * nm, cudaMemcpyHostToDevice, h->stream));
-            rc = launch_expand_fp64_sm(h->desc, h->nb, nm, h->q64, h->v, kn, h->nb_pad, h->phi, h->w, h->stream);
-            if (!rc) rc = launch_contract_fp64_t128(h->phi, h->w, h->nb_pad, kn, h->tm, h->nsplit, h->partial,
-                                                    h->stream);
+            rc = i8::prepare(h->ip, h->q64, h->v, nullptr, kn, h->stream);
+            if (!rc) rc = i8::contract(h->ip, kn, h->stream);
             SCP3_CUDA(cudaStreamSynchronize(h->stream));
         }
         if (rc) return rc;
@@ -735,6 +729,14 @@ int scp3gpu_hbuild_add_epot_grad(scp3gpu_hbuild* h, const double* q, const doubl
     return SCP3GPU_OK;
 }
 
+// The plan whose error flag a synchronising read-out reports (the matrix of an
+// unfinished pass reads NaN in any case); the split forms report it in build_dense.
+static const i8::Plan* integer_plan(const scp3gpu_hbuild* h)
+{
+    if (h->split_form || (h->gradient && h->sp.split)) return nullptr;
+    return h->gradient ? &h->sp.ip : &h->ip;
+}
+
 static int build_dense(scp3gpu_hbuild* h, int mode)
 {
     int rc;
@@ -754,7 +756,8 @@ static int build_dense(scp3gpu_hbuild* h, int mode)
     Timed t(h, 3);
     if (h->split_form) return tc::unpack(h->tcp, h->nb, divisor, diag, zpe, h->dense, h->nb, h->stream);
     if (h->gradient) return stein_unpack(h->sp, h->desc, divisor, diag, zpe, h->dense, h->nb, h->stream);
-    return launch_unpack(h->partial, h->tm, h->nsplit, h->nb, divisor, diag, zpe, h->dense, h->nb, h->stream);
+    return tc::launch_unpack(h->ip.partial, h->owner, h->nt, h->ip.ntiles, h->ip.nsplit, h->nb, divisor, diag, zpe, h->dense,
+                             h->nb, h->stream, h->ip.err);
 }
 
 int scp3gpu_hbuild_read(scp3gpu_hbuild* h, double* M, int64_t ld, int mode)
@@ -766,6 +769,7 @@ int scp3gpu_hbuild_read(scp3gpu_hbuild* h, double* M, int64_t ld, int mode)
     if (rc) return rc;
     SCP3_CUDA(cudaMemcpy2DAsync(M, sizeof(double) * ld, h->dense, sizeof(double) * h->nb, sizeof(double) * h->nb,
                                 h->nb, cudaMemcpyDeviceToHost, h->stream));
+    if (const i8::Plan* p = integer_plan(h)) return i8::check(*p, h->stream);
     SCP3_CUDA(cudaStreamSynchronize(h->stream));
     return SCP3GPU_OK;
 }
@@ -789,6 +793,7 @@ int scp3gpu_hbuild_eigvals(scp3gpu_hbuild* h, int64_t nsub, int k, double* evals
         return fail(SCP3GPU_ERR_ARG, "eigvals: bad arguments");
     DeviceGuard g(h->dev);
     int rc = build_dense(h, 1);
+    if (!rc && integer_plan(h)) rc = i8::check(*integer_plan(h), h->stream);
     if (rc) return rc;
     const int n = (int)nsub;
     double *A = nullptr, *W = nullptr, *work = nullptr;

@@ -7,6 +7,7 @@
 #include <vector>
 
 #include "../../include/scp3gpu.h"
+#include "contract_i8.h"
 
 namespace scp3 {
 
@@ -149,7 +150,7 @@ int launch_std_normal(int dims, int64_t index0, int64_t n, const int64_t* vdir, 
 int launch_expand_fp64(const uint32_t* desc, int nb, int nb_pad, int nm, const double* q, const double* v,
                        int64_t n, int64_t ldk, double* phi, double* w, cudaStream_t s);
 
-// Gradient (Stein) estimator, FP64, as products of reduced basis functions
+// Gradient (Stein) estimator, as products of reduced basis functions
 // (stein.cu).  Virtual rows (m, i): basis function i that excites mode m, ordered
 // by m then i, plus one last row for <0|V|0>.
 struct SteinPlan {
@@ -157,7 +158,7 @@ struct SteinPlan {
     int nv = 0, nv_pad = 0;          // virtual rows (with the ground row), padded to 128
     int rt = 0, ct = 0;              // 128-row tiles of the virtual rows and of the basis
     int nsplit = 1;                  // sample ranges of the products (C)
-    int dsplit = 1;                  // sample ranges of the same-mode pair sums (D), a multiple of nsplit
+    int dsplit = 1;                  // sample ranges of the same-mode pair sums (D)
     int64_t chunk = 0;               // samples per pass
     int64_t dsize = 0;               // doubles of the same-mode pair sums per split
     int ndtasks = 0;
@@ -168,13 +169,11 @@ struct SteinPlan {
     int4* dtasks = nullptr;          // [ndtasks] (m, row tile, column tile) of the tiled pair kernel
     int nftasks = 0;
     int* ftasks = nullptr;           // [nftasks] modes of the triangle-blocked pair kernel
-    double* W = nullptr;             // [chunk][nv_pad]  reduced function x Stein weight
-    double* Phi = nullptr;           // [chunk][nb_pad]  basis functions
-    double* C = nullptr;             // [nsplit][rt * ct][128 * 128]
     double* D = nullptr;             // [dsplit][dsize]
-    // Split form (BF16x3 products on the tensor cores): W and Phi as one operand of
-    // 32-slot boxes, W rows [0, nv_pad), Phi rows from nv_pad; C is then the
-    // 128 x 256 tiles' unit partials P.
+    // The products, on the tensor cores: W and Phi as one operand, W rows [0, nv_pad),
+    // Phi rows after the W_b rows.  FP64 form: integer products (contract_i8.cu).
+    i8::Plan ip;
+    // Split form: BF16x3, the operand in 32-slot boxes, unit partials P.
     bool split = false;
     int bpairs = 0;                  // Phi panel pairs (the last a one-panel tile when ct is odd)
     int ntiles2 = 0;                 // tiles (W panel, Phi pair): rt * bpairs
@@ -204,7 +203,7 @@ struct SteinPlan {
     double* P = nullptr;             // [nsplit][ntiles2][128 x 256] tile-local column-major
     int* err = nullptr;              // a bounded wait of the contraction expired
 };
-// split: BF16x3 products (tcgen05) instead of FP64 ones.
+// split: BF16x3 products instead of FP64 ones.
 int stein_create(SteinPlan& p, const std::vector<uint32_t>& desc, int nm, int64_t chunk, int sms,
                  bool split = false);
 // Samples of a pass holding nvalid samples (padding samples carry V = 0 and dV/dq = 0).
@@ -227,25 +226,6 @@ struct TileMap {
 // P[split][tile][tile*tile] += sum over this split's sample range of Phi_i W_j.
 int launch_contract_fp64(const double* phi, const double* w, int64_t ldk, int64_t k, int nb_pad,
                          const TileMap& tm, int nsplit, double* partial, cudaStream_t s);
-
-// The plain build's form: Phi and W sample-major ([k][ld], ld = tm.nt * 128),
-// P[split][tile][128*128] += sum over this split's sample range of Phi_i W_j.
-int launch_expand_fp64_sm(const uint32_t* desc, int nb, int nm, const double* q, const double* v, int64_t n,
-                          int64_t ld, double* phi, double* w, cudaStream_t s);
-int launch_contract_fp64_t128(const double* phi, const double* w, int64_t ld, int64_t k, const TileMap& tm,
-                              int nsplit, double* partial, cudaStream_t s);
-
-// P[split][ti * ct + tj][128*128] += sum over this split's sample range of
-// A[k][ti*128 + r] B[k][tj*128 + c] (sample-major operands, every tile of the
-// rt x ct rectangle).
-int launch_gemm_fp64_rect(const double* A, int64_t lda, const double* B, int64_t ldb, int64_t k, int rt, int ct,
-                          int nsplit, double* partial, cudaStream_t s);
-
-// Sum the splits of P into a dense column-major nb x nb matrix (upper triangle
-// mirrored to the lower), divided by `divisor`; with `diag` (length nb) the
-// diagonal becomes (v + diag[i]) + zpe, the order of SCP3.cpp:237-239.
-int launch_unpack(const double* partial, const TileMap& tm, int nsplit, int nb, double divisor, const double* diag,
-                  double zpe, double* M, int64_t ld, cudaStream_t s);
 
 // Upload the TTM3-F constants (combined monomer coefficients, damping widths)
 // to the current device once.

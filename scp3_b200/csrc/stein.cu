@@ -36,66 +36,14 @@
 #include <array>
 #include <map>
 
+#include "contract_i8.h"
+#include "hermite.cuh"
 #include "internal.h"
 #include "tc.h"
 
 namespace scp3 {
 
 namespace {
-
-// (mode, level) list of a basis descriptor (kind | m << 3 | n << 11 | p << 19)
-__host__ __device__ __forceinline__ int decode(uint32_t d, int* m, int* l)
-{
-    const int kind = (int)(d & 7u), a = (int)((d >> 3) & 255u), b = (int)((d >> 11) & 255u), c = (int)(d >> 19);
-    switch (kind) {
-        case kGround: return 0;
-        case kHo1: m[0] = a, l[0] = 1; return 1;
-        case kHo2: m[0] = a, l[0] = 2; return 1;
-        case kHo1Ho1: m[0] = a, l[0] = 1, m[1] = b, l[1] = 1; return 2;
-        case kHo3: m[0] = a, l[0] = 3; return 1;
-        case kHo2Ho1: m[0] = a, l[0] = 2, m[1] = b, l[1] = 1; return 2;
-        case kHo1Ho2: m[0] = a, l[0] = 1, m[1] = b, l[1] = 2; return 2;
-        default: m[0] = a, l[0] = 1, m[1] = b, l[1] = 1, m[2] = c, l[2] = 1; return 3;
-    }
-}
-
-// h_l(q) (HarmonicOscillatorBasis.cpp: 1, sqrt2 q, (2q^2 - 1)/sqrt2, (2q^3 - 3q)/sqrt3)
-__device__ __forceinline__ double ho(int l, double q)
-{
-    switch (l) {
-        case 0: return 1.0;
-        case 1: return 1.4142135623730951 * q;
-        case 2: return (2.0 * q * q - 1.0) * 0.70710678118654752;
-        default: return (2.0 * q * q - 3.0) * q * 0.57735026918962576;
-    }
-}
-
-// h_a(q), h_a(0), h_a'(q), d_a(q), d_a'(q) for the oscillator functions h_0..h_3
-__device__ __forceinline__ void ho_parts(int a, double q, double& h, double& h0, double& dh, double& d, double& dd)
-{
-    constexpr double s2 = 1.4142135623730951, is2 = 0.70710678118654752, is3 = 0.57735026918962576;
-    switch (a) {
-        case 0: h = 1, h0 = 1, dh = 0, d = 0, dd = 0; break;
-        case 1: h = s2 * q, h0 = 0, dh = s2, d = s2, dd = 0; break;
-        case 2: h = (2 * q * q - 1) * is2, h0 = -is2, dh = 2 * s2 * q, d = s2 * q, dd = s2; break;
-        default: h = (2 * q * q - 3) * q * is3, h0 = 0, dh = (6 * q * q - 3) * is3, d = (2 * q * q - 3) * is3,
-                 dd = 4 * q * is3; break;
-    }
-}
-
-// K_ab = u V + w dV/dq_m for mode m at q_m = x, levels (a, b)
-__device__ __forceinline__ double stein_weight(int a, int b, double x, double V, double Vm)
-{
-    double ha, ha0, dha, da, dda, hb, hb0, dhb, db, ddb;
-    ho_parts(a, x, ha, ha0, dha, da, dda);
-    ho_parts(b, x, hb, hb0, dhb, db, ddb);
-    const double r = da * hb + ha0 * db;
-    const double dr = dda * hb + da * dhb + ha0 * ddb;
-    double u = ha0 * hb0 + 0.5 * dr;
-    const double w = 0.5 * r;
-    if (a == 3 && b == 3) u = (2 * x * x - 3) * (x * x - 3) * (1.0 / 6.0);   // TripleExcitations.h:763-773
-    return u * V + w * Vm;
-}
 
 // Virtual row descriptor: m | a << 8 | m1 << 10 | l1 << 18 | m2 << 20 | l2 << 28,
 // (m1, l1), (m2, l2) the function's other factors (level 0: none); bit 30: the
@@ -111,58 +59,6 @@ __device__ __forceinline__ double reduced(uint32_t vd, const double* qs, int str
     return r;
 }
 
-constexpr int kExpS = 64, kExpR = 128;
-constexpr int kExpLd = kExpS + 1;   // odd row stride of the staged q: a warp's rows read different modes conflict-free
-
-// Phi [s][j] (ld nb_pad) and W [s][r] (ld nv_pad) for 64 samples; one thread per
-// row of the stacked [Phi rows | W rows], coalesced 1 KB stores per sample.
-__global__ void __launch_bounds__(kExpR) stein_expand_kernel(const uint32_t* __restrict__ desc, int nb, int nb_pad,
-                                                             const uint32_t* __restrict__ vrdesc, int nv,
-                                                             int nv_pad, int nm, const double* __restrict__ q,
-                                                             const double* __restrict__ v,
-                                                             const double* __restrict__ vq, int64_t n,
-                                                             double* __restrict__ Phi, double* __restrict__ W)
-{
-    extern __shared__ double st[];          // q [nm][65], vq [nm][65], V [64]
-    double* qs = st;
-    double* vqs = st + (size_t)nm * kExpLd;
-    double* vs = vqs + (size_t)nm * kExpLd;
-    const int t = threadIdx.x;
-    const int64_t s0 = (int64_t)blockIdx.x * kExpS;
-    for (int e = t; e < nm * kExpS; e += kExpR) {
-        const int ss = e / nm, m = e - ss * nm;          // coalesced reads of row s0 + ss
-        const bool ok = s0 + ss < n;
-        qs[m * kExpLd + ss] = ok ? q[(s0 + ss) * nm + m] : 0.0;
-        vqs[m * kExpLd + ss] = ok ? vq[(s0 + ss) * nm + m] : 0.0;
-    }
-    for (int ss = t; ss < kExpS; ss += kExpR) vs[ss] = s0 + ss < n ? v[s0 + ss] : 0.0;
-    __syncthreads();
-    const int ns = (int)min((int64_t)kExpS, n - s0);
-    const int row = blockIdx.y * kExpR + t;
-    if (row < nb_pad) {
-        int mm[3], ll[3], k = 0;
-        if (row < nb) k = decode(__ldg(desc + row), mm, ll);
-        for (int j = 0; j < ns; j++) {
-            double x = row < nb ? 1.0 : 0.0;
-            for (int u = 0; u < k; u++) x *= ho(ll[u], qs[mm[u] * kExpLd + j]);
-            Phi[(size_t)(s0 + j) * nb_pad + row] = x;
-        }
-    } else {
-        const int r = row - nb_pad;
-        const uint32_t vd = r < nv ? __ldg(vrdesc + r) : 0u;
-        const int m = vd & 255, a = (vd >> 8) & 3;
-        for (int j = 0; j < ns; j++) {
-            double x = 0.0;
-            if (r < nv) {
-                if (vd & kGroundRow) x = vs[j];
-                else x = reduced(vd, qs, kExpLd, j) *
-                         stein_weight(a, 0, qs[m * kExpLd + j], vs[j], vqs[m * kExpLd + j]);
-            }
-            W[(size_t)(s0 + j) * nv_pad + r] = x;
-        }
-    }
-}
-
 // Split form: x = hi + lo in BF16 for two values, each half packed in one
 // 32-bit word (the first value in the low 16 bits), round-to-nearest.
 __device__ __forceinline__ void split_bf16x2(float x0, float x1, uint32_t& hi, uint32_t& lo)
@@ -176,11 +72,11 @@ __device__ __forceinline__ void split_bf16x2(float x0, float x1, uint32_t& hi, u
 
 constexpr int kSxSlots = 32, kSxThreads = 256, kSxLd = 33;
 constexpr int kSxBlocksPerFlush = tc::kSlotsPerFlush / kSxSlots;   // 130: the last two hold only padding slots
-constexpr uint32_t kSxZeroRow = 0xffffffffu;                        // padding row: never written
+constexpr uint32_t kSxZeroRow = i8::kZeroRow;                        // padding row: never written
 constexpr int kSxMaxTable = 1024;                                   // table rows (10-bit indices)
 
 // Kinds of table rows (TableSpec: kind | a << 4 | b << 6 | mode << 8)
-enum : uint32_t { kTOne = 0, kTHo = 1, kTKa0 = 2, kTV = 3, kTKab = 4 };
+enum : uint32_t { kTOne = i8::kOne, kTHo = i8::kHo, kTKa0 = i8::kKa0, kTV = i8::kV, kTKab = i8::kKab };
 
 // h_a(q), h_a(0), h_a'(q), d_a(q), d_a'(q) in FP32 (as ho_parts)
 __device__ __forceinline__ void ho_parts_f(int a, float q, float& h, float& h0, float& dh, float& d, float& dd)
@@ -621,7 +517,6 @@ __global__ void __launch_bounds__(256) stein_rowsum_kernel(const float* __restri
 // split form's pair sums as products) the term of a pair exciting m in both
 // functions is C at W_b row (m, rank of r, level of c in m), column
 // red3(c without its mode-m factor).
-template <bool N256>
 __global__ void stein_unpack_kernel(const uint32_t* __restrict__ desc, const int* __restrict__ rank3,
                                     const int* __restrict__ voff, const int64_t* __restrict__ doff, int nb, int nv,
                                     int ct, int nsplit, int dsplit, const double* __restrict__ C,
@@ -630,7 +525,7 @@ __global__ void stein_unpack_kernel(const uint32_t* __restrict__ desc, const int
                                     double zpe, double* __restrict__ M, int64_t ld,
                                     const int* __restrict__ tile_of, const int* __restrict__ red3,
                                     const int* __restrict__ wb_off, const int* __restrict__ sum_off,
-                                    const double* __restrict__ sums)
+                                    const double* __restrict__ sums, const int* __restrict__ err)
 {
     const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= (int64_t)nb * nb) return;
@@ -639,12 +534,9 @@ __global__ void stein_unpack_kernel(const uint32_t* __restrict__ desc, const int
     // a term whose tile the plan did not make reads NaN into the element (never,
     // by construction; a visible result rather than an out-of-range read)
     auto cidx = [&](int vr, int col) -> int64_t {
-        if (N256) {
-            const int t = tile_of[(vr >> 7) * ct + (col >> 8)];
-            if (t < 0) return -1;
-            return (int64_t)t * (128 * 256) + (int64_t)(((col >> 7) & 1) * 128 + (col & 127)) * 128 + (vr & 127);
-        }
-        return ((int64_t)(vr >> 7) * ct + (col >> 7)) * (128 * 128) + (int64_t)(vr & 127) * 128 + (col & 127);
+        const int t = tile_of[(vr >> 7) * ct + (col >> 8)];
+        if (t < 0) return -1;
+        return (int64_t)t * (128 * 256) + (int64_t)(((col >> 7) & 1) * 128 + (col & 127)) * 128 + (vr & 127);
     };
     auto csum = [&](int64_t x) {
         if (x < 0) return __longlong_as_double(0x7ff8000000000000ll);
@@ -700,6 +592,7 @@ __global__ void stein_unpack_kernel(const uint32_t* __restrict__ desc, const int
     }
     val = val / divisor;
     if (diag && i == j) val = (val + diag[i]) + zpe;
+    if (*err) val = __longlong_as_double(0x7ff8000000000000ll);     // a pass did not finish
     M[(size_t)j * ld + i] = val;
 }
 
@@ -747,8 +640,8 @@ int stein_create(SteinPlan& p, const std::vector<uint32_t>& desc, int nm, int64_
     p.nb = (int)desc.size();
     p.nm = nm;
     p.nb_pad = (int)round_up(p.nb, 128);
-    if (sizeof(double) * (2 * (size_t)nm * kExpLd + kExpS) > 227 * 1024)
-        return fail(SCP3GPU_ERR_ARG, "stein: too many modes for the expansion's shared memory (at most 220)");
+    if (!split && 6 * nm + 2 > i8::table_room())
+        return fail(SCP3GPU_ERR_ARG, "stein: too many modes for the expansion's table (at most 140)");
     if (split && 6 * nm + 2 > kSxMaxTable)
         return fail(SCP3GPU_ERR_ARG, "stein: too many modes for the split expansion's table (at most 170)");
     // functions exciting each mode, in basis order; rank of each in its mode's list
@@ -824,148 +717,193 @@ int stein_create(SteinPlan& p, const std::vector<uint32_t>& desc, int nm, int64_
     p.dsize = std::max<int64_t>(dsz, 1);
     p.ndtasks = (int)tasks.size();
     p.nftasks = (int)ftasks.size();
+    // The products W Phi^T on the tensor cores: tiles of one W panel against a
+    // pair of Phi panels (one panel when ct is odd).
     int rc;
-    if (!split) {
-        // passes of 2^14 samples (fewer while W and Phi of a pass would pass ~4 GB);
-        // sample ranges per tile as the plain form chooses them, the C partials of
-        // all ranges held under ~8 GB (one range if a single one is larger)
-        int64_t chunk = chunk_cfg > 0 ? chunk_cfg : 16384;
-        while (chunk > 4096 && (int64_t)(p.nv_pad + p.nb_pad) * chunk * 8 > (4ll << 30)) chunk /= 2;
-        p.chunk = chunk;
-        const int64_t csize = (int64_t)p.rt * p.ct * 128 * 128;
-        double best = 1e300;
-        p.nsplit = 1;
-        for (int ns = 1; chunk / ns >= 2048 && chunk % (16ll * ns) == 0; ns *= 2) {
-            if (ns > 1 && (csize + p.dsize) * 8 * ns > (8ll << 30)) break;
-            const int64_t units = (int64_t)p.rt * p.ct * ns;
-            const double cost = (double)((units + sms - 1) / sms) / ns;
-            if (cost < best - 1e-9) best = cost, p.nsplit = ns;
+    p.split = split;
+    p.bpairs = (p.ct + 1) / 2;
+    // The same-mode pair sums as products too, when every function j exciting m
+    // is, without its mode-m factor, again a basis function (red3) and the
+    // expansion's table holds the weights of the level pairs present:
+    // T^m_ij = sum_s [R_i^m K^m_{a_i b_j}] Phi_{red(j, m)}.
+    bool closed = true;
+    const std::vector<int> red3 = reduced_functions(desc, &closed);
+    std::vector<int> levmask(nm, 0);
+    for (int m = 0; m < nm; m++)
+        for (int l : lev[m]) levmask[m] |= 1 << l;
+    // the expansion's table holds at most 1 + 3 nm Hermite values, 3 nm weights
+    // K_a0, V and 6 nm weights K_ab: 10-bit indices
+    p.tcpairs = closed && 12 * nm + 2 <= (split ? kSxMaxTable : i8::table_room());
+    // W_b blocks (m, b), one per level b present in mode m, e_m rows each: in the
+    // operand, or summed when every function of level b in m reduces to the
+    // constant (its only Phi column would be the ground function's)
+    std::vector<int> wb_off((size_t)nm * 4, -1), sum_off((size_t)nm * 4, -1);
+    auto reduces_to_ground = [&](int m, int b) {
+        for (size_t r = 0; r < E[m].size(); r++) {
+            if (lev[m][r] != b) continue;
+            int mm[3], ll[3];
+            const int k = decode(desc[E[m][r]], mm, ll);
+            for (int a = 0; a < k; a++)
+                if (mm[a] == m && red3[(size_t)3 * E[m][r] + a] != 0) return false;
         }
-        // sample ranges of the same-mode pair sums: a multiple of the products' (so a
-        // pass of 16 * nsplit samples divides), up to 4x finer while their sums stay
-        // small -- those kernels have one CTA per mode and range, too few for the GPU
-        // at the products' split (48 x 8 for the hexamer doubles basis)
-        p.dsplit = p.nsplit;
-        while (p.dsplit < 4 * p.nsplit && p.dsplit * 2 * p.dsize * 8 <= (256ll << 20)) p.dsplit *= 2;
-        if ((rc = dalloc(&p.W, (size_t)p.chunk * p.nv_pad)) || (rc = dalloc(&p.Phi, (size_t)p.chunk * p.nb_pad)) ||
-            (rc = dalloc(&p.C, (size_t)csize * p.nsplit))) {
+        return true;
+    };
+    // The products of the W_b blocks pay whole tiles for the few columns each
+    // needs: worth it while they add no more tiles than the direct terms have
+    // (hexamer doubles basis: 19 against 95); otherwise (triples bases, where
+    // each block reaches Phi pairs all over the basis) the pair sums stay FP64.
+    if (p.tcpairs) {
+        int64_t est = 0;
+        for (int m = 0; m < nm; m++)
+            for (int b = 1; b <= 3; b++) {
+                if (!((levmask[m] >> b) & 1) || reduces_to_ground(m, b)) continue;
+                std::vector<char> pairs((size_t)p.bpairs, 0);
+                for (size_t r = 0; r < E[m].size(); r++) {
+                    if (lev[m][r] != b) continue;
+                    int mm[3], ll[3];
+                    const int k = decode(desc[E[m][r]], mm, ll);
+                    for (int a = 0; a < k; a++)
+                        if (mm[a] == m) pairs[red3[(size_t)3 * E[m][r] + a] / 256] = 1;
+                }
+                int np = 0;
+                for (char c : pairs) np += c;
+                est += (int64_t)np * (int64_t)E[m].size();     // tile rows: 128 per tile
+            }
+        if (split && est > (int64_t)128 * p.rt * p.bpairs) p.tcpairs = false;
+        // FP64 form: a tile of the integer products costs what ~600 pair sums of
+        // the FP64 kernels do where those run well (hexamer doubles basis: 57,600
+        // pairs, 641 us per 2^14 samples, against 19 tiles, ~125 us) and ~150 where
+        // they do not (a trimer with triples: 7,600 pairs, 480 us).
+        const int64_t tiles_b = est / 128 + 1;
+        if (!split && (dsz / 2 < 200 * tiles_b || (tiles_b + (int64_t)p.rt * p.bpairs) * 128 * 256 * 8 > (8ll << 30)))
+            p.tcpairs = false;
+    }
+    int nwb = 0;
+    p.nsum = 0;
+    if (p.tcpairs)
+        for (int m = 0; m < nm; m++)
+            for (int b = 1; b <= 3; b++) {
+                if (!((levmask[m] >> b) & 1)) continue;
+                if (reduces_to_ground(m, b)) {
+                    sum_off[(size_t)m * 4 + b] = p.nsum;
+                    p.nsum += (int)E[m].size();
+                } else {
+                    wb_off[(size_t)m * 4 + b] = p.nv_pad + nwb;
+                    nwb += (int)E[m].size();
+                }
+            }
+    p.nwb_pad = (int)round_up(nwb, 128);
+    const int wpanels = (p.nv_pad + p.nwb_pad) / 128;
+    const int phi0 = p.nv_pad + p.nwb_pad;     // first Phi row
+    const int64_t rows = (int64_t)phi0 + p.nb_pad;
+    // tiles: every W panel of the direct terms against every Phi pair (pair-major,
+    // so a wave's tiles share their pairs), then every W_b panel against the pairs
+    // that hold its rows' reduced functions
+    std::vector<int4> tl;
+    std::vector<int> tile_of((size_t)wpanels * p.bpairs, -1);
+    auto add_tile = [&](int r, int q) {
+        const int b0 = phi0 + 2 * q * 128, b1 = 2 * q + 1 < p.ct ? b0 + 128 : b0;
+        tile_of[(size_t)r * p.bpairs + q] = (int)tl.size();
+        tl.push_back(make_int4(r * 128, b0, 0, b1));
+    };
+    for (int q = 0; q < p.bpairs; q++)
+        for (int r = 0; r < p.rt; r++) add_tile(r, q);
+    if (p.tcpairs) {
+        std::vector<std::vector<char>> need((size_t)wpanels, std::vector<char>((size_t)p.bpairs, 0));
+        for (int m = 0; m < nm; m++)
+            for (int b = 1; b <= 3; b++) {
+                const int o = wb_off[(size_t)m * 4 + b], en = (int)E[m].size();
+                if (o < 0) continue;
+                for (int r = 0; r < en; r++) {
+                    if (lev[m][r] != b) continue;
+                    int mm[3], ll[3];
+                    const int k = decode(desc[E[m][r]], mm, ll);
+                    for (int a = 0; a < k; a++)
+                        if (mm[a] == m)
+                            for (int pr = o / 128; pr <= (o + en - 1) / 128; pr++)
+                                need[pr][red3[(size_t)3 * E[m][r] + a] / 256] = 1;
+                }
+            }
+        for (int r = p.rt; r < wpanels; r++)
+            for (int q = 0; q < p.bpairs; q++)
+                if (need[r][q]) add_tile(r, q);
+    }
+    p.ntiles2 = (int)tl.size();
+    // per operand row, three indices into the expansion's table (0 = the constant 1);
+    // the table holds the entries the rows use, numbered as they are first needed
+    std::map<uint32_t, uint32_t> tslot;
+    std::vector<uint32_t> tspec{kTOne};
+    auto tab = [&](uint32_t kind, int a, int b, int m) -> uint32_t {
+        const uint32_t key = kind | (uint32_t)a << 4 | (uint32_t)b << 6 | (uint32_t)m << 8;
+        const auto it = tslot.find(key);
+        if (it != tslot.end()) return it->second;
+        const uint32_t i = (uint32_t)tspec.size();
+        tspec.push_back(key);
+        tslot[key] = i;
+        return i;
+    };
+    auto hidx = [&](int m, int l) { return l ? tab(kTHo, l, 0, m) : 0u; };
+    std::vector<uint32_t> xd((size_t)rows + p.nsum, kSxZeroRow);   // operand rows, then summed rows
+    for (int r = 0; r < p.nv; r++) {
+        const uint32_t vd = vrdesc[r];
+        if (vd & kGroundRow) {
+            xd[r] = tab(kTV, 0, 0, 0);
+            continue;
+        }
+        const int m = vd & 255, a = (vd >> 8) & 3;
+        xd[r] = tab(kTKa0, a, 0, m) | hidx((vd >> 10) & 255, (vd >> 18) & 3) << 10 |
+                hidx((vd >> 20) & 255, (vd >> 28) & 3) << 20;
+    }
+    for (int m = 0; m < nm; m++)        // W_b(m, r) = R^m_{E_m[r]} K^m_{a_r b}
+        for (int b = 1; b <= 3; b++) {
+            const int o = wb_off[(size_t)m * 4 + b] >= 0 ? wb_off[(size_t)m * 4 + b]
+                          : sum_off[(size_t)m * 4 + b] >= 0 ? (int)rows + sum_off[(size_t)m * 4 + b]
+                                                             : -1;
+            if (o < 0) continue;
+            for (size_t r = 0; r < E[m].size(); r++) {
+                const uint32_t vd = vrdesc[voff[m] + r];
+                const int a = lev[m][r];
+                xd[(size_t)o + r] = tab(kTKab, std::min(a, b), std::max(a, b), m) |
+                                    hidx((vd >> 10) & 255, (vd >> 18) & 3) << 10 |
+                                    hidx((vd >> 20) & 255, (vd >> 28) & 3) << 20;
+            }
+        }
+    for (int j = 0; j < p.nb; j++) {
+        int mm[3] = {0, 0, 0}, ll[3] = {0, 0, 0};
+        decode(desc[j], mm, ll);
+        xd[(size_t)phi0 + j] = hidx(mm[0], ll[0]) | hidx(mm[1], ll[1]) << 10 | hidx(mm[2], ll[2]) << 20;
+    }
+    p.trows = (int)tspec.size();
+    if ((rc = upload(&p.tile_of, tile_of.data(), tile_of.size())) ||
+        (p.tcpairs && ((rc = upload(&p.red3, red3.data(), red3.size())) ||
+                       (rc = upload(&p.wb_off, wb_off.data(), wb_off.size())) ||
+                       (rc = upload(&p.sum_off, sum_off.data(), sum_off.size()))))) {
+        stein_destroy(p);
+        return rc;
+    }
+    if (!split) {
+        // passes of 2^15 samples, fewer while their digits would pass ~4 GB
+        int64_t chunk = chunk_cfg > 0 ? chunk_cfg : 32768;
+        while (chunk > 4096 && rows * chunk * 7 > (4ll << 30)) chunk /= 2;
+        p.chunk = chunk;
+        p.nsplit = i8::plan_splits(p.ntiles2, chunk, sms);
+        if ((rc = i8::create(p.ip, tspec, xd, (int)rows, 0, p.nsum, nm, tl, p.nsplit, chunk, sms))) {
             stein_destroy(p);
             return rc;
         }
+        p.dsplit = 1;
+        while (!p.tcpairs && p.dsplit < i8::kKB && p.dsplit * 2 * p.dsize * 8 <= (256ll << 20)) p.dsplit *= 2;
     } else {
-        // The products W Phi^T on the tensor cores: tiles of one W panel against a
-        // pair of Phi panels (one panel when ct is odd), K slots in blocks of 4160
-        // per 4096 samples (the contraction's sign groups, here all positive).
-        // Passes of 2^16 samples (fewer while the operand would pass ~4 GB); sample
-        // ranges per tile minimising waves per range, at most 16, partials under ~4 GB.
-        p.split = true;
-        p.bpairs = (p.ct + 1) / 2;
-        // The same-mode pair sums as products too, when every function j exciting m
-        // is, without its mode-m factor, again a basis function (red3) and the
-        // expansion's table holds the weights of the level pairs present:
-        // T^m_ij = sum_s [R_i^m K^m_{a_i b_j}] Phi_{red(j, m)}.
-        bool closed = true;
-        const std::vector<int> red3 = reduced_functions(desc, &closed);
-        std::vector<int> levmask(nm, 0);
-        for (int m = 0; m < nm; m++)
-            for (int l : lev[m]) levmask[m] |= 1 << l;
-        // the expansion's table holds at most 1 + 3 nm Hermite values, 3 nm weights
-        // K_a0, V and 6 nm weights K_ab: 10-bit indices
-        p.tcpairs = closed && 12 * nm + 2 <= kSxMaxTable;
-        // W_b blocks (m, b), one per level b present in mode m, e_m rows each: in the
-        // operand, or summed when every function of level b in m reduces to the
-        // constant (its only Phi column would be the ground function's)
-        std::vector<int> wb_off((size_t)nm * 4, -1), sum_off((size_t)nm * 4, -1);
-        auto reduces_to_ground = [&](int m, int b) {
-            for (size_t r = 0; r < E[m].size(); r++) {
-                if (lev[m][r] != b) continue;
-                int mm[3], ll[3];
-                const int k = decode(desc[E[m][r]], mm, ll);
-                for (int a = 0; a < k; a++)
-                    if (mm[a] == m && red3[(size_t)3 * E[m][r] + a] != 0) return false;
-            }
-            return true;
-        };
-        // The products of the W_b blocks pay whole tiles for the few columns each
-        // needs: worth it while they add no more tiles than the direct terms have
-        // (hexamer doubles basis: 19 against 95); otherwise (triples bases, where
-        // each block reaches Phi pairs all over the basis) the pair sums stay FP64.
-        if (p.tcpairs) {
-            int64_t est = 0;
-            for (int m = 0; m < nm; m++)
-                for (int b = 1; b <= 3; b++) {
-                    if (!((levmask[m] >> b) & 1) || reduces_to_ground(m, b)) continue;
-                    std::vector<char> pairs((size_t)p.bpairs, 0);
-                    for (size_t r = 0; r < E[m].size(); r++) {
-                        if (lev[m][r] != b) continue;
-                        int mm[3], ll[3];
-                        const int k = decode(desc[E[m][r]], mm, ll);
-                        for (int a = 0; a < k; a++)
-                            if (mm[a] == m) pairs[red3[(size_t)3 * E[m][r] + a] / 256] = 1;
-                    }
-                    int np = 0;
-                    for (char c : pairs) np += c;
-                    est += (int64_t)np * (int64_t)E[m].size();     // tile rows: 128 per tile
-                }
-            if (est > (int64_t)128 * p.rt * p.bpairs) p.tcpairs = false;
-        }
-        int nwb = 0;
-        p.nsum = 0;
-        if (p.tcpairs)
-            for (int m = 0; m < nm; m++)
-                for (int b = 1; b <= 3; b++) {
-                    if (!((levmask[m] >> b) & 1)) continue;
-                    if (reduces_to_ground(m, b)) {
-                        sum_off[(size_t)m * 4 + b] = p.nsum;
-                        p.nsum += (int)E[m].size();
-                    } else {
-                        wb_off[(size_t)m * 4 + b] = p.nv_pad + nwb;
-                        nwb += (int)E[m].size();
-                    }
-                }
-        p.nwb_pad = (int)round_up(nwb, 128);
-        const int wpanels = (p.nv_pad + p.nwb_pad) / 128;
-        const int phi0 = p.nv_pad + p.nwb_pad;     // first Phi row
-        const int64_t rows = (int64_t)phi0 + p.nb_pad;
+        // K slots in blocks of 4160 per 4096 samples (the contraction's sign groups,
+        // here all positive).  Passes of 2^16 samples (fewer while the operand would
+        // pass ~4 GB); sample ranges per tile minimising waves per range, at most 16,
+        // partials under ~4 GB.
         auto slots_of = [](int64_t k) { return k / tc::kFlush * tc::kSlotsPerFlush; };
         int64_t chunk = chunk_cfg > 0 ? chunk_cfg : 65536;
         while (chunk > tc::kFlush && rows * slots_of(chunk) * 4 > (4ll << 30)) chunk /= 2;
         chunk = std::max<int64_t>(chunk / tc::kFlush * tc::kFlush, tc::kFlush);
         p.chunk = chunk;
         p.slots = slots_of(chunk);
-        // tiles: every W panel of the direct terms against every Phi pair (pair-major,
-        // so a wave's tiles share their pairs), then every W_b panel against the pairs
-        // that hold its rows' reduced functions
-        std::vector<int4> tl;
-        std::vector<int> tile_of((size_t)wpanels * p.bpairs, -1);
-        auto add_tile = [&](int r, int q) {
-            const int b0 = phi0 + 2 * q * 128, b1 = 2 * q + 1 < p.ct ? b0 + 128 : b0;
-            tile_of[(size_t)r * p.bpairs + q] = (int)tl.size();
-            tl.push_back(make_int4(r * 128, b0, 0, b1));
-        };
-        for (int q = 0; q < p.bpairs; q++)
-            for (int r = 0; r < p.rt; r++) add_tile(r, q);
-        if (p.tcpairs) {
-            std::vector<std::vector<char>> need((size_t)wpanels, std::vector<char>((size_t)p.bpairs, 0));
-            for (int m = 0; m < nm; m++)
-                for (int b = 1; b <= 3; b++) {
-                    const int o = wb_off[(size_t)m * 4 + b], en = (int)E[m].size();
-                    if (o < 0) continue;
-                    for (int r = 0; r < en; r++) {
-                        if (lev[m][r] != b) continue;
-                        int mm[3], ll[3];
-                        const int k = decode(desc[E[m][r]], mm, ll);
-                        for (int a = 0; a < k; a++)
-                            if (mm[a] == m)
-                                for (int pr = o / 128; pr <= (o + en - 1) / 128; pr++)
-                                    need[pr][red3[(size_t)3 * E[m][r] + a] / 256] = 1;
-                    }
-                }
-            for (int r = p.rt; r < wpanels; r++)
-                for (int q = 0; q < p.bpairs; q++)
-                    if (need[r][q]) add_tile(r, q);
-        }
-        p.ntiles2 = (int)tl.size();
         double best = 1e300;
         p.nsplit = 1;
         for (int m = 1; m <= 16; m++) {
@@ -978,66 +916,16 @@ int stein_create(SteinPlan& p, const std::vector<uint32_t>& desc, int nm, int64_
         while (!p.tcpairs && p.dsplit < 64 && p.dsplit * 2 * p.dsize * 8 <= (256ll << 20)) p.dsplit *= 2;
         const std::vector<int> nosign((size_t)(chunk / tc::kFlush), tc::kSlotsPerFlush / 16);
         const size_t xop_elems = (size_t)2 * rows * p.slots;
-        // per operand row, three indices into the expansion's table (0 = the constant 1);
-        // the table holds the entries the rows use, numbered as they are first needed
-        std::map<uint32_t, uint32_t> tslot;
-        std::vector<uint32_t> tspec{kTOne};
-        auto tab = [&](uint32_t kind, int a, int b, int m) -> uint32_t {
-            const uint32_t key = kind | (uint32_t)a << 4 | (uint32_t)b << 6 | (uint32_t)m << 8;
-            const auto it = tslot.find(key);
-            if (it != tslot.end()) return it->second;
-            const uint32_t i = (uint32_t)tspec.size();
-            tspec.push_back(key);
-            tslot[key] = i;
-            return i;
-        };
-        auto hidx = [&](int m, int l) { return l ? tab(kTHo, l, 0, m) : 0u; };
-        std::vector<uint32_t> xd((size_t)rows + p.nsum, kSxZeroRow);   // operand rows, then summed rows
-        for (int r = 0; r < p.nv; r++) {
-            const uint32_t vd = vrdesc[r];
-            if (vd & kGroundRow) {
-                xd[r] = tab(kTV, 0, 0, 0);
-                continue;
-            }
-            const int m = vd & 255, a = (vd >> 8) & 3;
-            xd[r] = tab(kTKa0, a, 0, m) | hidx((vd >> 10) & 255, (vd >> 18) & 3) << 10 |
-                    hidx((vd >> 20) & 255, (vd >> 28) & 3) << 20;
-        }
-        for (int m = 0; m < nm; m++)        // W_b(m, r) = R^m_{E_m[r]} K^m_{a_r b}
-            for (int b = 1; b <= 3; b++) {
-                const int o = wb_off[(size_t)m * 4 + b] >= 0 ? wb_off[(size_t)m * 4 + b]
-                              : sum_off[(size_t)m * 4 + b] >= 0 ? (int)rows + sum_off[(size_t)m * 4 + b]
-                                                                 : -1;
-                if (o < 0) continue;
-                for (size_t r = 0; r < E[m].size(); r++) {
-                    const uint32_t vd = vrdesc[voff[m] + r];
-                    const int a = lev[m][r];
-                    xd[(size_t)o + r] = tab(kTKab, std::min(a, b), std::max(a, b), m) |
-                                        hidx((vd >> 10) & 255, (vd >> 18) & 3) << 10 |
-                                        hidx((vd >> 20) & 255, (vd >> 28) & 3) << 20;
-                }
-            }
-        for (int j = 0; j < p.nb; j++) {
-            int mm[3] = {0, 0, 0}, ll[3] = {0, 0, 0};
-            decode(desc[j], mm, ll);
-            xd[(size_t)phi0 + j] = hidx(mm[0], ll[0]) | hidx(mm[1], ll[1]) << 10 | hidx(mm[2], ll[2]) << 20;
-        }
-        p.trows = (int)tspec.size();
         if (p.trows > kSxMaxTable) {
             stein_destroy(p);
             return fail(SCP3GPU_ERR_ARG, "stein: the split expansion's table exceeds 1024 rows");
         }
         if ((rc = upload(&p.xdesc, xd.data(), xd.size())) || (rc = upload(&p.tspec, tspec.data(), tspec.size())) ||
             (rc = upload(&p.tiles2, tl.data(), tl.size())) ||
-            (rc = upload(&p.tile_of, tile_of.data(), tile_of.size())) ||
-            (p.tcpairs && ((rc = upload(&p.red3, red3.data(), red3.size())) ||
-                           (rc = upload(&p.wb_off, wb_off.data(), wb_off.size())) ||
-                           (rc = upload(&p.sum_off, sum_off.data(), sum_off.size())))) ||
             (p.nsum && ((rc = dalloc(&p.spart, (size_t)(chunk / tc::kFlush) * kSxBlocksPerFlush * p.nsum)) ||
                         (rc = dalloc(&p.sums, (size_t)p.nsum)))) ||
-            (rc = upload(&p.nosign, nosign.data(), nosign.size())) ||
-            (rc = dalloc(&p.xop, xop_elems)) || (rc = dalloc(&p.P, (size_t)p.nsplit * p.ntiles2 * 128 * 256)) ||
-            (rc = dalloc(&p.err, (size_t)1))) {
+            (rc = upload(&p.nosign, nosign.data(), nosign.size())) || (rc = dalloc(&p.xop, xop_elems)) ||
+            (rc = dalloc(&p.P, (size_t)p.nsplit * p.ntiles2 * 128 * 256)) || (rc = dalloc(&p.err, (size_t)1))) {
             stein_destroy(p);
             return rc;
         }
@@ -1065,13 +953,14 @@ int stein_create(SteinPlan& p, const std::vector<uint32_t>& desc, int nm, int64_
 
 int64_t stein_pass_samples(const SteinPlan& p, int64_t nvalid)
 {
-    return p.split ? round_up(nvalid, tc::kFlush) : round_up(nvalid, 16ll * p.nsplit);
+    return p.split ? round_up(nvalid, tc::kFlush) : i8::pass_samples(nvalid);
 }
 
 void stein_destroy(SteinPlan& p)
 {
     cudaFree(p.vrdesc), cudaFree(p.rank3), cudaFree(p.voff), cudaFree(p.doff), cudaFree(p.dtasks), cudaFree(p.ftasks);
-    cudaFree(p.W), cudaFree(p.Phi), cudaFree(p.C), cudaFree(p.D);
+    i8::destroy(p.ip);
+    cudaFree(p.D);
     cudaFree(p.xop), cudaFree(p.xdesc), cudaFree(p.tiles2), cudaFree(p.nosign), cudaFree(p.P), cudaFree(p.err);
     cudaFree(p.tile_of), cudaFree(p.red3), cudaFree(p.wb_off), cudaFree(p.tspec);
     cudaFree(p.sum_off), cudaFree(p.spart), cudaFree(p.sums);
@@ -1083,8 +972,8 @@ int stein_zero(const SteinPlan& p, cudaStream_t s)
     if (p.split) {
         SCP3_CUDA(cudaMemsetAsync(p.P, 0, sizeof(double) * (size_t)p.nsplit * p.ntiles2 * 128 * 256, s));
         SCP3_CUDA(cudaMemsetAsync(p.err, 0, sizeof(int), s));
-    } else {
-        SCP3_CUDA(cudaMemsetAsync(p.C, 0, sizeof(double) * (size_t)p.rt * p.ct * 128 * 128 * p.nsplit, s));
+    } else if (int rc = i8::zero(p.ip, s)) {
+        return rc;
     }
     if (p.D) SCP3_CUDA(cudaMemsetAsync(p.D, 0, sizeof(double) * (size_t)p.dsize * p.dsplit, s));
     if (p.sums) SCP3_CUDA(cudaMemsetAsync(p.sums, 0, sizeof(double) * (size_t)p.nsum, s));
@@ -1123,14 +1012,7 @@ int stein_pass(const SteinPlan& p, const uint32_t* desc, const double* q, const 
                                  nflush * (tc::kSlotsPerFlush / tc::kKBlock2), p.nosign, false, p.P, p.err,
                                  std::min(units, sms), s);
     } else {
-        const size_t es = sizeof(double) * (2 * (size_t)p.nm * kExpLd + kExpS);
-        if (es > 48 * 1024)
-            SCP3_CUDA(cudaFuncSetAttribute(stein_expand_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)es));
-        dim3 eg((unsigned)((k + kExpS - 1) / kExpS), (unsigned)((p.nb_pad + p.nv_pad) / kExpR));
-        stein_expand_kernel<<<eg, kExpR, es, s>>>(desc, p.nb, p.nb_pad, p.vrdesc, p.nv, p.nv_pad, p.nm, q, v, vq, k,
-                                                  p.Phi, p.W);
-        SCP3_CUDA(cudaGetLastError());
-        rc = launch_gemm_fp64_rect(p.W, p.nv_pad, p.Phi, p.nb_pad, k, p.rt, p.ct, p.nsplit, p.C, s);
+        if (!(rc = i8::prepare(p.ip, q, v, vq, k, s))) rc = i8::contract(p.ip, k, s);
     }
     if (rc) return rc;
     if (p.tcpairs) return SCP3GPU_OK;      // the pair sums were part of the products
@@ -1166,17 +1048,12 @@ int stein_unpack(const SteinPlan& p, const uint32_t* desc, double divisor, const
         SCP3_CUDA(cudaMemcpyAsync(&err, p.err, sizeof(int), cudaMemcpyDeviceToHost, s));
         SCP3_CUDA(cudaStreamSynchronize(s));
         if (err) return fail(SCP3GPU_ERR_TIMEOUT, "tensor-core contraction: a bounded pipeline wait expired");
-        stein_unpack_kernel<true><<<grid, 256, 0, s>>>(desc, p.rank3, p.voff, p.doff, p.nb, p.nv, p.bpairs, p.nsplit,
-                                                       p.dsplit, p.P, p.D, (int64_t)p.ntiles2 * 128 * 256, p.dsize,
-                                                       divisor, diag, zpe, M, ld, p.tile_of, p.red3,
-                                                       p.tcpairs ? p.wb_off : nullptr,
-                                                       p.nsum ? p.sum_off : nullptr, p.sums);
-    } else {
-        stein_unpack_kernel<false><<<grid, 256, 0, s>>>(desc, p.rank3, p.voff, p.doff, p.nb, p.nv, p.ct, p.nsplit,
-                                                        p.dsplit, p.C, p.D, (int64_t)p.rt * p.ct * 128 * 128, p.dsize,
-                                                        divisor, diag, zpe, M, ld, nullptr, nullptr, nullptr,
-                                                        nullptr, nullptr);
     }
+    stein_unpack_kernel<<<grid, 256, 0, s>>>(desc, p.rank3, p.voff, p.doff, p.nb, p.nv, p.bpairs, p.nsplit, p.dsplit,
+                                             p.split ? p.P : p.ip.partial, p.D, (int64_t)p.ntiles2 * 128 * 256, p.dsize,
+                                             divisor, diag, zpe, M, ld, p.tile_of, p.red3,
+                                             p.tcpairs ? p.wb_off : nullptr, p.nsum ? p.sum_off : nullptr,
+                                             p.split ? p.sums : p.ip.sums, p.split ? p.err : p.ip.err);
     SCP3_CUDA(cudaGetLastError());
     return SCP3GPU_OK;
 }
