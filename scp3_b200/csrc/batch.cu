@@ -38,8 +38,7 @@ struct Cluster {
     uint64_t* shift = nullptr;
     double *x0 = nullptr, *MUa = nullptr, *omega = nullptr, *hodiag = nullptr;
     int* modes = nullptr;
-    uint32_t *tasks = nullptr, *factors = nullptr;
-    int ntasks = 0;
+    uint32_t* factors = nullptr;
 };
 
 constexpr int kBuffers = 2;
@@ -126,8 +125,6 @@ SampleArgs make_args(scp3gpu_batch* b, int c, int buf, int64_t index0, int64_t n
     a.modes = k.modes;
     a.vdir = k.vdir;
     a.shift = k.shift;
-    a.tasks = k.tasks;
-    a.ntasks = k.ntasks;
     a.normals = nullptr;
     a.index0 = index0;
     a.n = npad;
@@ -298,15 +295,13 @@ int upload_cluster(Cluster& k, const scp3gpu_config* c)
     std::vector<uint64_t> sh;
     int rc = sobol_tables(c->nmodes0, c->scramble, c->scramble_seed, vd, sh);
     if (rc) return rc;
-    const std::vector<uint32_t> tasks = pair_tasks(c->nw);
     const std::vector<uint32_t> fac = basis_factor_table(c->nmodes, c->n2, c->n3);
     const std::vector<double> hod = ho_diagonal(k.omega_sel, c->n2, c->n3);
-    k.ntasks = (int)tasks.size();
     const int N3 = 9 * c->nw;
     if ((rc = upload(&k.vdir, vd.data(), vd.size())) || (c->scramble && (rc = upload(&k.shift, sh.data(), sh.size()))) ||
         (rc = upload(&k.x0, c->x0, (size_t)N3)) || (rc = upload(&k.MUa, c->MUa, (size_t)N3 * c->nmodes0)) ||
         (rc = upload(&k.omega, c->omega, (size_t)c->nmodes0)) || (rc = upload(&k.modes, c->modes, (size_t)c->nmodes)) ||
-        (rc = upload(&k.tasks, tasks.data(), tasks.size())) || (rc = upload(&k.factors, fac.data(), fac.size())) ||
+        (rc = upload(&k.factors, fac.data(), fac.size())) ||
         (rc = upload(&k.hodiag, hod.data(), hod.size())))
         return rc;
     return SCP3GPU_OK;
@@ -324,7 +319,7 @@ int scp3gpu_batch_destroy(scp3gpu_batch* b)
     if (b->prep) cudaStreamSynchronize(b->prep);
     free_graph(b);
     for (Cluster& k : b->cl) {
-        void* ptrs[] = {k.vdir, k.shift, k.x0, k.MUa, k.omega, k.hodiag, k.modes, k.tasks, k.factors};
+        void* ptrs[] = {k.vdir, k.shift, k.x0, k.MUa, k.omega, k.hodiag, k.modes, k.factors};
         for (void* p : ptrs)
             if (p) cudaFree(p);
     }

@@ -46,7 +46,7 @@ struct scp3gpu_hbuild {
     cudaEvent_t prepared[2] = {nullptr, nullptr}, contracted[2] = {nullptr, nullptr};
     cudaEvent_t head_done[2] = {nullptr, nullptr};   // a pass's whole waves of contraction units done
     int64_t pass = 0;                 // split form: passes launched (buffer = pass & 1)
-    int nb = 0, ntasks = 0;
+    int nb = 0;
     int64_t chunk = 0;
     i8::Plan ip{};                    // plain form, direct estimator: operand, tiles, partials
     int nt = 0;                       // its 128-row panels
@@ -58,7 +58,7 @@ struct scp3gpu_hbuild {
     uint64_t* shift = nullptr;
     double *x0 = nullptr, *MUa = nullptr, *omega = nullptr;
     int* modes = nullptr;
-    uint32_t *tasks = nullptr, *desc = nullptr;
+    uint32_t* desc = nullptr;
     // per chunk
     double* q64 = nullptr;
     float* q32 = nullptr;             // split form: q32 / vv[buffer]
@@ -172,8 +172,6 @@ int launch_chunk(scp3gpu_hbuild* h, int64_t index0, int64_t nvalid, const double
     a.modes = h->modes;
     a.vdir = h->vdir;
     a.shift = h->shift;
-    a.tasks = h->tasks;
-    a.ntasks = h->ntasks;
     a.normals = normals_dev;
     a.normals32 = normals32_dev;
     a.index0 = index0;
@@ -362,12 +360,8 @@ int scp3gpu_pes_energy_dev(int pes, int nw, int64_t n, const double* crd_dev, do
     if (rc) return rc;
     DeviceGuard g(device);
     if (pes == SCP3GPU_PES_TTM3F && (rc = ttm_init_device())) return rc;
-    std::vector<uint32_t> t = pair_tasks(nw);
-    uint32_t* td = nullptr;
-    if ((rc = upload(&td, t.data(), t.size()))) return rc;
-    rc = launch_pes_energy(pes, nw, n, crd_dev, E_dev, nullptr, td, (int)t.size(), 0);
+    rc = launch_pes(pes, nw, n, crd_dev, E_dev, nullptr, nullptr, 0);
     cudaError_t e = cudaStreamSynchronize(0);
-    cudaFree(td);
     if (rc) return rc;
     if (e != cudaSuccess) return cuda_fail(e, "pes_energy");
     return SCP3GPU_OK;
@@ -385,23 +379,21 @@ int scp3gpu_pes_energy(int pes, int nw, int64_t n, const double* crd, double* E,
     int rc = check_device(dev);
     if (rc) return rc;
     if (pes == SCP3GPU_PES_TTM3F && (rc = ttm_init_device())) return rc;
-    std::vector<uint32_t> t = pair_tasks(nw);
-    uint32_t* td = nullptr;
     double *cd = nullptr, *ed = nullptr;
     int* id = nullptr;
-    if ((rc = upload(&td, t.data(), t.size())) || (rc = upload(&cd, crd, (size_t)n * 9 * nw)) ||
+    if ((rc = upload(&cd, crd, (size_t)n * 9 * nw)) ||
         (rc = dalloc(&ed, (size_t)n)) || (rc = dalloc(&id, (size_t)n))) {
-        cudaFree(td), cudaFree(cd), cudaFree(ed), cudaFree(id);
+        cudaFree(cd), cudaFree(ed), cudaFree(id);
         return rc;
     }
-    rc = launch_pes_energy(pes, nw, n, cd, ed, id, td, (int)t.size(), 0);
+    rc = launch_pes(pes, nw, n, cd, ed, nullptr, id, 0);
     std::vector<int> it(n);
     if (!rc) {
         cudaError_t e = cudaMemcpy(E, ed, sizeof(double) * n, cudaMemcpyDeviceToHost);
         if (e == cudaSuccess) e = cudaMemcpy(it.data(), id, sizeof(int) * n, cudaMemcpyDeviceToHost);
         if (e != cudaSuccess) rc = cuda_fail(e, "pes_energy copy-out");
     }
-    cudaFree(td), cudaFree(cd), cudaFree(ed), cudaFree(id);
+    cudaFree(cd), cudaFree(ed), cudaFree(id);
     if (rc) return rc;
     bool capped = false;
     for (int64_t k = 0; k < n; k++) {
@@ -424,16 +416,14 @@ int scp3gpu_pes_energy_grad(int pes, int nw, int64_t n, const double* crd, doubl
     int rc = check_device(dev);
     if (rc) return rc;
     if (pes == SCP3GPU_PES_TTM3F && (rc = ttm_init_device())) return rc;
-    std::vector<uint32_t> t = pair_tasks(nw);
-    uint32_t* td = nullptr;
     double *cd = nullptr, *ed = nullptr, *gd = nullptr;
     int* id = nullptr;
-    if ((rc = upload(&td, t.data(), t.size())) || (rc = upload(&cd, crd, (size_t)n * 9 * nw)) ||
+    if ((rc = upload(&cd, crd, (size_t)n * 9 * nw)) ||
         (rc = dalloc(&ed, (size_t)n)) || (rc = dalloc(&gd, (size_t)n * 9 * nw)) || (rc = dalloc(&id, (size_t)n))) {
-        cudaFree(td), cudaFree(cd), cudaFree(ed), cudaFree(gd), cudaFree(id);
+        cudaFree(cd), cudaFree(ed), cudaFree(gd), cudaFree(id);
         return rc;
     }
-    rc = launch_pes_energy_grad(pes, nw, n, cd, ed, gd, id, td, (int)t.size(), 0);
+    rc = launch_pes(pes, nw, n, cd, ed, gd, id, 0);
     std::vector<int> it(n);
     if (!rc) {
         cudaError_t e = cudaMemcpy(E, ed, sizeof(double) * n, cudaMemcpyDeviceToHost);
@@ -441,7 +431,7 @@ int scp3gpu_pes_energy_grad(int pes, int nw, int64_t n, const double* crd, doubl
         if (e == cudaSuccess) e = cudaMemcpy(it.data(), id, sizeof(int) * n, cudaMemcpyDeviceToHost);
         if (e != cudaSuccess) rc = cuda_fail(e, "pes_energy_grad copy-out");
     }
-    cudaFree(td), cudaFree(cd), cudaFree(ed), cudaFree(gd), cudaFree(id);
+    cudaFree(cd), cudaFree(ed), cudaFree(gd), cudaFree(id);
     if (rc) return rc;
     for (int64_t k = 0; k < n; k++)
         if (it[k] > kTtmMaxIter) return fail(SCP3GPU_ERR_NOT_CONVERGED, "TTM3-F dipoles hit the iteration cap");
@@ -485,7 +475,7 @@ int scp3gpu_hbuild_destroy(scp3gpu_hbuild* h)
     if (h->stream) cudaStreamSynchronize(h->stream);
     if (h->copy_stream) cudaStreamSynchronize(h->copy_stream);
     if (h->prep_stream) cudaStreamSynchronize(h->prep_stream);
-    void* ptrs[] = {h->sur_ws, h->vq, h->ybuf, h->vdir, h->shift, h->x0, h->MUa, h->omega, h->modes, h->tasks, h->desc, h->q64, h->q32b[0],
+    void* ptrs[] = {h->sur_ws, h->vq, h->ybuf, h->vdir, h->shift, h->x0, h->MUa, h->omega, h->modes, h->desc, h->q64, h->q32b[0],
                     h->q32b[1], h->vb[0], h->vb[1],
                     h->v, h->normals[0], h->normals[1], h->owner, h->dense, h->hodiag,
                     h->counters};
@@ -585,13 +575,12 @@ int scp3gpu_hbuild_create(const scp3gpu_config* c, scp3gpu_hbuild** out)
     std::vector<int64_t> vd;
     std::vector<uint64_t> sh;
     if ((rc = sobol_tables(nm0, c->scramble, c->scramble_seed, vd, sh))) return bail(rc);
-    std::vector<uint32_t> tasks = pair_tasks(c->nw), desc = basis_descriptors(c->nmodes, c->n2, c->n3);
-    h->ntasks = (int)tasks.size();
+    std::vector<uint32_t> desc = basis_descriptors(c->nmodes, c->n2, c->n3);
     if ((rc = upload(&h->vdir, vd.data(), vd.size())) ||
         (c->scramble && (rc = upload(&h->shift, sh.data(), sh.size()))) ||
         (rc = upload(&h->x0, c->x0, (size_t)N3)) || (rc = upload(&h->MUa, c->MUa, (size_t)N3 * nm0)) ||
         (rc = upload(&h->omega, c->omega, (size_t)nm0)) || (rc = upload(&h->modes, c->modes, (size_t)c->nmodes)) ||
-        (rc = upload(&h->tasks, tasks.data(), tasks.size())) || (rc = upload(&h->desc, desc.data(), desc.size())) ||
+        (rc = upload(&h->desc, desc.data(), desc.size())) ||
         (rc = dalloc(&h->counters, 2)))
         return bail(rc);
     SCP3_CUDA(cudaMemset(h->counters, 0, 2 * sizeof(unsigned long long)));
@@ -871,7 +860,7 @@ int scp3gpu_hbuild_sample(scp3gpu_hbuild* h, int64_t index0, int64_t n, float* q
         SampleArgs a{};
         a.nw = h->cfg.nw, a.nm0 = h->cfg.nmodes0, a.nm = nm;
         a.x0 = h->x0, a.MUa = h->MUa, a.omega = h->omega, a.modes = h->modes, a.vdir = h->vdir, a.shift = h->shift;
-        a.tasks = h->tasks, a.ntasks = h->ntasks, a.index0 = index0 + off, a.n = c, a.nvalid = c;
+        a.index0 = index0 + off, a.n = c, a.nvalid = c;
         a.q64 = h->split_form ? nullptr : h->q64;
         a.q32 = h->split_form ? h->q32b[0] : nullptr;
         a.v = h->split_form ? h->vb[0] : h->v;

@@ -96,12 +96,6 @@ std::vector<uint32_t> basis_descriptors(int nm, int n2, int n3);
 std::vector<double> ho_diagonal(const std::vector<double>& omega_sel, int n2, int n3);
 std::vector<uint32_t> basis_factor_table(int nm, int n2, int n3);
 
-// Pair tasks of the water potentials, in one list per cluster size: type in
-// bits 0..1 (0: M-site(i)/H(j), 1: H/H, 2: O/O, 3: M/M) and the two atom or
-// site indices in bits 2..16 and 17..31 (atoms index 3*water+{0,1,2}; M sites
-// index the water).
-std::vector<uint32_t> pair_tasks(int nw);
-
 // ---------------------------------------------------------------- launches
 struct SampleArgs {
     int nw, nm0, nm;              // waters, all modes, selected modes
@@ -111,8 +105,6 @@ struct SampleArgs {
     const int* modes;             // [nm]
     const int64_t* vdir;          // [62 x nm0] bit-major direction numbers
     const uint64_t* shift;        // [nm0] or nullptr
-    const uint32_t* tasks;        // pair tasks
-    int ntasks;
     const double* normals;        // [n x nm0] sample-major, or nullptr to draw Sobol points
     const float* normals32;       // the same in FP32 (read when normals is nullptr), or nullptr
     int64_t index0;               // first Sobol index
@@ -135,13 +127,9 @@ int launch_samples(int pes, bool fp32, const SampleArgs& a, cudaStream_t s);
 int launch_samples_batch(int pes, bool fp32, const SampleArgs* args_host, const SampleArgs* args_dev, int ncl,
                          int64_t n, cudaStream_t s);
 
-// Energies (kcal/mol) and gradients (kcal/mol/A, [n][9nw]) of n geometries, FP64;
-// iters (may be null): TTM3-F dipole sweeps per geometry
-int launch_pes_energy_grad(int pes, int nw, int64_t n, const double* crd, double* E, double* G, int* iters,
-                           const uint32_t* tasks, int ntasks, cudaStream_t s);
-
-int launch_pes_energy(int pes, int nw, int64_t n, const double* crd, double* E, int* iters,
-                      const uint32_t* tasks, int ntasks, cudaStream_t s);
+// Energies (kcal/mol) and, with G not null, gradients (kcal/mol/A, [n][9nw]) of n
+// geometries, FP64; iters (may be null): TTM3-F dipole sweeps per geometry
+int launch_pes(int pes, int nw, int64_t n, const double* crd, double* E, double* G, int* iters, cudaStream_t s);
 
 int launch_std_normal(int dims, int64_t index0, int64_t n, const int64_t* vdir, const uint64_t* shift,
                       double* out, cudaStream_t s);
@@ -234,7 +222,7 @@ int ttm_init_device();
 // SCP1 per-sample stage (SCP1.cpp:52-63): for points index0 + s, s < n, of the
 // unscrambled Sobol sequence in dim = 9 nw dimensions, y = std_normal % sqrt(d),
 // dq = isqrtM_U y, V = pes(bohr (q + dq)) / autokcal, G = dV/dr bohr / autokcal;
-// writes V[n], G[n][dim], D[n][dim] = dq (and the TTM3-F sweep counts).
+// writes V[n], G[n][dim], D[n][dim] = dq.
 struct Scp1Args {
     int nw, dim;
     const double* q;          // [dim] bohr
@@ -242,12 +230,10 @@ struct Scp1Args {
     const double* U;          // [dim x dim] isqrtM_U, column-major
     const int64_t* vdir;      // [62][dim]
     int64_t index0, n;
-    const uint32_t* tasks;
-    int ntasks;
     double* V;
     double* G;
     double* D;
-    int* iters;               // may be null
+    unsigned long long* not_converged;   // TTM3-F samples at the sweep cap, added to
 };
 int launch_scp1_samples(int pes, const Scp1Args& a, cudaStream_t s);
 

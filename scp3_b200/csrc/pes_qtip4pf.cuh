@@ -1,6 +1,5 @@
-// qTIP4P/f energy, warp-cooperative: one warp per geometry, the geometry and
-// M sites staged in the warp's shared memory, lanes strided over the pair
-// tasks and the monomers.  Same terms and constants as the reference
+// qTIP4P/f energies and gradients of four geometries per warp, the geometries and M
+// sites staged in the warp's shared memory.  Same terms and constants as the reference
 // (qtip4pf.cpp:57-145 monomer, 190-286 pair terms); kcal/mol, Angstrom.
 #pragma once
 #include "common.cuh"
@@ -43,22 +42,6 @@ __device__ __forceinline__ T monomer(const T* w)
     return v1 + v2 + T(0.5) * T(kKTheta) * dth * dth;
 }
 
-template <typename T>
-__device__ __forceinline__ T pair(uint32_t task, const T* crd, const T* ms)
-{
-    const uint32_t type = task & 3u, a = (task >> 2) & 0x7fffu, b = task >> 17;
-    switch (type) {
-        case 0: return T(kQH * kQM) * inv_sqrt(dist2(ms + 3 * a, crd + 3 * b));
-        case 1: return T(kQH * kQH) * inv_sqrt(dist2(crd + 3 * a, crd + 3 * b));
-        case 2: {
-            const T s2 = T(kSigma * kSigma) / dist2(crd + 3 * a, crd + 3 * b);
-            const T s6 = s2 * s2 * s2;
-            return T(4 * kEpsilon) * s6 * (s6 - T(1));
-        }
-        default: return T(kQM * kQM) * inv_sqrt(dist2(ms + 3 * a, ms + 3 * b));
-    }
-}
-
 // Water pair p of the row-major upper triangle of nw waters: a < b.
 __host__ __device__ __forceinline__ void water_pair_of(int p, int nw, int& a, int& b)
 {
@@ -73,8 +56,7 @@ __host__ __device__ __forceinline__ void water_pair_of(int p, int nw, int& a, in
 // The ten site pairs of waters a < b that the reference's pair loops visit
 // (qtip4pf.cpp:213-283): the M site of each water against the two H of the
 // other, the four H/H pairs, O/O (Lennard-Jones) and M/M.  The eight sites are
-// read once; each term is formed in T exactly as pair() forms it and summed in
-// FP64.
+// read once; each term is formed in T and summed in FP64.
 template <typename T>
 __device__ __forceinline__ double water_pair(int a, int b, const T* crd, const T* ms)
 {
@@ -137,25 +119,6 @@ __device__ double energy_warp4(const T* crd, int stride, T* ms, int nw, int ng, 
     return part;
 }
 
-// Energy of the geometry crd[9nw] (shared memory, T), all lanes return the sum.
-// ms is a 3nw shared scratch for the M sites.
-template <typename T>
-__device__ double energy_warp(const T* crd, T* ms, int nw, const uint32_t* __restrict__ tasks, int ntasks,
-                              int lane)
-{
-    double part = 0;     // terms in T, their sums in FP64
-    for (int i = lane; i < nw; i += 32) {
-        const T* w = crd + 9 * i;
-#pragma unroll
-        for (int k = 0; k < 3; k++) ms[3 * i + k] = T(kGammaM) * w[k] + T(kGamma1) * (w[3 + k] + w[6 + k]);
-        part += (double)monomer(w);
-    }
-    __syncwarp();
-    for (int t = lane; t < ntasks; t += 32) part += (double)pair(__ldg(tasks + t), crd, ms);
-    return warp_sum(part);
-}
-
-
 // ---------------------------------------------------------------- energy + gradient
 // qtip4pf.cpp:252-397 (the E+g operator of the gradient path): the same terms,
 // their derivatives in kcal/mol/A.  The M site is gammaM O + gamma1 (H1 + H2), so
@@ -164,7 +127,7 @@ __device__ double energy_warp(const T* crd, T* ms, int nw, const uint32_t* __res
 // each term's energy returned in FP64 and summed in FP64.
 
 template <typename T>
-__device__ __forceinline__ double monomer_grad(const T* w, T* g)
+__device__ __forceinline__ T monomer_grad(const T* w, T* gh1, T* gh2)
 {
     T d1[3], d2[3], r1 = 0, r2 = 0, c = 0;
 #pragma unroll
@@ -185,148 +148,31 @@ __device__ __forceinline__ double monomer_grad(const T* w, T* g)
     const T cs = c / (r1 * r2);
     const T dth = acos(cs) - T(kAHOHeqRad);
     const T de_dc = -T(kKTheta) * dth / sqrt(T(1.0) - cs * cs);                           // dE/dcos(theta)
+    const T i1 = T(1.0) / r1, i2 = T(1.0) / r2;
 #pragma unroll
     for (int k = 0; k < 3; k++) {
-        const T u1 = d1[k] / r1, u2 = d2[k] / r2;
-        const T gh1 = dv1 * u1 + de_dc * (u2 - cs * u1) / r1;
-        const T gh2 = dv2 * u2 + de_dc * (u1 - cs * u2) / r2;
-        atomicAdd(g + 3 + k, gh1);
-        atomicAdd(g + 6 + k, gh2);
-        atomicAdd(g + k, -(gh1 + gh2));
+        const T u1 = d1[k] * i1, u2 = d2[k] * i2;
+        gh1[k] = dv1 * u1 + de_dc * (u2 - cs * u1) * i1;
+        gh2[k] = dv2 * u2 + de_dc * (u1 - cs * u2) * i2;
     }
-    return (double)(v1 + v2 + T(0.5) * T(kKTheta) * dth * dth);
+    return v1 + v2 + T(0.5) * T(kKTheta) * dth * dth;
 }
 
-// q q' / |a - b|: energy; gradient into ga (at a) and gb (at b)
+// Energies and gradients of ng <= 4 geometries crd + j * stride at once: lane l works
+// for geometry l % 4 and for waters l / 4, l / 4 + 8, ..., whose forces it gathers in
+// registers over all other waters.  Every pair is formed from both ends, and nothing is
+// added in shared memory: FP64 and FP32 atomics there are compare-and-swap loops, which
+// bound this kernel before (hexamer, FP64 gradient path's per-sample kernel 382 us per
+// 2^15 samples before, 113 now; FP32 200 and 171 us per 2^16).  ms
+// [4][3nw] and g [4][9nw] (FP64) are shared, g complete after the call; lane l returns the
+// energy of geometry l % 4.
 template <typename T>
-__device__ __forceinline__ double coulomb_grad(double qq, const T* a, const T* b, T* ga, T* gb)
-{
-    const T d0 = a[0] - b[0], d1 = a[1] - b[1], d2 = a[2] - b[2];
-    const T ir = T(1.0) / sqrt(d0 * d0 + d1 * d1 + d2 * d2), e = T(qq) * ir, f = -e * ir * ir;
-    atomicAdd(ga + 0, f * d0), atomicAdd(ga + 1, f * d1), atomicAdd(ga + 2, f * d2);
-    atomicAdd(gb + 0, -f * d0), atomicAdd(gb + 1, -f * d1), atomicAdd(gb + 2, -f * d2);
-    return (double)e;
-}
-
-template <typename T>
-__device__ __forceinline__ double pair_grad(uint32_t task, const T* crd, const T* ms, T* g, T* gm)
-{
-    const uint32_t type = task & 3u, a = (task >> 2) & 0x7fffu, b = task >> 17;
-    switch (type) {
-        case 0: return coulomb_grad<T>(kQH * kQM, ms + 3 * a, crd + 3 * b, gm + 3 * a, g + 3 * b);
-        case 1: return coulomb_grad<T>(kQH * kQH, crd + 3 * a, crd + 3 * b, g + 3 * a, g + 3 * b);
-        case 2: {
-            const T d0 = crd[3 * a] - crd[3 * b], d1 = crd[3 * a + 1] - crd[3 * b + 1];
-            const T d2 = crd[3 * a + 2] - crd[3 * b + 2];
-            const T r2 = d0 * d0 + d1 * d1 + d2 * d2;
-            const T s2 = T(kSigma * kSigma) / r2, s6 = s2 * s2 * s2;
-            const T f = T(2.0 * 4 * kEpsilon) * (T(3.0) * s6 - T(6.0) * s6 * s6) / r2;   // 2 dE/d(r^2)
-            atomicAdd(g + 3 * a, f * d0), atomicAdd(g + 3 * a + 1, f * d1), atomicAdd(g + 3 * a + 2, f * d2);
-            atomicAdd(g + 3 * b, -f * d0), atomicAdd(g + 3 * b + 1, -f * d1), atomicAdd(g + 3 * b + 2, -f * d2);
-            return (double)(T(4 * kEpsilon) * s6 * (s6 - T(1.0)));
-        }
-        default: return coulomb_grad<T>(kQM * kQM, ms + 3 * a, ms + 3 * b, gm + 3 * a, gm + 3 * b);
-    }
-}
-
-// Energy (all lanes) and gradient g[9nw] (shared, complete after the call) of
-// the geometry crd; ms[3nw] and gm[3nw] are shared scratch (M sites, their forces).
-template <typename T>
-__device__ inline double energy_grad_warp(const T* crd, T* ms, T* g, T* gm, int nw,
-                                          const uint32_t* __restrict__ tasks, int ntasks, int lane)
-{
-    for (int c = lane; c < 9 * nw; c += 32) g[c] = T(0);
-    for (int c = lane; c < 3 * nw; c += 32) gm[c] = T(0);
-    for (int i = lane; i < nw; i += 32) {
-        const T* w = crd + 9 * i;
-#pragma unroll
-        for (int k = 0; k < 3; k++) ms[3 * i + k] = T(kGammaM) * w[k] + T(kGamma1) * (w[3 + k] + w[6 + k]);
-    }
-    __syncwarp();
-    double part = 0;
-    for (int i = lane; i < nw; i += 32) part += monomer_grad<T>(crd + 9 * i, g + 9 * i);
-    for (int t = lane; t < ntasks; t += 32) part += pair_grad<T>(__ldg(tasks + t), crd, ms, g, gm);
-    __syncwarp();
-    for (int i = lane; i < nw; i += 32)
-#pragma unroll
-        for (int k = 0; k < 3; k++) {
-            const T f = gm[3 * i + k];
-            g[9 * i + k] += T(kGammaM) * f;
-            g[9 * i + 3 + k] += T(kGamma1) * f;
-            g[9 * i + 6 + k] += T(kGamma1) * f;
-        }
-    __syncwarp();
-    return warp_sum(part);
-}
-
-// The ten site pairs of waters a < b with their gradients, as water_pair:
-// each term formed in T as pair_grad() forms it, the forces on the eight sites
-// gathered in registers and added to g (O, H1, H2) and gm (M) once per site.
-template <typename T>
-__device__ __forceinline__ double water_pair_grad(int a, int b, const T* crd, const T* ms, T* g, T* gm)
-{
-    T s[2][4][3], f[2][4][3];   // [water][O, H1, H2, M][x, y, z]: positions, forces
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-#pragma unroll
-        for (int l = 0; l < 3; l++) s[0][l][k] = crd[9 * a + 3 * l + k], s[1][l][k] = crd[9 * b + 3 * l + k];
-        s[0][3][k] = ms[3 * a + k];
-        s[1][3][k] = ms[3 * b + k];
-#pragma unroll
-        for (int l = 0; l < 4; l++) f[0][l][k] = f[1][l][k] = T(0);
-    }
-    double e = 0.0;
-    // q q' / |u - v| with its forces, u = site x of water w, v = site y of water 1 - w
-    auto coulomb = [&](T qq, int w, int x, int y) {
-        const T d0 = s[w][x][0] - s[1 - w][y][0], d1 = s[w][x][1] - s[1 - w][y][1], d2 = s[w][x][2] - s[1 - w][y][2];
-        const T ir = T(1.0) / sqrt(d0 * d0 + d1 * d1 + d2 * d2), eu = qq * ir, fu = -eu * ir * ir;
-        f[w][x][0] += fu * d0, f[w][x][1] += fu * d1, f[w][x][2] += fu * d2;
-        f[1 - w][y][0] -= fu * d0, f[1 - w][y][1] -= fu * d1, f[1 - w][y][2] -= fu * d2;
-        e += (double)eu;
-    };
-#pragma unroll
-    for (int w = 0; w < 2; w++)
-#pragma unroll
-        for (int l = 1; l < 3; l++) coulomb(T(kQH * kQM), w, 3, l);
-#pragma unroll
-    for (int l = 1; l < 3; l++)
-#pragma unroll
-        for (int m = 1; m < 3; m++) coulomb(T(kQH * kQH), 0, l, m);
-    {
-        const T d0 = s[0][0][0] - s[1][0][0], d1 = s[0][0][1] - s[1][0][1], d2 = s[0][0][2] - s[1][0][2];
-        const T r2 = d0 * d0 + d1 * d1 + d2 * d2;
-        const T s2 = T(kSigma * kSigma) / r2, s6 = s2 * s2 * s2;
-        const T fo = T(2.0 * 4 * kEpsilon) * (T(3.0) * s6 - T(6.0) * s6 * s6) / r2;   // 2 dE/d(r^2)
-        f[0][0][0] += fo * d0, f[0][0][1] += fo * d1, f[0][0][2] += fo * d2;
-        f[1][0][0] -= fo * d0, f[1][0][1] -= fo * d1, f[1][0][2] -= fo * d2;
-        e += (double)(T(4 * kEpsilon) * s6 * (s6 - T(1.0)));
-    }
-    coulomb(T(kQM * kQM), 0, 3, 3);
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-#pragma unroll
-        for (int l = 0; l < 3; l++) atomicAdd(g + 9 * a + 3 * l + k, f[0][l][k]), atomicAdd(g + 9 * b + 3 * l + k, f[1][l][k]);
-        atomicAdd(gm + 3 * a + k, f[0][3][k]);
-        atomicAdd(gm + 3 * b + k, f[1][3][k]);
-    }
-    return e;
-}
-
-// Energies and gradients of ng <= 4 geometries crd + j * stride at once (the
-// FP32 gradient path): lane l works for geometry l % 4 only, as energy_warp4;
-// ms [4][3nw], g [4][9nw] and gm [4][3nw] are shared scratch, g complete after
-// the call; lane l returns the energy of geometry l % 4.
-template <typename T>
-__device__ double energy_grad_warp4(const T* crd, int stride, T* ms, T* g, T* gm, int nw, int ng, int lane)
+__device__ double energy_grad_warp4(const T* crd, int stride, T* ms, double* g, int nw, int ng, int lane)
 {
     const int j = lane & 3;
     const bool on = j < ng;
     const T* cj = crd + j * stride;
     T* mj = ms + j * 3 * nw;
-    T* gj = g + j * 9 * nw;
-    T* gmj = gm + j * 3 * nw;
-    for (int c = lane; c < 4 * 9 * nw; c += 32) g[c] = T(0);
-    for (int c = lane; c < 4 * 3 * nw; c += 32) gm[c] = T(0);
     if (on)
         for (int i = lane >> 2; i < nw; i += 8) {
             const T* w = cj + 9 * i;
@@ -335,25 +181,60 @@ __device__ double energy_grad_warp4(const T* crd, int stride, T* ms, T* g, T* gm
         }
     __syncwarp();
     double part = 0;
-    if (on) {
-        for (int i = lane >> 2; i < nw; i += 8) part += monomer_grad<T>(cj + 9 * i, gj + 9 * i);
-        const int np = nw * (nw - 1) / 2;
-        for (int p = lane >> 2; p < np; p += 8) {
-            int a, b;
-            water_pair_of(p, nw, a, b);
-            part += water_pair_grad<T>(a, b, cj, mj, gj, gmj);
-        }
-    }
-    __syncwarp();
     if (on)
-        for (int i = lane >> 2; i < nw; i += 8)
+        for (int i = lane >> 2; i < nw; i += 8) {
+            T s[4][3], f[4][3];                 // O, H1, H2, M: positions, gradients
 #pragma unroll
             for (int k = 0; k < 3; k++) {
-                const T f = gmj[3 * i + k];
-                gj[9 * i + k] += T(kGammaM) * f;
-                gj[9 * i + 3 + k] += T(kGamma1) * f;
-                gj[9 * i + 6 + k] += T(kGamma1) * f;
+#pragma unroll
+                for (int l = 0; l < 3; l++) s[l][k] = cj[9 * i + 3 * l + k];
+                s[3][k] = mj[3 * i + k];
+                f[0][k] = f[1][k] = f[2][k] = f[3][k] = T(0);
             }
+            double e = 0.0;                     // pair terms, each counted from both ends
+#pragma unroll 1
+            for (int b = 0; b < nw; b++) {
+                if (b == i) continue;
+                T o[4][3];
+#pragma unroll
+                for (int k = 0; k < 3; k++) {
+#pragma unroll
+                    for (int l = 0; l < 3; l++) o[l][k] = cj[9 * b + 3 * l + k];
+                    o[3][k] = mj[3 * b + k];
+                }
+                auto coulomb = [&](T qq, int x, int y) {
+                    const T d0 = s[x][0] - o[y][0], d1 = s[x][1] - o[y][1], d2 = s[x][2] - o[y][2];
+                    const T ir = inv_sqrt(d0 * d0 + d1 * d1 + d2 * d2), eu = qq * ir, fu = -eu * (ir * ir);
+                    f[x][0] += fu * d0, f[x][1] += fu * d1, f[x][2] += fu * d2;
+                    e += (double)eu;
+                };
+#pragma unroll
+                for (int l = 1; l < 3; l++) {
+                    coulomb(T(kQH * kQM), 3, l);
+                    coulomb(T(kQH * kQM), l, 3);
+                    coulomb(T(kQH * kQH), l, 1);
+                    coulomb(T(kQH * kQH), l, 2);
+                }
+                coulomb(T(kQM * kQM), 3, 3);
+                const T d0 = s[0][0] - o[0][0], d1 = s[0][1] - o[0][1], d2 = s[0][2] - o[0][2];
+                const T ir2 = T(1.0) / (d0 * d0 + d1 * d1 + d2 * d2);
+                const T s2 = T(kSigma * kSigma) * ir2, s6 = s2 * s2 * s2;
+                const T fo = T(2.0 * 4 * kEpsilon) * (T(3.0) * s6 - T(6.0) * s6 * s6) * ir2;   // 2 dE/d(r^2)
+                f[0][0] += fo * d0, f[0][1] += fo * d1, f[0][2] += fo * d2;
+                e += (double)(T(4 * kEpsilon) * s6 * (s6 - T(1.0)));
+            }
+            T w[9], gh1[3], gh2[3];
+#pragma unroll
+            for (int k = 0; k < 9; k++) w[k] = s[k / 3][k % 3];
+            part += (double)monomer_grad(w, gh1, gh2) + 0.5 * e;
+            double* gw = g + j * 9 * nw + 9 * i;
+#pragma unroll
+            for (int k = 0; k < 3; k++) {
+                gw[k] = f[0][k] + T(kGammaM) * f[3][k] - (gh1[k] + gh2[k]);
+                gw[3 + k] = f[1][k] + T(kGamma1) * f[3][k] + gh1[k];
+                gw[6 + k] = f[2][k] + T(kGamma1) * f[3][k] + gh2[k];
+            }
+        }
     __syncwarp();
     part += __shfl_xor_sync(0xffffffffu, part, 4);
     part += __shfl_xor_sync(0xffffffffu, part, 8);

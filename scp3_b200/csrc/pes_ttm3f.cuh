@@ -1,33 +1,67 @@
-// TTM3-F energy, warp-cooperative: one warp per geometry.  Same model and
-// constants as the reference (ttm3f.cpp:92-321; Partridge-Schwenke monomer and
+// TTM3-F energies and gradients of four geometries per warp.  Same model and constants
+// as the reference (ttm3f.cpp:92-321, 325-720; Partridge-Schwenke monomer and
 // dipole-moment surface ps.cpp:470-836; smeared interactions
-// ttm3f-bits-smear.cpp:17-287):
-//   lanes 0..nw-1   one water each: M site, PS monomer energy, DMS charges
-//   all lanes       strided over the pair tasks: smeared potentials, fields,
-//                   the 3nw x 3nw dipole tensor (shared-memory atomics for the
-//                   per-site sums)
-//   lanes 0..3nw-1  one row each of the Jacobi sweep for the induced dipoles
-// The induced field is zeroed before the first sweep (the reference's fill at
-// ttm3f.cpp:108-109 starts at Efq and leaves Efd to whatever the heap held).
-// Every data-dependent loop is bounded: the incomplete-gamma series and
-// continued fraction at 1000 terms, the dipole iteration at 500 sweeps
-// (ttm3f.cpp:31), after which *iters reports 501 and the caller counts the
-// sample as not converged (the reference only asserts, and not under NDEBUG,
-// ttm3f.cpp:309).
+// ttm3f-bits-smear.cpp:17-287).
+//
+// Lane l works for water l / 4 of geometry l % 4 (nw <= 8; above, two geometries) and keeps what it sums for
+// that water in registers: it reads the other waters from shared memory in turn and
+// forms its own side of every pair, so nothing is accumulated in shared memory (the
+// energy alone needs H/H once per pair and M/H once per direction; a gradient forms
+// both sides).  The monomer polynomials are Horner forms over compile-time loops whose
+// coefficients are constant-bank operands; the incomplete gamma function costs one
+// exponential and a short polynomial (see smear_tail).  The induced dipoles iterate as the reference's
+// (ttm3f.cpp:268-307), all four geometries at once, each stopping on its own residual,
+// the dipole tensors in registers.
+// What bounds it: instruction issue at the 8 to 16 warps per SM the registers allow.
+// Per-sample kernel: hexamer FP32 energies 372 us per 2^16 samples (1864 before), trimer
+// FP64 gradients 268 us per 2^14 (1113 before), when a warp took one geometry, its
+// monomers on nw lanes, and added every pair term to shared memory by FP64 atomics.
+//
+// The induced field is zero before the first sweep (the reference's fill at
+// ttm3f.cpp:108-109 starts at Efq and leaves Efd to whatever the heap held).  Every
+// loop is bounded; the dipole iteration at 500 sweeps (ttm3f.cpp:31), after which the
+// sweep count reads 501 and the caller counts the sample as not converged (the
+// reference only asserts, and not under NDEBUG, ttm3f.cpp:309).
 #pragma once
 #include "common.cuh"
 
 namespace scp3 {
 namespace ttm {
 
+// Monomer polynomials by powers (I, J) of the two stretches: the energy's 25 groups
+// I >= J, I + J <= 8 with 15 - I - J powers of the bend each (ps.cpp idx1..3), the
+// charges' 28 groups I + J <= 6 with 7 - I - J (idxD0..2), both in ascending I, J.
+constexpr int kEI = 9, kES = 8, kEK = 15, kDI = 7, kDK = 7;
+constexpr int kETerms = 245, kDTerms = 84;
+__host__ __device__ constexpr int e_offset(int I, int J)
+{
+    int o = 0;
+    for (int i = 0; i < kEI; i++)
+        for (int j = 0; j <= i && i + j <= kES; j++) {
+            if (i == I && j == J) return o;
+            o += kEK - i - j;
+        }
+    return o;
+}
+__host__ __device__ constexpr int d_offset(int I, int J)
+{
+    int o = 0;
+    for (int i = 0; i < kDI; i++)
+        for (int j = 0; i + j < kDI; j++) {
+            if (i == I && j == J) return o;
+            o += kDK - i - j;
+        }
+    return o;
+}
+
 struct Consts {
-    double AA_HH, AA_HM, AA_MM;   // pow(polfac*polfac, 1/6), ttm3f.cpp:25-27
-    double aXX13;                 // pow(0.175, 1/3), ttm3f-bits-smear.cpp:201
-    double c5z[245];              // combined monomer coefficients, ps.cpp:508-511
-    double phh1;                  // f5z*phh1A*exp(phh2), ps.cpp:514
-    double coefD[84];
-    unsigned char idx1[245], idx2[245], idx3[245];
-    unsigned char idxD0[84], idxD1[84], idxD2[84];
+    double iAA_HH, iAA_HM, iAA_MM;   // 1 / pow(polfac*polfac, 1/6), ttm3f.cpp:25-27
+    double aXX13;                    // pow(0.175, 1/3), ttm3f-bits-smear.cpp:201
+    double c5z0, coefD0;             // the constant terms, outside the damped sums
+    double phh1;                     // f5z*phh1A*exp(phh2), ps.cpp:514
+    double e[kETerms], d[kDTerms];   // by group (e_offset, d_offset), powers of the bend ascending
+    double s[36];                    // 1 / (2/3)_(n+1)
+    float ef[kETerms], df[kDTerms], sf[36];
 };
 
 // Defined here: only sampling.cu includes this header (whole-program compilation).
@@ -39,85 +73,163 @@ constexpr double kChargeCon = 18.22234397655801030455;
 constexpr double kGammaM = 0.46, kGamma1 = 1.0 - kGammaM, kGamma2 = kGammaM / 2;  // ttm3f-bits.h:21-23
 constexpr double kVdwC = -0.72298855E+03, kVdwD = 0.10211829E+06, kVdwE = 0.37170376E+01;
 constexpr double kAXX = 0.175;
-constexpr int kSeriesCap = 1000;
+constexpr double kGamma23 = 1.3541179394264004169;  // Gamma(2/3)
 
-// scratch per warp, in elements of T: charge, phi, efq, dip, dipp, efd (3nw each),
-// ddt (3nw x 3nw), power tables (48 per water); with the gradient also the
-// charge derivatives (27 per water) and the M-site forces (3nw)
-__host__ __device__ inline size_t scratch_elems(int nw, bool grad = false)
+// scratch per warp beside crd and ms: the charges, [4][3nw] in T, and the dipoles in FP64,
+// [4][6nw]: every water's a second time nw places on, so water i's partners i + r lie in
+// a row
+template <typename T>
+__host__ __device__ inline size_t scratch_bytes(int nw)
 {
-    return (size_t)18 * nw + (size_t)9 * nw * nw + 48 * nw + (grad ? (size_t)30 * nw : 0);
+    return (sizeof(T) + 2 * sizeof(double)) * 12 * (size_t)nw;
 }
 
-template <typename T> struct Eps;
-template <> struct Eps<double> { static constexpr double v = 2.220446049250313e-16; static constexpr double fpmin = 2.2250738585072014e-308 / 2.220446049250313e-16; };
-template <> struct Eps<float> { static constexpr float v = 1.1920929e-07f; static constexpr float fpmin = 1.1754944e-38f / 1.1920929e-07f; };
-
-// gammq(2/3, x) * Gamma(2/3): series below 5/3, continued fraction above
-// (ttm3f-bits-smear.cpp:17-80).
 template <typename T>
-__device__ T gammq23(T x)
+__device__ __forceinline__ T ce(int k)
 {
-    const T a = T(2.0 / 3.0), eps = Eps<T>::v, fpmin = Eps<T>::fpmin;
-    if (x < T(5.0 / 3.0)) {
-        T ap = a, sum = T(1) / a, del = sum;
-        for (int it = 0; it < kSeriesCap; it++) {
-            ++ap;
-            del *= x / ap;
-            sum += del;
-            if (fabs(del) < fabs(sum) * eps) break;
+    if constexpr (sizeof(T) == 8) return kC.e[k];
+    else return kC.ef[k];
+}
+template <typename T>
+__device__ __forceinline__ T cd(int k)
+{
+    if constexpr (sizeof(T) == 8) return kC.d[k];
+    else return kC.df[k];
+}
+
+// v of the smeared charge-charge term (1 - v) / r: with x = a (r/A)^3, e1 = exp(-x) and
+// x13 = a^(1/3) r/A, the reference's 1 - e1 + x13 Gamma(2/3, x) (ttm3f-bits-smear.cpp:
+// 17-80, 213-231).  Gamma(2/3, x) = x^(2/3) e1 h(x), h the continued fraction 1/(x +
+// 1/3 - 1 (1/3)/(x + 7/3 - 2 (4/3)/(x + 13/3 - ...))), so v = e1 (1 - x h), x13 x^(2/3)
+// being x.  1 - x h is smooth: a polynomial of degree 16 (7 in FP32) on each of ten
+// intervals, two per octave of x from 1.5 to 48, interpolated at Chebyshev points from
+// the fraction (tail_tables; 1e-17 of it, 1e-8), takes 17 fused steps where the
+// fraction's recurrence takes 100 and more near its start.  Past x = 37 (17) v is below
+// rounding; below 1.5 Gamma(2/3) minus the series of the lower function, v = e1 (1 + x
+// S) - x13 Gamma(2/3), S = sum x^n / (2/3)_(n+1) (there the reference's own split, at 5/3;
+// further out the two terms would cancel).
+constexpr int kTailSpans = 10, kTailN = 17, kTailNf = 8;
+struct TailTable {
+    double scale[kTailSpans], shift[kTailSpans], c[kTailN][kTailSpans];       // t = x scale - shift in [-1, 1]
+    float scalef[kTailSpans], shiftf[kTailSpans], cf[kTailNf][kTailSpans];
+};
+__device__ TailTable kTail;
+
+template <typename T>
+__device__ __forceinline__ T smear_tail(T x, T e1, T x13)
+{
+    constexpr bool F = sizeof(T) == 4;
+    if (x > T(F ? 17.0 : 37.0)) return T(0);
+    if (x < T(1.5)) {
+        T s = T(0);
+#pragma unroll
+        for (int n = F ? 14 : 22; n >= 0; n--) {
+            if constexpr (F) s = s * x + kC.sf[n];
+            else s = s * x + kC.s[n];
         }
-        return T(1.354117939426400e+00) - sum * exp(-x + a * log(x));
+        return e1 * (T(1) + x * s) - x13 * T(kGamma23);
     }
-    T b = x + T(1) - a, c = T(1) / fpmin, d = T(1) / b, h = d;
-    for (int i = 1; i <= kSeriesCap; ++i) {
-        const T an = -i * (i - a);
-        b += T(2);
-        d = an * d + b;
-        if (fabs(d) < fpmin) d = fpmin;
-        c = b + an / c;
-        if (fabs(c) < fpmin) c = fpmin;
-        d = T(1) / d;
-        const T del = d * c;
-        h *= del;
-        if (fabs(del - T(1)) <= eps) break;
+    // two intervals per octave: exponent and first bit of the fraction, from 1.5 on
+    int i;
+    if constexpr (F) i = (__float_as_int(x) >> 22) - 255;
+    else i = (__double2hiint(x) >> 19) - 2047;
+    T s;
+    if constexpr (F) {
+        const T t = x * __ldg(kTail.scalef + i) - __ldg(kTail.shiftf + i);
+        s = __ldg(&kTail.cf[kTailNf - 1][i]);
+#pragma unroll
+        for (int k = kTailNf - 2; k >= 0; k--) s = s * t + __ldg(&kTail.cf[k][i]);
+    } else {
+        const T t = x * __ldg(kTail.scale + i) - __ldg(kTail.shift + i);
+        s = __ldg(&kTail.c[kTailN - 1][i]);
+#pragma unroll
+        for (int k = kTailN - 2; k >= 0; k--) s = s * t + __ldg(&kTail.c[k][i]);
     }
-    return exp(-x + a * log(x)) * h;
+    return e1 * s;
 }
 
-// smear0/01/012 (ttm3f-bits-smear.cpp:213-287): ts0 always, ts1/ts2 on request.
-template <typename T>
-__device__ __forceinline__ void smear(T r, T AA, T& ts0, T& ts1, T* ts2)
+// The table, in extended precision: Chebyshev interpolation of 1 - x h(x), as powers of t.
+inline void tail_tables(TailTable& o)
 {
-    const T dri = T(1) / r, drsqi = dri * dri;
-    const T rA = r / AA, rA3 = rA * rA * rA;
-    const T e1 = exp(-T(kAXX) * rA3);
-    ts0 = (T(1) - e1 + T(kC.aXX13) * rA * gammq23(T(kAXX) * rA3)) * dri;
-    ts1 = (T(1) - e1) * dri * drsqi;
-    if (ts2) *ts2 = (ts1 - e1 * T(kAXX) / (AA * AA * AA)) * drsqi;
-}
-
-template <typename T>
-__device__ __forceinline__ void powers(T x1, T x2, T x3, T* f /* [3][16] */)
-{
-    f[0] = f[16] = f[32] = T(0);
-    f[1] = f[17] = f[33] = T(1);
-    for (int j = 2; j < 16; j++) {
-        f[j] = f[j - 1] * x1;
-        f[16 + j] = f[16 + j - 1] * x2;
-        f[32 + j] = f[32 + j - 1] * x3;
+    auto w = [](long double x) {
+        const long double a = 2.0L / 3.0L;
+        long double b = x + 1.0L - a, A0 = 0.0L, A1 = 1.0L, B0 = 1.0L, B1 = b;
+        for (int k = 1; k <= 200; k++) {
+            const long double an = -k * (k - a);
+            b += 2.0L;
+            const long double A2 = b * A1 + an * A0, B2 = b * B1 + an * B0;
+            A0 = A1 / B2, A1 = A2 / B2, B0 = B1 / B2, B1 = 1.0L;
+        }
+        return 1.0L - x * A1 / B1;
+    };
+    const long double pi = 3.14159265358979323846264338327950288L;
+    for (int i = 0; i < kTailSpans; i++) {
+        const long double lo = ldexpl((i & 1) ? 1.0L : 1.5L, (i + 1) / 2), hi = lo + ldexpl(0.5L, (i + 1) / 2);
+        o.scale[i] = (double)(2.0L / (hi - lo)), o.shift[i] = (double)((hi + lo) / (hi - lo));
+        o.scalef[i] = (float)o.scale[i], o.shiftf[i] = (float)o.shift[i];
+        for (int n : {kTailN, kTailNf}) {
+            std::vector<long double> f(n), c(n, 0.0L), p(n, 0.0L), t0(n, 0.0L), t1(n, 0.0L);
+            for (int k = 0; k < n; k++) f[k] = w(0.5L * (lo + hi) + 0.5L * (hi - lo) * cosl(pi * (k + 0.5L) / n));
+            for (int j = 0; j < n; j++) {
+                for (int k = 0; k < n; k++) c[j] += f[k] * cosl(pi * j * (k + 0.5L) / n);
+                c[j] *= (j ? 2.0L : 1.0L) / n;
+            }
+            t0[0] = 1.0L, t1[1] = 1.0L;                    // T_0, T_1 as powers of t
+            for (int k = 0; k < n; k++) p[k] = c[0] * t0[k] + c[1] * t1[k];
+            for (int j = 2; j < n; j++) {
+                std::vector<long double> t2(n, 0.0L);
+                for (int k = 0; k < n; k++) t2[k] = (k ? 2.0L * t1[k - 1] : 0.0L) - t0[k];
+                for (int k = 0; k < n; k++) p[k] += c[j] * t2[k];
+                t0 = t1, t1 = t2;
+            }
+            for (int k = 0; k < n; k++)
+                if (n == kTailN) o.c[k][i] = (double)p[k];
+                else o.cf[k][i] = (float)p[k];
+        }
     }
 }
 
-// Monomer energy (pot_nasa, energy part) and charges (dms_nasa with ttm3=true),
-// kcal/mol and elementary charges, for the water at w[9].  f: 48 scratch.
+// Smeared interactions of two sites R apart (ttm3f-bits-smear.cpp:97-287); the members
+// a caller does not read are not formed.
 template <typename T>
-__device__ void monomer(const T* w, T* f, T& e, T q3[3])
+struct Smear {
+    T ri, x, e1, x13;
+    __device__ __forceinline__ Smear(T r2, T iAA)
+    {
+        ri = inv_sqrt(r2);
+        x13 = T(kC.aXX13) * (r2 * ri * iAA);
+        x = x13 * x13 * x13;
+        e1 = exp(-x);
+    }
+    __device__ __forceinline__ T ts0() const { return (T(1) - smear_tail(x, e1, x13)) * ri; }
+    __device__ __forceinline__ T ts1() const { return (T(1) - e1) * ri * (ri * ri); }
+    __device__ __forceinline__ T ts2(T ts1, T iAA) const { return (ts1 - e1 * (T(kAXX) * iAA * iAA * iAA)) * (ri * ri); }
+    __device__ __forceinline__ T ts3(T ts2, T iAA) const
+    {
+        const T c = T(kAXX) * iAA * iAA * iAA;
+        return (ts2 - T(0.6) * e1 * (c * c) / ri) * (ri * ri);
+    }
+};
+
+// A water's own terms: energy (kcal/mol) and the charges of H1 and H2 (elementary
+// charges); with G the energy's gradient on H1 and H2 and the charges' derivatives.
+template <typename T, bool G>
+struct Monomer {
+    T e, q1, q2;
+    T h1[3], h2[3];                               // kcal/mol/A on H1, H2 (O: minus their sum)
+    T f11, f12, f21, f22, g11, g12, g21, g22;     // d q1 / d H1 = f11 roh1 + f12 roh2, d q1 / d H2 = f21 roh1 + f22 roh2; g: q2
+};
+
+// pot_nasa and dms_nasa with ttm3 = true (ps.cpp:470-836) for the water at w[9].
+template <typename T, bool G>
+__device__ __forceinline__ void monomer(const T* w, Monomer<T, G>& o)
 {
     constexpr double reoh = 0.958649, b1 = 2.0, roh = 0.9519607159623009, alphaoh = 2.587949757553683;
     constexpr double deohA = 42290.92019288289, phh2 = 12.66426998162947, f5z = 0.999677885;
-    constexpr double costhe = -.24780227221366464506;
-    T roh1[3], roh2[3], rhh[3], d1 = 0, d2 = 0, dhh = 0;
+    constexpr double costhe = -.24780227221366464506, tocal = 0.00285914375100642899, xx = 0.529177249;
+    constexpr double ath0 = 1.82400520401572996557, dms1 = 0.5, dms2 = 0.9578, dms3 = 0.012;
+    T roh1[3], roh2[3], rhh[3], d1 = 0, d2 = 0, dhh = 0, dot = 0;
+#pragma unroll
     for (int i = 0; i < 3; i++) {
         roh1[i] = w[3 + i] - w[i];
         roh2[i] = w[6 + i] - w[i];
@@ -125,496 +237,389 @@ __device__ void monomer(const T* w, T* f, T& e, T q3[3])
         d1 += roh1[i] * roh1[i];
         d2 += roh2[i] * roh2[i];
         dhh += rhh[i] * rhh[i];
+        dot += roh1[i] * roh2[i];
     }
     d1 = sqrt(d1);
     d2 = sqrt(d2);
     dhh = sqrt(dhh);
-    const T costh = (roh1[0] * roh2[0] + roh1[1] * roh2[1] + roh1[2] * roh2[2]) / (d1 * d2);
-    // --- pot_nasa (ps.cpp:486-570)
-    const T deoh = T(f5z * deohA);
-    const T e1x = exp(-T(alphaoh) * (d1 - T(roh))), e2x = exp(-T(alphaoh) * (d2 - T(roh)));
-    const T va = deoh * (e1x * (e1x - T(2)) + e2x * (e2x - T(2)));
-    const T vb = T(kC.phh1) * exp(-T(phh2) * dhh);
-    const T x1 = (d1 - T(reoh)) / T(reoh), x2 = (d2 - T(reoh)) / T(reoh);
-    powers(x1, x2, costh - T(costhe), f);
-    const T dr1 = d1 - T(reoh), dr2 = d2 - T(reoh);
-    const T efac = exp(-T(b1) * (dr1 * dr1 + dr2 * dr2));
-    T sum0 = 0;
-    for (int j = 1; j < 245; j++) {
-        const int I = kC.idx1[j], J = kC.idx2[j], K = kC.idx3[j];
-        sum0 += T(kC.c5z[j]) * (f[I] * f[16 + J] + f[J] * f[16 + I]) * f[32 + K];
-    }
-    e = (va + vb + (T(2) * T(kC.c5z[0]) + efac * sum0) + T(0.44739574026257)) * T(0.00285914375100642899);
-    // --- dms_nasa (ps.cpp:605-790), charges only
-    const T efacD = exp(-(dr1 * dr1 + dr2 * dr2));   // b1D = 1
-    T p1 = 0, p2 = 0;
-    const T pl1 = costh, pl2 = T(0.5) * (T(3) * pl1 * pl1 - T(1));
-    for (int j = 1; j < 84; j++) {
-        const int I = kC.idxD0[j], J = kC.idxD1[j], K = kC.idxD2[j];
-        p1 += T(kC.coefD[j]) * f[I] * f[16 + J] * f[32 + K];
-        p2 += T(kC.coefD[j]) * f[J] * f[16 + I] * f[32 + K];
-    }
-    const T xx = T(0.529177249);
-    const T pc0 = T(0.2999) * (pow(d1, T(-0.6932)) + pow(d2, T(-0.6932))) *
-                  (T(1.0099) + pl1 * T(-0.1801) + pl2 * T(0.0892));
-    p1 = T(kC.coefD[0]) + p1 * efacD + pc0 * xx;
-    p2 = T(kC.coefD[0]) + p2 * efacD + pc0 * xx;
-    T axb[3] = {roh1[1] * roh2[2] - roh1[2] * roh2[1], -roh1[0] * roh2[2] + roh1[2] * roh2[0],
-                roh1[0] * roh2[1] - roh1[1] * roh2[0]};
-    const T sinth = sqrt(axb[0] * axb[0] + axb[1] * axb[1] + axb[2] * axb[2]) / (d1 * d2);
-    const T ang = atan2(sinth, costh);
-    const T m1 = T(0.5) * (d1 - T(0.9578)) + T(0.012) * (ang - T(1.82400520401572996557));
-    const T m2 = T(0.5) * (d2 - T(0.9578)) + T(0.012) * (ang - T(1.82400520401572996557));
-    q3[0] = -(p1 + p2) - (m1 + m2);
-    q3[1] = p1 + m1;
-    q3[2] = p2 + m2;
-}
-
-// Energy (kcal/mol) of crd[9nw] (shared, T); ms: 3nw shared; sc: scratch_elems(nw).
-// Returns the sum on all lanes; *iters = Jacobi sweeps (kTtmMaxIter+1 if capped).
-template <typename T>
-__device__ double energy_warp(const T* crd, T* ms, T* sc, int nw, const uint32_t* __restrict__ tasks, int ntasks,
-                              int lane, int* iters)
-{
-    const int n3 = 3 * nw;
-    T *chg = sc, *phi = chg + n3, *efq = phi + n3, *dip = efq + n3, *dipp = dip + n3, *efd = dipp + n3,
-      *ddt = efd + n3, *fpow = ddt + n3 * n3;
-    for (int i = lane; i < n3 * n3; i += 32) ddt[i] = T(0);
-    for (int i = lane; i < n3; i += 32) phi[i] = efq[i] = efd[i] = T(0);
-    double part = 0;
-    for (int i = lane; i < nw; i += 32) {
-        const T* w = crd + 9 * i;
-        for (int k = 0; k < 3; k++) ms[3 * i + k] = T(kGamma1) * w[k] + T(kGamma2) * (w[3 + k] + w[6 + k]);
-        T e, q3[3];
-        monomer(w, fpow + 48 * i, e, q3);
-        part += (double)e;
-        const T t = T(kGamma2 / kGamma1);
-        chg[3 * i + 0] = T(kChargeCon) * q3[0] / T(kGamma1);
-        chg[3 * i + 1] = T(kChargeCon) * (q3[1] + t * (q3[1] + q3[2]));
-        chg[3 * i + 2] = T(kChargeCon) * (q3[2] + t * (q3[1] + q3[2]));
-    }
-    __syncwarp();
-    for (int t = lane; t < ntasks; t += 32) {
-        const uint32_t task = __ldg(tasks + t), type = task & 3u, a = (task >> 2) & 0x7fffu, b = task >> 17;
-        if (type == 0) {            // M site of water a, H atom b  (ttm3f.cpp:149-174)
-            const int ia = 3 * a;
-            T R[3];
-            for (int k = 0; k < 3; k++) R[k] = ms[ia + k] - crd[3 * b + k];
-            T ts0, ts1;
-            smear<T>(sqrt(R[0] * R[0] + R[1] * R[1] + R[2] * R[2]), T(kC.AA_HM), ts0, ts1, nullptr);
-            const int jb = b;        // charge index of atom b = 3*water + l
-            atomicAdd(phi + ia, ts0 * chg[jb]);
-            atomicAdd(phi + jb, ts0 * chg[ia]);
-            for (int k = 0; k < 3; k++) atomicAdd(efq + ia + k, chg[jb] * ts1 * R[k]);
-        } else if (type == 1) {     // H/H  (ttm3f.cpp:183-200)
-            T ts0, ts1;
-            smear<T>(sqrt(dist2(crd + 3 * a, crd + 3 * b)), T(kC.AA_HH), ts0, ts1, nullptr);
-            atomicAdd(phi + a, chg[b] * ts0);
-            atomicAdd(phi + b, chg[a] * ts0);
-        } else if (type == 2) {     // O/O van der Waals  (ttm3f.cpp:204-219)
-            const T r2 = dist2(crd + 3 * a, crd + 3 * b);
-            part += (double)(T(kVdwC) / (r2 * r2 * r2) + T(kVdwD) * exp(-T(kVdwE) * sqrt(r2)));
-        } else {                    // M/M  (ttm3f.cpp:222-256)
-            const int i3 = 3 * a, j3 = 3 * b;
-            T R[3];
-            for (int k = 0; k < 3; k++) R[k] = ms[i3 + k] - ms[j3 + k];
-            T ts0, ts1, ts2;
-            smear<T>(sqrt(R[0] * R[0] + R[1] * R[1] + R[2] * R[2]), T(kC.AA_MM), ts0, ts1, &ts2);
-            atomicAdd(phi + i3, ts0 * chg[j3]);
-            atomicAdd(phi + j3, ts0 * chg[i3]);
-            for (int k = 0; k < 3; k++) {
-                atomicAdd(efq + i3 + k, chg[j3] * ts1 * R[k]);
-                atomicAdd(efq + j3 + k, -(chg[i3] * ts1 * R[k]));
-            }
-            for (int k = 0; k < 3; k++)
-                for (int l = k; l < 3; l++) {
-                    const T d = T(3) * ts2 * R[k] * R[l] - (k == l ? ts1 : T(0));
-                    ddt[n3 * (i3 + k) + j3 + l] = d;
-                    ddt[n3 * (j3 + k) + i3 + l] = d;
-                    ddt[n3 * (i3 + l) + j3 + k] = d;
-                    ddt[n3 * (j3 + l) + i3 + k] = d;
+    const T costh = dot / (d1 * d2);
+    const T dr1 = d1 - T(reoh), dr2 = d2 - T(reoh), x3 = costh - T(costhe);
+    T p[kEI], q[kEI];                              // powers of the two stretches
+    p[0] = q[0] = T(1);
+    p[1] = dr1 / T(reoh), q[1] = dr2 / T(reoh);
+#pragma unroll
+    for (int k = 2; k < kEI; k++) p[k] = p[k - 1] * p[1], q[k] = q[k - 1] * q[1];
+    const T g2 = dr1 * dr1 + dr2 * dr2;
+    // --- pot_nasa (ps.cpp:486-603)
+    {
+        const T deoh = T(f5z * deohA);
+        const T e1x = exp(-T(alphaoh) * (d1 - T(roh))), e2x = exp(-T(alphaoh) * (d2 - T(roh)));
+        const T va = deoh * (e1x * (e1x - T(2)) + e2x * (e2x - T(2)));
+        const T vb = T(kC.phh1) * exp(-T(phh2) * dhh);
+        const T efac = exp(-T(b1) * g2);
+        T s0 = 0, s1 = 0, s2 = 0, s3 = 0;
+#pragma unroll
+        for (int I = 0; I < kEI; I++)
+#pragma unroll
+            for (int J = 0; J < kEI; J++) {
+                if (J > I || I + J > kES) continue;
+                const int off = e_offset(I, J), n = kEK - I - J;
+                T a = ce<T>(off + n - 1), da = T(0);
+#pragma unroll
+                for (int k = kEK - 2; k >= 0; k--) {
+                    if (k > n - 2) continue;
+                    if (G) da = da * x3 + a;
+                    a = a * x3 + ce<T>(off + k);
                 }
+                const T sym = I == J ? T(2) * p[I] * q[I] : p[I] * q[J] + p[J] * q[I];
+                s0 += a * sym;
+                if (G) {
+                    T t1 = T(0), t2 = T(0);
+                    if (I) t1 += T(I) * p[I - 1] * q[J], t2 += T(I) * p[J] * q[I - 1];
+                    if (J) t1 += T(J) * p[J - 1] * q[I], t2 += T(J) * p[I] * q[J - 1];
+                    s1 += a * t1, s2 += a * t2, s3 += da * sym;
+                }
+            }
+        o.e = (va + vb + (T(2) * T(kC.c5z0) + efac * s0) + T(0.44739574026257)) * T(tocal);
+        if (G) {
+            const T dva1 = T(2.0 * alphaoh) * deoh * e1x * (T(1) - e1x) / d1;
+            const T dva2 = T(2.0 * alphaoh) * deoh * e2x * (T(1) - e2x) / d2;
+            const T dvb = -T(phh2) * vb / dhh;
+            const T dvc1 = (-T(2 * b1) * efac * dr1 * s0 + efac * s1 / T(reoh)) / d1;
+            const T dvc2 = (-T(2 * b1) * efac * dr2 * s0 + efac * s2 / T(reoh)) / d2;
+            const T dvcc = efac * s3;
+#pragma unroll
+            for (int i = 0; i < 3; i++) {
+                o.h1[i] = T(tocal) * (dva1 * roh1[i] + dvb * rhh[i] + dvc1 * roh1[i] +
+                                      dvcc * (roh2[i] / (d1 * d2) - costh * roh1[i] / (d1 * d1)));
+                o.h2[i] = T(tocal) * (dva2 * roh2[i] - dvb * rhh[i] + dvc2 * roh2[i] +
+                                      dvcc * (roh1[i] / (d1 * d2) - costh * roh2[i] / (d2 * d2)));
+            }
         }
     }
+    // --- dms_nasa (ps.cpp:605-836)
+    const T efacD = exp(-g2);   // b1D = 1
+    T p1 = 0, p2 = 0, dp1r1 = 0, dp1r2 = 0, dp1c = 0, dp2r1 = 0, dp2r2 = 0, dp2c = 0;
+#pragma unroll
+    for (int I = 0; I < kDI; I++)
+#pragma unroll
+        for (int J = 0; J < kDI; J++) {
+            if (I + J >= kDI) continue;
+            const int off = d_offset(I, J), n = kDK - I - J;
+            T a = cd<T>(off + n - 1), da = T(0);
+#pragma unroll
+            for (int k = kDK - 2; k >= 0; k--) {
+                if (k > n - 2) continue;
+                if (G) da = da * x3 + a;
+                a = a * x3 + cd<T>(off + k);
+            }
+            p1 += a * (p[I] * q[J]);
+            p2 += a * (p[J] * q[I]);
+            if (G) {
+                if (I) dp1r1 += a * (T(I) * p[I - 1] * q[J]), dp2r2 += a * (T(I) * p[J] * q[I - 1]);
+                if (J) dp1r2 += a * (T(J) * p[I] * q[J - 1]), dp2r1 += a * (T(J) * p[J - 1] * q[I]);
+                dp1c += da * (p[I] * q[J]);
+                dp2c += da * (p[J] * q[I]);
+            }
+        }
+    constexpr double pa = 0.2999, pb = -0.6932, pc0c = 1.0099, pc1 = -0.1801, pc2 = 0.0892;
+    const T pl2 = T(0.5) * (T(3) * costh * costh - T(1));
+    const T ang_f = T(pc0c) + costh * T(pc1) + pl2 * T(pc2);
+    const T w1 = exp(T(pb) * log(d1)), w2 = exp(T(pb) * log(d2));
+    const T pc0 = T(pa) * (w1 + w2) * ang_f;
+    const T axb[3] = {roh1[1] * roh2[2] - roh1[2] * roh2[1], -roh1[0] * roh2[2] + roh1[2] * roh2[0],
+                      roh1[0] * roh2[1] - roh1[1] * roh2[0]};
+    const T sinth = sqrt(axb[0] * axb[0] + axb[1] * axb[1] + axb[2] * axb[2]) / (d1 * d2);
+    const T ang = T(dms3) * (atan2(sinth, costh) - T(ath0));
+    o.q1 = T(kC.coefD0) + p1 * efacD + pc0 * T(xx) + T(dms1) * (d1 - T(dms2)) + ang;
+    o.q2 = T(kC.coefD0) + p2 * efacD + pc0 * T(xx) + T(dms1) * (d2 - T(dms2)) + ang;
+    if (G) {
+        // derivatives by d1, d2 and cos; those of p by a stretch carry 1 / reoh
+        const T dw1 = T(pa * pb * xx) * w1 / d1 * ang_f, dw2 = T(pa * pb * xx) * w2 / d2 * ang_f;
+        const T dwc = T(pa * xx) * (w1 + w2) * (T(pc1) + T(3.0 * pc2) * costh);
+        const T ef1 = -T(2) * dr1 * efacD, ef2 = -T(2) * dr2 * efacD;
+        const T a11 = dp1r1 * efacD / T(reoh) + p1 * ef1 + dw1 + T(dms1);
+        const T a12 = dp1r2 * efacD / T(reoh) + p1 * ef2 + dw2;
+        const T a1c = dp1c * efacD + dwc - T(dms3) / sinth;
+        const T a21 = dp2r1 * efacD / T(reoh) + p2 * ef1 + dw1;
+        const T a22 = dp2r2 * efacD / T(reoh) + p2 * ef2 + dw2 + T(dms1);
+        const T a2c = dp2c * efacD + dwc - T(dms3) / sinth;
+        const T i12 = T(1) / (d1 * d2);
+        o.f11 = (a11 - a1c * costh / d1) / d1, o.f12 = a1c * i12;
+        o.f22 = (a12 - a1c * costh / d2) / d2, o.f21 = a1c * i12;
+        o.g11 = (a21 - a2c * costh / d1) / d1, o.g12 = a2c * i12;
+        o.g22 = (a22 - a2c * costh / d2) / d2, o.g21 = a2c * i12;
+    }
+}
+
+template <typename T>
+__device__ __forceinline__ void load3(const T* a, T* r)
+{
+    r[0] = a[0], r[1] = a[1], r[2] = a[2];
+}
+template <typename T>
+__device__ __forceinline__ T dot3(const T* a, const T* b)
+{
+    return a[0] * b[0] + a[1] * b[1] + a[2] * b[2];
+}
+template <int NG>
+__device__ __forceinline__ double sum_geometry(double x)      // over the lanes of a geometry
+{
+#pragma unroll
+    for (int o = NG; o < 32; o <<= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+    return x;
+}
+
+// Energies (kcal/mol) of ng <= 4 geometries crd + j * stride (shared memory, T), and with
+// G their gradients g + j * 9 nw (shared, kcal/mol/A, complete after the call); ms
+// [4][3nw] and sc (scratch_bytes) shared scratch.  Lane l returns the energy of geometry
+// l % 4, *iters its Jacobi sweeps (kTtmMaxIter + 1 if capped).  NG = 2: two geometries
+// of up to 16 waters instead, lane l on water l / 2 of geometry l % 2.
+template <typename T, bool G, int NG = 4>
+__device__ double energy_warp4(const T* crd, int stride, T* ms, char* sc, double* g, int nw, int ng, int lane, int* iters)
+{
+    constexpr int kMaxNw = 32 / NG;
+    const int j = lane % NG, i = lane / NG, n3 = 3 * nw;
+    const bool on = j < ng && i < nw;
+    const T* cj = crd + j * stride;
+    T* mj = ms + j * n3;
+    double* dip = reinterpret_cast<double*>(sc) + j * 2 * n3;
+    T* chg = reinterpret_cast<T*>(sc + sizeof(double) * 8 * n3) + j * n3;
+    T xO[3], xH[2][3], xM[3], qM = 0, qH[2] = {0, 0};
+    double part = 0;
+    Monomer<T, G> mo;
+    if (on) {
+        const T* w = cj + 9 * i;
+        load3(w, xO), load3(w + 3, xH[0]), load3(w + 6, xH[1]);
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            xM[k] = T(kGamma1) * xO[k] + T(kGamma2) * (xH[0][k] + xH[1][k]);
+            mj[3 * i + k] = xM[k];
+        }
+        T w9[9];
+#pragma unroll
+        for (int k = 0; k < 9; k++) w9[k] = w[k];
+        monomer<T, G>(w9, mo);
+        part = (double)mo.e;
+        const T t = T(kGamma2 / kGamma1), s = mo.q1 + mo.q2;
+        qM = -T(kChargeCon) * s / T(kGamma1);
+        qH[0] = T(kChargeCon) * (mo.q1 + t * s);
+        qH[1] = T(kChargeCon) * (mo.q2 + t * s);
+        chg[3 * i] = qM, chg[3 * i + 1] = qH[0], chg[3 * i + 2] = qH[1];
+    }
     __syncwarp();
-    // induced dipoles (ttm3f.cpp:268-307); the iterate is carried in FP64 so the
-    // FP32 form can still reach its residual target
+    const T iHH = T(kC.iAA_HH), iHM = T(kC.iAA_HM), iMM = T(kC.iAA_MM);
+    T phi[3] = {0, 0, 0}, gO[3] = {0, 0, 0}, gH[2][3] = {{0, 0, 0}, {0, 0, 0}};   // potentials at M, H1, H2
+    double efq[3] = {0, 0, 0}, el = 0.0, vdw = 0.0;
+    // pair terms, the water's own side (ttm3f.cpp:144-257, 403-520)
+    if (on)
+#pragma unroll 1
+        for (int r = 1; r < nw; r++) {
+            const int b = i + r < nw ? i + r : i + r - nw;
+            const T* w = cj + 9 * b;
+            T yO[3], yH[2][3], yM[3], R[3];
+            load3(w, yO), load3(w + 3, yH[0]), load3(w + 6, yH[1]), load3(mj + 3 * b, yM);
+            const T pM = chg[3 * b], pH[2] = {chg[3 * b + 1], chg[3 * b + 2]};
+#pragma unroll
+            for (int l = 0; l < 2; l++) {       // own M, other H
+#pragma unroll
+                for (int k = 0; k < 3; k++) R[k] = xM[k] - yH[l][k];
+                const Smear<T> s(dot3(R, R), iHM);
+                const T t0 = s.ts0(), t1 = pH[l] * s.ts1();
+                if (G) phi[0] += t0 * pH[l];
+                else el += (double)(t0 * pH[l] * qM);
+#pragma unroll
+                for (int k = 0; k < 3; k++) efq[k] += (double)(t1 * R[k]);
+            }
+            if (G) {
+#pragma unroll
+                for (int l = 0; l < 2; l++) {   // own H, other M
+#pragma unroll
+                    for (int k = 0; k < 3; k++) R[k] = yM[k] - xH[l][k];
+                    const Smear<T> s(dot3(R, R), iHM);
+                    phi[1 + l] += s.ts0() * pM;
+                    const T f = pM * qH[l] * s.ts1();
+#pragma unroll
+                    for (int k = 0; k < 3; k++) gH[l][k] += f * R[k];
+                }
+            }
+            // H/H: both sides of a gradient; the energy takes the waters i and i + r, r up
+            // to nw / 2 (that one from both ends, at half weight)
+            if (G || 2 * r <= nw) {
+                const T half = 2 * r == nw ? T(0.5) : T(1);
+#pragma unroll
+                for (int l = 0; l < 2; l++)
+#pragma unroll
+                    for (int m = 0; m < 2; m++) {
+#pragma unroll
+                        for (int k = 0; k < 3; k++) R[k] = xH[l][k] - yH[m][k];
+                        const Smear<T> s(dot3(R, R), iHH);
+                        const T t0 = s.ts0();
+                        if (G) {
+                            phi[1 + l] += t0 * pH[m];
+                            const T f = -pH[m] * qH[l] * s.ts1();
+#pragma unroll
+                            for (int k = 0; k < 3; k++) gH[l][k] += f * R[k];
+                        } else {
+                            el += (double)(half * t0 * pH[m] * qH[l]);
+                        }
+                    }
+            }
+            {                                   // O/O van der Waals, half of it this water's
+#pragma unroll
+                for (int k = 0; k < 3; k++) R[k] = xO[k] - yO[k];
+                const T r2 = dot3(R, R), rr = sqrt(r2), c6 = T(kVdwC) / (r2 * r2 * r2), ex = T(kVdwD) * exp(-T(kVdwE) * rr);
+                vdw += (double)(c6 + ex);
+                if (G) {
+                    const T f = -(T(6) * c6) / r2 - T(kVdwE) * ex / rr;
+#pragma unroll
+                    for (int k = 0; k < 3; k++) gO[k] += f * R[k];
+                }
+            }
+            {                                   // M/M
+#pragma unroll
+                for (int k = 0; k < 3; k++) R[k] = xM[k] - yM[k];
+                const Smear<T> s(dot3(R, R), iMM);
+                const T t0 = s.ts0(), t1 = pM * s.ts1();
+                if (G) phi[0] += t0 * pM;
+                else el += 0.5 * (double)(t0 * pM * qM);
+#pragma unroll
+                for (int k = 0; k < 3; k++) efq[k] += (double)(t1 * R[k]);
+            }
+        }
+    // induced dipoles (ttm3f.cpp:239-307); the iterate is carried in FP64 so the FP32
+    // form can still reach its residual target
+    double tens[kMaxNw - 1][6];                 // 3 ts2 R R^T - ts1 towards water i + r
+#pragma unroll
+    for (int r = 1; r < kMaxNw; r++)
+        if (on && r < nw) {
+            const int b = i + r < nw ? i + r : i + r - nw;
+            T R[3];
+#pragma unroll
+            for (int k = 0; k < 3; k++) R[k] = xM[k] - mj[3 * b + k];
+            const Smear<T> s(dot3(R, R), iMM);
+            const T t1 = s.ts1(), t2 = T(3) * s.ts2(t1, iMM);
+            tens[r - 1][0] = (double)(t2 * R[0] * R[0] - t1);
+            tens[r - 1][1] = (double)(t2 * R[0] * R[1]);
+            tens[r - 1][2] = (double)(t2 * R[0] * R[2]);
+            tens[r - 1][3] = (double)(t2 * R[1] * R[1] - t1);
+            tens[r - 1][4] = (double)(t2 * R[1] * R[2]);
+            tens[r - 1][5] = (double)(t2 * R[2] * R[2] - t1);
+        }
     const double tol = sizeof(T) == 8 ? 1.0e-15 : 1.0e-8;
     const double stath = kDebye / kChargeCon / sqrt((double)nw);
-    double dcur = 0.0, dprev = 0.0, efqk = 0.0;
-    if (lane < n3) {
-        efqk = (double)efq[lane];
-        dcur = dprev = kPolarM * efqk;
-        dip[lane] = (T)dcur;
-    }
-    __syncwarp();
-    int it = 0;
-    for (; it < kTtmMaxIter; it++) {
-        double ef = 0.0, del2 = 0.0;
-        if (lane < n3) {
-            const T* row = ddt + n3 * lane;
-            for (int l = 0; l < n3; l++) ef += (double)row[l] * (double)dip[l];
-            double d = kPolarM * (efqk + ef);
-            d = 0.7 * d + (1.0 - 0.7) * dprev;
-            const double del = d - dprev;
-            del2 = del * del;
-            dcur = d;
-        }
-        del2 = warp_sum(del2);
-        __syncwarp();
-        if (lane < n3) dip[lane] = (T)dcur;
-        __syncwarp();
-        if (sqrt(del2) * stath < tol) break;
-        dprev = dcur;
-    }
-    *iters = (it < kTtmMaxIter) ? it + 1 : kTtmMaxIter + 1;
-    double el = 0.0, ind = 0.0;
-    if (lane < n3) {
-        el = (double)phi[lane] * (double)chg[lane];
-        ind = -dcur * efqk;
-    }
-    const double tot = warp_sum(part) + warp_sum(el) / 2 + warp_sum(ind) / 2;
-    __syncwarp();
-    return tot;
-}
-
-// ---------------------------------------------------------------- energy + gradient
-// The E+g operator (ttm3f.cpp:325-720), FP64: the monomer energy with its
-// gradient (pot_nasa with dr, ps.cpp:486-603), the charges with their
-// derivatives (dms_nasa with dq3, ps.cpp:605-836), the smeared pair terms with
-// their forces, the induced dipoles as in energy_warp, then the charge-dipole
-// and dipole-dipole forces, the M-site forces spread over O, H, H, and the
-// terms of the geometry-dependent charges.
-
-__device__ __forceinline__ void smear123(double r, double AA, double& ts1, double& ts2, double& ts3)
-{
-    const double dri = 1.0 / r, drsqi = dri * dri;
-    const double rA = r / AA, rA3 = rA * rA * rA;
-    const double e1 = exp(-kAXX * rA3);
-    const double AA3 = AA * AA * AA;
-    ts1 = (1.0 - e1) * dri * drsqi;
-    ts2 = (ts1 - e1 * kAXX / AA3) * drsqi;
-    ts3 = (ts2 - 0.6 * e1 * r * kAXX * kAXX / (AA3 * AA3)) * drsqi;
-}
-
-// Monomer at w[9]: energy e (kcal/mol), its gradient g9 (written), the charges
-// q3 and the derivatives of the scaled site charges grdq[27] (GRDQ layout of
-// ttm3f.cpp:371-393: [atom H1, H2, O][charge H1, H2, M][xyz], times CHARGECON).
-__device__ inline void monomer_grad(const double* w, double* f, double& e, double q3[3], double* g9, double* grdq)
-{
-    constexpr double reoh = 0.958649, b1 = 2.0, roh = 0.9519607159623009, alphaoh = 2.587949757553683;
-    constexpr double deohA = 42290.92019288289, phh2 = 12.66426998162947, f5z = 0.999677885;
-    constexpr double costhe = -.24780227221366464506, tocal = 0.00285914375100642899;
-    constexpr double ath0 = 1.82400520401572996557, dms1 = 0.5, dms2 = 0.9578, dms3 = 0.012;
-    double roh1[3], roh2[3], rhh[3], d1 = 0, d2 = 0, dhh = 0;
-    for (int i = 0; i < 3; i++) {
-        roh1[i] = w[3 + i] - w[i];
-        roh2[i] = w[6 + i] - w[i];
-        rhh[i] = w[3 + i] - w[6 + i];
-        d1 += roh1[i] * roh1[i];
-        d2 += roh2[i] * roh2[i];
-        dhh += rhh[i] * rhh[i];
-    }
-    d1 = sqrt(d1);
-    d2 = sqrt(d2);
-    dhh = sqrt(dhh);
-    const double costh = (roh1[0] * roh2[0] + roh1[1] * roh2[1] + roh1[2] * roh2[2]) / (d1 * d2);
-    // --- pot_nasa with its derivatives
-    const double deoh = f5z * deohA;
-    const double e1x = exp(-alphaoh * (d1 - roh)), e2x = exp(-alphaoh * (d2 - roh));
-    const double va = deoh * (e1x * (e1x - 2.0) + e2x * (e2x - 2.0));
-    const double vb = kC.phh1 * exp(-phh2 * dhh);
-    const double dva1 = 2.0 * alphaoh * deoh * e1x * (1.0 - e1x) / d1;
-    const double dva2 = 2.0 * alphaoh * deoh * e2x * (1.0 - e2x) / d2;
-    const double dvb = -phh2 * vb / dhh;
-    const double x1 = (d1 - reoh) / reoh, x2 = (d2 - reoh) / reoh;
-    powers(x1, x2, costh - costhe, f);
-    const double dr1 = d1 - reoh, dr2 = d2 - reoh;
-    const double efac = exp(-b1 * (dr1 * dr1 + dr2 * dr2));
-    double s0 = 0, s1 = 0, s2 = 0, s3 = 0;
-    for (int j = 1; j < 245; j++) {
-        const int I = kC.idx1[j], J = kC.idx2[j], K = kC.idx3[j];
-        const double c = kC.c5z[j];
-        const double sym = f[I] * f[16 + J] + f[J] * f[16 + I];
-        s0 += c * sym * f[32 + K];
-        s1 += c * ((I - 1) * f[I - 1] * f[16 + J] + (J - 1) * f[J - 1] * f[16 + I]) * f[32 + K];
-        s2 += c * ((J - 1) * f[I] * f[16 + J - 1] + (I - 1) * f[J] * f[16 + I - 1]) * f[32 + K];
-        s3 += c * sym * (K - 1) * f[32 + K - 1];
-    }
-    e = (va + vb + (2.0 * kC.c5z[0] + efac * s0) + 0.44739574026257) * tocal;
-    const double dvc1 = (-2 * b1 * efac * dr1 * s0 + efac * s1 / reoh) / d1;
-    const double dvc2 = (-2 * b1 * efac * dr2 * s0 + efac * s2 / reoh) / d2;
-    const double dvcc = efac * s3;
-    for (int i = 0; i < 3; i++) {
-        const double h1 = dva1 * roh1[i] + dvb * rhh[i] + dvc1 * roh1[i] +
-                          dvcc * (roh2[i] / (d1 * d2) - costh * roh1[i] / (d1 * d1));
-        const double h2 = dva2 * roh2[i] - dvb * rhh[i] + dvc2 * roh2[i] +
-                          dvcc * (roh1[i] / (d1 * d2) - costh * roh2[i] / (d2 * d2));
-        g9[3 + i] = h1 * tocal;
-        g9[6 + i] = h2 * tocal;
-        g9[i] = -(h1 + h2) * tocal;
-    }
-    // --- dms_nasa with dq3
-    const double efacD = exp(-(dr1 * dr1 + dr2 * dr2));   // b1D = 1
-    double p1 = 0, p2 = 0, dp1r1 = 0, dp1r2 = 0, dp1c = 0, dp2r1 = 0, dp2r2 = 0, dp2c = 0;
-    const double pl1 = costh, pl2 = 0.5 * (3 * pl1 * pl1 - 1.0);
-    for (int j = 1; j < 84; j++) {
-        const int I = kC.idxD0[j], J = kC.idxD1[j], K = kC.idxD2[j];
-        const double c = kC.coefD[j];
-        p1 += c * f[I] * f[16 + J] * f[32 + K];
-        p2 += c * f[J] * f[16 + I] * f[32 + K];
-        dp1r1 += c * (I - 1) * f[I - 1] * f[16 + J] * f[32 + K];
-        dp1r2 += c * (J - 1) * f[I] * f[16 + J - 1] * f[32 + K];
-        dp1c += c * (K - 1) * f[I] * f[16 + J] * f[32 + K - 1];
-        dp2r1 += c * (J - 1) * f[J - 1] * f[16 + I] * f[32 + K];
-        dp2r2 += c * (I - 1) * f[J] * f[16 + I - 1] * f[32 + K];
-        dp2c += c * (K - 1) * f[J] * f[16 + I] * f[32 + K - 1];
-    }
-    const double xx = 0.529177249, xx2 = xx * xx;
-    dp1r1 /= reoh / xx;
-    dp1r2 /= reoh / xx;
-    dp2r1 /= reoh / xx;
-    dp2r2 /= reoh / xx;
-    const double pa = 0.2999, pb = -0.6932, pc0c = 1.0099, pc1 = -0.1801, pc2 = 0.0892;
-    const double ang_f = pc0c + pl1 * pc1 + pl2 * pc2;
-    const double pc0 = pa * (pow(d1, pb) + pow(d2, pb)) * ang_f;
-    const double dpc0r1 = pa * pb * pow(d1, pb - 1) * ang_f * xx2;
-    const double dpc0r2 = pa * pb * pow(d2, pb - 1) * ang_f * xx2;
-    const double dpc0c = pa * (pow(d1, pb) + pow(d2, pb)) * (pc1 + 0.5 * (6.0 * pl1) * pc2) * xx;
-    const double defr1 = -2.0 * dr1 * efacD * xx, defr2 = -2.0 * dr2 * efacD * xx;
-    dp1r1 = dp1r1 * efacD + p1 * defr1 + dpc0r1;
-    dp1r2 = dp1r2 * efacD + p1 * defr2 + dpc0r2;
-    dp1c = dp1c * efacD + dpc0c;
-    dp2r1 = dp2r1 * efacD + p2 * defr1 + dpc0r1;
-    dp2r2 = dp2r2 * efacD + p2 * defr2 + dpc0r2;
-    dp2c = dp2c * efacD + dpc0c;
-    p1 = kC.coefD[0] + p1 * efacD + pc0 * xx;
-    p2 = kC.coefD[0] + p2 * efacD + pc0 * xx;
-    dp1r1 /= xx;
-    dp1r2 /= xx;
-    dp2r1 /= xx;
-    dp2r2 /= xx;
-    const double axb[3] = {roh1[1] * roh2[2] - roh1[2] * roh2[1], -roh1[0] * roh2[2] + roh1[2] * roh2[0],
-                           roh1[0] * roh2[1] - roh1[1] * roh2[0]};
-    const double sinth = sqrt(axb[0] * axb[0] + axb[1] * axb[1] + axb[2] * axb[2]) / (d1 * d2);
-    const double ang = atan2(sinth, costh);
-    const double m1 = dms1 * (d1 - dms2) + dms3 * (ang - ath0);
-    const double m2 = dms1 * (d2 - dms2) + dms3 * (ang - ath0);
-    q3[0] = -(p1 + p2) - (m1 + m2);
-    q3[1] = p1 + m1;
-    q3[2] = p2 + m2;
-    dp1r1 += dms1;
-    dp2r2 += dms1;
-    dp1c -= dms3 / sinth;
-    dp2c -= dms3 / sinth;
-    const double f1q1r13 = (dp1r1 - dp1c * costh / d1) / d1, f1q1r23 = dp1c / (d1 * d2);
-    const double f2q1r23 = (dp1r2 - dp1c * costh / d2) / d2, f2q1r13 = dp1c / (d2 * d1);
-    const double f1q2r13 = (dp2r1 - dp2c * costh / d1) / d1, f1q2r23 = dp2c / (d1 * d2);
-    const double f2q2r23 = (dp2r2 - dp2c * costh / d2) / d2, f2q2r13 = dp2c / (d2 * d1);
-    double dq[27];   // [atom H1, H2, O][charge h1, h2, O][xyz]
+    double cur[3];
+#pragma unroll
     for (int k = 0; k < 3; k++) {
-        dq[0 * 9 + 0 * 3 + k] = f1q1r13 * roh1[k] + f1q1r23 * roh2[k];
-        dq[1 * 9 + 0 * 3 + k] = f2q1r13 * roh1[k] + f2q1r23 * roh2[k];
-        dq[2 * 9 + 0 * 3 + k] = -(dq[k] + dq[9 + k]);
-        dq[0 * 9 + 1 * 3 + k] = f1q2r13 * roh1[k] + f1q2r23 * roh2[k];
-        dq[1 * 9 + 1 * 3 + k] = f2q2r13 * roh1[k] + f2q2r23 * roh2[k];
-        dq[2 * 9 + 1 * 3 + k] = -(dq[3 + k] + dq[9 + 3 + k]);
-        dq[0 * 9 + 2 * 3 + k] = -(dq[k] + dq[3 + k]);
-        dq[1 * 9 + 2 * 3 + k] = -(dq[9 + k] + dq[9 + 3 + k]);
-        dq[2 * 9 + 2 * 3 + k] = -(dq[18 + k] + dq[18 + 3 + k]);
+        cur[k] = kPolarM * efq[k];
+        if (on) dip[3 * i + k] = dip[n3 + 3 * i + k] = cur[k];
     }
-    const double t = kGamma2 / kGamma1;
-    for (int a = 0; a < 3; a++)
-        for (int k = 0; k < 3; k++) {
-            const double h1 = dq[9 * a + k], h2 = dq[9 * a + 3 + k], o = dq[9 * a + 6 + k];
-            grdq[9 * a + 0 + k] = kChargeCon * (h1 + t * (h1 + h2));
-            grdq[9 * a + 3 + k] = kChargeCon * (h2 + t * (h2 + h1));
-            grdq[9 * a + 6 + k] = kChargeCon * (o - 2 * t * (h1 + h2));
-        }
-}
-
-// Energy (kcal/mol, all lanes) and gradient g[9nw] (kcal/mol/A, shared, complete
-// after the call) of crd[9nw] (shared); ms 3nw shared; sc: scratch_elems(nw, true).
-__device__ inline double energy_grad_warp(const double* crd, double* ms, double* sc, double* g, int nw,
-                                          const uint32_t* __restrict__ tasks, int ntasks, int lane, int* iters)
-{
-    const int n3 = 3 * nw;
-    double *chg = sc, *phi = chg + n3, *efq = phi + n3, *dip = efq + n3, *dipp = dip + n3, *efd = dipp + n3,
-           *ddt = efd + n3, *fpow = ddt + n3 * n3, *grdq = fpow + 48 * nw, *dM = grdq + 27 * nw;
-    for (int i = lane; i < n3 * n3; i += 32) ddt[i] = 0.0;
-    for (int i = lane; i < n3; i += 32) phi[i] = efq[i] = efd[i] = dM[i] = 0.0;
-    double part = 0;
-    for (int i = lane; i < nw; i += 32) {
-        const double* w = crd + 9 * i;
-        for (int k = 0; k < 3; k++) ms[3 * i + k] = kGamma1 * w[k] + kGamma2 * (w[3 + k] + w[6 + k]);
-        double e, q3[3];
-        monomer_grad(w, fpow + 48 * i, e, q3, g + 9 * i, grdq + 27 * i);
-        part += e;
-        const double t = kGamma2 / kGamma1;
-        chg[3 * i + 0] = kChargeCon * q3[0] / kGamma1;
-        chg[3 * i + 1] = kChargeCon * (q3[1] + t * (q3[1] + q3[2]));
-        chg[3 * i + 2] = kChargeCon * (q3[2] + t * (q3[1] + q3[2]));
-    }
-    __syncwarp();
-    // pair terms with their forces (ttm3f.cpp:403-520)
-    for (int t = lane; t < ntasks; t += 32) {
-        const uint32_t task = __ldg(tasks + t), type = task & 3u, a = (task >> 2) & 0x7fffu, b = task >> 17;
-        if (type == 0) {            // M site of water a, H atom b
-            const int ia = 3 * a;
-            double R[3];
-            for (int k = 0; k < 3; k++) R[k] = ms[ia + k] - crd[3 * b + k];
-            double ts0, ts1;
-            smear<double>(sqrt(R[0] * R[0] + R[1] * R[1] + R[2] * R[2]), kC.AA_HM, ts0, ts1, nullptr);
-            atomicAdd(phi + ia, ts0 * chg[b]);
-            atomicAdd(phi + b, ts0 * chg[ia]);
-            const double tmp1 = chg[b] * ts1, tmp2 = chg[ia] * tmp1;
-            for (int k = 0; k < 3; k++) {
-                atomicAdd(efq + ia + k, tmp1 * R[k]);
-                atomicAdd(g + 3 * b + k, tmp2 * R[k]);
-            }
-        } else if (type == 1) {     // H/H
-            double R[3];
-            for (int k = 0; k < 3; k++) R[k] = crd[3 * a + k] - crd[3 * b + k];
-            double ts0, ts1;
-            smear<double>(sqrt(R[0] * R[0] + R[1] * R[1] + R[2] * R[2]), kC.AA_HH, ts0, ts1, nullptr);
-            atomicAdd(phi + a, chg[b] * ts0);
-            atomicAdd(phi + b, chg[a] * ts0);
-            const double qq = chg[a] * chg[b] * ts1;
-            for (int k = 0; k < 3; k++) {
-                atomicAdd(g + 3 * a + k, -qq * R[k]);
-                atomicAdd(g + 3 * b + k, qq * R[k]);
-            }
-        } else if (type == 2) {     // O/O van der Waals
-            double R[3];
-            for (int k = 0; k < 3; k++) R[k] = crd[3 * a + k] - crd[3 * b + k];
-            const double r2 = R[0] * R[0] + R[1] * R[1] + R[2] * R[2], r = sqrt(r2), r6 = r2 * r2 * r2;
-            const double expon = kVdwD * exp(-kVdwE * r);
-            part += kVdwC / r6 + expon;
-            const double tmp = -(6.0 * kVdwC / r6) / r2 - kVdwE * expon / r;
-            for (int k = 0; k < 3; k++) {
-                atomicAdd(g + 3 * a + k, tmp * R[k]);
-                atomicAdd(g + 3 * b + k, -tmp * R[k]);
-            }
-        } else {                    // M/M
-            const int i3 = 3 * a, j3 = 3 * b;
-            double R[3];
-            for (int k = 0; k < 3; k++) R[k] = ms[i3 + k] - ms[j3 + k];
-            double ts0, ts1, ts2;
-            smear<double>(sqrt(R[0] * R[0] + R[1] * R[1] + R[2] * R[2]), kC.AA_MM, ts0, ts1, &ts2);
-            atomicAdd(phi + i3, ts0 * chg[j3]);
-            atomicAdd(phi + j3, ts0 * chg[i3]);
-            for (int k = 0; k < 3; k++) {
-                atomicAdd(efq + i3 + k, chg[j3] * ts1 * R[k]);
-                atomicAdd(efq + j3 + k, -(chg[i3] * ts1 * R[k]));
-            }
-            for (int k = 0; k < 3; k++)
-                for (int l = k; l < 3; l++) {
-                    const double d = 3.0 * ts2 * R[k] * R[l] - (k == l ? ts1 : 0.0);
-                    ddt[n3 * (i3 + k) + j3 + l] = d;
-                    ddt[n3 * (j3 + k) + i3 + l] = d;
-                    ddt[n3 * (i3 + l) + j3 + k] = d;
-                    ddt[n3 * (j3 + l) + i3 + k] = d;
-                }
-        }
-    }
-    __syncwarp();
-    // induced dipoles (ttm3f.cpp:528-581)
-    const double stath = kDebye / kChargeCon / sqrt((double)nw);
-    double dcur = 0.0, dprev = 0.0, efqk = 0.0;
-    if (lane < n3) {
-        efqk = efq[lane];
-        dcur = dprev = kPolarM * efqk;
-        dip[lane] = dcur;
-    }
-    __syncwarp();
+    bool busy = j < ng;
     int it = 0;
-    for (; it < kTtmMaxIter; it++) {
-        double ef = 0.0, del2 = 0.0;
-        if (lane < n3) {
-            const double* row = ddt + n3 * lane;
-            for (int l = 0; l < n3; l++) ef += row[l] * dip[l];
-            double d = kPolarM * (efqk + ef);
-            d = 0.7 * d + (1.0 - 0.7) * dprev;
-            const double del = d - dprev;
-            del2 = del * del;
-            dcur = d;
-        }
-        del2 = warp_sum(del2);
+    for (int sweep = 0; sweep < kTtmMaxIter; sweep++) {
         __syncwarp();
-        if (lane < n3) dip[lane] = dcur;
+        double ef[3] = {0, 0, 0}, del2 = 0.0;
+        if (on && busy) {
+#pragma unroll
+            for (int r = 1; r < kMaxNw; r++)
+                if (r < nw) {
+                    const double* d = dip + 3 * (i + r);
+                    const double* t = tens[r - 1];
+                    const double dx = d[0], dy = d[1], dz = d[2];
+                    ef[0] += t[0] * dx + t[1] * dy + t[2] * dz;
+                    ef[1] += t[1] * dx + t[3] * dy + t[4] * dz;
+                    ef[2] += t[2] * dx + t[4] * dy + t[5] * dz;
+                }
+#pragma unroll
+            for (int k = 0; k < 3; k++) {
+                const double prev = cur[k];
+                double d = kPolarM * (efq[k] + ef[k]);
+                d = 0.7 * d + (1.0 - 0.7) * prev;
+                cur[k] = d;
+                del2 += (d - prev) * (d - prev);
+            }
+        }
+        del2 = sum_geometry<NG>(del2);
         __syncwarp();
-        if (sqrt(del2) * stath < 1.0e-15) break;
-        dprev = dcur;
-    }
-    *iters = (it < kTtmMaxIter) ? it + 1 : kTtmMaxIter + 1;
-    double el = 0.0, ind = 0.0;
-    if (lane < n3) {
-        el = phi[lane] * chg[lane];
-        ind = -dcur * efqk;
-    }
-    const double tot = warp_sum(part) + warp_sum(el) / 2 + warp_sum(ind) / 2;
-    __syncwarp();
-    // charge-dipole and dipole-dipole forces (ttm3f.cpp:594-676)
-    for (int t = lane; t < ntasks; t += 32) {
-        const uint32_t task = __ldg(tasks + t), type = task & 3u, a = (task >> 2) & 0x7fffu, b = task >> 17;
-        if (type == 0) {            // dipole of M(a), charge of H atom b
-            const int i3 = 3 * a;
-            double R[3], diR = 0;
-            for (int k = 0; k < 3; k++) {
-                R[k] = ms[i3 + k] - crd[3 * b + k];
-                diR += dip[i3 + k] * R[k];
-            }
-            const double r = sqrt(R[0] * R[0] + R[1] * R[1] + R[2] * R[2]);
-            const double dri = 1.0 / r, drsqi = dri * dri, rA = r / kC.AA_HM, e1 = exp(-kAXX * rA * rA * rA);
-            const double ts1 = (1.0 - e1) * dri * drsqi;
-            const double ts2 = (ts1 - e1 * kAXX / (kC.AA_HM * kC.AA_HM * kC.AA_HM)) * drsqi;   // smear12
-            for (int k = 0; k < 3; k++) {
-                const double derij = chg[b] * (3 * ts2 * diR * R[k] - ts1 * dip[i3 + k]);
-                atomicAdd(dM + i3 + k, derij);
-                atomicAdd(g + 3 * b + k, -derij);
-            }
-            atomicAdd(phi + b, -ts1 * diR);
-        } else if (type == 3) {     // M(a), M(b): both charge-dipole directions, dipole-dipole once
-            const int i3 = 3 * a, j3 = 3 * b;
-            double R[3], diR = 0, djR = 0, didj = 0;
-            for (int k = 0; k < 3; k++) {
-                R[k] = ms[i3 + k] - ms[j3 + k];
-                diR += dip[i3 + k] * R[k];
-                djR += dip[j3 + k] * R[k];
-                didj += dip[i3 + k] * dip[j3 + k];
-            }
-            double ts1, ts2, ts3;
-            smear123(sqrt(R[0] * R[0] + R[1] * R[1] + R[2] * R[2]), kC.AA_MM, ts1, ts2, ts3);
-            for (int k = 0; k < 3; k++) {
-                // (i, j): dipole of i, charge of j, added to i and taken from j;
-                // (j, i): R and dip_j.R change sign together, added to j and taken from i
-                const double dij = chg[j3] * (3 * ts2 * diR * R[k] - ts1 * dip[i3 + k]);
-                const double dji = chg[i3] * (3 * ts2 * djR * R[k] - ts1 * dip[j3 + k]);
-                const double dd = -3 * ts2 * (didj * R[k] + djR * dip[i3 + k] + diR * dip[j3 + k]) +
-                                  15 * ts3 * diR * djR * R[k];
-                atomicAdd(dM + i3 + k, dij - dji + dd);
-                atomicAdd(dM + j3 + k, -(dij - dji + dd));
-            }
-            atomicAdd(phi + j3, -ts1 * diR);
-            atomicAdd(phi + i3, ts1 * djR);
+        if (busy) {
+            if (on)
+#pragma unroll
+                for (int k = 0; k < 3; k++) dip[3 * i + k] = dip[n3 + 3 * i + k] = cur[k];
+            it++;
+            if (sqrt(del2) * stath < tol) busy = false;
         }
+        if (!__any_sync(0xffffffffu, busy)) break;
     }
+    *iters = busy ? kTtmMaxIter + 1 : it;
     __syncwarp();
-    // M-site forces onto O, H, H, and the charges' geometry dependence (ttm3f.cpp:680-716)
-    for (int i = lane; i < nw; i += 32) {
-        const int i3 = 3 * i;
-        const double* gq = grdq + 27 * i;
-        for (int k = 0; k < 3; k++) {
-            const double tmp = dM[i3 + k] - chg[i3] * efq[i3 + k];
-            g[9 * i + k] += kGamma1 * tmp + gq[18 + 0 + k] * phi[i3 + 1] + gq[18 + 3 + k] * phi[i3 + 2] +
-                            gq[18 + 6 + k] * phi[i3];
-            g[9 * i + 3 + k] += kGamma2 * tmp + gq[0 + k] * phi[i3 + 1] + gq[3 + k] * phi[i3 + 2] +
-                                gq[6 + k] * phi[i3];
-            g[9 * i + 6 + k] += kGamma2 * tmp + gq[9 + k] * phi[i3 + 1] + gq[9 + 3 + k] * phi[i3 + 2] +
-                                gq[9 + 6 + k] * phi[i3];
+    if (G) el = 0.5 * ((double)phi[0] * (double)qM + (double)phi[1] * (double)qH[0] + (double)phi[2] * (double)qH[1]);
+    const double ind = -(cur[0] * efq[0] + cur[1] * efq[1] + cur[2] * efq[2]);
+    const double tot = sum_geometry<NG>(on ? part + el + 0.5 * vdw + 0.5 * ind : 0.0);
+    if constexpr (G) {
+        // charge-dipole and dipole-dipole forces (ttm3f.cpp:594-676), the water's own side
+        if (on) {
+            T d[3], dM[3] = {0, 0, 0};
+#pragma unroll
+            for (int k = 0; k < 3; k++) d[k] = (T)cur[k];
+#pragma unroll 1
+            for (int r = 1; r < nw; r++) {
+                const int b = i + r < nw ? i + r : i + r - nw;
+                const T* w = cj + 9 * b;
+                T yM[3], R[3], db[3];
+                load3(mj + 3 * b, yM);
+#pragma unroll
+                for (int k = 0; k < 3; k++) db[k] = (T)dip[3 * b + k];
+                const T pM = chg[3 * b];
+#pragma unroll
+                for (int l = 0; l < 2; l++) {   // own dipole, other H
+#pragma unroll
+                    for (int k = 0; k < 3; k++) R[k] = xM[k] - w[3 + 3 * l + k];
+                    const Smear<T> s(dot3(R, R), iHM);
+                    const T t1 = s.ts1(), t2 = s.ts2(t1, iHM), p = chg[3 * b + 1 + l], c = T(3) * t2 * dot3(d, R);
+#pragma unroll
+                    for (int k = 0; k < 3; k++) dM[k] += p * (c * R[k] - t1 * d[k]);
+                }
+#pragma unroll
+                for (int l = 0; l < 2; l++) {   // own H, other dipole
+#pragma unroll
+                    for (int k = 0; k < 3; k++) R[k] = yM[k] - xH[l][k];
+                    const Smear<T> s(dot3(R, R), iHM);
+                    const T t1 = s.ts1(), t2 = s.ts2(t1, iHM), dR = dot3(db, R), c = T(3) * t2 * dR;
+#pragma unroll
+                    for (int k = 0; k < 3; k++) gH[l][k] -= qH[l] * (c * R[k] - t1 * db[k]);
+                    phi[1 + l] -= t1 * dR;
+                }
+#pragma unroll
+                for (int k = 0; k < 3; k++) R[k] = xM[k] - yM[k];
+                const Smear<T> s(dot3(R, R), iMM);
+                const T t1 = s.ts1(), t2 = s.ts2(t1, iMM), t3 = s.ts3(t2, iMM);
+                const T diR = dot3(d, R), djR = dot3(db, R), dd = dot3(d, db);
+#pragma unroll
+                for (int k = 0; k < 3; k++)
+                    dM[k] += pM * (T(3) * t2 * diR * R[k] - t1 * d[k]) - qM * (T(3) * t2 * djR * R[k] - t1 * db[k]) -
+                             T(3) * t2 * (dd * R[k] + djR * d[k] + diR * db[k]) + T(15) * t3 * diR * djR * R[k];
+                phi[0] += t1 * djR;
+            }
+            // the M site's force onto O, H, H, and the charges' geometry dependence
+            // (ttm3f.cpp:680-716, GRDQ of 371-393)
+            const T t = T(kGamma2 / kGamma1), P0 = (T(1) + T(2) * t) * phi[0];
+            const T A1 = T(kChargeCon) * ((T(1) + t) * phi[1] + t * phi[2] - P0);
+            const T A2 = T(kChargeCon) * ((T(1) + t) * phi[2] + t * phi[1] - P0);
+            const T u1 = A1 * mo.f11 + A2 * mo.g11, u2 = A1 * mo.f12 + A2 * mo.g12;
+            const T v1 = A1 * mo.f21 + A2 * mo.g21, v2 = A1 * mo.f22 + A2 * mo.g22;
+            double* gw = g + j * 9 * nw + 9 * i;
+#pragma unroll
+            for (int k = 0; k < 3; k++) {
+                const T r1 = xH[0][k] - xO[k], r2 = xH[1][k] - xO[k];
+                const T c1 = u1 * r1 + u2 * r2 + mo.h1[k], c2 = v1 * r1 + v2 * r2 + mo.h2[k];
+                const T f = dM[k] - qM * (T)efq[k];
+                gw[k] = gO[k] + T(kGamma1) * f - (c1 + c2);
+                gw[3 + k] = gH[0][k] + T(kGamma2) * f + c1;
+                gw[6 + k] = gH[1][k] + T(kGamma2) * f + c2;
+            }
         }
+        __syncwarp();
     }
-    __syncwarp();
     return tot;
 }
 

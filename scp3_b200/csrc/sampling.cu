@@ -1,8 +1,7 @@
 // Per-sample kernels: Sobol point (optionally scrambled) -> BSM -> q = y/sqrt(2)
 // -> Cartesian back-transform -> water potential -> anharmonic residual.
-// One warp per sample; the sample's q and geometry live in the warp's slice of
-// shared memory, lanes split the dimensions, the coordinates and the potential's
-// pair terms.  The FP64 form follows SCP3.cpp:196-223 operation for operation
+// A warp takes four samples at a time; their q and geometries live in the warp's slice
+// of shared memory, lanes split the dimensions, the coordinates and the waters.  The FP64 form follows SCP3.cpp:196-223 operation for operation
 // where that is cheap (division by sqrt(2), x0 + MUa q then times bohr).
 #include "common.cuh"
 #include "internal.h"
@@ -32,62 +31,123 @@ struct WarpSlot {
     T* q;           // [group][qs] normal coordinates (the form's precision)
     T* crd;         // [group][9nw] geometries
     T* ms;          // [group][3nw] M sites
-    T* ttm;         // TTM3-F scratch
-    double* g;      // 9nw gradient (gradient path)
-    double* gm;     // 3nw forces on the M sites
-    uint64_t* xs;   // FP32 form: [group][nm0] Sobol states of the group
-    uint16_t* tl;   // FP32 form: [group * nm0] items that take the inverse CDF's tail branch
+    uint64_t* xs;   // [group][nm0] Sobol states of the group (dead once the normals are formed)
+    uint16_t* tl;   // [group * nm0] items that take the inverse CDF's tail branch
+    double* g;      // [group][9nw] gradients (gradient path), over xs and tl
+    char* sc;       // TTM3-F scratch, after g
     int qs;         // q stride: nm0 rounded up to even (16-byte aligned rows)
 };
 
-// Gradient storage of a warp slot: [9nw] + [3nw] in FP64, or in the FP32 form
-// the four geometries' [4][9nw] + [4][3nw].
+constexpr size_t round16(size_t b) { return (b + 15) & ~(size_t)15; }
+
 template <typename T>
-__host__ __device__ inline size_t grad_bytes(int nw, int group)
+__host__ __device__ inline size_t slot_bytes(int pes, int nm0, int nw, bool grad = false)
 {
-    return sizeof(T) == 4 ? sizeof(float) * (size_t)(12 * nw * group) : sizeof(double) * (size_t)(12 * nw);
+    const size_t fixed = round16(sizeof(T) * kGroup * (((nm0 + 1) & ~1) + (size_t)(12 * nw)));
+    const size_t normals = round16((size_t)kGroup * nm0 * (sizeof(uint64_t) + sizeof(uint16_t)));
+    const size_t force = (grad ? round16(sizeof(double) * kGroup * 9 * (size_t)nw) : 0) +
+                         (pes == SCP3GPU_PES_TTM3F ? round16(ttm::scratch_bytes<T>(nw)) : 0);
+    return fixed + (normals > force ? normals : force);
 }
 
 template <typename T>
-__host__ __device__ inline size_t slot_bytes(int pes, int nm0, int nw, bool grad = false, int group = 1)
-{
-    size_t b = sizeof(T) * ((size_t)group * ((nm0 + 1) & ~1) + (size_t)(12 * nw * group));
-    if (pes == SCP3GPU_PES_TTM3F) b += sizeof(T) * ttm::scratch_elems(nw, grad);
-    b = (b + 7) & ~(size_t)7;
-    if (grad) b += grad_bytes<T>(nw, group);
-    if (sizeof(T) == 4) b += (size_t)group * nm0 * (sizeof(uint64_t) + sizeof(uint16_t));
-    return (b + 15) & ~(size_t)15;
-}
-
-template <typename T>
-__device__ inline WarpSlot<T> warp_slot(char* base, int pes, int nm0, int nw, bool grad = false, int group = 1)
+__device__ inline WarpSlot<T> warp_slot(char* base, int nm0, int nw, bool grad = false)
 {
     WarpSlot<T> s;
     s.qs = (nm0 + 1) & ~1;
     s.q = reinterpret_cast<T*>(base);
-    s.crd = s.q + (size_t)group * s.qs;
-    s.ms = s.crd + 9 * nw * group;
-    s.ttm = s.ms + 3 * nw * group;
-    size_t off = sizeof(T) * ((size_t)group * s.qs + (size_t)(12 * nw * group));
-    if (pes == SCP3GPU_PES_TTM3F) off += sizeof(T) * ttm::scratch_elems(nw, grad);
-    off = (off + 7) & ~(size_t)7;
-    s.g = grad ? reinterpret_cast<double*>(base + off) : nullptr;
-    s.gm = grad ? s.g + 9 * nw : nullptr;
-    if (grad) off += grad_bytes<T>(nw, group);
-    s.xs = sizeof(T) == 4 ? reinterpret_cast<uint64_t*>(base + off) : nullptr;
-    s.tl = sizeof(T) == 4 ? reinterpret_cast<uint16_t*>(base + off + sizeof(uint64_t) * (size_t)group * nm0) : nullptr;
+    s.crd = s.q + (size_t)kGroup * s.qs;
+    s.ms = s.crd + 9 * nw * kGroup;
+    char* over = base + round16(sizeof(T) * kGroup * (s.qs + (size_t)(12 * nw)));
+    s.xs = reinterpret_cast<uint64_t*>(over);
+    s.tl = reinterpret_cast<uint16_t*>(s.xs + (size_t)kGroup * nm0);
+    s.g = reinterpret_cast<double*>(over);
+    s.sc = over + (grad ? round16(sizeof(double) * kGroup * 9 * (size_t)nw) : 0);
     return s;
 }
 
-template <int PES, typename T>
-__device__ inline double potential(const T* crd, const WarpSlot<T>& w, int nw, const uint32_t* tasks, int ntasks,
-                                   int lane, int* iters)
+// Energies (and with G gradients) of a group's gn geometries in one warp pass: lane l
+// returns the energy of geometry l % 4.
+template <int PES, typename T, bool G, int NG = kGroup>
+__device__ __forceinline__ double potential4(const WarpSlot<T>& w, int nw, int gn, int lane, int* iters)
 {
-    if (PES == SCP3GPU_PES_QTIP4PF) {
+    if constexpr (PES == SCP3GPU_PES_QTIP4PF) {
         *iters = 0;
-        return qt::energy_warp<T>(crd, w.ms, nw, tasks, ntasks, lane);
+        if constexpr (G) return qt::energy_grad_warp4<T>(w.crd, 9 * nw, w.ms, w.g, nw, gn, lane);
+        else return qt::energy_warp4<T>(w.crd, 9 * nw, w.ms, nw, gn, lane);
+    } else {
+        return ttm::energy_warp4<T, G, NG>(w.crd, 9 * nw, w.ms, w.sc, w.g, nw, gn, lane, iters);
     }
-    return ttm::energy_warp<T>(crd, w.ms, w.ttm, nw, tasks, ntasks, lane, iters);
+}
+
+constexpr int kDimsPerLane = 4;           // dimensions up to 128 keep their Sobol state in registers
+
+// Standard normals of samples s0 .. s0 + gn - 1 of a warp's range (first sample s_first,
+// Sobol index index0 + s): put(j, d, y) for sample s0 + j and dimension d.
+// (a) the group's Sobol states, lane-owned by dimension, staged as [sample][dimension]
+// (padding samples, s >= nvalid, get u = 0.5, so y = 0); (b) the central branch over all
+// gn * dims items, the warp's lanes strided over them, the tail items listed; (c) the
+// tail branch (16 % of the items, two logarithms) over the list.
+template <typename T, typename Put>
+__device__ __forceinline__ void group_normals(const int64_t* __restrict__ vdir, const uint64_t* __restrict__ shift,
+                                              int dims, int64_t index0, int64_t s0, int64_t s_first, int64_t nvalid,
+                                              int gn, uint64_t* st, uint64_t* xs, uint16_t* tl, int lane, Put put)
+{
+    for (int j = 0; j < gn; j++) {
+        const int64_t s = s0 + j;
+        const uint64_t idx = (uint64_t)(index0 + s);
+        uint64_t* xj = xs + j * dims;
+        if (s >= nvalid) {
+            for (int d = lane; d < dims; d += 32) xj[d] = 1ull << 61;
+            continue;
+        }
+#pragma unroll
+        for (int jd = 0; jd < kDimsPerLane; jd++) {
+            const int d = lane + 32 * jd;
+            if (d >= dims) break;
+            if (s == s_first) st[jd] = sobol_state(vdir, dims, d, idx);
+            else st[jd] ^= (uint64_t)__ldg(vdir + (size_t)(__ffsll((long long)idx) - 1) * dims + d);
+            xj[d] = shift ? st[jd] ^ __ldg(shift + d) : st[jd];
+        }
+        for (int d = lane + 32 * kDimsPerLane; d < dims; d += 32)
+            xj[d] = (shift ? __ldg(shift + d) : 0ull) ^ sobol_state(vdir, dims, d, idx);
+    }
+    __syncwarp();
+    const int items = gn * dims;
+    const float inv = 1.0f / (float)dims;      // item i is (i / dims, i % dims); exact for i < 2^16
+    // two items per lane and round (i, i + 32): two independent chains; every item runs
+    // the central formula, the tail items' values are dropped (their denominator may
+    // vanish; nothing reads the quotient)
+    int ntail = 0;
+    const unsigned below = (1u << lane) - 1u;
+    for (int i0 = 0; i0 < items; i0 += 64) {
+        const int ia = i0 + lane, ib = ia + 32;
+        const T ya = ia < items ? bsm_centred<T>(xs[ia]) : T(0);
+        const T yb = ib < items ? bsm_centred<T>(xs[ib]) : T(0);
+        const T va = bsm_central<T>(ya), vb = bsm_central<T>(yb);
+        const bool ta = ia < items && !(fabs(ya) < T(0.42));
+        const bool tb = ib < items && !(fabs(yb) < T(0.42));
+        if (ia < items && !ta) {
+            const int j = (int)(((float)ia + 0.5f) * inv);
+            put(j, ia - j * dims, va);
+        }
+        if (ib < items && !tb) {
+            const int j = (int)(((float)ib + 0.5f) * inv);
+            put(j, ib - j * dims, vb);
+        }
+        const unsigned ma = __ballot_sync(0xffffffffu, ta);
+        if (ta) tl[ntail + __popc(ma & below)] = (uint16_t)ia;
+        ntail += __popc(ma);
+        const unsigned mb = __ballot_sync(0xffffffffu, tb);
+        if (tb) tl[ntail + __popc(mb & below)] = (uint16_t)ib;
+        ntail += __popc(mb);
+    }
+    __syncwarp();
+    for (int t = lane; t < ntail; t += 32) {
+        const int i = tl[t];
+        const int j = (int)(((float)i + 0.5f) * inv);
+        put(j, i - j * dims, bsm_tail<T>(xs[i]));
+    }
 }
 
 // MUa is staged in shared memory, in the form's precision, when it fits this
@@ -129,11 +189,18 @@ struct Pair<float> {
 template <int PES, typename T, bool G = false>
 __device__ __forceinline__ void samples_body(const SampleArgs& a, char* smem);
 
+// Blocks per SM the registers must allow: qTIP4P/f, 4 for the FP32 energies (64
+// registers), 3 for the FP32 gradients (85), 2 for FP64; TTM3-F keeps its dipole tensors
+// in registers: 2 for the energies, 1 for the gradients.
 template <int PES, typename T, bool G>
-// Blocks per SM the registers must allow: 4 for the FP32 energy path (64
-// registers), 3 for the FP32 gradient path (85: a few spills, 1.3x faster than
-// at 2), 2 for FP64.
-__global__ void __launch_bounds__(kWarpsPerBlock * 32, sizeof(T) == 4 ? (G ? 3 : 4) : 2)
+constexpr int sample_blocks()
+{
+    if (PES == SCP3GPU_PES_TTM3F) return G ? 1 : 2;
+    return sizeof(T) == 4 ? (G ? 3 : 4) : 2;
+}
+
+template <int PES, typename T, bool G>
+__global__ void __launch_bounds__(kWarpsPerBlock * 32, sample_blocks<PES, T, G>())
     samples_kernel(SampleArgs a)
 {
     extern __shared__ __align__(16) char smem[];
@@ -142,7 +209,8 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, sizeof(T) == 4 ? (G ? 3 :
 
 // Several clusters of a batch: cluster blockIdx.y takes args[blockIdx.y].
 template <int PES, typename T>
-__global__ void __launch_bounds__(kWarpsPerBlock * 32) samples_batch_kernel(const SampleArgs* __restrict__ args)
+__global__ void __launch_bounds__(kWarpsPerBlock * 32, sample_blocks<PES, T, false>())
+    samples_batch_kernel(const SampleArgs* __restrict__ args)
 {
     extern __shared__ __align__(16) char smem[];
     // the cluster's arguments in shared memory, read where used (a register copy
@@ -185,117 +253,36 @@ __device__ __forceinline__ void samples_body(const SampleArgs& a, char* smem)
         __syncthreads();
     }
     char* slots = smem + (mua_in_smem ? mua_b : 0) + (muat_in_smem ? muat_smem_bytes(nw, a.nm) : 0);
-    WarpSlot<T> w = warp_slot<T>(slots + wib * slot_bytes<T>(PES, nm0, nw, grad, kGroup), PES, nm0, nw, grad, kGroup);
+    WarpSlot<T> w = warp_slot<T>(slots + wib * slot_bytes<T>(PES, nm0, nw, grad), nm0, nw, grad);
     // Each warp takes one contiguous range of samples, the ranges balanced to
     // within one sample (the grid is sized to the SMs, so there is no tail wave):
     // the Sobol state of the first is formed from the Gray code of its index, the
     // next ones by one XOR per dimension (index k differs from k-1 in direction
     // number ctz(k)).  The range goes in groups of kGroup samples: normals for
-    // the group, one back-transform pass for the group, then the potential per
-    // sample.
+    // the group, one back-transform pass and one potential pass for the group, then
+    // V, q and dV/dq.
     const int64_t nwarps = (int64_t)gridDim.x * kWarpsPerBlock;
     const int64_t gw = (int64_t)blockIdx.x * kWarpsPerBlock + wib;
-    constexpr int kDimsPerLane = 4;           // dimensions up to 128 keep their state in registers
     uint64_t st[kDimsPerLane];
     const int64_t s_first = a.n * gw / nwarps, s_end = a.n * (gw + 1) / nwarps;
     const bool sobol = a.normals == nullptr && a.normals32 == nullptr;
     for (int64_t s0 = s_first; s0 < s_end; s0 += kGroup) {
         const int gn = (int)(s_end - s0 < kGroup ? s_end - s0 : kGroup);
         // 1. standard normals -> q   (SCP3.cpp:196-201)
-        bool done = false;
-        if constexpr (sizeof(T) == 4) {
-            if (sobol) {
-                // FP32 form: (a) the group's Sobol states, lane-owned by dimension,
-                // staged as [sample][dimension] (padding samples get u = 0.5, so
-                // q = 0); (b) the central branch over all gn * nm0 items, the warp's
-                // lanes strided over them, the tail items listed; (c) the tail
-                // branch over the list.
-                for (int j = 0; j < gn; j++) {
-                    const int64_t s = s0 + j;
-                    const uint64_t idx = (uint64_t)(a.index0 + s);
-                    uint64_t* xj = w.xs + j * nm0;
-                    if (s >= a.nvalid) {
-                        for (int d = lane; d < nm0; d += 32) xj[d] = 1ull << 61;
-                        continue;
-                    }
-#pragma unroll
-                    for (int jd = 0; jd < kDimsPerLane; jd++) {
-                        const int d = lane + 32 * jd;
-                        if (d >= nm0) break;
-                        if (s == s_first) st[jd] = sobol_state(a.vdir, nm0, d, idx);
-                        else st[jd] ^= (uint64_t)__ldg(a.vdir + (size_t)(__ffsll((long long)idx) - 1) * nm0 + d);
-                        xj[d] = a.shift ? st[jd] ^ __ldg(a.shift + d) : st[jd];
-                    }
-                    for (int d = lane + 32 * kDimsPerLane; d < nm0; d += 32)
-                        xj[d] = (a.shift ? __ldg(a.shift + d) : 0ull) ^ sobol_state(a.vdir, nm0, d, idx);
+        if (sobol) {
+            group_normals<T>(a.vdir, a.shift, nm0, a.index0, s0, s_first, a.nvalid, gn, st, w.xs, w.tl, lane,
+                             [&](int j, int d, T y) {
+                                 w.q[j * w.qs + d] = sizeof(T) == 4 ? y * T(0.70710678f) : y / T(1.4142135623730951);
+                             });
+        } else {
+            for (int j = 0; j < gn; j++) {
+                const int64_t s = s0 + j;
+                T* q = w.q + j * w.qs;
+                for (int d = lane; d < nm0; d += 32) {
+                    double y = 0.0;             // padding sample (the range's tail): contributes nothing
+                    if (s < a.nvalid) y = a.normals ? a.normals[s * nm0 + d] : (double)a.normals32[s * nm0 + d];
+                    q[d] = (T)(y / 1.4142135623730951);   // by /= sqrt(2.0)
                 }
-                __syncwarp();
-                const int items = gn * nm0;
-                const float inv_nm0 = 1.0f / (float)nm0;   // item i is (i / nm0, i % nm0); exact for i < 2^16
-                // two items per lane and round (i, i + 32): two independent chains;
-                // every item runs the central formula, the tail items' values are
-                // dropped (their denominator may vanish; nothing reads the quotient)
-                int ntail = 0;
-                const unsigned below = (1u << lane) - 1u;
-                for (int i0 = 0; i0 < items; i0 += 64) {
-                    const int ia = i0 + lane, ib = ia + 32;
-                    const float ya = ia < items ? bsm_centred_f32(w.xs[ia]) : 0.0f;
-                    const float yb = ib < items ? bsm_centred_f32(w.xs[ib]) : 0.0f;
-                    const float va = bsm_central_f32(ya), vb = bsm_central_f32(yb);
-                    const bool ta = ia < items && !(fabsf(ya) < 0.42f);
-                    const bool tb = ib < items && !(fabsf(yb) < 0.42f);
-                    if (ia < items && !ta) {
-                        const int j = (int)(((float)ia + 0.5f) * inv_nm0);
-                        w.q[j * w.qs + (ia - j * nm0)] = (T)(va * 0.70710678f);
-                    }
-                    if (ib < items && !tb) {
-                        const int j = (int)(((float)ib + 0.5f) * inv_nm0);
-                        w.q[j * w.qs + (ib - j * nm0)] = (T)(vb * 0.70710678f);
-                    }
-                    const unsigned ma = __ballot_sync(0xffffffffu, ta);
-                    if (ta) w.tl[ntail + __popc(ma & below)] = (uint16_t)ia;
-                    ntail += __popc(ma);
-                    const unsigned mb = __ballot_sync(0xffffffffu, tb);
-                    if (tb) w.tl[ntail + __popc(mb & below)] = (uint16_t)ib;
-                    ntail += __popc(mb);
-                }
-                __syncwarp();
-                for (int t = lane; t < ntail; t += 32) {
-                    const int i = w.tl[t];
-                    const int j = (int)(((float)i + 0.5f) * inv_nm0);
-                    w.q[j * w.qs + (i - j * nm0)] = (T)(bsm_tail_f32(w.xs[i]) * 0.70710678f);
-                }
-                done = true;
-            }
-        }
-        for (int j = 0; j < gn && !done; j++) {
-            const int64_t s = s0 + j;
-            T* q = w.q + j * w.qs;
-            if (s >= a.nvalid) {        // padding sample (the range's tail): contributes nothing
-                for (int d = lane; d < nm0; d += 32) q[d] = T(0);
-                continue;
-            }
-            const uint64_t idx = (uint64_t)(a.index0 + s);
-#pragma unroll
-            for (int jd = 0; jd < kDimsPerLane; jd++) {
-                const int d = lane + 32 * jd;
-                if (d >= nm0) break;
-                double y;
-                if (!sobol) {
-                    y = a.normals ? a.normals[s * nm0 + d] : (double)a.normals32[s * nm0 + d];
-                } else {
-                    if (s == s_first) st[jd] = sobol_state(a.vdir, nm0, d, idx);
-                    else st[jd] ^= (uint64_t)__ldg(a.vdir + (size_t)(__ffsll((long long)idx) - 1) * nm0 + d);
-                    const uint64_t x = a.shift ? st[jd] ^ __ldg(a.shift + d) : st[jd];
-                    y = bsm(sobol_uniform(x));
-                }
-                q[d] = (T)(y / 1.4142135623730951);   // by /= sqrt(2.0)
-            }
-            for (int d = lane + 32 * kDimsPerLane; d < nm0; d += 32) {   // beyond 128 dimensions
-                double y = sobol ? bsm(sobol_uniform((a.shift ? __ldg(a.shift + d) : 0ull) ^
-                                                     sobol_state(a.vdir, nm0, d, idx)))
-                                 : a.normals ? a.normals[s * nm0 + d] : (double)a.normals32[s * nm0 + d];
-                q[d] = (T)(y / 1.4142135623730951);
             }
         }
         __syncwarp();
@@ -360,30 +347,33 @@ __device__ __forceinline__ void samples_body(const SampleArgs& a, char* smem)
             }
         }
         __syncwarp();
-        // qTIP4P/f energies of the whole group in one warp pass
+        // 3. V and, on the gradient path (SCP3.cpp:209-216), dV/dr of the whole group in
+        // one warp pass, then dV_anh/dq = MUa^T (bohr dV/dr / autokcal) - omega % q of the
+        // group's (sample, selected mode) items over the lanes, summed in FP64
         double e4 = 0.0;
-        if constexpr (PES == SCP3GPU_PES_QTIP4PF) {
-            if (!a.skip_pes && !grad) e4 = qt::energy_warp4<T>(w.crd, N3, w.ms, nw, gn, lane);
-        }
-        if constexpr (PES == SCP3GPU_PES_QTIP4PF && sizeof(T) == 4) {
+        int iters4 = 0;
+        if (!a.skip_pes) {
             if (grad) {
-                // FP32 gradient path (the split form's products): energies and
-                // gradients of the group in one warp pass, then dV_anh/dq of the
-                // group's (sample, mode) items over the lanes, summed in FP64
-                T* g4 = reinterpret_cast<T*>(w.g);
-                T* gm4 = g4 + 4 * 9 * nw;
-                e4 = qt::energy_grad_warp4<T>(w.crd, N3, w.ms, g4, gm4, nw, gn, lane);
+                if constexpr (G) e4 = potential4<PES, T, true>(w, nw, gn, lane, &iters4);
+            } else {
+                e4 = potential4<PES, T, false>(w, nw, gn, lane, &iters4);
+            }
+        }
+        if constexpr (G) {
+            if (grad) {
                 for (int it = lane; it < gn * a.nm; it += 32) {
                     const int j = it / a.nm, m = it - j * a.nm;
+                    const int64_t s = s0 + j;
                     const int k = __ldg(a.modes + m);
-                    const T* gj = g4 + j * 9 * nw;
+                    const double* gj = w.g + j * N3;
                     double acc = 0.0;
                     if (muat_in_smem)
-                        for (int c = 0; c < N3; c++) acc += muat[(size_t)c * a.nm + m] * (double)gj[c];
+                        for (int c = 0; c < N3; c++) acc += muat[(size_t)c * a.nm + m] * gj[c];
                     else
-                        for (int c = 0; c < N3; c++) acc += MUa[(size_t)k * N3 + c] * (double)gj[c];
-                    a.vq[(s0 + j) * a.nm + m] =
-                        acc * (kBohr / kAuToKcalPerMol) - __ldg(a.omega + k) * (double)w.q[j * w.qs + k];
+                        for (int c = 0; c < N3; c++) acc += MUa[(size_t)k * N3 + c] * gj[c];
+                    a.vq[s * a.nm + m] = s < a.nvalid ? acc * (kBohr / kAuToKcalPerMol) -
+                                                            __ldg(a.omega + k) * (double)w.q[j * w.qs + k]
+                                                      : 0.0;
                 }
                 __syncwarp();
             }
@@ -391,60 +381,19 @@ __device__ __forceinline__ void samples_body(const SampleArgs& a, char* smem)
         for (int j = 0; j < gn; j++) {
             const int64_t s = s0 + j;
             const T* q = w.q + j * w.qs;
-            const T* crd = w.crd + j * N3;
-            const double e4j = __shfl_sync(0xffffffffu, e4, j);
+            const double e = __shfl_sync(0xffffffffu, e4, j);
+            const int iters = PES == SCP3GPU_PES_TTM3F ? __shfl_sync(0xffffffffu, iters4, j) : 0;
             if (s >= a.nvalid) {
                 if (lane == 0) a.v[s] = 0.0;
                 for (int m = lane; m < a.nm; m += 32) {
                     if (a.q64) a.q64[s * a.nm + m] = 0.0;
                     if (a.q32) a.q32[s * a.nm + m] = 0.0f;
-                    if (a.vq) a.vq[s * a.nm + m] = 0.0;
                 }
                 continue;
             }
-            // 3. V in hartree, anharmonic residual   (SCP3.cpp:219-223)
-            int iters = 0;
+            // V in hartree, anharmonic residual   (SCP3.cpp:219-223)
             double V = 0.0;
-            if constexpr (sizeof(T) == 8) {
-                if (grad) {
-                    // gradient path (SCP3.cpp:209-216): V and dV/dr, then
-                    // dV_anh/dq = MUa^T (bohr dV/dr / autokcal) - omega % q, selected modes
-                    double e;
-                    if constexpr (PES == SCP3GPU_PES_QTIP4PF)
-                        e = qt::energy_grad_warp(reinterpret_cast<const double*>(crd),
-                                                 reinterpret_cast<double*>(w.ms), w.g, w.gm, nw, a.tasks, a.ntasks,
-                                                 lane);
-                    else
-                        e = ttm::energy_grad_warp(reinterpret_cast<const double*>(crd),
-                                                  reinterpret_cast<double*>(w.ms), reinterpret_cast<double*>(w.ttm),
-                                                  w.g, nw, a.tasks, a.ntasks, lane, &iters);
-                    double h = 0.0;
-                    for (int d = lane; d < nm0; d += 32) h += (double)q[d] * (__ldg(a.omega + d) * (double)q[d]);
-                    h = warp_sum(h);
-                    V = e / kAuToKcalPerMol - 0.5 * h;
-                    for (int m = lane; m < a.nm; m += 32) {
-                        const int k = __ldg(a.modes + m);
-                        double acc = 0.0;
-                        if (muat_in_smem)
-                            for (int c = 0; c < N3; c++) acc += muat[(size_t)c * a.nm + m] * w.g[c];
-                        else
-                            for (int c = 0; c < N3; c++) acc += MUa[(size_t)k * N3 + c] * w.g[c];
-                        a.vq[s * a.nm + m] = acc * (kBohr / kAuToKcalPerMol) - __ldg(a.omega + k) * (double)q[k];
-                    }
-                }
-            } else if constexpr (PES == SCP3GPU_PES_QTIP4PF) {
-                if (grad) {
-                    // the FP32 form: the group's energies and dV/dq came from the
-                    // group pass above
-                    double h = 0.0;
-                    for (int d = lane; d < nm0; d += 32) h += (double)q[d] * (__ldg(a.omega + d) * (double)q[d]);
-                    h = warp_sum(h);
-                    V = e4j / kAuToKcalPerMol - 0.5 * h;
-                }
-            }
-            if (!a.skip_pes && !grad) {
-                const double e = PES == SCP3GPU_PES_QTIP4PF ? e4j
-                                                             : potential<PES, T>(crd, w, nw, a.tasks, a.ntasks, lane, &iters);
+            if (!a.skip_pes) {
                 double h = 0.0;
                 for (int d = lane; d < nm0; d += 32) h += (double)q[d] * (__ldg(a.omega + d) * (double)q[d]);
                 h = warp_sum(h);
@@ -466,125 +415,91 @@ __device__ __forceinline__ void samples_body(const SampleArgs& a, char* smem)
     }
 }
 
-template <int PES>
-__global__ void __launch_bounds__(kWarpsPerBlock * 32)
-    pes_energy_kernel(int nw, int64_t n, const double* __restrict__ crd, double* __restrict__ E,
-                      int* __restrict__ iters_out, const uint32_t* __restrict__ tasks, int ntasks)
+// Energies (and with G gradients) of n geometries, FP64, NG per warp (four; two for TTM3-F
+// with more than eight waters); one warp per CTA, so that a few geometries (a Hessian's
+// 2N) spread over the SMs.
+template <int PES, bool G, int NG = kGroup>
+__global__ void __launch_bounds__(32) pes_kernel(int nw, int64_t n, const double* __restrict__ crd,
+                                                 double* __restrict__ E, double* __restrict__ grad,
+                                                 int* __restrict__ iters_out)
 {
     extern __shared__ __align__(16) char smem[];
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    WarpSlot<double> w = warp_slot<double>(smem + wib * slot_bytes<double>(PES, 0, nw), PES, 0, nw);
-    const int64_t nwarps = (int64_t)gridDim.x * kWarpsPerBlock;
-    for (int64_t g = (int64_t)blockIdx.x * kWarpsPerBlock + wib; g < n; g += nwarps) {
-        for (int c = lane; c < 9 * nw; c += 32) w.crd[c] = crd[g * 9 * nw + c];
+    const int lane = threadIdx.x, N3 = 9 * nw;
+    const WarpSlot<double> w = warp_slot<double>(smem, 0, nw, G);
+    for (int64_t g0 = (int64_t)blockIdx.x * NG; g0 < n; g0 += (int64_t)gridDim.x * NG) {
+        const int gn = (int)(n - g0 < NG ? n - g0 : NG);
+        for (int c = lane; c < gn * N3; c += 32) w.crd[c] = crd[g0 * N3 + c];
         __syncwarp();
         int iters = 0;
-        const double e = potential<PES, double>(w.crd, w, nw, tasks, ntasks, lane, &iters);
-        if (lane == 0) {
-            E[g] = e;
-            if (iters_out) iters_out[g] = iters;
+        const double e = potential4<PES, double, G, NG>(w, nw, gn, lane, &iters);
+        if (lane < gn) {
+            E[g0 + lane] = e;
+            if (iters_out) iters_out[g0 + lane] = iters;
         }
+        if (G)
+            for (int c = lane; c < gn * N3; c += 32) grad[g0 * N3 + c] = w.g[c];
         __syncwarp();
     }
 }
 
-// qTIP4P/f energy and gradient of n geometries, one warp each (the E+g operator,
-// qtip4pf.cpp:252-397).
-template <int PES>
-__global__ void __launch_bounds__(kWarpsPerBlock * 32)
-    pes_energy_grad_kernel(int nw, int64_t n, const double* __restrict__ crd, double* __restrict__ E,
-                           double* __restrict__ G, int* __restrict__ iters_out, const uint32_t* __restrict__ tasks,
-                           int ntasks)
-{
-    extern __shared__ __align__(16) double gsm[];
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    const size_t per = 24 * (size_t)nw + (PES == SCP3GPU_PES_TTM3F ? ttm::scratch_elems(nw, true) : 0);
-    double* x = gsm + (size_t)wib * per;
-    double *ms = x + 9 * nw, *g = ms + 3 * nw, *gm = g + 9 * nw, *sc = gm + 3 * nw;
-    const int64_t nwarps = (int64_t)gridDim.x * kWarpsPerBlock;
-    for (int64_t k = (int64_t)blockIdx.x * kWarpsPerBlock + wib; k < n; k += nwarps) {
-        for (int c = lane; c < 9 * nw; c += 32) x[c] = crd[k * 9 * nw + c];
-        __syncwarp();
-        int iters = 0;
-        double e;
-        if constexpr (PES == SCP3GPU_PES_QTIP4PF) e = qt::energy_grad_warp(x, ms, g, gm, nw, tasks, ntasks, lane);
-        else e = ttm::energy_grad_warp(x, ms, sc, g, nw, tasks, ntasks, lane, &iters);
-        if (lane == 0) {
-            E[k] = e;
-            if (iters_out) iters_out[k] = iters;
-        }
-        for (int c = lane; c < 9 * nw; c += 32) G[k * 9 * nw + c] = g[c];
-        __syncwarp();
-    }
-}
-
-// SCP1 per-sample stage (SCP1.cpp:52-63): one warp per sample, contiguous
-// balanced ranges per warp with the Gray-code Sobol walk, isqrtM_U staged in
-// shared memory, the potential's energy and gradient (the gradient estimator's
-// warp code).
+// SCP1 per-sample stage (SCP1.cpp:52-63): contiguous balanced sample ranges per warp with
+// the Gray-code Sobol walk, in groups of four samples as the builds' per-sample kernel;
+// isqrtM_U staged in shared memory.
 constexpr int kS1Warps = 8;
 
 __host__ __device__ inline size_t scp1_slot(int pes, int nw, int dim)
 {
-    return 2 * (size_t)dim + 24 * (size_t)nw + (pes == SCP3GPU_PES_TTM3F ? ttm::scratch_elems(nw, true) : 0);
+    return slot_bytes<double>(pes, dim, nw, true) + sizeof(double) * kGroup * (size_t)dim;
 }
 
 template <int PES>
-__global__ void __launch_bounds__(kS1Warps * 32) scp1_samples_kernel(Scp1Args a)
+__global__ void __launch_bounds__(kS1Warps * 32, PES == SCP3GPU_PES_TTM3F ? 1 : 2) scp1_samples_kernel(Scp1Args a)
 {
     extern __shared__ __align__(16) double s1[];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const int nw = a.nw, dim = a.dim;
     double* U = s1;
     for (int e = threadIdx.x; e < dim * dim; e += blockDim.x) U[e] = a.U[e];
-    double* y = s1 + (size_t)dim * dim + (size_t)wib * scp1_slot(PES, nw, dim);
-    double* dq = y + dim;
-    double* x = dq + dim;
-    double* ms = x + 9 * nw;
-    double* g = ms + 3 * nw;
-    double* gm = g + 9 * nw;
-    double* sc = gm + 3 * nw;
+    char* slot = reinterpret_cast<char*>(s1) + round16(sizeof(double) * dim * dim) + (size_t)wib * scp1_slot(PES, nw, dim);
+    const WarpSlot<double> w = warp_slot<double>(slot, dim, nw, true);      // w.q: y = std_normal % sqrt(d)
+    double* dq = reinterpret_cast<double*>(slot + slot_bytes<double>(PES, dim, nw, true));   // [group][dim]
     __syncthreads();
     const int64_t nwarps = (int64_t)gridDim.x * kS1Warps;
     const int64_t gw = (int64_t)blockIdx.x * kS1Warps + wib;
     const int64_t s_first = a.n * gw / nwarps, s_end = a.n * (gw + 1) / nwarps;
-    constexpr int kDimsPerLane = 4;
     uint64_t st[kDimsPerLane];
-    for (int64_t s = s_first; s < s_end; s++) {
-        const uint64_t idx = (uint64_t)(a.index0 + s);
+    for (int64_t s0 = s_first; s0 < s_end; s0 += kGroup) {
+        const int gn = (int)(s_end - s0 < kGroup ? s_end - s0 : kGroup);
         // y = std_normal % sqrt(d)   (SCP1.cpp:54-58)
-#pragma unroll
-        for (int jd = 0; jd < kDimsPerLane; jd++) {
-            const int d = lane + 32 * jd;
-            if (d >= dim) break;
-            if (s == s_first) st[jd] = sobol_state(a.vdir, dim, d, idx);
-            else st[jd] ^= (uint64_t)__ldg(a.vdir + (size_t)(__ffsll((long long)idx) - 1) * dim + d);
-            y[d] = bsm(sobol_uniform(st[jd])) * __ldg(a.sqd + d);
-        }
-        for (int d = lane + 32 * kDimsPerLane; d < dim; d += 32)
-            y[d] = bsm(sobol_uniform(sobol_state(a.vdir, dim, d, idx))) * __ldg(a.sqd + d);
+        group_normals<double>(a.vdir, nullptr, dim, a.index0, s0, s_first, a.n, gn, st, w.xs, w.tl, lane,
+                              [&](int j, int d, double y) { w.q[j * w.qs + d] = y * __ldg(a.sqd + d); });
         __syncwarp();
         // dq = isqrtM_U y, r = bohr (q + dq)   (SCP1.cpp:60-61), k in order
         for (int c = lane; c < dim; c += 32) {
-            double acc = 0.0;
-            for (int k = 0; k < dim; k++) acc += U[(size_t)k * dim + c] * y[k];
-            dq[c] = acc;
-            x[c] = kBohr * (__ldg(a.q + c) + acc);
+            double acc[kGroup] = {};
+            for (int k = 0; k < dim; k++) {
+                const double u = U[(size_t)k * dim + c];
+#pragma unroll
+                for (int j = 0; j < kGroup; j++) acc[j] += u * w.q[j * w.qs + k];   // past gn: stale, not used
+            }
+            const double q0 = __ldg(a.q + c);
+#pragma unroll
+            for (int j = 0; j < kGroup; j++) {
+                if (j >= gn) break;
+                dq[j * dim + c] = acc[j];
+                w.crd[j * dim + c] = kBohr * (q0 + acc[j]);
+            }
         }
         __syncwarp();
         int it = 0;
-        double e;
-        if constexpr (PES == SCP3GPU_PES_QTIP4PF)
-            e = qt::energy_grad_warp(x, ms, g, gm, nw, a.tasks, a.ntasks, lane);
-        else
-            e = ttm::energy_grad_warp(x, ms, sc, g, nw, a.tasks, a.ntasks, lane, &it);
-        if (lane == 0) {
-            a.V[s] = e / kAuToKcalPerMol;
-            if (a.iters) a.iters[s] = it;
+        const double e = potential4<PES, double, true>(w, nw, gn, lane, &it);
+        if (lane < gn) {
+            a.V[s0 + lane] = e / kAuToKcalPerMol;
+            if (it > kTtmMaxIter) atomicAdd(a.not_converged, 1ull);
         }
-        for (int c = lane; c < dim; c += 32) {
-            a.G[s * dim + c] = g[c] * (kBohr / kAuToKcalPerMol);    // UX_ *= bohr/autokcalpmol
-            a.D[s * dim + c] = dq[c];
+        for (int c = lane; c < gn * dim; c += 32) {
+            a.G[s0 * dim + c] = w.g[c] * (kBohr / kAuToKcalPerMol);    // UX_ *= bohr/autokcalpmol
+            a.D[s0 * dim + c] = dq[c];
         }
         __syncwarp();
     }
@@ -632,9 +547,11 @@ int launch_samples_t(const SampleArgs& a, cudaStream_t s)
 {
     const size_t mua_b = mua_smem_bytes<T>(a.nw, a.nm0);
     const size_t muat_b = muat_smem_bytes(a.nw, a.nm);
-    const size_t sm = kWarpsPerBlock * slot_bytes<T>(PES, a.nm0, a.nw, a.vq != nullptr, kGroup) +
+    const size_t sm = kWarpsPerBlock * slot_bytes<T>(PES, a.nm0, a.nw, a.vq != nullptr) +
                       (mua_b <= kMuaSmemMax ? mua_b : 0) + (a.vq && muat_b <= kMuaTSmemMax ? muat_b : 0);
-    auto kern = a.vq ? samples_kernel<PES, T, true> : samples_kernel<PES, T, false>;
+    // the FP32 gradient is qTIP4P/f's only (launch_samples)
+    constexpr bool kGrad = PES == SCP3GPU_PES_QTIP4PF || sizeof(T) == 8;
+    auto kern = a.vq ? samples_kernel<PES, T, kGrad> : samples_kernel<PES, T, false>;
     if (sm > 48 * 1024) SCP3_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
     kern<<<sample_grid(kern, sm, a.n), kWarpsPerBlock * 32, sm, s>>>(a);
     SCP3_CUDA(cudaGetLastError());
@@ -655,7 +572,7 @@ int launch_samples_batch_t(const SampleArgs* args_host, const SampleArgs* args_d
         const size_t b = mua_smem_bytes<T>(args_host[c].nw, args_host[c].nm0);
         if (b <= kMuaSmemMax) mua = std::max(mua, b);
     }
-    const size_t sm = kWarpsPerBlock * slot_bytes<T>(PES, nm0, nw, false, kGroup) + mua;
+    const size_t sm = kWarpsPerBlock * slot_bytes<T>(PES, nm0, nw, false) + mua;
     if (sm > 48 * 1024) SCP3_CUDA(cudaFuncSetAttribute(samples_batch_kernel<PES, T>,
                                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
     const int per = grid_for((n + kRun - 1) / kRun);   // per cluster; the clusters share the SMs
@@ -689,25 +606,31 @@ int ttm_init_device()
     if (dev < 0 || dev >= 128) return fail(SCP3GPU_ERR_ARG, "device ordinal out of range");
     if (done[dev]) return SCP3GPU_OK;
     ttm::Consts c;
-    c.AA_HH = std::pow(0.496 * 0.496, 1.0 / 6.0);
-    c.AA_HM = std::pow(0.496 * 0.837, 1.0 / 6.0);
-    c.AA_MM = std::pow(0.837 * 0.837, 1.0 / 6.0);
+    c.iAA_HH = 1.0 / std::pow(0.496 * 0.496, 1.0 / 6.0);
+    c.iAA_HM = 1.0 / std::pow(0.496 * 0.837, 1.0 / 6.0);
+    c.iAA_MM = 1.0 / std::pow(0.837 * 0.837, 1.0 / 6.0);
     c.aXX13 = std::pow(0.175, 1.0 / 3.0);
-    for (int i = 0; i < 245; i++)   // ps.cpp:508-511: f5z, fbasis, fcore, frest
-        c.c5z[i] = 0.999677885 * scp3_ps_c5zA[i] + 0.15860145369897 * scp3_ps_cbasis[i] +
-                   -1.6351695982132 * scp3_ps_ccore[i] + 1.0 * scp3_ps_crest[i];
     c.phh1 = 0.999677885 * 16.94879431193463 * std::exp(12.66426998162947);
-    for (int i = 0; i < 84; i++) c.coefD[i] = scp3_ps_coefD[i];
-    for (int i = 0; i < 245; i++) {
-        c.idx1[i] = scp3_ps_idx1[i];
-        c.idx2[i] = scp3_ps_idx2[i];
-        c.idx3[i] = scp3_ps_idx3[i];
+    for (int i = 0; i < ttm::kETerms; i++) {   // ps.cpp:508-511: f5z, fbasis, fcore, frest
+        const double c5z = 0.999677885 * scp3_ps_c5zA[i] + 0.15860145369897 * scp3_ps_cbasis[i] +
+                           -1.6351695982132 * scp3_ps_ccore[i] + 1.0 * scp3_ps_crest[i];
+        const int I = scp3_ps_idx1[i] - 1, J = scp3_ps_idx2[i] - 1, K = scp3_ps_idx3[i] - 1;
+        if (i == 0) c.c5z0 = c5z;
+        c.e[ttm::e_offset(I, J) + K] = i ? c5z : 0.0;
     }
-    for (int i = 0; i < 84; i++) {
-        c.idxD0[i] = scp3_ps_idxD0[i];
-        c.idxD1[i] = scp3_ps_idxD1[i];
-        c.idxD2[i] = scp3_ps_idxD2[i];
+    for (int i = 0; i < ttm::kDTerms; i++) {
+        const int I = scp3_ps_idxD0[i] - 1, J = scp3_ps_idxD1[i] - 1, K = scp3_ps_idxD2[i] - 1;
+        if (i == 0) c.coefD0 = scp3_ps_coefD[i];
+        c.d[ttm::d_offset(I, J) + K] = i ? scp3_ps_coefD[i] : 0.0;
     }
+    double ser = 1.0;
+    for (int n = 0; n < 36; n++) c.s[n] = ser /= 2.0 / 3.0 + n;
+    for (int i = 0; i < ttm::kETerms; i++) c.ef[i] = (float)c.e[i];
+    for (int i = 0; i < ttm::kDTerms; i++) c.df[i] = (float)c.d[i];
+    for (int n = 0; n < 36; n++) c.sf[n] = (float)c.s[n];
+    ttm::TailTable tail;
+    ttm::tail_tables(tail);
+    SCP3_CUDA(cudaMemcpyToSymbol(ttm::kTail, &tail, sizeof(tail)));
     SCP3_CUDA(cudaMemcpyToSymbol(ttm::kC, &c, sizeof(c)));
     done[dev] = true;
     return SCP3GPU_OK;
@@ -727,16 +650,25 @@ int launch_samples(int pes, bool fp32, const SampleArgs& a, cudaStream_t s)
     return fail(SCP3GPU_ERR_ARG, "unknown potential id");
 }
 
-int launch_pes_energy_grad(int pes, int nw, int64_t n, const double* crd, double* E, double* G, int* iters,
-                           const uint32_t* tasks, int ntasks, cudaStream_t s)
+int launch_pes(int pes, int nw, int64_t n, const double* crd, double* E, double* G, int* iters, cudaStream_t s)
 {
     if (n <= 0) return SCP3GPU_OK;
-    const bool ttm = pes == SCP3GPU_PES_TTM3F;
-    const size_t per = 24 * (size_t)nw + (ttm ? ttm::scratch_elems(nw, true) : 0);
-    const size_t sm = sizeof(double) * kWarpsPerBlock * per;
-    auto kern = ttm ? pes_energy_grad_kernel<SCP3GPU_PES_TTM3F> : pes_energy_grad_kernel<SCP3GPU_PES_QTIP4PF>;
-    if (sm > 48 * 1024) SCP3_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-    kern<<<grid_for(n), kWarpsPerBlock * 32, sm, s>>>(nw, n, crd, E, G, iters, tasks, ntasks);
+    if (pes != SCP3GPU_PES_QTIP4PF && pes != SCP3GPU_PES_TTM3F) return fail(SCP3GPU_ERR_ARG, "unknown potential id");
+    const size_t sm = slot_bytes<double>(pes, 0, nw, G != nullptr);      // under 32 KB at 16 waters
+    auto kern = pes == SCP3GPU_PES_TTM3F
+                    ? (G ? pes_kernel<SCP3GPU_PES_TTM3F, true> : pes_kernel<SCP3GPU_PES_TTM3F, false>)
+                    : (G ? pes_kernel<SCP3GPU_PES_QTIP4PF, true> : pes_kernel<SCP3GPU_PES_QTIP4PF, false>);
+    int ng = kGroup;
+    if (pes == SCP3GPU_PES_TTM3F && nw > 8) {
+        if (G) return fail(SCP3GPU_ERR_ARG, "TTM3-F gradients: at most 8 waters");
+        kern = pes_kernel<SCP3GPU_PES_TTM3F, false, 2>;
+        ng = 2;
+    }
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const unsigned grid = (unsigned)std::min<int64_t>((n + ng - 1) / ng, (int64_t)sms * 32);
+    kern<<<grid, 32, sm, s>>>(nw, n, crd, E, G, iters);
     SCP3_CUDA(cudaGetLastError());
     return SCP3GPU_OK;
 }
@@ -745,7 +677,7 @@ int launch_scp1_samples(int pes, const Scp1Args& a, cudaStream_t s)
 {
     if (a.n <= 0) return SCP3GPU_OK;
     if (pes != SCP3GPU_PES_QTIP4PF && pes != SCP3GPU_PES_TTM3F) return fail(SCP3GPU_ERR_ARG, "unknown potential id");
-    const size_t sm = sizeof(double) * ((size_t)a.dim * a.dim + kS1Warps * scp1_slot(pes, a.nw, a.dim));
+    const size_t sm = round16(sizeof(double) * a.dim * a.dim) + kS1Warps * scp1_slot(pes, a.nw, a.dim);
     auto kern = pes == SCP3GPU_PES_QTIP4PF ? scp1_samples_kernel<SCP3GPU_PES_QTIP4PF>
                                             : scp1_samples_kernel<SCP3GPU_PES_TTM3F>;
     SCP3_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
@@ -756,27 +688,6 @@ int launch_scp1_samples(int pes, const Scp1Args& a, cudaStream_t s)
     const int64_t want = (a.n + 4 * kS1Warps - 1) / (4 * kS1Warps);     // >= 4 samples per warp
     const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(want, (int64_t)per * sms));
     kern<<<grid, kS1Warps * 32, sm, s>>>(a);
-    SCP3_CUDA(cudaGetLastError());
-    return SCP3GPU_OK;
-}
-
-int launch_pes_energy(int pes, int nw, int64_t n, const double* crd, double* E, int* iters, const uint32_t* tasks,
-                      int ntasks, cudaStream_t s)
-{
-    if (n <= 0) return SCP3GPU_OK;
-    const size_t sm = kWarpsPerBlock * slot_bytes<double>(pes, 0, nw);
-    if (pes == SCP3GPU_PES_QTIP4PF) {
-        pes_energy_kernel<SCP3GPU_PES_QTIP4PF><<<grid_for(n), kWarpsPerBlock * 32, sm, s>>>(nw, n, crd, E, iters,
-                                                                                          tasks, ntasks);
-    } else if (pes == SCP3GPU_PES_TTM3F) {
-        if (sm > 48 * 1024)
-            SCP3_CUDA(cudaFuncSetAttribute(pes_energy_kernel<SCP3GPU_PES_TTM3F>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-        pes_energy_kernel<SCP3GPU_PES_TTM3F><<<grid_for(n), kWarpsPerBlock * 32, sm, s>>>(nw, n, crd, E, iters,
-                                                                                        tasks, ntasks);
-    } else {
-        return fail(SCP3GPU_ERR_ARG, "unknown potential id");
-    }
     SCP3_CUDA(cudaGetLastError());
     return SCP3GPU_OK;
 }

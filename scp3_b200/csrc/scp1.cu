@@ -35,8 +35,6 @@ struct scp3gpu_scp1 {
     int blocks = 0;                 // reduction blocks (fixed per handle)
     cudaStream_t stream = nullptr;
     int64_t* vdir = nullptr;        // [62][dim] direction numbers
-    uint32_t* tasks = nullptr;
-    int ntasks = 0;
     double* q = nullptr;            // [dim]
     double* sqd = nullptr;          // [dim] sqrt(d)
     double* U = nullptr;            // [dim*dim] isqrtM_U, column-major
@@ -45,7 +43,7 @@ struct scp3gpu_scp1 {
     double* D = nullptr;            // [chunk][dim]
     double* P = nullptr;            // [blocks][(dim+1)^2] block partials
     double* R = nullptr;            // [(dim+1)^2]
-    int* iters = nullptr;           // [chunk] TTM3-F dipole iterations
+    unsigned long long* capped = nullptr;   // [1] TTM3-F samples at the sweep cap, all calls
     long long not_converged = 0;
 };
 
@@ -108,7 +106,7 @@ __global__ void scp1_sum_kernel(int E, int blocks, const double* __restrict__ P,
 
 void free_all(scp3gpu_scp1* h)
 {
-    void* p[] = {h->vdir, h->tasks, h->q, h->sqd, h->U, h->V, h->G, h->D, h->P, h->R, h->iters};
+    void* p[] = {h->vdir, h->q, h->sqd, h->U, h->V, h->G, h->D, h->P, h->R, h->capped};
     for (void* x : p)
         if (x) cudaFree(x);
     if (h->stream) cudaStreamDestroy(h->stream);
@@ -145,18 +143,17 @@ int scp3gpu_scp1_create(int pes, int nw, int64_t chunk, int device, scp3gpu_scp1
     const int dim = h->dim, E = (dim + 1) * (dim + 1);
     std::vector<int64_t> v;
     std::vector<uint64_t> sh;
-    const std::vector<uint32_t> t = pair_tasks(nw);
-    h->ntasks = (int)t.size();
     if ((rc = sobol_tables(dim, 0, 0, v, sh)) || (rc = upload(&h->vdir, v.data(), v.size())) ||
-        (rc = upload(&h->tasks, t.data(), t.size())) || (rc = dalloc(&h->q, dim)) || (rc = dalloc(&h->sqd, dim)) ||
+        (rc = dalloc(&h->q, dim)) || (rc = dalloc(&h->sqd, dim)) ||
         (rc = dalloc(&h->U, (size_t)dim * dim)) || (rc = dalloc(&h->V, h->chunk)) ||
         (rc = dalloc(&h->G, (size_t)h->chunk * dim)) || (rc = dalloc(&h->D, (size_t)h->chunk * dim)) ||
-        (rc = dalloc(&h->P, (size_t)h->blocks * E)) || (rc = dalloc(&h->R, E)) || (rc = dalloc(&h->iters, h->chunk))) {
+        (rc = dalloc(&h->P, (size_t)h->blocks * E)) || (rc = dalloc(&h->R, E)) || (rc = dalloc(&h->capped, 1))) {
         free_all(h);
         delete h;
         return rc;
     }
-    if (cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) != cudaSuccess) {
+    if (cudaMemset(h->capped, 0, sizeof(*h->capped)) != cudaSuccess ||
+        cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) != cudaSuccess) {
         free_all(h);
         delete h;
         return fail(SCP3GPU_ERR_CUDA, "scp1: stream creation failed");
@@ -185,28 +182,24 @@ int scp3gpu_scp1_average(scp3gpu_scp1* h, const double* q, const double* d, cons
     SCP3_CUDA(cudaMemcpyAsync(h->sqd, sqd.data(), sizeof(double) * dim, cudaMemcpyHostToDevice, s));
     SCP3_CUDA(cudaMemcpyAsync(h->U, isqrtM_U, sizeof(double) * dim * dim, cudaMemcpyHostToDevice, s));
     SCP3_CUDA(cudaMemsetAsync(h->P, 0, sizeof(double) * (size_t)h->blocks * E, s));
-    std::vector<int> it;
     int rc = SCP3GPU_OK;
     for (int64_t c0 = i0; c0 < i1; c0 += h->chunk) {
         const int64_t n = std::min<int64_t>(h->chunk, i1 - c0);
-        Scp1Args a{h->nw, dim, h->q, h->sqd, h->U, h->vdir, skip + c0, n, h->tasks, h->ntasks, h->V, h->G, h->D,
-                   h->iters};
+        Scp1Args a{h->nw, dim, h->q, h->sqd, h->U, h->vdir, skip + c0, n, h->V, h->G, h->D, h->capped};
         if ((rc = launch_scp1_samples(h->pes, a, s))) return rc;
         const int pages = (E + kRedThreads * kRedPer - 1) / (kRedThreads * kRedPer);
         scp1_reduce_kernel<<<dim3(h->blocks, pages), kRedThreads, 0, s>>>(dim, n, h->V, h->G, h->D, h->P);
         SCP3_CUDA(cudaGetLastError());
-        if (h->pes == SCP3GPU_PES_TTM3F) {
-            it.resize(n);
-            SCP3_CUDA(cudaMemcpyAsync(it.data(), h->iters, sizeof(int) * n, cudaMemcpyDeviceToHost, s));
-            SCP3_CUDA(cudaStreamSynchronize(s));
-            for (int64_t k = 0; k < n; k++) h->not_converged += it[k] > kTtmMaxIter;
-        }
     }
     scp1_sum_kernel<<<(E + 255) / 256, 256, 0, s>>>(E, h->blocks, h->P, h->R);
     SCP3_CUDA(cudaGetLastError());
     std::vector<double> R(E);
+    unsigned long long capped = 0;
     SCP3_CUDA(cudaMemcpyAsync(R.data(), h->R, sizeof(double) * E, cudaMemcpyDeviceToHost, s));
+    if (h->pes == SCP3GPU_PES_TTM3F)
+        SCP3_CUDA(cudaMemcpyAsync(&capped, h->capped, sizeof(capped), cudaMemcpyDeviceToHost, s));
     SCP3_CUDA(cudaStreamSynchronize(s));
+    h->not_converged = (long long)capped;
     for (int j = 0; j < dim; j++)
         for (int i = 0; i < dim; i++) UX_q[(size_t)j * dim + i] = R[(size_t)j * E1 + i];
     for (int i = 0; i < dim; i++) UX[i] = R[(size_t)dim * E1 + i];

@@ -1,5 +1,5 @@
 // Host-side tables of the build: Sobol direction numbers (+ scramble), basis
-// descriptors and pair tasks of the water potentials.
+// descriptors.
 #include <cstring>
 
 #include "internal.h"
@@ -96,29 +96,6 @@ std::vector<uint32_t> basis_descriptors(int nm, int n2, int n3)
         for (int n = m + 1; n < n3; n++)
             for (int p = n + 1; p < n3; p++) put(kHo1Ho1Ho1, m, n, p);
     return d;
-}
-
-// Same pair set as the reference's loops (qtip4pf.cpp:213-283, ttm3f.cpp:144-257):
-// for every ordered i != j the two H of j against the M site of i, and for i < j
-// the four H/H pairs, O/O and M/M.
-std::vector<uint32_t> pair_tasks(int nw)
-{
-    std::vector<uint32_t> t;
-    auto put = [&](uint32_t type, int a, int b) { t.push_back(type | ((uint32_t)a << 2) | ((uint32_t)b << 17)); };
-    // grouped by type so that the lanes of a warp mostly take the same branch
-    for (int i = 0; i < nw; i++)
-        for (int j = 0; j < nw; j++)
-            if (i != j)
-                for (int l = 1; l < 3; l++) put(0, i, 3 * j + l);
-    for (int i = 0; i < nw; i++)
-        for (int j = i + 1; j < nw; j++)
-            for (int a = 1; a < 3; a++)
-                for (int b = 1; b < 3; b++) put(1, 3 * i + a, 3 * j + b);
-    for (int i = 0; i < nw; i++)
-        for (int j = i + 1; j < nw; j++) put(2, 3 * i, 3 * j);
-    for (int i = 0; i < nw; i++)
-        for (int j = i + 1; j < nw; j++) put(3, i, j);
-    return t;
 }
 
 // Each basis function as a product of three entries of a per-sample table
