@@ -544,10 +544,7 @@ int scp3gpu_batch_read(scp3gpu_batch* b, int c, double* M, int64_t ld, int mode)
                             mode == 1 ? (double)b->count : 1.0, mode == 1 ? k.hodiag : nullptr,
                             mode == 1 ? k.zpe_inactive : 0.0, b->dense, k.nb, b->stream);
     if (rc) return rc;
-    SCP3_CUDA(cudaMemcpy2DAsync(M, sizeof(double) * ld, b->dense, sizeof(double) * k.nb, sizeof(double) * k.nb, k.nb,
-                                cudaMemcpyDeviceToHost, b->stream));
-    SCP3_CUDA(cudaStreamSynchronize(b->stream));
-    return SCP3GPU_OK;
+    return staging::copy_out(M, sizeof(double) * ld, b->dense, sizeof(double) * k.nb, (size_t)k.nb, b->stream);
 }
 
 int scp3gpu_batch_status(scp3gpu_batch* b, int c, int64_t* nonfinite, int64_t* not_converged)

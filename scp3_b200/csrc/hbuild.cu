@@ -367,6 +367,50 @@ int scp3gpu_pes_energy_dev(int pes, int nw, int64_t n, const double* crd_dev, do
     return SCP3GPU_OK;
 }
 
+// Energies (and gradients) of host geometries on the legacy default stream of the current
+// device.  Small calls (a Hessian's 2N gradients) go through a slot of the transfer pool:
+// no allocation, one copy each way.
+static int host_pes(int pes, int nw, int64_t n, const double* crd, double* E, double* grad, int* it)
+{
+    const size_t xb = sizeof(double) * (size_t)n * 9 * nw, eb = sizeof(double) * (size_t)n, gb = grad ? xb : 0,
+                 ib = sizeof(int) * (size_t)n, total = xb + gb + eb + ib;
+    staging::Slot slot;
+    char* d = nullptr;
+    const bool pooled = total <= staging::kScratchMax;
+    int rc = pooled ? slot.acquire() : SCP3GPU_OK;
+    if (!rc) rc = pooled ? slot.scratch(total, &d) : dalloc(&d, total);
+    if (rc) return rc;
+    // geometries, then gradients, energies, sweeps
+    double *dx = (double*)d, *dg = (double*)(d + xb), *de = (double*)(d + xb + gb);
+    int* di = (int*)(d + xb + gb + eb);
+    auto body = [&]() -> int {
+        const bool small = total <= staging::kPinned;
+        if (small) {
+            std::memcpy(slot.pinned(), crd, xb);
+            SCP3_CUDA(cudaMemcpyAsync(dx, slot.pinned(), xb, cudaMemcpyHostToDevice, 0));
+        } else {
+            SCP3_CUDA(cudaMemcpy(dx, crd, xb, cudaMemcpyHostToDevice));
+        }
+        if (int r = launch_pes(pes, nw, n, dx, de, grad ? dg : nullptr, di, 0)) return r;
+        if (small) {
+            char* p = slot.pinned();
+            SCP3_CUDA(cudaMemcpyAsync(p, dg, gb + eb + ib, cudaMemcpyDeviceToHost, 0));
+            SCP3_CUDA(cudaStreamSynchronize(0));
+            if (grad) std::memcpy(grad, p, gb);
+            std::memcpy(E, p + gb, eb);
+            std::memcpy(it, p + gb + eb, ib);
+            return SCP3GPU_OK;
+        }
+        int r = grad ? staging::copy_out(grad, gb / n, dg, gb / n, (size_t)n, 0) : SCP3GPU_OK;
+        if (!r) r = staging::copy_out(E, sizeof(double), de, sizeof(double), (size_t)n, 0);
+        return r ? r : staging::copy_out(it, sizeof(int), di, sizeof(int), (size_t)n, 0);
+    };
+    rc = body();
+    if (rc) cudaStreamSynchronize(0);        // nothing of the slot in flight when it goes back
+    if (!pooled) cudaFree(d);
+    return rc;
+}
+
 int scp3gpu_pes_energy(int pes, int nw, int64_t n, const double* crd, double* E, int* iters)
 {
     (void)cudaGetLastError();   // a pending error of an earlier, unrelated call is not this call's
@@ -379,22 +423,8 @@ int scp3gpu_pes_energy(int pes, int nw, int64_t n, const double* crd, double* E,
     int rc = check_device(dev);
     if (rc) return rc;
     if (pes == SCP3GPU_PES_TTM3F && (rc = ttm_init_device())) return rc;
-    double *cd = nullptr, *ed = nullptr;
-    int* id = nullptr;
-    if ((rc = upload(&cd, crd, (size_t)n * 9 * nw)) ||
-        (rc = dalloc(&ed, (size_t)n)) || (rc = dalloc(&id, (size_t)n))) {
-        cudaFree(cd), cudaFree(ed), cudaFree(id);
-        return rc;
-    }
-    rc = launch_pes(pes, nw, n, cd, ed, nullptr, id, 0);
     std::vector<int> it(n);
-    if (!rc) {
-        cudaError_t e = cudaMemcpy(E, ed, sizeof(double) * n, cudaMemcpyDeviceToHost);
-        if (e == cudaSuccess) e = cudaMemcpy(it.data(), id, sizeof(int) * n, cudaMemcpyDeviceToHost);
-        if (e != cudaSuccess) rc = cuda_fail(e, "pes_energy copy-out");
-    }
-    cudaFree(cd), cudaFree(ed), cudaFree(id);
-    if (rc) return rc;
+    if ((rc = host_pes(pes, nw, n, crd, E, nullptr, it.data()))) return rc;
     bool capped = false;
     for (int64_t k = 0; k < n; k++) {
         if (iters) iters[k] = it[k];
@@ -416,23 +446,8 @@ int scp3gpu_pes_energy_grad(int pes, int nw, int64_t n, const double* crd, doubl
     int rc = check_device(dev);
     if (rc) return rc;
     if (pes == SCP3GPU_PES_TTM3F && (rc = ttm_init_device())) return rc;
-    double *cd = nullptr, *ed = nullptr, *gd = nullptr;
-    int* id = nullptr;
-    if ((rc = upload(&cd, crd, (size_t)n * 9 * nw)) ||
-        (rc = dalloc(&ed, (size_t)n)) || (rc = dalloc(&gd, (size_t)n * 9 * nw)) || (rc = dalloc(&id, (size_t)n))) {
-        cudaFree(cd), cudaFree(ed), cudaFree(gd), cudaFree(id);
-        return rc;
-    }
-    rc = launch_pes(pes, nw, n, cd, ed, gd, id, 0);
     std::vector<int> it(n);
-    if (!rc) {
-        cudaError_t e = cudaMemcpy(E, ed, sizeof(double) * n, cudaMemcpyDeviceToHost);
-        if (e == cudaSuccess) e = cudaMemcpy(grad, gd, sizeof(double) * n * 9 * nw, cudaMemcpyDeviceToHost);
-        if (e == cudaSuccess) e = cudaMemcpy(it.data(), id, sizeof(int) * n, cudaMemcpyDeviceToHost);
-        if (e != cudaSuccess) rc = cuda_fail(e, "pes_energy_grad copy-out");
-    }
-    cudaFree(cd), cudaFree(ed), cudaFree(gd), cudaFree(id);
-    if (rc) return rc;
+    if ((rc = host_pes(pes, nw, n, crd, E, grad, it.data()))) return rc;
     for (int64_t k = 0; k < n; k++)
         if (it[k] > kTtmMaxIter) return fail(SCP3GPU_ERR_NOT_CONVERGED, "TTM3-F dipoles hit the iteration cap");
     return SCP3GPU_OK;
@@ -756,11 +771,9 @@ int scp3gpu_hbuild_read(scp3gpu_hbuild* h, double* M, int64_t ld, int mode)
     DeviceGuard g(h->dev);
     int rc = build_dense(h, mode);
     if (rc) return rc;
-    SCP3_CUDA(cudaMemcpy2DAsync(M, sizeof(double) * ld, h->dense, sizeof(double) * h->nb, sizeof(double) * h->nb,
-                                h->nb, cudaMemcpyDeviceToHost, h->stream));
-    if (const i8::Plan* p = integer_plan(h)) return i8::check(*p, h->stream);
-    SCP3_CUDA(cudaStreamSynchronize(h->stream));
-    return SCP3GPU_OK;
+    rc = staging::copy_out(M, sizeof(double) * ld, h->dense, sizeof(double) * h->nb, (size_t)h->nb, h->stream);
+    if (!rc && integer_plan(h)) rc = i8::check(*integer_plan(h), h->stream);
+    return rc;
 }
 
 int scp3gpu_hbuild_read_dev(scp3gpu_hbuild* h, double* M_dev, int64_t ld, int mode)

@@ -8,6 +8,7 @@
 
 #include "../../include/scp3gpu.h"
 #include "contract_i8.h"
+#include "staging.h"
 
 namespace scp3 {
 
@@ -30,7 +31,13 @@ inline int dalloc(T** p, size_t count)
 {
     *p = nullptr;
     if (count == 0) return SCP3GPU_OK;
-    SCP3_CUDA(cudaMalloc((void**)p, count * sizeof(T)));
+    cudaError_t e = cudaMalloc((void**)p, count * sizeof(T));
+    if (e == cudaErrorMemoryAllocation) {       // the transfer pool's idle memory first
+        (void)cudaGetLastError();
+        staging::trim();
+        e = cudaMalloc((void**)p, count * sizeof(T));
+    }
+    SCP3_CUDA(e);
     return SCP3GPU_OK;
 }
 
