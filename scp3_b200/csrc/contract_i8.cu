@@ -56,17 +56,19 @@ constexpr int kDigits = 7, kSweeps = 4, kTile = 128, kN = 256;
 constexpr int kBox = kTile * kKB;                  // 8 KB: one digit of 128 rows x 64 samples
 constexpr int kSlot = 3 * kBox, kRing = 9;         // A box, two B boxes
 constexpr int kRunKB = 288;                        // k-blocks per run: 7 * 2^14 * 18432 < 2^31
-constexpr int kSmem = kRing * kSlot + 1024 + 256;
+constexpr int kSmem = kRing * kSlot + 1024 + 256 + kN * (int)sizeof(double);
 constexpr int kThreads = 320, kEpiWarps = 8;
 // kind::i8: D S32, A and B signed 8-bit, K-major
 constexpr uint32_t kIdesc = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kN >> 3) << 17) |
                             ((uint32_t)(kTile >> 4) << 24);
+constexpr uint32_t kIdescHalf = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kTile >> 3) << 17) |
+                                ((uint32_t)(kTile >> 4) << 24);      // N = 128: tiles of one B panel
 
-__device__ __forceinline__ void mma_i8(uint32_t d, uint64_t a, uint64_t b, uint32_t acc)
+__device__ __forceinline__ void mma_i8(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc)
 {
     asm volatile(
         "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n}\n" ::"r"(d),
-        "l"(a), "l"(b), "r"(kIdesc), "r"(acc));
+        "l"(a), "l"(b), "r"(idesc), "r"(acc));
 }
 
 // 16 columns of each of two accumulators
@@ -114,6 +116,8 @@ __device__ __forceinline__ double row_unit(int hi)     // value of one unit of t
     return hi >= 0x7ff00000 ? __longlong_as_double(0x7ff8000000000000ll) : pow2(row_exp(hi) - 54);
 }
 
+__device__ __forceinline__ double zero_unit(int hi) { return hi ? row_unit(hi) : 0.0; }
+
 __global__ void __launch_bounds__(kThreads, 1)
     contract_i8_kernel(const uint8_t* __restrict__ x, long long nkb_alloc, const int* __restrict__ rowmax,
                        const int4* __restrict__ tiles, int ntiles, int nsplit, int nkb_pass, int units,
@@ -128,6 +132,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     uint64_t* drain = acc_empty + 1;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain + 1);
     volatile int* abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    double* cunit = reinterpret_cast<double*>(smem + kRing * kSlot + 256);    // [256] units of the tile's columns
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     auto krange = [&](int u, int& lo, int& hi) {
@@ -177,11 +182,11 @@ __global__ void __launch_bounds__(kThreads, 1)
                                     break;
                                 }
                                 uint8_t* st = smem + slot * kSlot;
-                                mbar_expect_tx(full + slot, kSlot);
+                                mbar_expect_tx(full + slot, ti.z ? 2 * kBox : kSlot);
                                 const size_t o = ((size_t)kb * kDigits + chain_digit(t, e) - 1) * kBox;
                                 bulk_load(st, pa + o, kBox, full + slot);
                                 bulk_load(st + kBox, pb0 + o, kBox, full + slot);
-                                bulk_load(st + 2 * kBox, pb1 + o, kBox, full + slot);
+                                if (!ti.z) bulk_load(st + 2 * kBox, pb1 + o, kBox, full + slot);
                                 issued |= 1u << slot;
                                 issued_phase = (issued_phase & ~(1u << slot)) | phase << slot;
                                 if (++slot == kRing) {
@@ -206,6 +211,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
                 int lo, hi;
                 krange(u, lo, hi);
+                const uint32_t idesc = tiles[u % ntiles].z ? kIdescHalf : kIdesc;
                 for (int r0 = lo; r0 < hi && ok; r0 += kRunKB)
                     for (int t = 0; t < kSweeps && ok; t++, use++) {
                         const int n = sweep_digits(t);
@@ -228,15 +234,15 @@ __global__ void __launch_bounds__(kThreads, 1)
                                 if (e) {
                                     const uint32_t d = tmem + (in_large(t, e) ? 0u : (uint32_t)kN);
                                     const uint32_t acc = kb != r0 || e > 2;
-                                    mma_i8(d, pa, cb, acc);
-                                    mma_i8(d, pa + 2, cb + 2, 1);
-                                    mma_i8(d, ca, pb, 1);
-                                    mma_i8(d, ca + 2, pb + 2, 1);
+                                    mma_i8(d, pa, cb, idesc, acc);
+                                    mma_i8(d, pa + 2, cb + 2, idesc, 1);
+                                    mma_i8(d, ca, pb, idesc, 1);
+                                    mma_i8(d, ca + 2, pb + 2, idesc, 1);
                                     mma_commit(empty + prev);
                                 }
                                 if (e == n - 1) {      // in sweep 3 the smaller sum's first
-                                    mma_i8(tmem + kN, ca, cb, kb != r0 || n > 2);
-                                    mma_i8(tmem + kN, ca + 2, cb + 2, 1);
+                                    mma_i8(tmem + kN, ca, cb, idesc, kb != r0 || n > 2);
+                                    mma_i8(tmem + kN, ca + 2, cb + 2, idesc, 1);
                                     mma_commit(empty + slot);
                                 }
                                 pa = ca, pb = cb, prev = slot;
@@ -263,8 +269,13 @@ __global__ void __launch_bounds__(kThreads, 1)
             int lo, hi;
             krange(u, lo, hi);
             const int4 ti = tiles[u % ntiles];
-            const double ra = row_unit(rowmax[ti.x + row]);
-            const int* cmax = rowmax + (half ? ti.w : ti.y);
+            const double ra = zero_unit(rowmax[ti.x + row]);
+            // the columns' units, for the eight warps (the last unit's are no longer read)
+            asm volatile("bar.sync 1, %0;" ::"n"(kEpiWarps * 32) : "memory");
+            const int et = threadIdx.x - 64;
+            cunit[et] = zero_unit(rowmax[(et < kTile ? ti.y : ti.w) + (et & (kTile - 1))]);
+            asm volatile("bar.sync 1, %0;" ::"n"(kEpiWarps * 32) : "memory");
+            const double* cu = cunit + half * kTile;
             double* P = partial + (size_t)u * (size_t)(kTile * kN) + (size_t)half * kTile * kTile + row;
             for (int r0 = lo; r0 < hi && ok; r0 += kRunKB)
                 for (int t = 0; t < kSweeps; t++, use++) {
@@ -275,16 +286,25 @@ __global__ void __launch_bounds__(kThreads, 1)
                     tc_fence_after();
                     const double w = ra * pow2(8 * (5 + 2 * t));     // the larger digit sum: 2^(8 (14 - (9 - 2t)))
                     const uint32_t base = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(half * kTile);
+                    // a tile of one panel has no second half; rows that are zero throughout
+                    // (padding among them; unit 0) add nothing, unless to values that are
+                    // not finite (unit NaN)
 #pragma unroll 1
-                    for (int c0 = 0; c0 < kTile; c0 += 16) {
+                    for (int c0 = 0; c0 < (half && ti.z ? 0 : kTile); c0 += 16) {
+                        double un[16];
+                        bool any = false;
+#pragma unroll
+                        for (int j = 0; j < 16; j++) any |= (un[j] = cu[c0 + j]) != 0.0;
+                        if (!any) continue;
                         int a0[16], a1[16];
                         tmem_ld16x2(base + c0, base + kN + c0, a0, a1);
 #pragma unroll
                         for (int j = 0; j < 16; j++) {
                             // |.| < 2^40: exact through the bits of 1.5 * 2^52
                             const long long d = ((long long)a1[j] << 8) + a0[j] + 0x4338000000000000ll;
-                            add_f64(P + (size_t)(c0 + j) * kTile,
-                                    (__longlong_as_double(d) - 6755399441055744.0) * w * row_unit(cmax[c0 + j]));
+                            if ((w != 0.0 && un[j] != 0.0) || w != w || un[j] != un[j])
+                                add_f64(P + (size_t)(c0 + j) * kTile,
+                                        (__longlong_as_double(d) - 6755399441055744.0) * w * un[j]);
                         }
                     }
                     tc_fence_before();

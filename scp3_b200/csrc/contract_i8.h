@@ -29,7 +29,7 @@ struct Plan {
     int scan_per = 0;              // rows per CTA of the scan
     int16_t* entries = nullptr;    // [nm][12] table entry of each kind of each mode, -1 = none
     uint32_t* xdesc = nullptr;
-    int4* tiles = nullptr;         // (A row, B rows 0..127, -, B rows 128..255)
+    int4* tiles = nullptr;         // (A row, B rows 0..127, 1 = that panel only, B rows 128..255)
     double* partial = nullptr;     // [nsplit][ntiles][128 x 256] tile-local column-major
     double* spart = nullptr;       // [blocks of the scan][nsum]
     double* sums = nullptr;        // [nsum]

@@ -305,50 +305,69 @@ __global__ void __launch_bounds__(kThreads, 1)
 // as itself or transposed (block_owner = 4 t + 2 transposed + h); its value is
 // the sum over the splits, in order, of unit (split * ntiles + t) at row
 // r % 128 and column 128 h + c % 128 (transposed: row c % 128, column
-// 128 h + r % 128).
-// `err` (may be null): a non-zero flag makes every element NaN.  kGroups > 1: that
-// many threads per element, each summing a contiguous share of the splits, the
-// shares then added in order (bases of a few tiles have up to one split per SM, and
-// one thread's chain of 148 loads took 35 us).
-template <int kGroups>
-__global__ void __launch_bounds__(256) unpack_n256_kernel(const double* __restrict__ partial,
-                                                          const int* __restrict__ block_owner, int nt, int ntiles,
-                                                          int nsplit, int nb, double divisor,
-                                                          const double* __restrict__ diag, double zpe,
-                                                          double* __restrict__ M, int64_t ld,
-                                                          const int* __restrict__ err)
+// 128 h + r % 128).  `err` (may be null): a non-zero flag makes every element NaN.
+//
+// CTA: 32 x kY elements of a needed block (every part of one above the diagonal, those of
+// a diagonal block that hold upper elements), read along the partials' rows and written to
+// both triangles, the mirror through shared memory (one thread per element of the full
+// matrix read half of them across the partials' columns: 3825 functions 392 us, now 136).
+// blockDim (32, 8 kGroups): group g of a CTA sums a contiguous share of the splits, the
+// shares then added in order; kY = 8 and four groups for bases of a few tiles, which have
+// up to one split per SM.
+template <int kGroups, int kY>
+__global__ void __launch_bounds__(256 * kGroups) unpack_n256_kernel(const double* __restrict__ partial,
+                                                                    const int* __restrict__ block_owner, int nt,
+                                                                    int nblk, int ntiles, int nsplit, int nb,
+                                                                    double divisor, const double* __restrict__ diag,
+                                                                    double zpe, double* __restrict__ M, int64_t ld,
+                                                                    const int* __restrict__ err)
 {
-    constexpr int kPer = 256 / kGroups;                 // elements per CTA
-    const int x = threadIdx.x % kPer, g = threadIdx.x / kPer;
-    const int64_t e = (int64_t)blockIdx.x * kPer + x;
-    const bool in = e < (int64_t)nb * nb;
-    const int j = in ? (int)(e / nb) : 0, i = in ? (int)(e - (int64_t)j * nb) : 0;
-    double val = 0.0;
-    if (in) {
-        const int r = min(i, j), c = max(i, j);
-        const int ti = r / kTile, tj = c / kTile;
-        const int own = block_owner[ti * nt + tj];
-        const int t = own >> 2, h = own & 1;
-        const int rr = r - ti * kTile, cc = c - tj * kTile;
-        const size_t off = (own & 2) ? (size_t)(h * kTile + rr) * kTile + cc : (size_t)(h * kTile + cc) * kTile + rr;
-        const int s1 = nsplit * (g + 1) / kGroups;
-#pragma unroll 4
-        for (int s = nsplit * g / kGroups; s < s1; s++)
-            val += partial[((size_t)s * ntiles + t) * (size_t)(kTile * kN2) + off];
-    }
-    if (kGroups > 1) {
-        __shared__ double part[kGroups][kPer];
-        part[g][x] = val;
-        __syncthreads();
-        if (g) return;
+    constexpr int kParts = kTile / 32 * (kTile / kY);
+    __shared__ double v[kGroups][kY][33];
+    // block (ti, tj), row-major over ti <= tj < nblk, and its part
+    int p = blockIdx.x / kParts, ti = 0;
+    while (p >= nblk - ti) p -= nblk - ti, ti++;
+    const int tj = ti + p, part = blockIdx.x % kParts;
+    const int own = block_owner[ti * nt + tj], t = own >> 2, h = own & 1;
+    const bool tr = own & 2, diagonal = ti == tj;      // a diagonal block is never transposed
+    // x along the partials' rows, y along their columns
+    const int x0 = (part & 3) * 32, y0 = (part >> 2) * kY;
+    const int gx0 = (tr ? tj : ti) * kTile + x0, gy0 = (tr ? ti : tj) * kTile + y0;
+    if (gx0 >= nb || gy0 >= nb || (diagonal && gx0 >= gy0 + kY)) return;
+    const int x = threadIdx.x, y8 = threadIdx.y & 7, g = threadIdx.y >> 3;
+    const size_t unit = (size_t)ntiles * (kTile * kN2);
+    const double* P = partial + (size_t)t * (kTile * kN2) + (size_t)(h * kTile + y0) * kTile + x0 + x;
+    const int s1 = nsplit * (g + 1) / kGroups;
+    double sum[kY / 8] = {};
+#pragma unroll 8
+    for (int s = nsplit * g / kGroups; s < s1; s++)
 #pragma unroll
-        for (int k = 1; k < kGroups; k++) val += part[k][x];
+        for (int k = 0; k < kY / 8; k++) sum[k] += P[s * unit + (size_t)(y8 + 8 * k) * kTile];
+#pragma unroll
+    for (int k = 0; k < kY / 8; k++) v[g][y8 + 8 * k][x] = sum[k];
+    __syncthreads();
+    const bool bad = err && *err;
+    if (g == 0) {
+#pragma unroll
+        for (int k = 0; k < kY / 8; k++) {
+            const int y = y8 + 8 * k;
+            double val = v[0][y][x];
+#pragma unroll
+            for (int q = 1; q < kGroups; q++) val += v[q][y][x];
+            val = val / divisor;
+            if (diag && gx0 + x == gy0 + y) val = (val + diag[gx0 + x]) + zpe;
+            if (bad) val = __longlong_as_double(0x7ff8000000000000ll);
+            v[0][y][x] = val;
+            if (gx0 + x < nb && gy0 + y < nb && !(diagonal && gx0 + x > gy0 + y))
+                M[(size_t)(gy0 + y) * ld + gx0 + x] = val;
+        }
     }
-    if (!in) return;
-    val = val / divisor;
-    if (diag && i == j) val = (val + diag[i]) + zpe;
-    if (err && *err) val = __longlong_as_double(0x7ff8000000000000ll);
-    M[(size_t)j * ld + i] = val;
+    __syncthreads();
+    if (g) return;
+    for (int e = threadIdx.y * 32 + x; e < 32 * kY; e += 256) {
+        const int gy = gy0 + e % kY, gx = gx0 + e / kY;
+        if (gx < nb && gy < nb && !(diagonal && gx >= gy)) M[(size_t)gx * ld + gy] = v[0][e % kY][e / kY];
+    }
 }
 
 // One CTA of 1024 threads per 4096-sample block (4 samples per thread): stable
@@ -815,12 +834,14 @@ int launch_unpack(const double* partial, const int* owner, int nt, int ntiles, i
 {
     const int64_t total = (int64_t)nb * nb;
     if (total <= 0) return SCP3GPU_OK;
+    const int nblk = (nb + kTile - 1) / kTile;
+    const unsigned grid = (unsigned)(nblk * (nblk + 1) / 2 * 16);
     if (nsplit < 16)
-        unpack_n256_kernel<1><<<(unsigned)((total + 255) / 256), 256, 0, s>>>(partial, owner, nt, ntiles, nsplit, nb,
-                                                                              divisor, diag, zpe, M, ld, err);
+        unpack_n256_kernel<1, 32><<<grid, dim3(32, 8), 0, s>>>(partial, owner, nt, nblk, ntiles, nsplit, nb, divisor,
+                                                               diag, zpe, M, ld, err);
     else
-        unpack_n256_kernel<8><<<(unsigned)((total + 31) / 32), 256, 0, s>>>(partial, owner, nt, ntiles, nsplit, nb,
-                                                                            divisor, diag, zpe, M, ld, err);
+        unpack_n256_kernel<4, 8><<<4 * grid, dim3(32, 32), 0, s>>>(partial, owner, nt, nblk, ntiles, nsplit, nb,
+                                                                   divisor, diag, zpe, M, ld, err);
     SCP3_CUDA(cudaGetLastError());
     return SCP3GPU_OK;
 }

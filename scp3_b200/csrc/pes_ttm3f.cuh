@@ -374,11 +374,11 @@ __device__ __forceinline__ double sum_geometry(double x)      // over the lanes 
 // G their gradients g + j * 9 nw (shared, kcal/mol/A, complete after the call); ms
 // [4][3nw] and sc (scratch_bytes) shared scratch.  Lane l returns the energy of geometry
 // l % 4, *iters its Jacobi sweeps (kTtmMaxIter + 1 if capped).  NG = 2: two geometries
-// of up to 16 waters instead, lane l on water l / 2 of geometry l % 2.
-template <typename T, bool G, int NG = 4>
+// of up to 16 waters instead, lane l on water l / 2 of geometry l % 2.  kMaxNw: most
+// waters the instance's registers hold dipole tensors for.
+template <typename T, bool G, int NG = 4, int kMaxNw = 32 / NG>
 __device__ double energy_warp4(const T* crd, int stride, T* ms, char* sc, double* g, int nw, int ng, int lane, int* iters)
 {
-    constexpr int kMaxNw = 32 / NG;
     const int j = lane % NG, i = lane / NG, n3 = 3 * nw;
     const bool on = j < ng && i < nw;
     const T* cj = crd + j * stride;

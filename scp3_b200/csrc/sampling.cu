@@ -68,7 +68,7 @@ __device__ inline WarpSlot<T> warp_slot(char* base, int nm0, int nw, bool grad =
 
 // Energies (and with G gradients) of a group's gn geometries in one warp pass: lane l
 // returns the energy of geometry l % 4.
-template <int PES, typename T, bool G, int NG = kGroup>
+template <int PES, typename T, bool G, int NG = kGroup, int NW = 32 / NG>
 __device__ __forceinline__ double potential4(const WarpSlot<T>& w, int nw, int gn, int lane, int* iters)
 {
     if constexpr (PES == SCP3GPU_PES_QTIP4PF) {
@@ -76,7 +76,7 @@ __device__ __forceinline__ double potential4(const WarpSlot<T>& w, int nw, int g
         if constexpr (G) return qt::energy_grad_warp4<T>(w.crd, 9 * nw, w.ms, w.g, nw, gn, lane);
         else return qt::energy_warp4<T>(w.crd, 9 * nw, w.ms, nw, gn, lane);
     } else {
-        return ttm::energy_warp4<T, G, NG>(w.crd, 9 * nw, w.ms, w.sc, w.g, nw, gn, lane, iters);
+        return ttm::energy_warp4<T, G, NG, NW>(w.crd, 9 * nw, w.ms, w.sc, w.g, nw, gn, lane, iters);
     }
 }
 
@@ -186,25 +186,27 @@ struct Pair<float> {
 
 // G: the gradient path (dV/dq) is compiled in; the energy-only instances keep
 // their registers for the energy path.
-template <int PES, typename T, bool G = false>
+template <int PES, typename T, bool G = false, int NW = 8>
 __device__ __forceinline__ void samples_body(const SampleArgs& a, char* smem);
 
 // Blocks per SM the registers must allow: qTIP4P/f, 4 for the FP32 energies (64
 // registers), 3 for the FP32 gradients (85), 2 for FP64; TTM3-F keeps its dipole tensors
-// in registers: 2 for the energies, 1 for the gradients.
-template <int PES, typename T, bool G>
+// in registers: 2 for the energies, 1 for the gradients, 2 for those of clusters of up to
+// NW = 4 waters (three tensors per lane instead of seven; trimer gradients, 2^14
+// samples: 268 us at one block).
+template <int PES, typename T, bool G, int NW = 8>
 constexpr int sample_blocks()
 {
-    if (PES == SCP3GPU_PES_TTM3F) return G ? 1 : 2;
+    if (PES == SCP3GPU_PES_TTM3F) return G && NW > 4 ? 1 : 2;
     return sizeof(T) == 4 ? (G ? 3 : 4) : 2;
 }
 
-template <int PES, typename T, bool G>
-__global__ void __launch_bounds__(kWarpsPerBlock * 32, sample_blocks<PES, T, G>())
+template <int PES, typename T, bool G, int NW = 8>
+__global__ void __launch_bounds__(kWarpsPerBlock * 32, sample_blocks<PES, T, G, NW>())
     samples_kernel(SampleArgs a)
 {
     extern __shared__ __align__(16) char smem[];
-    samples_body<PES, T, G>(a, smem);
+    samples_body<PES, T, G, NW>(a, smem);
 }
 
 // Several clusters of a batch: cluster blockIdx.y takes args[blockIdx.y].
@@ -221,7 +223,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, sample_blocks<PES, T, fal
     samples_body<PES, T>(a, smem);
 }
 
-template <int PES, typename T, bool G>
+template <int PES, typename T, bool G, int NW>
 __device__ __forceinline__ void samples_body(const SampleArgs& a, char* smem)
 {
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
@@ -354,9 +356,9 @@ __device__ __forceinline__ void samples_body(const SampleArgs& a, char* smem)
         int iters4 = 0;
         if (!a.skip_pes) {
             if (grad) {
-                if constexpr (G) e4 = potential4<PES, T, true>(w, nw, gn, lane, &iters4);
+                if constexpr (G) e4 = potential4<PES, T, true, kGroup, NW>(w, nw, gn, lane, &iters4);
             } else {
-                e4 = potential4<PES, T, false>(w, nw, gn, lane, &iters4);
+                e4 = potential4<PES, T, false, kGroup, NW>(w, nw, gn, lane, &iters4);
             }
         }
         if constexpr (G) {
@@ -552,6 +554,8 @@ int launch_samples_t(const SampleArgs& a, cudaStream_t s)
     // the FP32 gradient is qTIP4P/f's only (launch_samples)
     constexpr bool kGrad = PES == SCP3GPU_PES_QTIP4PF || sizeof(T) == 8;
     auto kern = a.vq ? samples_kernel<PES, T, kGrad> : samples_kernel<PES, T, false>;
+    if constexpr (PES == SCP3GPU_PES_TTM3F)
+        if (a.nw <= 4) kern = a.vq ? samples_kernel<PES, T, kGrad, 4> : samples_kernel<PES, T, false, 4>;
     if (sm > 48 * 1024) SCP3_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
     kern<<<sample_grid(kern, sm, a.n), kWarpsPerBlock * 32, sm, s>>>(a);
     SCP3_CUDA(cudaGetLastError());

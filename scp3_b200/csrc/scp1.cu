@@ -50,57 +50,102 @@ struct scp3gpu_scp1 {
 namespace scp3 {
 namespace {
 
-constexpr int kRedThreads = 256, kRedPer = 16, kRedRows = 32;
+constexpr int kRedThreads = 256, kRedRows = 32, kRedTile = 8, kRedLd = 80;   // dim + 1 <= 80
+constexpr int kRedStage = 2 * kRedRows * kRedLd;     // rows of [g, V], then of [dq, 1]
+constexpr size_t kRedSmem = sizeof(double) * 2 * kRedStage;
+static_assert(kRedLd * kRedLd <= 2 * kRedStage, "the sums go over the stages");
 
 // P[block] += sum over the block's samples of [g, V] [dq, 1]^T, column-major
-// (dim+1) x (dim+1); element page blockIdx.y of kRedThreads * kRedPer elements.
+// (dim+1) x (dim+1).  nt = ceil((dim+1) / 8): thread (ti, tj) of a group of nt^2 threads
+// owns the 64 elements (ti + nt a, tj + nt b), and the CTA's groups take the staged rows
+// in turn, so a row costs a thread 16 conflict-free reads for 64 FMAs; the groups' sums
+// are added in order.  It was 16 elements per thread on pairs of reads each, bound by
+// shared memory: hexamer, 141 us per 2^16 samples.
 __global__ void __launch_bounds__(kRedThreads) scp1_reduce_kernel(int dim, int64_t n, const double* __restrict__ V,
                                                                   const double* __restrict__ G,
                                                                   const double* __restrict__ D, double* __restrict__ P)
 {
-    __shared__ double sg[kRedRows][80], sd[kRedRows][80];    // dim + 1 <= 80
-    const int E1 = dim + 1, E = E1 * E1;
-    const int t = threadIdx.x;
-    const int e0 = blockIdx.y * kRedThreads * kRedPer;
-    int ia[kRedPer], ib[kRedPer];
-    double acc[kRedPer];
-#pragma unroll
-    for (int k = 0; k < kRedPer; k++) {
-        const int e = e0 + t + kRedThreads * k;
-        ia[k] = e < E ? e % E1 : 0;
-        ib[k] = e < E ? e / E1 : 0;
-        acc[k] = 0.0;
-    }
+    extern __shared__ double sm[];                 // two stages; later the sums
+    const int E1 = dim + 1, E = E1 * E1, nt = (E1 + kRedTile - 1) / kRedTile;
+    const int t = threadIdx.x, groups = kRedThreads / (nt * nt), g = t / (nt * nt), u = t - g * nt * nt;
+    const int ti = u % nt, tj = u / nt, lane = t & 31;
+    double acc[kRedTile][kRedTile] = {};
+    // columns past E1 stay zero, the last column of dq's rows 1
+    for (int e = t; e < 2 * kRedStage; e += kRedThreads)
+        sm[e] = e % kRedStage >= kRedRows * kRedLd && e % kRedLd == dim ? 1.0 : 0.0;
+    __syncthreads();
     const int64_t s0 = n * blockIdx.x / gridDim.x, s1 = n * (blockIdx.x + 1) / gridDim.x;
-    for (int64_t c0 = s0; c0 < s1; c0 += kRedRows) {
-        const int rows = (int)(s1 - c0 < kRedRows ? s1 - c0 : kRedRows);
-        __syncthreads();
-        for (int e = t; e < rows * E1; e += kRedThreads) {
-            const int r = e / E1, c = e - r * E1;
+    auto copy8 = [](double* dst, const double* src) {
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+                     : "memory");
+    };
+    auto fetch = [&](int64_t c0, int stage) {
+        double *sg = sm + stage * kRedStage, *sd = sg + kRedRows * kRedLd;
+        for (int r = t >> 5; r < kRedRows && c0 + r < s1; r += kRedThreads / 32) {
             const int64_t s = c0 + r;
-            sg[r][c] = c < dim ? G[s * dim + c] : V[s];
-            sd[r][c] = c < dim ? D[s * dim + c] : 1.0;
+            for (int c = lane; c < dim; c += 32) {
+                copy8(sg + r * kRedLd + c, G + s * dim + c);
+                copy8(sd + r * kRedLd + c, D + s * dim + c);
+            }
+            if (lane == 0) copy8(sg + r * kRedLd + dim, V + s);
         }
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    };
+    fetch(s0, 0);
+    int stage = 0;
+    for (int64_t c0 = s0; c0 < s1; c0 += kRedRows, stage ^= 1) {
+        const int rows = (int)(s1 - c0 < kRedRows ? s1 - c0 : kRedRows);
+        fetch(c0 + kRedRows, stage ^ 1);           // an empty group past the end
+        asm volatile("cp.async.wait_group 1;\n" ::: "memory");
         __syncthreads();
-        for (int r = 0; r < rows; r++) {
+        const double *sg = sm + stage * kRedStage, *sd = sg + kRedRows * kRedLd;
+        if (g < groups)
+            for (int r = g; r < rows; r += groups) {
+                double a[kRedTile], b[kRedTile];
 #pragma unroll
-            for (int k = 0; k < kRedPer; k++) acc[k] += sg[r][ia[k]] * sd[r][ib[k]];
-        }
+                for (int k = 0; k < kRedTile; k++) a[k] = sg[r * kRedLd + ti + nt * k], b[k] = sd[r * kRedLd + tj + nt * k];
+#pragma unroll
+                for (int i = 0; i < kRedTile; i++)
+#pragma unroll
+                    for (int j = 0; j < kRedTile; j++) acc[i][j] = fma(a[i], b[j], acc[i][j]);
+            }
+        __syncthreads();                           // the stage is free for the next fetch
     }
-    double* Pb = P + (size_t)blockIdx.x * E;
+    asm volatile("cp.async.wait_all;\n" ::: "memory");
+    for (int q = 0; q < groups; q++) {
+        __syncthreads();
+        if (g == q)
 #pragma unroll
-    for (int k = 0; k < kRedPer; k++) {
-        const int e = e0 + t + kRedThreads * k;
-        if (e < E) Pb[e] += acc[k];
+            for (int i = 0; i < kRedTile; i++)
+#pragma unroll
+                for (int j = 0; j < kRedTile; j++) {
+                    double* p = sm + (tj + nt * j) * kRedLd + ti + nt * i;
+                    *p = q ? *p + acc[i][j] : acc[i][j];
+                }
+    }
+    __syncthreads();
+    double* Pb = P + (size_t)blockIdx.x * E;
+    for (int e = t; e < E; e += kRedThreads) {
+        const int j = e / E1;
+        Pb[e] += sm[j * kRedLd + (e - j * E1)];
     }
 }
 
-__global__ void scp1_sum_kernel(int E, int blocks, const double* __restrict__ P, double* __restrict__ R)
+// R[e] = sum of the block partials: warp w of a CTA adds the blocks w, w + 8, ... of 32
+// elements in order, the eight warp sums are then added in order
+__global__ void __launch_bounds__(256) scp1_sum_kernel(int E, int blocks, const double* __restrict__ P,
+                                                       double* __restrict__ R)
 {
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= E) return;
+    __shared__ double ws[8][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, e = blockIdx.x * 32 + lane;
     double s = 0.0;
-    for (int b = 0; b < blocks; b++) s += P[(size_t)b * E + e];
+    if (e < E)
+        for (int b = w; b < blocks; b += 8) s += P[(size_t)b * E + e];
+    ws[w][lane] = s;
+    __syncthreads();
+    if (w || e >= E) return;
+#pragma unroll
+    for (int k = 1; k < 8; k++) s += ws[k][lane];
     R[e] = s;
 }
 
@@ -139,7 +184,7 @@ int scp3gpu_scp1_create(int pes, int nw, int64_t chunk, int device, scp3gpu_scp1
     h->chunk = chunk > 0 ? (chunk + 31) / 32 * 32 : (1 << 16);
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    h->blocks = 2 * sms;
+    h->blocks = sms;
     const int dim = h->dim, E = (dim + 1) * (dim + 1);
     std::vector<int64_t> v;
     std::vector<uint64_t> sh;
@@ -187,11 +232,11 @@ int scp3gpu_scp1_average(scp3gpu_scp1* h, const double* q, const double* d, cons
         const int64_t n = std::min<int64_t>(h->chunk, i1 - c0);
         Scp1Args a{h->nw, dim, h->q, h->sqd, h->U, h->vdir, skip + c0, n, h->V, h->G, h->D, h->capped};
         if ((rc = launch_scp1_samples(h->pes, a, s))) return rc;
-        const int pages = (E + kRedThreads * kRedPer - 1) / (kRedThreads * kRedPer);
-        scp1_reduce_kernel<<<dim3(h->blocks, pages), kRedThreads, 0, s>>>(dim, n, h->V, h->G, h->D, h->P);
+        SCP3_CUDA(cudaFuncSetAttribute(scp1_reduce_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRedSmem));
+        scp1_reduce_kernel<<<h->blocks, kRedThreads, kRedSmem, s>>>(dim, n, h->V, h->G, h->D, h->P);
         SCP3_CUDA(cudaGetLastError());
     }
-    scp1_sum_kernel<<<(E + 255) / 256, 256, 0, s>>>(E, h->blocks, h->P, h->R);
+    scp1_sum_kernel<<<(E + 31) / 32, 256, 0, s>>>(E, h->blocks, h->P, h->R);
     SCP3_CUDA(cudaGetLastError());
     std::vector<double> R(E);
     unsigned long long capped = 0;

@@ -517,7 +517,8 @@ __global__ void __launch_bounds__(256) stein_rowsum_kernel(const float* __restri
 // split form's pair sums as products) the term of a pair exciting m in both
 // functions is C at W_b row (m, rank of r, level of c in m), column
 // red3(c without its mode-m factor).
-__global__ void stein_unpack_kernel(const uint32_t* __restrict__ desc, const int* __restrict__ rank3,
+template <int kY>
+__global__ void __launch_bounds__(256) stein_unpack_kernel(const uint32_t* __restrict__ desc, const int* __restrict__ rank3,
                                     const int* __restrict__ voff, const int64_t* __restrict__ doff, int nb, int nv,
                                     int ct, int nsplit, int dsplit, const double* __restrict__ C,
                                     const double* __restrict__ D,
@@ -527,10 +528,15 @@ __global__ void stein_unpack_kernel(const uint32_t* __restrict__ desc, const int
                                     const int* __restrict__ wb_off, const int* __restrict__ sum_off,
                                     const double* __restrict__ sums, const int* __restrict__ err)
 {
-    const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= (int64_t)nb * nb) return;
-    const int j = (int)(e / nb), i = (int)(e - (int64_t)j * nb);
-    const int r = min(i, j), c = max(i, j);
+    // CTA: 32 rows x kY columns of block (a, b) of 32 x 32 elements, a <= b, row-major over
+    // the upper blocks; thread (x, y) forms (r, c) = (r0 + x, c0 + y) and columns y + 8, ...;
+    // the mirror is written through shared memory
+    __shared__ double v[kY][33];
+    const int nblk = (nb + 31) / 32;
+    int p = blockIdx.x / (32 / kY), a0 = 0;
+    while (p >= nblk - a0) p -= nblk - a0, a0++;
+    const int r0 = 32 * a0, c0 = 32 * (a0 + p) + kY * (blockIdx.x % (32 / kY));
+    const bool bad = *err != 0;
     // a term whose tile the plan did not make reads NaN into the element (never,
     // by construction; a visible result rather than an out-of-range read)
     auto cidx = [&](int vr, int col) -> int64_t {
@@ -544,56 +550,67 @@ __global__ void stein_unpack_kernel(const uint32_t* __restrict__ desc, const int
         for (int s = 0; s < nsplit; s++) t += C[s * csize + x];
         return t;
     };
-    int mr[3], lr[3], mc[3], lc[3];
-    const int nr = decode(desc[r], mr, lr), ncn = decode(desc[c], mc, lc);
-    double val = 0.0;
-    if (nr + ncn == 0) {   // <0|V|0>
-        const int64_t x = cidx(nv - 1, 0);
-        val += csum(x);
-    } else {
-        int ns = 0;
-        for (int a = 0; a < nr; a++) {
-            int b = -1;
-            for (int k = 0; k < ncn; k++)
-                if (mc[k] == mr[a]) b = k;
-            const int m = mr[a];
-            double t = 0.0;
-            if (b < 0) {
-                const int64_t x = cidx(voff[m] + rank3[3 * r + a], c);
-                t += csum(x);
-            } else if (sum_off && sum_off[m * 4 + lc[b]] >= 0) {
-                // summed row (m, rank of r, level of c in m): c without m is the constant
-                t = sums[sum_off[m * 4 + lc[b]] + rank3[3 * r + a]];
-            } else if (wb_off) {
-                // W_b row (m, rank of r, level of c in m) against Phi of c without m
-                const int64_t x = cidx(wb_off[m * 4 + lc[b]] + rank3[3 * r + a], red3[3 * c + b]);
-                t += csum(x);
-            } else {
-                // D holds the upper triangle of ranks (functions ordered by level in m)
-                const int en = voff[m + 1] - voff[m];
-                const int ra = rank3[3 * r + a], rb = rank3[3 * c + b];
-                const int64_t x = doff[m] + (int64_t)min(ra, rb) * en + max(ra, rb);
-                for (int s = 0; s < dsplit; s++) t += D[s * dsize + x];
+    const int x = threadIdx.x & 31, y8 = threadIdx.x >> 5;
+    for (int y = y8; y < kY; y += 8) {
+        const int r = r0 + x, c = c0 + y;
+        if (r >= nb || c >= nb || r > c) continue;
+        int mr[3], lr[3], mc[3], lc[3];
+        const int nr = decode(desc[r], mr, lr), ncn = decode(desc[c], mc, lc);
+        double val = 0.0;
+        if (nr + ncn == 0) {   // <0|V|0>
+            const int64_t x = cidx(nv - 1, 0);
+            val += csum(x);
+        } else {
+            int ns = 0;
+            for (int a = 0; a < nr; a++) {
+                int b = -1;
+                for (int k = 0; k < ncn; k++)
+                    if (mc[k] == mr[a]) b = k;
+                const int m = mr[a];
+                double t = 0.0;
+                if (b < 0) {
+                    const int64_t x = cidx(voff[m] + rank3[3 * r + a], c);
+                    t += csum(x);
+                } else if (sum_off && sum_off[m * 4 + lc[b]] >= 0) {
+                    // summed row (m, rank of r, level of c in m): c without m is the constant
+                    t = sums[sum_off[m * 4 + lc[b]] + rank3[3 * r + a]];
+                } else if (wb_off) {
+                    // W_b row (m, rank of r, level of c in m) against Phi of c without m
+                    const int64_t x = cidx(wb_off[m * 4 + lc[b]] + rank3[3 * r + a], red3[3 * c + b]);
+                    t += csum(x);
+                } else {
+                    // D holds the upper triangle of ranks (functions ordered by level in m)
+                    const int en = voff[m + 1] - voff[m];
+                    const int ra = rank3[3 * r + a], rb = rank3[3 * c + b];
+                    const int64_t x = doff[m] + (int64_t)min(ra, rb) * en + max(ra, rb);
+                    for (int s = 0; s < dsplit; s++) t += D[s * dsize + x];
+                }
+                val += t;
+                ns++;
             }
-            val += t;
-            ns++;
+            for (int b = 0; b < ncn; b++) {
+                bool shared = false;
+                for (int a = 0; a < nr; a++) shared |= mr[a] == mc[b];
+                if (shared) continue;
+                const int64_t x = cidx(voff[mc[b]] + rank3[3 * c + b], r);
+                double t = 0.0;
+                t += csum(x);
+                val += t;
+                ns++;
+            }
+            val /= (double)ns;
         }
-        for (int b = 0; b < ncn; b++) {
-            bool shared = false;
-            for (int a = 0; a < nr; a++) shared |= mr[a] == mc[b];
-            if (shared) continue;
-            const int64_t x = cidx(voff[mc[b]] + rank3[3 * c + b], r);
-            double t = 0.0;
-            t += csum(x);
-            val += t;
-            ns++;
-        }
-        val /= (double)ns;
+        val = val / divisor;
+        if (diag && r == c) val = (val + diag[r]) + zpe;
+        if (bad) val = __longlong_as_double(0x7ff8000000000000ll);     // a pass did not finish
+        v[y][x] = val;
+        M[(size_t)c * ld + r] = val;
     }
-    val = val / divisor;
-    if (diag && i == j) val = (val + diag[i]) + zpe;
-    if (*err) val = __longlong_as_double(0x7ff8000000000000ll);     // a pass did not finish
-    M[(size_t)j * ld + i] = val;
+    __syncthreads();
+    for (int e = threadIdx.x; e < 32 * kY; e += 256) {
+        const int c = c0 + e % kY, r = r0 + e / kY;
+        if (c < nb && r < c) M[(size_t)r * ld + c] = v[e % kY][e / kY];
+    }
 }
 
 int64_t round_up(int64_t a, int64_t b) { return (a + b - 1) / b * b; }
@@ -804,7 +821,7 @@ int stein_create(SteinPlan& p, const std::vector<uint32_t>& desc, int nm, int64_
     auto add_tile = [&](int r, int q) {
         const int b0 = phi0 + 2 * q * 128, b1 = 2 * q + 1 < p.ct ? b0 + 128 : b0;
         tile_of[(size_t)r * p.bpairs + q] = (int)tl.size();
-        tl.push_back(make_int4(r * 128, b0, 0, b1));
+        tl.push_back(make_int4(r * 128, b0, !split && b1 == b0, b1));     // z: the split form's sign-table offset
     };
     for (int q = 0; q < p.bpairs; q++)
         for (int r = 0; r < p.rt; r++) add_tile(r, q);
@@ -1041,15 +1058,17 @@ int stein_pass(const SteinPlan& p, const uint32_t* desc, const double* q, const 
 int stein_unpack(const SteinPlan& p, const uint32_t* desc, double divisor, const double* diag, double zpe,
                  double* M, int64_t ld, cudaStream_t s)
 {
-    const int64_t total = (int64_t)p.nb * p.nb;
-    const unsigned grid = (unsigned)((total + 255) / 256);
+    const int nblk = (p.nb + 31) / 32;
+    const unsigned grid = (unsigned)(nblk * (nblk + 1) / 2);
+    const bool fine = grid < 600;       // fewer CTAs than a GPU holds: a quarter of the columns each
+    auto kern = fine ? stein_unpack_kernel<8> : stein_unpack_kernel<32>;
     if (p.split) {
         int err = 0;
         SCP3_CUDA(cudaMemcpyAsync(&err, p.err, sizeof(int), cudaMemcpyDeviceToHost, s));
         SCP3_CUDA(cudaStreamSynchronize(s));
         if (err) return fail(SCP3GPU_ERR_TIMEOUT, "tensor-core contraction: a bounded pipeline wait expired");
     }
-    stein_unpack_kernel<<<grid, 256, 0, s>>>(desc, p.rank3, p.voff, p.doff, p.nb, p.nv, p.bpairs, p.nsplit, p.dsplit,
+    kern<<<fine ? 4 * grid : grid, 256, 0, s>>>(desc, p.rank3, p.voff, p.doff, p.nb, p.nv, p.bpairs, p.nsplit, p.dsplit,
                                              p.split ? p.P : p.ip.partial, p.D, (int64_t)p.ntiles2 * 128 * 256, p.dsize,
                                              divisor, diag, zpe, M, ld, p.tile_of, p.red3,
                                              p.tcpairs ? p.wb_off : nullptr, p.nsum ? p.sum_off : nullptr,

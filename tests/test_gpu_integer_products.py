@@ -78,7 +78,11 @@ def test_zero_and_not_finite(api):
         V = rng.normal(size=200)
         V[77] = bad
         assert not np.isfinite(me.addEpot(q.T, V, np.zeros((nb, nb), order="F"))).any()
+    # a mode at rest: rows of zeros inside the panels
     V = rng.normal(size=200)
+    qz = q.copy()
+    qz[:, 4] = 0.0
+    check(me.addEpot(qz.T, V, np.zeros((nb, nb), order="F")), qz, V, 12, 0)
     qb = q.copy()
     qb[5, 3] = np.nan            # only the functions that excite mode 3
     M = me.addEpot(qb.T, V, np.zeros((nb, nb), order="F"))
