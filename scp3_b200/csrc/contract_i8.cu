@@ -325,17 +325,18 @@ __global__ void __launch_bounds__(kThreads, 1)
 // ---------------------------------------------------------------- the operand
 // A CTA tabulates the entries the rows use for 32 samples in FP64, one (mode, sample)
 // per thread at a time; thread (g, r) then takes 16 of the samples (half g; the scan 8)
-// of rows
-// 4r .. 4r+3 and on in steps of the CTA: consecutive rows mostly share their first factor, read
-// once.  Table entry i, 16-byte chunk c (0..7) of half g lies at chunk 8 g + (c ^ (i &
-// 7)), and half 1 reads its chunks in the order c ^ 4, so that four rows with
-// consecutive entries read without bank conflicts (the eight lanes of a 16-byte phase).
+// of rows 4r .. 4r+3 and on in steps of the CTA: consecutive rows mostly share their
+// first factor, read once.  Table entry i, 16-byte chunk c (0..7) of half g lies at chunk
+// 8 g + (c ^ (i / 4 & 7)), and half 1 reads its chunks in the order c ^ 4: the eight
+// lanes of a 16-byte phase hold rows four apart, whose entries mostly are four apart too,
+// and so meet no bank conflict (with the key i & 7 they did: 2^15 samples of the hexamer
+// gradient's digits 381 us, now 308).
 constexpr int kS = 32, kScanThreads = 512, kDigitThreads = 256;
 constexpr int kModeKinds = 12;     // h1 h2 h3 K10 K20 K30 K11 K12 K13 K22 K23 K33
 
 __device__ __forceinline__ void put_entry(double* tab, int r, int l, double val)
 {
-    if (r >= 0) tab[r * kS + ((((l >> 4) << 3) + (((l >> 1) & 7) ^ (r & 7))) << 1) + (l & 1)] = val;
+    if (r >= 0) tab[r * kS + ((((l >> 4) << 3) + (((l >> 1) & 7) ^ ((r >> 2) & 7))) << 1) + (l & 1)] = val;
 }
 
 // entries[m][kind]: table entry or -1; v_entry: V's, or -1
@@ -374,7 +375,7 @@ __device__ __forceinline__ void read16(const double* tab, uint32_t i, int g, dou
     const double2* t = reinterpret_cast<const double2*>(tab + (size_t)i * kS) + 8 * g;
 #pragma unroll
     for (int k = 0; k < 8; k++) {
-        const double2 d = t[(k ^ (g << 2)) ^ (i & 7)];
+        const double2 d = t[(k ^ (g << 2)) ^ ((i >> 2) & 7)];
         o[2 * k] = d.x, o[2 * k + 1] = d.y;
     }
 }
@@ -384,7 +385,7 @@ __device__ __forceinline__ void mul16(const double* tab, uint32_t i, int g, doub
     const double2* t = reinterpret_cast<const double2*>(tab + (size_t)i * kS) + 8 * g;
 #pragma unroll
     for (int k = 0; k < 8; k++) {
-        const double2 d = t[(k ^ (g << 2)) ^ (i & 7)];
+        const double2 d = t[(k ^ (g << 2)) ^ ((i >> 2) & 7)];
         o[2 * k] *= d.x, o[2 * k + 1] *= d.y;
     }
 }
@@ -397,7 +398,7 @@ __device__ __forceinline__ void read8(const double* tab, uint32_t i, int g, doub
     const double2* t = reinterpret_cast<const double2*>(tab + (size_t)i * kS) + 8 * (g >> 1);
 #pragma unroll
     for (int k = 0; k < 4; k++) {
-        const double2 d = t[(4 * (g & 1) + (k ^ (g & 2))) ^ (i & 7)];
+        const double2 d = t[(4 * (g & 1) + (k ^ (g & 2))) ^ ((i >> 2) & 7)];
         if (kMul) o[2 * k] *= d.x, o[2 * k + 1] *= d.y;
         else o[2 * k] = d.x, o[2 * k + 1] = d.y;
     }
@@ -585,19 +586,22 @@ __global__ void __launch_bounds__(kDigitThreads, 2)
     for (int rb = r0 + 4 * rl; rb < r1; rb += 2 * kDigitThreads) {
         uint32_t pia = kZeroRow;
         uint4 d4 = __ldg(reinterpret_cast<const uint4*>(xdesc + rb));
+        int4 m4 = __ldg(reinterpret_cast<const int4*>(rowmax + rb)), w4 = make_int4(0, 0, 0, 0);
+        if (dual) w4 = __ldg(reinterpret_cast<const int4*>(rowmax + dual + rb));
 #pragma unroll 1
         for (int u = 0; u < 4; u++) {
-            const int row = rb + u;
+            const int row = rb + u, hi = m4.x, hiw = w4.x;
             const uint32_t d = d4.x;
             d4 = make_uint4(d4.y, d4.z, d4.w, kZeroRow);
+            m4 = make_int4(m4.y, m4.z, m4.w, 0), w4 = make_int4(w4.y, w4.z, w4.w, 0);
             if (d == kZeroRow) continue;
             double o[16];
             row16(tab, d, g, pia, fa, o);
-            put_digits(o, __ldg(rowmax + row), g, box(row));
+            put_digits(o, hi, g, box(row));
             if (dual) {
 #pragma unroll
                 for (int k = 0; k < 16; k++) o[k] *= vv[k];
-                put_digits(o, __ldg(rowmax + dual + row), g, box(dual + row));
+                put_digits(o, hiw, g, box(dual + row));
             }
         }
     }

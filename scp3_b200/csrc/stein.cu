@@ -113,12 +113,12 @@ __host__ __device__ __forceinline__ int level_pair(int a, int b)
 }
 
 // Table entry of row r for slot l (0..31): slots 8g..8g+3 at 4g..4g+3 and
-// 8g+4..8g+7 at 16+4g..16+4g+3, the two halves swapped on odd rows, so that the
-// 4 threads of an operand row read 64 contiguous bytes per load and rows of
-// different parity fall in different banks.
+// 8g+4..8g+7 at 16+4g..16+4g+3, the two halves swapped where r / 4 is odd: the 4
+// threads of an operand row read 64 contiguous bytes per load, and the next threads' row
+// is four on, its entries mostly too, and so in the other banks.
 __device__ __forceinline__ int sx_col(int r, int l)
 {
-    return ((((l >> 2) & 1) << 4) ^ ((r & 1) << 4)) | ((l >> 3) << 2) | (l & 3);
+    return ((((l >> 2) & 1) << 4) ^ (((r >> 2) & 1) << 4)) | ((l >> 3) << 2) | (l & 3);
 }
 
 // The split operand of a pass: the W rows (reduced function x Stein weight K^m_a0,
@@ -188,7 +188,7 @@ __global__ void __launch_bounds__(kSxThreads) stein_expand_split_kernel(
     const float4* tab4 = reinterpret_cast<const float4*>(tx);
     const int64_t box_k = kb;                                  // the block's 32-slot box
     auto rd = [&](uint32_t i, float4& lo4, float4& hi4) {
-        const uint32_t sw = (i & 1u) << 2;                      // swapped halves (in float4 units)
+        const uint32_t sw = i & 4u;                             // swapped halves (in float4 units)
         lo4 = tab4[i * (kSxSlots / 4) + (sw ^ 0u) + g];
         hi4 = tab4[i * (kSxSlots / 4) + (sw ^ 4u) + g];
     };
