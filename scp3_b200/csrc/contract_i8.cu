@@ -275,8 +275,12 @@ __global__ void __launch_bounds__(kThreads, 1)
             const int et = threadIdx.x - 64;
             cunit[et] = zero_unit(rowmax[(et < kTile ? ti.y : ti.w) + (et & (kTile - 1))]);
             asm volatile("bar.sync 1, %0;" ::"n"(kEpiWarps * 32) : "memory");
-            const double* cu = cunit + half * kTile;
-            double* P = partial + (size_t)u * (size_t)(kTile * kN) + (size_t)half * kTile * kTile + row;
+            // the warp's `span` columns of the tile from cb: a half, or of one panel a
+            // quarter (dimer, 2^14 samples: with four warps at a panel's 128 columns 158.5 us
+            // a pass on one card and 163.9 on another, with eight 156.2 and 153.3)
+            const int span = ti.z ? kTile / 2 : kTile, cb = half * span;
+            const double* cu = cunit + cb;
+            double* P = partial + (size_t)u * (size_t)(kTile * kN) + (size_t)cb * kTile + row;
             for (int r0 = lo; r0 < hi && ok; r0 += kRunKB)
                 for (int t = 0; t < kSweeps; t++, use++) {
                     if (!mbar_wait(acc_full, use & 1, abort)) {
@@ -285,12 +289,11 @@ __global__ void __launch_bounds__(kThreads, 1)
                     }
                     tc_fence_after();
                     const double w = ra * pow2(8 * (5 + 2 * t));     // the larger digit sum: 2^(8 (14 - (9 - 2t)))
-                    const uint32_t base = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(half * kTile);
-                    // a tile of one panel has no second half; rows that are zero throughout
-                    // (padding among them; unit 0) add nothing, unless to values that are
-                    // not finite (unit NaN)
+                    const uint32_t base = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)cb;
+                    // rows that are zero throughout (padding among them; unit 0) add
+                    // nothing, unless to values that are not finite (unit NaN)
 #pragma unroll 1
-                    for (int c0 = 0; c0 < (half && ti.z ? 0 : kTile); c0 += 16) {
+                    for (int c0 = 0; c0 < span; c0 += 16) {
                         double un[16];
                         bool any = false;
 #pragma unroll
