@@ -199,6 +199,7 @@ __global__ void __launch_bounds__(kSxThreads) stein_expand_split_kernel(
     for (int rb = r0 + 4 * rl; rb < r1; rb += kSxThreads) {
         uint32_t pia = 0xffffffffu;
         float4 f0 = make_float4(0.f, 0.f, 0.f, 0.f), f1 = f0;
+        float xs[4] = {};                  // summed rows: this thread's 8 slots
 #pragma unroll
         for (int u = 0; u < 4; u++) {
             const int row = rb + u;
@@ -227,12 +228,7 @@ __global__ void __launch_bounds__(kSxThreads) stein_expand_split_kernel(
                 }
             }
             if (row >= rows) {
-                // a summed row: its 32 values added, in FP32, into this block's partial
-                float x = has ? ((a0.x + a0.y) + (a0.z + a0.w)) + ((a1.x + a1.y) + (a1.z + a1.w)) : 0.0f;
-                const unsigned grp = 0xfu << (threadIdx.x & 28);     // the 4 lanes of this row
-                x += __shfl_xor_sync(grp, x, 1);
-                x += __shfl_xor_sync(grp, x, 2);
-                if (g == 0) spart[(size_t)kb * nsum + (row - rows)] = x;
+                if (has) xs[u] = ((a0.x + a0.y) + (a0.z + a0.w)) + ((a1.x + a1.y) + (a1.z + a1.w));
                 continue;
             }
             if (!has) continue;
@@ -246,6 +242,17 @@ __global__ void __launch_bounds__(kSxThreads) stein_expand_split_kernel(
             const int off = rin * tc::kKBlock2 + ((g ^ ((rin >> 1) & 3)) << 3);
             *reinterpret_cast<uint4*>(box + off) = hi;
             *reinterpret_cast<uint4*>(box + tc::kTile * tc::kKBlock2 + off) = lo;
+        }
+        // summed rows (operand rows are a multiple of 4): the four lanes of four rows add
+        // their shares in FP32 and each keeps one row, so a warp stores 32 consecutive
+        // partials
+        if (rb >= rows) {
+            const unsigned grp = 0xfu << (threadIdx.x & 28);
+            const bool o1 = g & 1, o2 = g & 2;
+            const float y0 = (o1 ? xs[1] : xs[0]) + __shfl_xor_sync(grp, o1 ? xs[0] : xs[1], 1);
+            const float y1 = (o1 ? xs[3] : xs[2]) + __shfl_xor_sync(grp, o1 ? xs[2] : xs[3], 1);
+            const float y = (o2 ? y1 : y0) + __shfl_xor_sync(grp, o2 ? y0 : y1, 2);
+            if (rb + g < r1) spart[(size_t)kb * nsum + (rb + g - rows)] = y;
         }
     }
 }
@@ -479,13 +486,15 @@ __global__ void __launch_bounds__(kTriThreads) stein_pairs_tri_kernel(const int*
 
 // sums[i] += the summed rows' partials of a pass (the last two blocks of every
 // 4096-sample block hold only padding slots and are skipped).  CTA: 32 rows;
-// warp w adds the blocks b = w mod 8 (a coalesced 128-byte read per block), the
-// eight warp sums are then added in warp order, so the result does not depend
-// on scheduling.
-__global__ void __launch_bounds__(256) stein_rowsum_kernel(const float* __restrict__ spart, int nsum, int nblocks,
+// warp w adds the blocks b = w mod 32 (a coalesced 128-byte read per block), the
+// warp sums are then added in warp order, so the result does not depend on scheduling.
+// Latency of its reads: 2352 rows of 2048 blocks 25.8 us with 8 warps, 14.9 with 32.
+constexpr int kRowSumWarps = 32;
+
+__global__ void __launch_bounds__(32 * kRowSumWarps) stein_rowsum_kernel(const float* __restrict__ spart, int nsum, int nblocks,
                                                            double* __restrict__ sums)
 {
-    __shared__ double ws[8][32];
+    __shared__ double ws[kRowSumWarps][32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int i = blockIdx.x * 32 + lane;
     constexpr int kValid = tc::kFlush / kSxSlots;     // 128 sample blocks per 130
@@ -493,7 +502,7 @@ __global__ void __launch_bounds__(256) stein_rowsum_kernel(const float* __restri
     double acc = 0.0;
     if (i < nsum) {
 #pragma unroll 8
-        for (int vb = w; vb < nvalid; vb += 8) {
+        for (int vb = w; vb < nvalid; vb += kRowSumWarps) {
             const int b = vb / kValid * kSxBlocksPerFlush + vb % kValid;
             acc += (double)__ldg(spart + (size_t)b * nsum + i);
         }
@@ -502,7 +511,7 @@ __global__ void __launch_bounds__(256) stein_rowsum_kernel(const float* __restri
     __syncthreads();
     if (w == 0 && i < nsum) {
         double t = 0.0;
-        for (int k = 0; k < 8; k++) t += ws[k][lane];
+        for (int k = 0; k < kRowSumWarps; k++) t += ws[k][lane];
         sums[i] += t;
     }
 }
@@ -1018,7 +1027,7 @@ int stein_pass(const SteinPlan& p, const uint32_t* desc, const double* q, const 
                                                              v, vq, k, p.slots / tc::kKBlock2, p.xop, p.spart);
         SCP3_CUDA(cudaGetLastError());
         if (p.nsum)
-            stein_rowsum_kernel<<<(p.nsum + 31) / 32, 256, 0, s>>>(p.spart, p.nsum, nflush * kSxBlocksPerFlush,
+            stein_rowsum_kernel<<<(p.nsum + 31) / 32, 32 * kRowSumWarps, 0, s>>>(p.spart, p.nsum, nflush * kSxBlocksPerFlush,
                                                                    p.sums);
         SCP3_CUDA(cudaGetLastError());
         const int units = p.ntiles2 * p.nsplit;
