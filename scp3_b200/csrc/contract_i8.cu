@@ -566,6 +566,10 @@ __device__ __forceinline__ void put_digits(const double* o, int hi, int g, uint8
 }
 
 // CTA (x, y): the 32 samples of block x, rows of chunk y (`per` rows, a multiple of 4).
+// Two kernels, and V read from the table like any factor: with V's 16 values kept in
+// registers too it spilled (hexamer, 2^16 samples direct 264 us, now 229, the operand's
+// 1.1 GB alone 172; gradient, 2^15 samples 309 us, now 270, of 206).
+template <bool kDual>
 __global__ void __launch_bounds__(kDigitThreads, 2)
     digits_kernel(const int16_t* __restrict__ entries, int v_entry, const uint32_t* __restrict__ xdesc, int ndesc,
                   int dual, int per, int nm, const double* __restrict__ q, const double* __restrict__ v,
@@ -583,14 +587,13 @@ __global__ void __launch_bounds__(kDigitThreads, 2)
         return x + ((size_t)(row / kTile) * nkb_alloc + kb) * (kDigits * kBox) + rin * kKB +
                ((c ^ ((rin >> 1) & 3)) << 4);
     };
-    double vv[16], fa[16];
-    if (dual) read16(tab, v_entry, g, vv);
+    double fa[16];
     const int r0 = blockIdx.y * per, r1 = min(ndesc, r0 + per);
     for (int rb = r0 + 4 * rl; rb < r1; rb += 2 * kDigitThreads) {
         uint32_t pia = kZeroRow;
         uint4 d4 = __ldg(reinterpret_cast<const uint4*>(xdesc + rb));
         int4 m4 = __ldg(reinterpret_cast<const int4*>(rowmax + rb)), w4 = make_int4(0, 0, 0, 0);
-        if (dual) w4 = __ldg(reinterpret_cast<const int4*>(rowmax + dual + rb));
+        if (kDual) w4 = __ldg(reinterpret_cast<const int4*>(rowmax + dual + rb));
 #pragma unroll 1
         for (int u = 0; u < 4; u++) {
             const int row = rb + u, hi = m4.x, hiw = w4.x;
@@ -601,9 +604,8 @@ __global__ void __launch_bounds__(kDigitThreads, 2)
             double o[16];
             row16(tab, d, g, pia, fa, o);
             put_digits(o, hi, g, box(row));
-            if (dual) {
-#pragma unroll
-                for (int k = 0; k < 16; k++) o[k] *= vv[k];
+            if (kDual) {
+                mul16(tab, v_entry, g, o);
                 put_digits(o, hiw, g, box(dual + row));
             }
         }
@@ -730,7 +732,8 @@ int prepare(const Plan& p, const double* q, const double* v, const double* vq, i
     const int ndesc = described(p), nblk = (int)(k / kS), nx = scan_blocks(p, k);
     SCP3_CUDA(cudaMemsetAsync(p.rowmax, 0, sizeof(int) * (size_t)p.rows, s));
     SCP3_CUDA(cudaFuncSetAttribute(scan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scan_smem(p)));
-    SCP3_CUDA(cudaFuncSetAttribute(digits_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)digits_smem(p)));
+    const auto digits = p.dual ? digits_kernel<true> : digits_kernel<false>;
+    SCP3_CUDA(cudaFuncSetAttribute(digits, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)digits_smem(p)));
     scan_kernel<<<dim3(nx, scan_chunks(p)), kScanThreads, scan_smem(p), s>>>(p.entries, p.v_entry, p.trows, p.xdesc,
                                                                             ndesc, p.dual, p.nsum, p.scan_per, p.nm, q,
                                                                             v, vq, nblk, p.rowmax, p.spart);
@@ -740,7 +743,7 @@ int prepare(const Plan& p, const double* q, const double* v, const double* vq, i
     // all rows of a block in one CTA (the table is built once) where there are blocks enough
     const int want = std::max(1, 4 * p.sms / nblk);
     const int per = std::max(kDigitThreads, ((ndesc + want - 1) / want + 3) / 4 * 4);
-    digits_kernel<<<dim3(nblk, (ndesc + per - 1) / per), kDigitThreads, digits_smem(p), s>>>(
+    digits<<<dim3(nblk, (ndesc + per - 1) / per), kDigitThreads, digits_smem(p), s>>>(
         p.entries, p.v_entry, p.xdesc, ndesc, p.dual, per, p.nm, q, v, vq, p.rowmax, p.nkb, p.x);
     SCP3_CUDA(cudaGetLastError());
     return SCP3GPU_OK;
