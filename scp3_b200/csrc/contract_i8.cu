@@ -121,7 +121,7 @@ __device__ __forceinline__ double zero_unit(int hi) { return hi ? row_unit(hi) :
 __global__ void __launch_bounds__(kThreads, 1)
     contract_i8_kernel(const uint8_t* __restrict__ x, long long nkb_alloc, const int* __restrict__ rowmax,
                        const int4* __restrict__ tiles, int ntiles, int nsplit, int nkb_pass, int units,
-                       double* __restrict__ partial, int* __restrict__ err_flag)
+                       double* __restrict__ partial, int* __restrict__ filled, int* __restrict__ err_flag)
 {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -270,6 +270,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             krange(u, lo, hi);
             const int4 ti = tiles[u % ntiles];
             const double ra = zero_unit(rowmax[ti.x + row]);
+            const bool empty = filled[u] == 0;     // the partial holds nothing yet
             // the columns' units, for the eight warps (the last unit's are no longer read)
             asm volatile("bar.sync 1, %0;" ::"n"(kEpiWarps * 32) : "memory");
             const int et = threadIdx.x - 64;
@@ -288,6 +289,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                         break;
                     }
                     tc_fence_after();
+                    const bool store = empty && r0 == lo && t == 0;
                     const double w = ra * pow2(8 * (5 + 2 * t));     // the larger digit sum: 2^(8 (14 - (9 - 2t)))
                     const uint32_t base = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)cb;
                     // rows that are zero throughout (padding among them; unit 0) add
@@ -298,22 +300,25 @@ __global__ void __launch_bounds__(kThreads, 1)
                         bool any = false;
 #pragma unroll
                         for (int j = 0; j < 16; j++) any |= (un[j] = cu[c0 + j]) != 0.0;
-                        if (!any) continue;
+                        if (!any && !store) continue;
                         int a0[16], a1[16];
                         tmem_ld16x2(base + c0, base + kN + c0, a0, a1);
 #pragma unroll
                         for (int j = 0; j < 16; j++) {
                             // |.| < 2^40: exact through the bits of 1.5 * 2^52
                             const long long d = ((long long)a1[j] << 8) + a0[j] + 0x4338000000000000ll;
-                            if ((w != 0.0 && un[j] != 0.0) || w != w || un[j] != un[j])
-                                add_f64(P + (size_t)(c0 + j) * kTile,
-                                        (__longlong_as_double(d) - 6755399441055744.0) * w * un[j]);
+                            const bool add = (w != 0.0 && un[j] != 0.0) || w != w || un[j] != un[j];
+                            const double val = (__longlong_as_double(d) - 6755399441055744.0) * w * un[j];
+                            double* e = P + (size_t)(c0 + j) * kTile;
+                            if (store) *e = add ? val : 0.0;
+                            else if (add) add_f64(e, val);
                         }
                     }
                     tc_fence_before();
                     __syncwarp();
                     if (lane == 0) mbar_arrive(acc_empty);
                 }
+            if (et == 0 && lo < hi) filled[u] = 1;     // all eight warps have read it
         }
     }
     tc_fence_before();
@@ -692,12 +697,13 @@ int create(Plan& p, const std::vector<uint32_t>& tspec, const std::vector<uint32
     int rc;
     if ((rc = upload(&p.entries, entries.data(), entries.size())) || (rc = upload(&p.xdesc, desc4.data(), desc4.size())) ||
         (rc = upload(&p.tiles, tiles.data(), tiles.size())) || (rc = dalloc(&p.x, xbytes)) ||
-        (rc = dalloc(&p.rowmax, (size_t)rows)) || (rc = dalloc(&p.err, (size_t)1)) ||
+        (rc = dalloc(&p.rowmax, (size_t)rows)) || (rc = dalloc(&p.filled, (size_t)p.nsplit * p.ntiles + 1)) ||
         (rc = dalloc(&p.partial, (size_t)p.nsplit * p.ntiles * kTile * kN)) ||
         (nsum && ((rc = dalloc(&p.spart, (size_t)scan_blocks(p, chunk) * nsum)) || (rc = dalloc(&p.sums, (size_t)nsum))))) {
         destroy(p);
         return rc;
     }
+    p.err = p.filled + (size_t)p.nsplit * p.ntiles;
     // padding rows are never written: zero the row blocks that hold any
     const size_t block = (size_t)p.nkb * kDigits * kBox;
     for (int rb = 0; rb < described(p) / kTile; rb++)
@@ -705,13 +711,13 @@ int create(Plan& p, const std::vector<uint32_t>& tspec, const std::vector<uint32
             SCP3_CUDA(cudaMemset(p.x + rb * block, 0, block));
             if (dual) SCP3_CUDA(cudaMemset(p.x + (rb + dual / kTile) * block, 0, block));
         }
-    SCP3_CUDA(cudaMemset(p.err, 0, sizeof(int)));
+    SCP3_CUDA(cudaMemset(p.filled, 0, sizeof(int) * ((size_t)p.nsplit * p.ntiles + 1)));
     return SCP3GPU_OK;
 }
 
 void destroy(Plan& p)
 {
-    void* ptrs[] = {p.x, p.rowmax, p.entries, p.xdesc, p.tiles, p.partial, p.spart, p.sums, p.err};
+    void* ptrs[] = {p.x, p.rowmax, p.entries, p.xdesc, p.tiles, p.partial, p.spart, p.sums, p.filled};
     for (void* q : ptrs)
         if (q) cudaFree(q);
     p = Plan{};
@@ -719,9 +725,8 @@ void destroy(Plan& p)
 
 int zero(const Plan& p, cudaStream_t s)
 {
-    SCP3_CUDA(cudaMemsetAsync(p.partial, 0, sizeof(double) * (size_t)p.nsplit * p.ntiles * kTile * kN, s));
     if (p.nsum) SCP3_CUDA(cudaMemsetAsync(p.sums, 0, sizeof(double) * (size_t)p.nsum, s));
-    SCP3_CUDA(cudaMemsetAsync(p.err, 0, sizeof(int), s));
+    SCP3_CUDA(cudaMemsetAsync(p.filled, 0, sizeof(int) * ((size_t)p.nsplit * p.ntiles + 1), s));     // and err
     return SCP3GPU_OK;
 }
 
@@ -755,7 +760,7 @@ int contract(const Plan& p, int64_t k, cudaStream_t s)
     const int units = p.ntiles * p.nsplit;
     SCP3_CUDA(cudaFuncSetAttribute(contract_i8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
     contract_i8_kernel<<<std::min(units, p.sms), kThreads, kSmem, s>>>(p.x, (long long)p.nkb, p.rowmax, p.tiles, p.ntiles,
-                                                                       p.nsplit, (int)(k / kKB), units, p.partial, p.err);
+                                                                       p.nsplit, (int)(k / kKB), units, p.partial, p.filled, p.err);
     SCP3_CUDA(cudaGetLastError());
     return SCP3GPU_OK;
 }

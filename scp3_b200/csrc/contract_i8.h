@@ -33,6 +33,10 @@ struct Plan {
     double* partial = nullptr;     // [nsplit][ntiles][128 x 256] tile-local column-major
     double* spart = nullptr;       // [blocks of the scan][nsum]
     double* sums = nullptr;        // [nsum]
+    // per unit (split, tile): whether its partial holds sums.  Resetting clears these
+    // instead of the partials, whose first drain stores; read-outs skip the other units
+    // (dimer, 2^14 samples: 151 us a pass, now 141; hexamer gradient 7893, now 7833).
+    int* filled = nullptr;         // [nsplit][ntiles], then err
     int* err = nullptr;            // a bounded wait expired
 };
 

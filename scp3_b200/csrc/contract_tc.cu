@@ -306,6 +306,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 // the sum over the splits, in order, of unit (split * ntiles + t) at row
 // r % 128 and column 128 h + c % 128 (transposed: row c % 128, column
 // 128 h + r % 128).  `err` (may be null): a non-zero flag makes every element NaN.
+// `filled` (kFilled; [nsplit][ntiles]): units whose flag is zero hold no sums.
 //
 // CTA: 32 x kY elements of a needed block (every part of one above the diagonal, those of
 // a diagonal block that hold upper elements), read along the partials' rows and written to
@@ -314,13 +315,14 @@ __global__ void __launch_bounds__(kThreads, 1)
 // blockDim (32, 8 kGroups): group g of a CTA sums a contiguous share of the splits, the
 // shares then added in order; kY = 8 and four groups for bases of a few tiles, which have
 // up to one split per SM.
-template <int kGroups, int kY>
+template <int kGroups, int kY, bool kFilled>
 __global__ void __launch_bounds__(256 * kGroups) unpack_n256_kernel(const double* __restrict__ partial,
                                                                     const int* __restrict__ block_owner, int nt,
                                                                     int nblk, int ntiles, int nsplit, int nb,
                                                                     double divisor, const double* __restrict__ diag,
                                                                     double zpe, double* __restrict__ M, int64_t ld,
-                                                                    const int* __restrict__ err)
+                                                                    const int* __restrict__ err,
+                                                                    const int* __restrict__ filled)
 {
     constexpr int kParts = kTile / 32 * (kTile / kY);
     __shared__ double v[kGroups][kY][33];
@@ -340,9 +342,12 @@ __global__ void __launch_bounds__(256 * kGroups) unpack_n256_kernel(const double
     const int s1 = nsplit * (g + 1) / kGroups;
     double sum[kY / 8] = {};
 #pragma unroll 8
-    for (int s = nsplit * g / kGroups; s < s1; s++)
+    for (int s = nsplit * g / kGroups; s < s1; s++) {
+        const bool on = !kFilled || __ldg(filled + (size_t)s * ntiles + t) != 0;
 #pragma unroll
-        for (int k = 0; k < kY / 8; k++) sum[k] += P[s * unit + (size_t)(y8 + 8 * k) * kTile];
+        for (int k = 0; k < kY / 8; k++)
+            if (on) sum[k] += P[s * unit + (size_t)(y8 + 8 * k) * kTile];
+    }
 #pragma unroll
     for (int k = 0; k < kY / 8; k++) v[g][y8 + 8 * k][x] = sum[k];
     __syncthreads();
@@ -830,18 +835,18 @@ int launch_contract(const uint16_t* x, int64_t nkb_alloc, const int4* tiles, int
 }
 
 int launch_unpack(const double* partial, const int* owner, int nt, int ntiles, int nsplit, int nb, double divisor,
-                   const double* diag, double zpe, double* M, int64_t ld, cudaStream_t s, const int* err)
+                   const double* diag, double zpe, double* M, int64_t ld, cudaStream_t s, const int* err,
+                   const int* filled)
 {
     const int64_t total = (int64_t)nb * nb;
     if (total <= 0) return SCP3GPU_OK;
     const int nblk = (nb + kTile - 1) / kTile;
     const unsigned grid = (unsigned)(nblk * (nblk + 1) / 2 * 16);
-    if (nsplit < 16)
-        unpack_n256_kernel<1, 32><<<grid, dim3(32, 8), 0, s>>>(partial, owner, nt, nblk, ntiles, nsplit, nb, divisor,
-                                                               diag, zpe, M, ld, err);
-    else
-        unpack_n256_kernel<4, 8><<<4 * grid, dim3(32, 32), 0, s>>>(partial, owner, nt, nblk, ntiles, nsplit, nb,
-                                                                   divisor, diag, zpe, M, ld, err);
+    const bool few = nsplit < 16;
+    const auto kern = few ? (filled ? unpack_n256_kernel<1, 32, true> : unpack_n256_kernel<1, 32, false>)
+                          : (filled ? unpack_n256_kernel<4, 8, true> : unpack_n256_kernel<4, 8, false>);
+    kern<<<few ? grid : 4 * grid, dim3(32, few ? 8 : 32), 0, s>>>(partial, owner, nt, nblk, ntiles, nsplit, nb, divisor,
+                                                                  diag, zpe, M, ld, err, filled);
     SCP3_CUDA(cudaGetLastError());
     return SCP3GPU_OK;
 }

@@ -766,7 +766,7 @@ static int build_dense(scp3gpu_hbuild* h, int mode, double* dst = nullptr, int64
     if (h->split_form) return tc::unpack(h->tcp, h->nb, divisor, diag, zpe, dst, ld, h->stream);
     if (h->gradient) return stein_unpack(h->sp, h->desc, divisor, diag, zpe, dst, ld, h->stream);
     return tc::launch_unpack(h->ip.partial, h->owner, h->nt, h->ip.ntiles, h->ip.nsplit, h->nb, divisor, diag, zpe, dst, ld,
-                             h->stream, h->ip.err);
+                             h->stream, h->ip.err, h->ip.filled);
 }
 
 int scp3gpu_hbuild_read(scp3gpu_hbuild* h, double* M, int64_t ld, int mode)

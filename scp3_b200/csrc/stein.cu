@@ -532,8 +532,10 @@ __global__ void __launch_bounds__(32 * kRowSumWarps) stein_rowsum_kernel(const f
 // with `ct` = column panel pairs, tile-local column-major.  With wb_off (the
 // split form's pair sums as products) the term of a pair exciting m in both
 // functions is C at W_b row (m, rank of r, level of c in m), column
-// red3(c without its mode-m factor).
-template <int kY>
+// red3(c without its mode-m factor).  `filled` (kFilled, the FP64 form): units whose
+// flag is zero hold no sums; their values are read all the same, so that the loads do not
+// wait on the flags, and dropped.
+template <int kY, bool kFilled>
 __global__ void __launch_bounds__(256) stein_unpack_kernel(const uint32_t* __restrict__ desc, const int* __restrict__ rank3,
                                     const int* __restrict__ voff, const int64_t* __restrict__ doff, int nb, int nv,
                                     int ct, int nsplit, int dsplit, const double* __restrict__ C,
@@ -542,7 +544,8 @@ __global__ void __launch_bounds__(256) stein_unpack_kernel(const uint32_t* __res
                                     double zpe, double* __restrict__ M, int64_t ld,
                                     const int* __restrict__ tile_of, const int* __restrict__ red3,
                                     const int* __restrict__ wb_off, const int* __restrict__ sum_off,
-                                    const double* __restrict__ sums, const int* __restrict__ err)
+                                    const double* __restrict__ sums, const int* __restrict__ err,
+                                    const int* __restrict__ filled)
 {
     // CTA: 32 rows x kY columns of block (a, b) of 32 x 32 elements, a <= b, row-major over
     // the upper blocks; thread (x, y) forms (r, c) = (r0 + x, c0 + y) and columns y + 8, ...;
@@ -563,7 +566,17 @@ __global__ void __launch_bounds__(256) stein_unpack_kernel(const uint32_t* __res
     auto csum = [&](int64_t x) {
         if (x < 0) return __longlong_as_double(0x7ff8000000000000ll);
         double t = 0.0;
-        for (int s = 0; s < nsplit; s++) t += C[s * csize + x];
+        if (kFilled) {
+            const int64_t nt = csize / (128 * 256);
+            const int* fl = filled + x / (128 * 256);
+#pragma unroll 4
+            for (int s = 0; s < nsplit; s++) {
+                const double c = C[s * csize + x];
+                t += __ldg(fl + s * nt) ? c : 0.0;
+            }
+        } else {
+            for (int s = 0; s < nsplit; s++) t += C[s * csize + x];
+        }
         return t;
     };
     const int x = threadIdx.x & 31, y8 = threadIdx.x >> 5;
@@ -1078,7 +1091,8 @@ int stein_unpack(const SteinPlan& p, const uint32_t* desc, double divisor, const
     const int nblk = (p.nb + 31) / 32;
     const unsigned grid = (unsigned)(nblk * (nblk + 1) / 2);
     const bool fine = grid < 600;       // fewer CTAs than a GPU holds: a quarter of the columns each
-    auto kern = fine ? stein_unpack_kernel<8> : stein_unpack_kernel<32>;
+    auto kern = p.split ? (fine ? stein_unpack_kernel<8, false> : stein_unpack_kernel<32, false>)
+                        : (fine ? stein_unpack_kernel<8, true> : stein_unpack_kernel<32, true>);
     if (p.split) {
         int err = 0;
         SCP3_CUDA(cudaMemcpyAsync(&err, p.err, sizeof(int), cudaMemcpyDeviceToHost, s));
@@ -1089,7 +1103,8 @@ int stein_unpack(const SteinPlan& p, const uint32_t* desc, double divisor, const
                                              p.split ? p.P : p.ip.partial, p.D, (int64_t)p.ntiles2 * 128 * 256, p.dsize,
                                              divisor, diag, zpe, M, ld, p.tile_of, p.red3,
                                              p.tcpairs ? p.wb_off : nullptr, p.nsum ? p.sum_off : nullptr,
-                                             p.split ? p.sums : p.ip.sums, p.split ? p.err : p.ip.err);
+                                             p.split ? p.sums : p.ip.sums, p.split ? p.err : p.ip.err,
+                                             p.split ? nullptr : p.ip.filled);
     SCP3_CUDA(cudaGetLastError());
     return SCP3GPU_OK;
 }

@@ -83,9 +83,11 @@ int launch_contract(const uint16_t* x, int64_t nkb_alloc, const int4* tiles, int
                     const int* neg, bool f16, double* partial, int* err_flag, int grid, cudaStream_t s,
                     int u_begin = 0, int u_end = -1);
 // dense column-major nb x nb of one cluster (its block-owner table) from the unit partials;
-// NaN throughout when the flag err (may be null) is set
+// NaN throughout when the flag err (may be null) is set; units whose flag in filled
+// ([nsplit][ntiles], may be null) is zero count as zero
 int launch_unpack(const double* partial, const int* owner, int nt, int ntiles, int nsplit, int nb, double divisor,
-                  const double* diag, double zpe, double* M, int64_t ld, cudaStream_t s, const int* err = nullptr);
+                  const double* diag, double zpe, double* M, int64_t ld, cudaStream_t s, const int* err = nullptr,
+                  const int* filled = nullptr);
 constexpr int kKBlock2 = 32;      // K slots per k-block of the 128 x 256 contraction's operand
 
 }  // namespace tc

@@ -123,3 +123,28 @@ def test_gradient_products(api, n3):
     iu = np.triu_indices(hb.nb)
     # terms of one sample are at most ~50 |V| or |Vq|; n 2^-51 of the rows' largest as above
     assert np.abs(M[iu] - ref[iu]).max() <= n * 2.0 ** -51 * 50 * 50 * max(np.abs(V).max(), np.abs(Vq).max())
+
+
+@pytest.mark.parametrize("estimator", ["direct", "gradient"])
+@pytest.mark.parametrize("nm,n", [(9, 1), (12, 65), (12, 4097)])
+def test_reset_leaves_nothing(api, estimator, nm, n):
+    """After a reset the sums are those of a new handle, bit for bit, also where the next
+    pass is too small to reach every unit of the plan; passes add up; nothing
+    accumulated reads as zero."""
+    c = load_hbuild_case("dimer_qtip4pf")
+    new = lambda: api.HBuild(2, c["x0"], c["MUa"], c["omega"], modes=np.arange(nm), n2=nm, n3=0, estimator=estimator)
+    hb = new()
+    assert not hb.read(0).any()
+    hb.accumulate(3, 20000)
+    full = hb.read(0)
+    hb.reset()
+    assert not hb.read(0).any()
+    hb.accumulate(50000, n)
+    small = hb.read(0)
+    other = new()
+    other.accumulate(50000, n)
+    assert np.array_equal(small, other.read(0)) and small.any()
+    hb.accumulate(3, 20000)
+    both = hb.read(0)
+    # two sums of FP64 values: a rounding of each of at most 148 partials
+    assert np.abs(both - (full + small)).max() <= 150 * 2.0 ** -53 * (np.abs(full) + np.abs(small)).max() * 2
