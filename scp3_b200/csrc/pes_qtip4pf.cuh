@@ -68,19 +68,20 @@ __device__ __forceinline__ double water_pair(int a, int b, const T* crd, const T
         s[0][3][k] = ms[3 * a + k];
         s[1][3][k] = ms[3 * b + k];
     }
+    // a site of one water with the other's three charges, which add up to zero: the sums
+    // stay small
     double e = 0.0;
 #pragma unroll
-    for (int w = 0; w < 2; w++)
+    for (int l = 1; l < 4; l++) {
+        const double ql = l == 3 ? kQM : kQH;
+        double t = (double)(T(ql * kQM) * inv_sqrt(dist2(s[0][l], s[1][3])));
 #pragma unroll
-        for (int l = 1; l < 3; l++) e += (double)(T(kQH * kQM) * inv_sqrt(dist2(s[w][3], s[1 - w][l])));
-#pragma unroll
-    for (int l = 1; l < 3; l++)
-#pragma unroll
-        for (int m = 1; m < 3; m++) e += (double)(T(kQH * kQH) * inv_sqrt(dist2(s[0][l], s[1][m])));
+        for (int m = 1; m < 3; m++) t += (double)(T(ql * kQH) * inv_sqrt(dist2(s[0][l], s[1][m])));
+        e += t;
+    }
     const T s2 = T(kSigma * kSigma) / dist2(s[0][0], s[1][0]);
     const T s6 = s2 * s2 * s2;
     e += (double)(T(4 * kEpsilon) * s6 * (s6 - T(1)));
-    e += (double)(T(kQM * kQM) * inv_sqrt(dist2(s[0][3], s[1][3])));
     return e;
 }
 
@@ -202,20 +203,20 @@ __device__ double energy_grad_warp4(const T* crd, int stride, T* ms, double* g, 
                     for (int l = 0; l < 3; l++) o[l][k] = cj[9 * b + 3 * l + k];
                     o[3][k] = mj[3 * b + k];
                 }
-                auto coulomb = [&](T qq, int x, int y) {
+                auto coulomb = [&](T qq, int x, int y) -> double {
                     const T d0 = s[x][0] - o[y][0], d1 = s[x][1] - o[y][1], d2 = s[x][2] - o[y][2];
                     const T ir = inv_sqrt(d0 * d0 + d1 * d1 + d2 * d2), eu = qq * ir, fu = -eu * (ir * ir);
                     f[x][0] += fu * d0, f[x][1] += fu * d1, f[x][2] += fu * d2;
-                    e += (double)eu;
+                    return (double)eu;
                 };
 #pragma unroll
-                for (int l = 1; l < 3; l++) {
-                    coulomb(T(kQH * kQM), 3, l);
-                    coulomb(T(kQH * kQM), l, 3);
-                    coulomb(T(kQH * kQH), l, 1);
-                    coulomb(T(kQH * kQH), l, 2);
+                for (int l = 1; l < 4; l++) {       // neutral groups, as in water_pair
+                    const double ql = l == 3 ? kQM : kQH;
+                    double t = coulomb(T(ql * kQM), l, 3);
+                    t += coulomb(T(ql * kQH), l, 1);
+                    t += coulomb(T(ql * kQH), l, 2);
+                    e += t;
                 }
-                coulomb(T(kQM * kQM), 3, 3);
                 const T d0 = s[0][0] - o[0][0], d1 = s[0][1] - o[0][1], d2 = s[0][2] - o[0][2];
                 const T ir2 = T(1.0) / (d0 * d0 + d1 * d1 + d2 * d2);
                 const T s2 = T(kSigma * kSigma) * ir2, s6 = s2 * s2 * s2;
