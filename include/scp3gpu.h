@@ -113,8 +113,8 @@ typedef struct scp3gpu_config {
     int chunk;              /* samples per device pass; multiple of 4096, 0 = auto:
                                2^18 for the split forms (halved while one pass's
                                operand would exceed ~6 GB); 2^16 for the FP64 form
-                               (halved while its Phi and W would exceed ~4 GB); for
-                               the gradient estimator 2^14 (FP64 products) or 2^16
+                               (halved while its digits would exceed ~4 GB); for
+                               the gradient estimator 2^15 (FP64 products) or 2^16
                                (BF16x3 products), halved while a pass's operands
                                would exceed ~4 GB                                     */
     int device;             /* CUDA device ordinal                                     */
