@@ -34,6 +34,21 @@ def test_read_equals_read_dev(api, n2, pad):
     assert np.isnan(out[hb.nb:]).all()
 
 
+@pytest.mark.parametrize("pad", [0, 7])
+def test_read_into_pinned_memory(api, pad):
+    """A pinned destination takes one copy: the same bytes as a pageable one, padding untouched."""
+    import torch
+    from scp3_b200 import inputs
+    nw, x0, MUa, omega = inputs.load("prism_qtip4pf")
+    hb = api.HBuild(nw, x0, MUa, omega, n2=48, precision="bf16x3", chunk=4096)
+    hb.accumulate(3, 4096)
+    block = torch.full((hb.nb, hb.nb + pad), float("nan"), dtype=torch.float64).pin_memory()
+    out = block.numpy().T
+    hb.read(1, out=out)
+    assert np.array_equal(out[:hb.nb], hb.read(1))
+    assert np.isnan(out[hb.nb:]).all()
+
+
 # one call's buffers within a pool slot's pinned memory, its device memory, and neither
 @pytest.mark.parametrize("n", [3, 20000, 60000])
 def test_potential_from_several_threads(api, n):
