@@ -23,6 +23,9 @@
 // sweep count reads 501 and the caller counts the sample as not converged (the
 // reference only asserts, and not under NDEBUG, ttm3f.cpp:309).
 #pragma once
+#include <cstring>
+#include <vector>
+
 #include "common.cuh"
 
 namespace scp3 {
@@ -115,11 +118,35 @@ struct TailTable {
 };
 __device__ TailTable kTail;
 
+// Interval of x, 0 .. kTailSpans - 1; -1 where the table has none: below 1.5, past the
+// last one, and for a NaN (coincident sites, coordinates that are not finite).  Two
+// intervals per octave: exponent and first bit of the fraction, from 1.5 on.
+template <typename T>
+__host__ __device__ __forceinline__ int tail_span(T x)
+{
+    constexpr bool F = sizeof(T) == 4;
+    if (!(x >= T(1.5) && x <= T(F ? 17.0 : 37.0))) return -1;
+#ifdef __CUDA_ARCH__
+    if constexpr (F) return (__float_as_int(x) >> 22) - 255;
+    else return (__double2hiint(x) >> 19) - 2047;
+#else
+    // the same bits by way of memory
+    if constexpr (F) {
+        int32_t b;
+        std::memcpy(&b, &x, sizeof(b));
+        return (b >> 22) - 255;
+    } else {
+        int64_t b;
+        std::memcpy(&b, &x, sizeof(b));
+        return (int)(b >> 51) - 2047;
+    }
+#endif
+}
+
 template <typename T>
 __device__ __forceinline__ T smear_tail(T x, T e1, T x13)
 {
     constexpr bool F = sizeof(T) == 4;
-    if (x > T(F ? 17.0 : 37.0)) return T(0);
     if (x < T(1.5)) {
         T s = T(0);
 #pragma unroll
@@ -129,10 +156,8 @@ __device__ __forceinline__ T smear_tail(T x, T e1, T x13)
         }
         return e1 * (T(1) + x * s) - x13 * T(kGamma23);
     }
-    // two intervals per octave: exponent and first bit of the fraction, from 1.5 on
-    int i;
-    if constexpr (F) i = (__float_as_int(x) >> 22) - 255;
-    else i = (__double2hiint(x) >> 19) - 2047;
+    const int i = tail_span(x);
+    if (i < 0) return x > T(1.5) ? T(0) : x;       // past the table; a NaN stays one
     T s;
     if constexpr (F) {
         const T t = x * __ldg(kTail.scalef + i) - __ldg(kTail.shiftf + i);

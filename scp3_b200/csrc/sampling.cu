@@ -708,6 +708,13 @@ int launch_std_normal(int dims, int64_t index0, int64_t n, const int64_t* vdir, 
 
 }  // namespace scp3
 
+// Host-only view of TTM3-F's smearing table, for tests: the interval (0..9) x is looked
+// up in, -1 where the table is not read.
+extern "C" int scp3gpu_internal_tail_span(double x, int fp32)
+{
+    return fp32 ? scp3::ttm::tail_span((float)x) : scp3::ttm::tail_span(x);
+}
+
 // Host-only view of the water-pair items of the four-sample qTIP4P/f kernels, for
 // tests: ab[2 p], ab[2 p + 1] = the waters a < b of pair p, p < nw (nw - 1) / 2.
 extern "C" int scp3gpu_internal_water_pairs(int nw, int* ab)
