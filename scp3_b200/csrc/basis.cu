@@ -66,8 +66,7 @@ int launch_expand_fp64(const uint32_t* desc, int nb, int nb_pad, int nm, const d
 {
     if (n <= 0) return SCP3GPU_OK;
     const size_t sm = sizeof(double) * nm * kExpSamples;
-    if (sm > 48 * 1024)
-        SCP3_CUDA(cudaFuncSetAttribute(expand_fp64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    if (int rc = allow_smem(expand_fp64_kernel)) return rc;
     dim3 grid((unsigned)((n + kExpSamples - 1) / kExpSamples), (unsigned)((nb_pad + kExpRows - 1) / kExpRows));
     expand_fp64_kernel<<<grid, kExpSamples, sm, s>>>(desc, nb, nb_pad, nm, q, v, n, ldk, phi, w);
     SCP3_CUDA(cudaGetLastError());

@@ -736,9 +736,9 @@ int prepare(const Plan& p, const double* q, const double* v, const double* vq, i
     if (k > p.chunk || k % kKB) return fail(SCP3GPU_ERR_ARG, "contract_i8: pass not in k-blocks");
     const int ndesc = described(p), nblk = (int)(k / kS), nx = scan_blocks(p, k);
     SCP3_CUDA(cudaMemsetAsync(p.rowmax, 0, sizeof(int) * (size_t)p.rows, s));
-    SCP3_CUDA(cudaFuncSetAttribute(scan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scan_smem(p)));
     const auto digits = p.dual ? digits_kernel<true> : digits_kernel<false>;
-    SCP3_CUDA(cudaFuncSetAttribute(digits, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)digits_smem(p)));
+    if (int rc = allow_smem(scan_kernel)) return rc;
+    if (int rc = allow_smem(digits)) return rc;
     scan_kernel<<<dim3(nx, scan_chunks(p)), kScanThreads, scan_smem(p), s>>>(p.entries, p.v_entry, p.trows, p.xdesc,
                                                                             ndesc, p.dual, p.nsum, p.scan_per, p.nm, q,
                                                                             v, vq, nblk, p.rowmax, p.spart);
@@ -758,7 +758,7 @@ int contract(const Plan& p, int64_t k, cudaStream_t s)
 {
     if (k <= 0) return SCP3GPU_OK;
     const int units = p.ntiles * p.nsplit;
-    SCP3_CUDA(cudaFuncSetAttribute(contract_i8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
+    if (int rc = allow_smem(contract_i8_kernel)) return rc;
     contract_i8_kernel<<<std::min(units, p.sms), kThreads, kSmem, s>>>(p.x, (long long)p.nkb, p.rowmax, p.tiles, p.ntiles,
                                                                        p.nsplit, (int)(k / kKB), units, p.partial, p.filled, p.err);
     SCP3_CUDA(cudaGetLastError());

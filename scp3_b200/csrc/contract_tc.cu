@@ -828,7 +828,7 @@ int launch_contract(const uint16_t* x, int64_t nkb_alloc, const int4* tiles, int
 {
     if (u_end < 0) u_end = ntiles * nsplit;
     if (ntiles <= 0 || nsplit <= 0 || grid <= 0 || u_end <= u_begin) return SCP3GPU_OK;
-    SCP3_CUDA(cudaFuncSetAttribute(contract_n256_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes2));
+    if (int rc = allow_smem(contract_n256_kernel)) return rc;
     contract_n256_kernel<<<grid, kThreads, kSmemBytes2, s>>>(x, (long long)nkb_alloc, tiles, ntiles, nsplit, nkb_pass,
                                                              u_begin, u_end, neg, (int)f16, partial,
                                                              err_flag);
@@ -896,7 +896,6 @@ int create(Plan& p, int nb, int nm, int n2_for_factors, int n3_for_factors, int 
     SCP3_CUDA(cudaMalloc(&p.partial, sizeof(double) * (size_t)p.nsplit * p.ntiles * kTile * kN2));
     SCP3_CUDA(cudaMalloc(&p.err_flag, sizeof(int)));
     SCP3_CUDA(cudaMemset(p.err_flag, 0, sizeof(int)));
-    SCP3_CUDA(cudaFuncSetAttribute(contract_n256_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes2));
     return SCP3GPU_OK;
 }
 
@@ -937,7 +936,7 @@ int launch_expand(const ExpandDesc* descs_dev, int nclusters, int max_nb_pad, in
     const bool staged = expand_smem(max_nm, true) <= kMaxSmem;
     const size_t sm = expand_smem(max_nm, staged);
     auto kern = f16 ? expand_split_kernel<true> : expand_split_kernel<false>;
-    if (sm > 48 * 1024) SCP3_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    if (int rc = allow_smem(kern)) return rc;
     int dev = 0, sms = 148, per = 0;
     SCP3_CUDA(cudaGetDevice(&dev));
     SCP3_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));

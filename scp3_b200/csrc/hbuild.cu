@@ -32,6 +32,32 @@ int cuda_fail(cudaError_t e, const char* what)
     return e == cudaErrorMemoryAllocation ? SCP3GPU_ERR_NOMEM : SCP3GPU_ERR_CUDA;
 }
 
+int allow_smem_of(const void* kernel)
+{
+    // no heap: the calls that allocate nothing come here too
+    constexpr int kKernels = 64, kDevices = 128;
+    static std::mutex mu;
+    static struct {
+        const void* kernel;
+        uint64_t devices[kDevices / 64];
+    } done[kKernels];
+    int dev = 0, most = 0, k = 0;
+    SCP3_CUDA(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> lock(mu);
+    while (k < kKernels && done[k].kernel && done[k].kernel != kernel) k++;
+    const bool room = k < kKernels && dev < kDevices;
+    if (room && ((done[k].devices[dev / 64] >> (dev % 64)) & 1)) return SCP3GPU_OK;
+    cudaFuncAttributes at{};
+    SCP3_CUDA(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    SCP3_CUDA(cudaFuncGetAttributes(&at, kernel));
+    SCP3_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)at.sharedSizeBytes));
+    if (room) {
+        done[k].kernel = kernel;
+        done[k].devices[dev / 64] |= 1ull << (dev % 64);
+    }
+    return SCP3GPU_OK;
+}
+
 }  // namespace scp3
 
 using namespace scp3;

@@ -26,6 +26,17 @@ int cuda_fail(cudaError_t e, const char* what);
     } while (0)
 
 // ---------------------------------------------------------------- device helpers
+// Lets a kernel use all the dynamic shared memory a CTA of the current device can have,
+// once per kernel and device.  The limit belongs to the function, not to the launch: a
+// handle that set it to its own need would lower it between another thread's set and
+// launch, or under an older handle.
+int allow_smem_of(const void* kernel);
+template <typename K>
+inline int allow_smem(K* kernel)
+{
+    return allow_smem_of(reinterpret_cast<const void*>(kernel));
+}
+
 template <typename T>
 inline int dalloc(T** p, size_t count)
 {

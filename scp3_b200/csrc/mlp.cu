@@ -220,7 +220,7 @@ int launch_layer(const __nv_bfloat16* X, const __nv_bfloat16* W, const float* b,
 {
     if (N % 32 || N > 256 || K % 32 || K > 256) return fail(SCP3GPU_ERR_ARG, "mlp layer: shape out of range");
     const size_t sm = tc_smem_bytes(N, K);
-    SCP3_CUDA(cudaFuncSetAttribute(gemm_bias_gelu_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    if (int rc = allow_smem(gemm_bias_gelu_tc)) return rc;
     int dev = 0, sms = 148;
     SCP3_CUDA(cudaGetDevice(&dev));
     SCP3_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));

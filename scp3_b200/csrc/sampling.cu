@@ -556,7 +556,7 @@ int launch_samples_t(const SampleArgs& a, cudaStream_t s)
     auto kern = a.vq ? samples_kernel<PES, T, kGrad> : samples_kernel<PES, T, false>;
     if constexpr (PES == SCP3GPU_PES_TTM3F)
         if (a.nw <= 4) kern = a.vq ? samples_kernel<PES, T, kGrad, 4> : samples_kernel<PES, T, false, 4>;
-    if (sm > 48 * 1024) SCP3_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    if (int rc = allow_smem(kern)) return rc;
     kern<<<sample_grid(kern, sm, a.n), kWarpsPerBlock * 32, sm, s>>>(a);
     SCP3_CUDA(cudaGetLastError());
     return SCP3GPU_OK;
@@ -577,8 +577,7 @@ int launch_samples_batch_t(const SampleArgs* args_host, const SampleArgs* args_d
         if (b <= kMuaSmemMax) mua = std::max(mua, b);
     }
     const size_t sm = kWarpsPerBlock * slot_bytes<T>(PES, nm0, nw, false) + mua;
-    if (sm > 48 * 1024) SCP3_CUDA(cudaFuncSetAttribute(samples_batch_kernel<PES, T>,
-                                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    if (int rc = allow_smem(samples_batch_kernel<PES, T>)) return rc;
     const int per = grid_for((n + kRun - 1) / kRun);   // per cluster; the clusters share the SMs
     samples_batch_kernel<PES, T><<<dim3((unsigned)per, (unsigned)ncl), kWarpsPerBlock * 32, sm, s>>>(args_dev);
     SCP3_CUDA(cudaGetLastError());
@@ -684,7 +683,7 @@ int launch_scp1_samples(int pes, const Scp1Args& a, cudaStream_t s)
     const size_t sm = round16(sizeof(double) * a.dim * a.dim) + kS1Warps * scp1_slot(pes, a.nw, a.dim);
     auto kern = pes == SCP3GPU_PES_QTIP4PF ? scp1_samples_kernel<SCP3GPU_PES_QTIP4PF>
                                             : scp1_samples_kernel<SCP3GPU_PES_TTM3F>;
-    SCP3_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    if (int rc = allow_smem(kern)) return rc;
     int dev = 0, sms = 148, per = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);

@@ -232,7 +232,7 @@ int scp3gpu_scp1_average(scp3gpu_scp1* h, const double* q, const double* d, cons
         const int64_t n = std::min<int64_t>(h->chunk, i1 - c0);
         Scp1Args a{h->nw, dim, h->q, h->sqd, h->U, h->vdir, skip + c0, n, h->V, h->G, h->D, h->capped};
         if ((rc = launch_scp1_samples(h->pes, a, s))) return rc;
-        SCP3_CUDA(cudaFuncSetAttribute(scp1_reduce_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRedSmem));
+        if ((rc = allow_smem(scp1_reduce_kernel))) return rc;
         scp1_reduce_kernel<<<h->blocks, kRedThreads, kRedSmem, s>>>(dim, n, h->V, h->G, h->D, h->P);
         SCP3_CUDA(cudaGetLastError());
     }

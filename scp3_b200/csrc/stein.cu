@@ -982,10 +982,6 @@ int stein_create(SteinPlan& p, const std::vector<uint32_t>& desc, int nm, int64_
             SCP3_CUDA(cudaMemset(p.spart, 0,
                                  sizeof(float) * (size_t)(chunk / tc::kFlush) * kSxBlocksPerFlush * p.nsum));
         SCP3_CUDA(cudaMemset(p.err, 0, sizeof(int)));
-        const size_t es = sizeof(float) * ((size_t)p.trows * kSxSlots + 2 * (size_t)nm * kSxLd + kSxSlots);
-        if (es > 48 * 1024)
-            SCP3_CUDA(cudaFuncSetAttribute(stein_expand_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)es));
     }
     if ((rc = upload(&p.vrdesc, vrdesc.data(), vrdesc.size())) || (rc = upload(&p.rank3, rank3.data(), rank3.size())) ||
         (rc = upload(&p.voff, voff.data(), voff.size())) || (rc = upload(&p.doff, doff.data(), doff.size())) ||
@@ -1044,6 +1040,7 @@ int stein_pass(const SteinPlan& p, const uint32_t* desc, const double* q, const 
         const int vrows = rows + p.nsum;   // operand rows, then summed rows
         const int ny = (vrows + 16383) / 16384, per = (int)round_up((vrows + ny - 1) / ny, 64);
         dim3 eg((unsigned)(nflush * kSxBlocksPerFlush), (unsigned)ny);
+        if ((rc = allow_smem(stein_expand_split_kernel))) return rc;
         stein_expand_split_kernel<<<eg, kSxThreads, es, s>>>(p.tspec, p.trows, p.xdesc, rows, p.nsum, per, p.nm, q,
                                                              v, vq, k, p.slots / tc::kKBlock2, p.xop, p.spart);
         SCP3_CUDA(cudaGetLastError());
@@ -1065,8 +1062,7 @@ int stein_pass(const SteinPlan& p, const uint32_t* desc, const double* q, const 
     if (p.tcpairs) return SCP3GPU_OK;      // the pair sums were part of the products
     if (p.ndtasks) {
         const size_t ps = sizeof(double) * ((size_t)kPS * p.nm + 2 * kPS + 2 * kPS * kPT + 16 * kPS);
-        if (ps > 48 * 1024)
-            SCP3_CUDA(cudaFuncSetAttribute(stein_pairs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ps));
+        if ((rc = allow_smem(stein_pairs_kernel))) return rc;
         dim3 pg((unsigned)p.ndtasks, (unsigned)p.dsplit);
         stein_pairs_kernel<<<pg, 256, ps, s>>>(p.dtasks, p.vrdesc, p.voff, p.doff, p.nm, q, v, vq, k / p.dsplit,
                                                p.dsize, p.D);
@@ -1074,9 +1070,7 @@ int stein_pass(const SteinPlan& p, const uint32_t* desc, const double* q, const 
     }
     if (p.nftasks) {
         const size_t fsm = sizeof(double) * ((size_t)kFS * p.nm + 2 * kFS + (size_t)kFS * kTriMax + 16 * kFS);
-        if (fsm > 48 * 1024)
-            SCP3_CUDA(cudaFuncSetAttribute(stein_pairs_tri_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)fsm));
+        if ((rc = allow_smem(stein_pairs_tri_kernel))) return rc;
         dim3 fg((unsigned)p.nftasks, (unsigned)p.dsplit);
         stein_pairs_tri_kernel<<<fg, kTriThreads, fsm, s>>>(p.ftasks, p.vrdesc, p.voff, p.doff, p.nm, q, v, vq,
                                                             k / p.dsplit, p.dsize, p.D);

@@ -1,0 +1,70 @@
+"""A handle belongs to one host thread; several threads build with handles of their own."""
+import threading
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def api():
+    import torch
+    assert torch.cuda.is_available()
+    import scp3_b200
+    return scp3_b200
+
+
+def build(api, name, precision, estimator, nm, n2, n3, pes="qtip4pf"):
+    from scp3_b200 import inputs
+    nw, x0, MUa, omega = inputs.load(name)
+    return api.HBuild(nw, x0, MUa, omega, modes=np.arange(omega.size)[-nm:], n2=n2, n3=n3, pes=pes,
+                      precision=precision, estimator=estimator)
+
+
+# small and large tables and operands beside one another
+@pytest.mark.parametrize("estimator,precision", [("direct", "fp64"), ("gradient", "fp64"), ("gradient", "bf16x3"),
+                                                 ("direct", "bf16x3")])
+def test_two_handles_in_two_threads(api, estimator, precision):
+    sizes = [("cluster_2_800", 3, 3, 0), ("cluster_6_100", 40, 12, 2)]
+    rounds, out, errors = 300, [None, None], []
+    want = []
+    for s in sizes:
+        h = build(api, s[0], precision, estimator, *s[1:])
+        h.accumulate(100, 500)
+        want.append(h.read(0))
+        h.close()
+    gate = threading.Barrier(2)
+
+    def work(k):
+        try:
+            h = build(api, sizes[k][0], precision, estimator, *sizes[k][1:])
+            gate.wait()
+            for _ in range(rounds):
+                h.reset()
+                h.accumulate(100, 500)
+            out[k] = h.read(0)
+            h.close()
+        except Exception as e:
+            errors.append(e)
+
+    ts = [threading.Thread(target=work, args=(k,)) for k in range(2)]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    assert not errors, errors
+    for k in range(2):
+        assert np.array_equal(out[k], want[k])
+
+
+def test_smaller_handle_leaves_the_larger_one(api):
+    """A second, smaller handle does not take shared memory from the first one's kernels."""
+    first = build(api, "cluster_8_0", "bf16x3", "gradient", 66, 66, 0)
+    first.accumulate(100, 300)
+    want = first.read(0)
+    second = build(api, "cluster_7_500", "bf16x3", "gradient", 57, 57, 0)
+    second.accumulate(100, 300)
+    first.reset()
+    first.accumulate(100, 300)
+    assert np.array_equal(first.read(0), want)
