@@ -197,8 +197,8 @@ int scp3gpu_scp1_create(int pes, int nw, int64_t chunk, int device, scp3gpu_scp1
         delete h;
         return rc;
     }
-    if (cudaMemset(h->capped, 0, sizeof(*h->capped)) != cudaSuccess ||
-        cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) != cudaSuccess) {
+    if (cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) != cudaSuccess ||
+        cudaMemsetAsync(h->capped, 0, sizeof(*h->capped), h->stream) != cudaSuccess) {
         free_all(h);
         delete h;
         return fail(SCP3GPU_ERR_CUDA, "scp1: stream creation failed");

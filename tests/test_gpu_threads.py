@@ -68,3 +68,34 @@ def test_smaller_handle_leaves_the_larger_one(api):
     first.reset()
     first.accumulate(100, 300)
     assert np.array_equal(first.read(0), want)
+
+
+def test_new_handle_beside_default_stream_work(api):
+    """A new handle's buffers are cleared before its first pass, also while another thread
+    keeps the default stream busy: the same matrix, bit for bit."""
+    import torch
+    h = build(api, "cluster_6_100", "fp64", "direct", 48, 10, 0)
+    h.accumulate(100, 1 << 17)
+    want = h.read(0)
+    h.close()
+    stop = threading.Event()
+
+    def busy():
+        a = torch.randn(2048, 2048, device="cuda")
+        while not stop.is_set():
+            for _ in range(20):
+                torch.mm(a, a)
+            torch.cuda.current_stream().synchronize()
+
+    t = threading.Thread(target=busy)
+    t.start()
+    try:
+        for _ in range(8):
+            h = build(api, "cluster_6_100", "fp64", "direct", 48, 10, 0)
+            h.accumulate(100, 1 << 17)
+            got = h.read(0)
+            h.close()
+            assert np.array_equal(got, want)
+    finally:
+        stop.set()
+        t.join()
