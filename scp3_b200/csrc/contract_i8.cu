@@ -56,8 +56,8 @@ constexpr int kDigits = 7, kSweeps = 4, kTile = 128, kN = 256;
 constexpr int kBox = kTile * kKB;                  // 8 KB: one digit of 128 rows x 64 samples
 constexpr int kSlot = 3 * kBox, kRing = 9;         // A box, two B boxes
 constexpr int kRunKB = 288;                        // k-blocks per run: 7 * 2^14 * 18432 < 2^31
-constexpr int kSmem = kRing * kSlot + 1024 + 256 + kN * (int)sizeof(double);
 constexpr int kThreads = 320, kEpiWarps = 8;
+constexpr int kSmem = kRing * kSlot + 1024 + 256 + kEpiWarps * kTile * (int)sizeof(double);
 // kind::i8: D S32, A and B signed 8-bit, K-major
 constexpr uint32_t kIdesc = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kN >> 3) << 17) |
                             ((uint32_t)(kTile >> 4) << 24);
@@ -132,7 +132,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     uint64_t* drain = acc_empty + 1;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain + 1);
     volatile int* abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
-    double* cunit = reinterpret_cast<double*>(smem + kRing * kSlot + 256);    // [256] units of the tile's columns
+    double* cunit = reinterpret_cast<double*>(smem + kRing * kSlot + 256);    // [8 warps][128] units of a warp's columns
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     auto krange = [&](int u, int& lo, int& hi) {
@@ -271,20 +271,22 @@ __global__ void __launch_bounds__(kThreads, 1)
             const int4 ti = tiles[u % ntiles];
             const double ra = zero_unit(rowmax[ti.x + row]);
             const bool empty = filled[u] == 0;     // the partial holds nothing yet
-            // the columns' units, for the eight warps (the last unit's are no longer read)
-            asm volatile("bar.sync 1, %0;" ::"n"(kEpiWarps * 32) : "memory");
-            const int et = threadIdx.x - 64;
-            cunit[et] = zero_unit(rowmax[(et < kTile ? ti.y : ti.w) + (et & (kTile - 1))]);
-            asm volatile("bar.sync 1, %0;" ::"n"(kEpiWarps * 32) : "memory");
             // the warp's `span` columns of the tile from cb: a half, or of one panel a
             // quarter (dimer, 2^14 samples: with four warps at a panel's 128 columns 158.5 us
             // a pass on one card and 163.9 on another, with eight 156.2 and 153.3)
             const int span = ti.z ? kTile / 2 : kTile, cb = half * span;
-            const double* cu = cunit + cb;
+            // their units; each warp its own copy: warps that met at a barrier here could wait
+            // for one whose bounded wait has expired and that has left the loop
+            double* cu = cunit + (warp - 2) * kTile;
+            __syncwarp();
+            for (int c = lane; c < span; c += 32)
+                cu[c] = zero_unit(rowmax[(cb + c < kTile ? ti.y : ti.w) + ((cb + c) & (kTile - 1))]);
+            __syncwarp();
             double* P = partial + (size_t)u * (size_t)(kTile * kN) + (size_t)cb * kTile + row;
             for (int r0 = lo; r0 < hi && ok; r0 += kRunKB)
                 for (int t = 0; t < kSweeps; t++, use++) {
-                    if (!mbar_wait(acc_full, use & 1, abort)) {
+                    // warp-uniform: the TMEM loads below are warp-collective
+                    if (!__all_sync(0xffffffffu, mbar_wait(acc_full, use & 1, abort))) {
                         ok = false;
                         break;
                     }
@@ -318,7 +320,9 @@ __global__ void __launch_bounds__(kThreads, 1)
                     __syncwarp();
                     if (lane == 0) mbar_arrive(acc_empty);
                 }
-            if (et == 0 && lo < hi) filled[u] = 1;     // all eight warps have read it
+            // the others have read it: the last sweep's sums came after their arrivals for the
+            // sweep before
+            if (threadIdx.x == 64 && lo < hi) filled[u] = 1;
         }
     }
     tc_fence_before();

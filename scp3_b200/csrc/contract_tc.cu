@@ -267,7 +267,8 @@ __global__ void __launch_bounds__(kThreads, 1)
             double* P = partial + (size_t)u * (size_t)(kTile * kN2);
             for (int k = 0; k < nruns; k++, use++) {
                 const int a = use & 1;
-                if (!mbar_wait(acc_full + a, (use >> 1) & 1, abort)) {
+                // warp-uniform: the TMEM loads below are warp-collective
+                if (!__all_sync(0xffffffffu, mbar_wait(acc_full + a, (use >> 1) & 1, abort))) {
                     ok = false;
                     break;
                 }
