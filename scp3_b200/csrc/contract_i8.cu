@@ -7,18 +7,36 @@
 // is worth 4 FP64 pipes or so (the clock is lower under this load).  The DFMA kernel this replaces ran at 0.72 of that pipe:
 // 8.9 ms per 2^17 samples of the hexamer doubles basis.
 //
-// Digits.  Within a pass every operand row has one power-of-two scale, 2^e above
-// its largest |value|; a value is rounded to the integer x 2^(54 - e) (|.| <= 2^54,
-// the rounding is half a unit of FP64's last place for values near the largest) and
-// written as seven balanced base-256 digits, each -128..127, most significant first.
+// Digits.  Within a pass every operand row has one power-of-two scale, 2^e just above
+// its largest |value|; a value is rounded to the integer x 2^(55 - e) (|.| < 0.9961 2^55)
+// and written as seven balanced base-256 digits, each -128..127, most significant first.
 // The product of two rows is sum over digit pairs (i, j) of 2^(8 (14 - i - j)) D_ij;
-// the 34 pairs with i + j <= 9 are formed.  Measured against compensated sums of the
-// same values, 2^13 samples: norm-wise error 1.6e-16 (dimer), 7.7e-17 (hexamer) and
-// 4.9e-16 (trimer, |V| up to 34 times its rms), against 4.2e-16, 4.9e-16 and 7.2e-16 of
-// an FP64 product; with i + j <= 8 only (28 pairs) 4.8e-15, 1.4e-15 and 1.5e-14.  D_ij is accumulated in 32-bit integers,
-// exactly: a run is at most 18432 samples, so a group of equal i + j (up to 7 pairs of
-// 2^14) stays below 2^31.  A row whose values are not all finite reads NaN in every
-// element it enters.
+// the 34 pairs with i + j <= 9 are formed.  Against extended-precision sums of the
+// same values, 2^13 samples, norm-wise, and of an FP64 product in brackets: 3.3e-16
+// (4.4e-16) for a dimer, 3.0e-16 (5.1e-16) a trimer with TTM3-F, 5.6e-16 (1.1e-15) the
+// hexamer; with i + j <= 8 only (28 pairs) about ten times as much.  D_ij is accumulated in
+// 32-bit integers, exactly: a run is at most 18432 samples, so a group of equal i + j (up to
+// 7 pairs of 2^14) stays below 2^31.
+//
+// Range.  A value 2^-k of its row's largest keeps 55 - k bits, so a sample that dwarfs the
+// others would cost them their bits, above all in the elements where its own term is
+// small.  Samples whose |V|, |q_m| or |dV/dq_m| is more than 2^9, 2^4 and 2^9 times that
+// quantity's geometric mean over 128 samples of the pass, or not finite, are therefore left
+// out of the digits (zero) and of the scales, and their products added in FP64 at the end
+// of contract_i8_kernel (add_heavy).  2^4 lies above every point of the Sobol sequence
+// (|q| < 6.3), 2^9 above the largest |V| of 2^17 points of the clusters looked at (8 to 490
+// times the mean), so ordinary builds have such samples rarely or not at all: the limits
+// cost a launch of 4 us in place of a memset.  One V of 2^14 at 1, 10^2, 10^3, 10^6 and
+// 10^12 times the others' rms, elements in which it vanishes, largest error over the sum
+// of |terms|: 2.8e-17, 8.7e-17, 2.8e-17, 2.8e-17, 2.8e-17 (an FP64 product 5.7e-17 in each;
+// without the limits 4.9e-17, 2.1e-16, 2.2e-15, 1.5e-12, 1.9e-6).  Hexamer, 2^16 samples,
+// 2.0 ms: 0.1 % of them heavy add 2 % to the pass, 1 % a tenth, 10 % as much again and 60 %
+// (V spread evenly over 24 decades) 3.3 times as much, 1.6 times an FP64 kernel's time.
+// Elements are NaN or infinite where the FP64 products would be; a finite row whose
+// products overflow reads NaN.
+//
+// The splitting into exact partial products is the published one for matrix products on
+// narrow units (Ozaki, Ogita, Oishi and Rump); the order of the digits below is this file's.
 //
 // Operand layout: [row block of 128][k-block of 64 samples][digit][128 rows x 64 B],
 // each 8 KB box in the 64-byte-swizzled order the MMA descriptors read (16-byte chunk
@@ -109,19 +127,162 @@ __host__ __device__ __forceinline__ bool in_large(int t, int e) { return ((e & 1
 
 __device__ __forceinline__ double pow2(int e) { return __hiloint2double((1023 + e) << 20, 0); }
 
-// Exponent e with every |value| of the row below 2^e, from the high word of the largest
-__device__ __forceinline__ int row_exp(int hi) { return max((hi >> 20) - 1022, -960); }
+// Exponent e with every |value| of the row below 0.996 2^e, from the high word of the
+// largest: seven balanced digits hold integers up to 0x7f7f7f7f7f7f7f = 0.9961 2^55
+__device__ __forceinline__ int row_exp(int hi) { return max(((hi + 0x2100) >> 20) - 1022, -960); }
 __device__ __forceinline__ double row_unit(int hi)     // value of one unit of the row's integers
 {
-    return hi >= 0x7ff00000 ? __longlong_as_double(0x7ff8000000000000ll) : pow2(row_exp(hi) - 54);
+    return hi >= 0x7ff00000 ? __longlong_as_double(0x7ff8000000000000ll) : pow2(row_exp(hi) - 55);
 }
 
 __device__ __forceinline__ double zero_unit(int hi) { return hi ? row_unit(hi) : 0.0; }
 
+// ---------------------------------------------------------------- heavy samples
+// The high word of a pass's limit of |x|: kLimitV or kLimitQ octaves above the geometric
+// mean of kLimitSamples of its values.
+constexpr int kLimitV = 9, kLimitQ = 4, kLimitSamples = 128, kLimitValues = 8;
+constexpr int kLimitThreads = kLimitSamples * kLimitValues;
+
+__device__ __forceinline__ int high_word(double x) { return __double2hiint(x) & 0x7fffffff; }
+
+// Limits of V, q and dV/dq, kLimitValues of these per block, from samples spread over the
+// pass; zeros (padding samples among them) and values that are not finite do not count,
+// and with nothing left any value but zero is over the limit.  The high word is the
+// logarithm's piecewise linear form, so the sums are integers.  The blocks from lblocks on
+// clear rowmax.
+__global__ void __launch_bounds__(kLimitThreads) limits_kernel(const double* __restrict__ q, const double* __restrict__ v,
+                                                               const double* __restrict__ vq, int nm, long long k,
+                                                               int* __restrict__ limits, uint32_t* __restrict__ any,
+                                                               int lblocks, int* __restrict__ rowmax, int rows)
+{
+    const int t = threadIdx.x;
+    if ((int)blockIdx.x >= lblocks) {
+        const int r = ((int)blockIdx.x - lblocks) * kLimitThreads + t;
+        if (r < rows) rowmax[r] = 0;
+        return;
+    }
+    __shared__ int sum[kLimitValues], count[kLimitValues];
+    if (t < kLimitValues) sum[t] = count[t] = 0;
+    if (blockIdx.x == 0 && t == 0) *any = 0;
+    __syncthreads();
+    const int ns = (int)min((long long)kLimitSamples, k), nq = 1 + nm + (vq ? nm : 0);
+    const int j = t / kLimitValues, i = (int)blockIdx.x * kLimitValues + t % kLimitValues;
+    int h = 0;
+    if (j < ns && i < nq) {
+        const long long s = k * j / ns;
+        h = high_word(i == 0 ? v[s] : i <= nm ? q[s * nm + i - 1] : vq[s * nm + i - 1 - nm]);
+    }
+    if (h > 0 && h < 0x7ff00000) {
+        atomicAdd(sum + t % kLimitValues, h >> 10);      // below 2^21 each
+        atomicAdd(count + t % kLimitValues, 1);
+    }
+    __syncthreads();
+    if (t < kLimitValues && i < nq) {
+        const int octaves = i == 0 || i > nm ? kLimitV : kLimitQ;
+        limits[i] = count[t] ? (int)min(((long long)(sum[t] / count[t]) << 10) + ((long long)octaves << 20), 0x7fefffffll) : 0;
+    }
+}
+
+// Value of a table entry (kind | a << 4 | b << 6 | mode << 8) at the sample with
+// coordinates q, potential V and derivatives vq
+__device__ __forceinline__ double entry_value(uint32_t sp, const double* q, double V, const double* vq)
+{
+    const int kind = sp & 15, a = (sp >> 4) & 3, b = (sp >> 6) & 3, m = sp >> 8;
+    if (kind == kOne) return 1.0;
+    if (kind == kV) return V;
+    return kind == kHo ? ho(a, q[m]) : stein_weight(a, kind == kKab ? b : 0, q[m], V, vq[m]);
+}
+
+struct HeavyArgs {
+    const uint32_t *heavy, *any, *tspec, *xdesc;
+    int dual, nm;
+    const double *q, *v, *vq;
+};
+
+constexpr int kHeavy = 32;                         // samples added at a time
+
+// Adds the heavy samples of a unit's blocks of 32, [w0, w1), to its partial P: the products
+// of their row values in FP64, in the order of the samples, kHeavy at a time (8 x 4 elements
+// of a 128 x 64 block per thread and round).  All threads of the CTA; buf: kHeavyBytes.
+constexpr int kHeavyBytes = kHeavy * (kTile + kN) * (int)sizeof(double) + kHeavy * (int)sizeof(int);
+__device__ __forceinline__ void add_heavy(const HeavyArgs& a, int4 ti, int w0, int w1, double* P, uint8_t* buf)
+{
+    double *sa = reinterpret_cast<double*>(buf), *sb = sa + kHeavy * kTile;     // [sample][row], [sample][column]
+    int* list = reinterpret_cast<int*>(sb + kHeavy * kN);
+    const int t = threadIdx.x, lane = t & 31, tx = t & 15, ty = t >> 4;
+    int nh = 0;
+    for (int wb = w0;; wb += 32) {
+        const bool end = wb >= w1;
+        const uint32_t word = wb + lane < w1 ? a.heavy[wb + lane] : 0u;
+        uint32_t words = __ballot_sync(0xffffffffu, word != 0), bits = 0;
+        int base = 0;
+        for (;;) {                                 // every warp takes the same steps
+            while (nh < kHeavy && (bits | words)) {
+                if (!bits) {
+                    const int l = __ffs((int)words) - 1;
+                    words &= words - 1;
+                    bits = __shfl_sync(0xffffffffu, word, l);
+                    base = (wb + l) * 32;
+                }
+                if (t == 0) list[nh] = base + __ffs((int)bits) - 1;
+                bits &= bits - 1;
+                nh++;
+            }
+            if (nh < kHeavy && !(end && nh)) break;
+            __syncthreads();
+            for (int e = t; e < nh * (kTile + kN); e += kThreads) {
+                const int h = e / (kTile + kN), c = e - h * (kTile + kN);
+                if (c >= 2 * kTile && ti.z) continue;
+                const int64_t s = list[h];
+                int row = c < kTile ? ti.x + c : c < 2 * kTile ? ti.y + c - kTile : ti.w + c - 2 * kTile;
+                const bool timesV = a.dual && row >= a.dual;
+                if (timesV) row -= a.dual;
+                const uint32_t d = a.xdesc[row];
+                const double V = a.v[s], *q = a.q + s * a.nm, *vq = a.vq + s * a.nm;
+                double val = 0.0;
+                if (d != kZeroRow) {
+                    val = entry_value(a.tspec[d & 1023u], q, V, vq);
+                    if ((d >> 10) & 1023u) val *= entry_value(a.tspec[(d >> 10) & 1023u], q, V, vq);
+                    if (d >> 20) val *= entry_value(a.tspec[d >> 20], q, V, vq);
+                    if (timesV) val *= V;
+                }
+                if (c < kTile) sa[h * kTile + c] = val;
+                else sb[h * kN + c - kTile] = val;
+            }
+            __syncthreads();
+            if (t < 256)
+#pragma unroll 1
+                for (int c0 = 0; c0 < (ti.z ? kTile : kN); c0 += 64) {
+                    double acc[8][4] = {};
+#pragma unroll 1
+                    for (int h = 0; h < nh; h++) {
+                        double x[8], y[4];
+#pragma unroll
+                        for (int i = 0; i < 8; i++) x[i] = sa[h * kTile + tx + 16 * i];
+#pragma unroll
+                        for (int j = 0; j < 4; j++) y[j] = sb[h * kN + c0 + ty + 16 * j];
+#pragma unroll
+                        for (int i = 0; i < 8; i++)
+#pragma unroll
+                            for (int j = 0; j < 4; j++) acc[i][j] = fma(x[i], y[j], acc[i][j]);
+                    }
+#pragma unroll
+                    for (int i = 0; i < 8; i++)
+#pragma unroll
+                        for (int j = 0; j < 4; j++)
+                            add_f64(P + (size_t)(c0 + ty + 16 * j) * kTile + tx + 16 * i, acc[i][j]);
+                }
+            __syncthreads();
+            nh = 0;
+        }
+        if (end) return;
+    }
+}
+
 __global__ void __launch_bounds__(kThreads, 1)
     contract_i8_kernel(const uint8_t* __restrict__ x, long long nkb_alloc, const int* __restrict__ rowmax,
                        const int4* __restrict__ tiles, int ntiles, int nsplit, int nkb_pass, int units,
-                       double* __restrict__ partial, int* __restrict__ filled, int* __restrict__ err_flag)
+                       double* __restrict__ partial, int* __restrict__ filled, int* __restrict__ err_flag, HeavyArgs ha)
 {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -332,6 +493,13 @@ __global__ void __launch_bounds__(kThreads, 1)
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem));
     }
+    if (*ha.any == 0 || *abort) return;
+    // the ring is free: every copy has been consumed
+    for (int u = blockIdx.x; u < units; u += gridDim.x) {
+        int lo, hi;
+        krange(u, lo, hi);
+        add_heavy(ha, tiles[u % ntiles], 2 * lo, 2 * hi, partial + (size_t)u * (size_t)(kTile * kN), smem);
+    }
 }
 
 // ---------------------------------------------------------------- the operand
@@ -351,24 +519,29 @@ __device__ __forceinline__ void put_entry(double* tab, int r, int l, double val)
     if (r >= 0) tab[r * kS + ((((l >> 4) << 3) + (((l >> 1) & 7) ^ ((r >> 2) & 7))) << 1) + (l & 1)] = val;
 }
 
-// entries[m][kind]: table entry or -1; v_entry: V's, or -1
-template <int kThreadsPerCta>
+// entries[m][kind]: table entry or -1; v_entry: V's, or -1.  kFlag: the samples over a
+// limit are marked in *heavy (shared, cleared).
+template <int kThreadsPerCta, bool kFlag>
 __device__ __forceinline__ void build_table(const int16_t* __restrict__ entries, int v_entry, int nm,
                                             const double* __restrict__ q, const double* __restrict__ v,
-                                            const double* __restrict__ vq, int64_t s0, double* tab)
+                                            const double* __restrict__ vq, int64_t s0, double* tab,
+                                            const int* __restrict__ limits = nullptr, uint32_t* heavy = nullptr)
 {
     const int l = threadIdx.x & 31;
     const int64_t s = s0 + l;
     const double V = v[s];
+    bool over = kFlag && high_word(V) > __ldg(limits);
     if (threadIdx.x < kS) put_entry(tab, 0, l, 1.0);
     else if (threadIdx.x < 2 * kS) put_entry(tab, v_entry, l, V);
     for (int m = threadIdx.x >> 5; m < nm; m += kThreadsPerCta / 32) {
         const double x = __ldg(q + s * nm + m);
+        if (kFlag) over |= high_word(x) > __ldg(limits + 1 + m);
         const int16_t* e = entries + m * kModeKinds;
 #pragma unroll
         for (int a = 1; a <= 3; a++) put_entry(tab, e[a - 1], l, ho(a, x));
         if (!vq) continue;
         const double Vm = __ldg(vq + s * nm + m);
+        if (kFlag) over |= high_word(Vm) > __ldg(limits + 1 + nm + m);
 #pragma unroll
         for (int a = 1; a <= 3; a++) {
             put_entry(tab, e[2 + a], l, stein_weight(a, 0, x, V, Vm));
@@ -378,6 +551,10 @@ __device__ __forceinline__ void build_table(const int16_t* __restrict__ entries,
                 if (e[k] >= 0) put_entry(tab, e[k], l, stein_weight(a, b, x, V, Vm));
             }
         }
+    }
+    if (kFlag) {
+        const uint32_t bits = __ballot_sync(0xffffffffu, over);
+        if (bits && l == 0) atomicOr(heavy, bits);
     }
 }
 
@@ -416,6 +593,14 @@ __device__ __forceinline__ void read8(const double* tab, uint32_t i, int g, doub
     }
 }
 
+// zero in every table entry at the marked samples
+__device__ __forceinline__ void drop_samples(double* tab, int trows, uint32_t marked)
+{
+#pragma unroll 1
+    for (int e = threadIdx.x; e < trows * kS; e += blockDim.x)
+        if ((marked >> (e & 31)) & 1) put_entry(tab, e >> 5, e & 31, 0.0);
+}
+
 // Row values of `d` (entry indices); `fa` caches the first factor of entry `pia`.
 __device__ __forceinline__ void row16(const double* tab, uint32_t d, int g, uint32_t& pia, double* fa, double* o)
 {
@@ -438,76 +623,96 @@ __device__ __forceinline__ int max_hi8(const double* o)
     return m;
 }
 
-// Largest |value| of every row over the pass (its high word), and the sums of the
-// summed rows.  CTA (x, y): sample blocks x, x + gridDim.x, ..., rows of chunk y.
+// Largest |value| of every row over the pass's samples within the limits (its high word;
+// the others are marked in heavy), and the sums of the summed rows over all of them.  CTA (x, y): sample blocks x, x + gridDim.x, ..., rows of chunk y.
 // dual: row dual + r is V times row r; the summed rows follow the described ones, and
 // xdesc ends on a multiple of four rows.
 __global__ void __launch_bounds__(kScanThreads, 1)
     scan_kernel(const int16_t* __restrict__ entries, int v_entry, int trows, const uint32_t* __restrict__ xdesc,
                 int ndesc, int dual, int nsum, int per, int nm, const double* __restrict__ q,
                 const double* __restrict__ v, const double* __restrict__ vq, int nblk, int* __restrict__ rowmax,
-                double* __restrict__ spart)
+                double* __restrict__ spart, const int* __restrict__ limits, uint32_t* __restrict__ heavy,
+                uint32_t* __restrict__ any)
 {
-    extern __shared__ __align__(16) double tab[];      // [trows][32], then [per] doubles
+    extern __shared__ __align__(16) double tab[];      // [trows][32], then [per] doubles and two words
     double* keep = tab + (size_t)trows * kS;           // (max, max of V times the row) or the sum
     int2* mx = reinterpret_cast<int2*>(keep);
+    uint32_t* marks = reinterpret_cast<uint32_t*>(keep + per);     // of this block and of the next
+    if (threadIdx.x < 2) marks[threadIdx.x] = 0;
     const int r0 = blockIdx.y * per, r1 = min(ndesc + nsum, r0 + per);
     for (int r = threadIdx.x; r < r1 - r0; r += kScanThreads) keep[r] = 0.0;
     const int g = threadIdx.x & 3, rl = threadIdx.x >> 2, w0 = 4 * (rl & 7);     // w0: rows below in the warp
-    for (int b = blockIdx.x; b < nblk; b += gridDim.x) {
+    for (int b = blockIdx.x, odd = 0; b < nblk; b += gridDim.x, odd ^= 1) {
         __syncthreads();
-        build_table<kScanThreads>(entries, v_entry, nm, q, v, vq, (int64_t)b * kS, tab);
+        build_table<kScanThreads, true>(entries, v_entry, nm, q, v, vq, (int64_t)b * kS, tab, limits, marks + odd);
         __syncthreads();
-        double vv[8], fa[8];
-        if (dual) read8<false>(tab, v_entry, g, vv);
-        // whole warps take the same number of rounds: the quarters meet in shuffles
-        for (int rb = r0 + 4 * rl; rb - w0 < r1; rb += kScanThreads) {
-            uint32_t pia = kZeroRow;
-            uint32_t d4[4] = {kZeroRow, kZeroRow, kZeroRow, kZeroRow};
-            if (rb < r1) *reinterpret_cast<uint4*>(d4) = __ldg(reinterpret_cast<const uint4*>(xdesc + rb));
-            const bool sum = rb - w0 + 32 > ndesc;     // the warp holds summed rows
+        const uint32_t hw = marks[odd];
+        if (threadIdx.x == 0) {
+            marks[odd ^ 1] = 0;                        // read by all before the barrier above
+            if (blockIdx.y == 0) heavy[b] = hw;
+            if (hw) *any = 1;
+        }
+        // one round over the rows; with marked samples first the summed rows, then, these
+        // samples dropped, the others
+#pragma unroll 1
+        for (int part = 0; part < (hw ? 2 : 1); part++) {
+            const int ra = hw && part == 0 ? max(r0, ndesc) : r0, re = part ? min(r1, ndesc) : r1;
+            if (part) {
+                __syncthreads();
+                drop_samples(tab, trows, hw);
+                __syncthreads();
+            }
+            double vv[8], fa[8];
+            if (dual) read8<false>(tab, v_entry, g, vv);
+            // whole warps take the same number of rounds: the quarters meet in shuffles
+            for (int rb = ra + 4 * rl; rb - w0 < re; rb += kScanThreads) {
+                uint32_t pia = kZeroRow;
+                uint32_t d4[4] = {kZeroRow, kZeroRow, kZeroRow, kZeroRow};
+                if (rb < re) *reinterpret_cast<uint4*>(d4) = __ldg(reinterpret_cast<const uint4*>(xdesc + rb));
+                const bool sum = rb - w0 + 32 > ndesc;     // the warp holds summed rows
 #pragma unroll
-            for (int u = 0; u < 4; u++) {
-                const int row = rb + u;
-                const uint32_t d = d4[u];
-                double o[8];
-                int m = 0, mv = 0;
-                double t = 0.0;
-                if (d != kZeroRow) {
-                    const uint32_t ia = d & 1023u, ib = (d >> 10) & 1023u, ic = d >> 20;
-                    if (ia != pia) {
-                        read8<false>(tab, ia, g, fa);
-                        pia = ia;
-                    }
-#pragma unroll
-                    for (int k = 0; k < 8; k++) o[k] = fa[k];
-                    if (ib) read8<true>(tab, ib, g, o);
-                    if (ic) read8<true>(tab, ic, g, o);
-                    if (row < ndesc) {
-                        m = max_hi8(o);
-                        if (dual) {
-#pragma unroll
-                            for (int k = 0; k < 8; k++) o[k] *= vv[k];
-                            mv = max_hi8(o);
+                for (int u = 0; u < 4; u++) {
+                    const int row = rb + u;
+                    const uint32_t d = d4[u];
+                    double o[8];
+                    int m = 0, mv = 0;
+                    double t = 0.0;
+                    if (d != kZeroRow) {
+                        const uint32_t ia = d & 1023u, ib = (d >> 10) & 1023u, ic = d >> 20;
+                        if (ia != pia) {
+                            read8<false>(tab, ia, g, fa);
+                            pia = ia;
                         }
-                    } else {
-                        t = ((o[0] + o[1]) + (o[2] + o[3])) + ((o[4] + o[5]) + (o[6] + o[7]));
+#pragma unroll
+                        for (int k = 0; k < 8; k++) o[k] = fa[k];
+                        if (ib) read8<true>(tab, ib, g, o);
+                        if (ic) read8<true>(tab, ic, g, o);
+                        if (row < ndesc) {
+                            m = max_hi8(o);
+                            if (dual) {
+#pragma unroll
+                                for (int k = 0; k < 8; k++) o[k] *= vv[k];
+                                mv = max_hi8(o);
+                            }
+                        } else {
+                            t = ((o[0] + o[1]) + (o[2] + o[3])) + ((o[4] + o[5]) + (o[6] + o[7]));
+                        }
                     }
+                    if (sum) {
+                        t += __shfl_xor_sync(0xffffffffu, t, 1);
+                        t += __shfl_xor_sync(0xffffffffu, t, 2);
+                        if (g == 0 && row >= ndesc && d != kZeroRow) keep[row - r0] += t;
+                        if (rb - w0 >= ndesc) continue;
+                    }
+                    m = max(m, __shfl_xor_sync(0xffffffffu, m, 1));
+                    m = max(m, __shfl_xor_sync(0xffffffffu, m, 2));
+                    if (dual) {
+                        mv = max(mv, __shfl_xor_sync(0xffffffffu, mv, 1));
+                        mv = max(mv, __shfl_xor_sync(0xffffffffu, mv, 2));
+                    }
+                    if (g == 0 && row < ndesc && d != kZeroRow)
+                        mx[row - r0] = make_int2(max(mx[row - r0].x, m), max(mx[row - r0].y, mv));
                 }
-                if (sum) {
-                    t += __shfl_xor_sync(0xffffffffu, t, 1);
-                    t += __shfl_xor_sync(0xffffffffu, t, 2);
-                    if (g == 0 && row >= ndesc && d != kZeroRow) keep[row - r0] += t;
-                    if (rb - w0 >= ndesc) continue;
-                }
-                m = max(m, __shfl_xor_sync(0xffffffffu, m, 1));
-                m = max(m, __shfl_xor_sync(0xffffffffu, m, 2));
-                if (dual) {
-                    mv = max(mv, __shfl_xor_sync(0xffffffffu, mv, 1));
-                    mv = max(mv, __shfl_xor_sync(0xffffffffu, mv, 2));
-                }
-                if (g == 0 && row < ndesc && d != kZeroRow)
-                    mx[row - r0] = make_int2(max(mx[row - r0].x, m), max(mx[row - r0].y, mv));
             }
         }
     }
@@ -544,7 +749,7 @@ __global__ void __launch_bounds__(256) add_sums_kernel(const double* __restrict_
 // chunk of each digit's box: the bytes of x + sum 128 256^b, each xor 0x80.
 __device__ __forceinline__ void put_digits(const double* o, int hi, int g, uint8_t* p)
 {
-    const double inv = hi >= 0x7ff00000 ? 0.0 : pow2(54 - row_exp(hi));
+    const double inv = hi >= 0x7ff00000 ? 0.0 : pow2(55 - row_exp(hi));
     uint32_t w[kDigits][4];
 #pragma unroll
     for (int j = 0; j < 4; j++) {
@@ -580,14 +785,18 @@ __device__ __forceinline__ void put_digits(const double* o, int hi, int g, uint8
 // 1.1 GB alone 172; gradient, 2^15 samples 309 us, now 270, of 206).
 template <bool kDual>
 __global__ void __launch_bounds__(kDigitThreads, 2)
-    digits_kernel(const int16_t* __restrict__ entries, int v_entry, const uint32_t* __restrict__ xdesc, int ndesc,
-                  int dual, int per, int nm, const double* __restrict__ q, const double* __restrict__ v,
-                  const double* __restrict__ vq, const int* __restrict__ rowmax, int64_t nkb_alloc,
-                  uint8_t* __restrict__ x)
+    digits_kernel(const int16_t* __restrict__ entries, int v_entry, int trows, const uint32_t* __restrict__ xdesc,
+                  int ndesc, int dual, int per, int nm, const double* __restrict__ q, const double* __restrict__ v,
+                  const double* __restrict__ vq, const int* __restrict__ rowmax, const uint32_t* __restrict__ heavy,
+                  int64_t nkb_alloc, uint8_t* __restrict__ x)
 {
     extern __shared__ __align__(16) double tab[];
-    build_table<kDigitThreads>(entries, v_entry, nm, q, v, vq, (int64_t)blockIdx.x * kS, tab);
+    build_table<kDigitThreads, false>(entries, v_entry, nm, q, v, vq, (int64_t)blockIdx.x * kS, tab);
     __syncthreads();
+    if (const uint32_t hw = __ldg(heavy + blockIdx.x)) {       // their digits are zero: every row's first factor is
+        drop_samples(tab, trows, hw);
+        __syncthreads();
+    }
     const int g = threadIdx.x & 1, rl = threadIdx.x >> 1;
     const int64_t kb = blockIdx.x >> 1;
     const int c = ((blockIdx.x & 1) << 1) | g;          // 16-byte chunk of the box rows
@@ -622,7 +831,7 @@ __global__ void __launch_bounds__(kDigitThreads, 2)
 }
 
 size_t digits_smem(const Plan& p) { return sizeof(double) * (size_t)p.trows * kS; }
-size_t scan_smem(const Plan& p) { return digits_smem(p) + sizeof(double) * (size_t)p.scan_per; }
+size_t scan_smem(const Plan& p) { return digits_smem(p) + sizeof(double) * (size_t)p.scan_per + 2 * sizeof(uint32_t); }
 int described(const Plan& p) { return p.dual ? p.dual : p.rows; }
 int scan_chunks(const Plan& p) { return (described(p) + p.nsum + p.scan_per - 1) / p.scan_per; }
 int scan_blocks(const Plan& p, int64_t k)
@@ -694,20 +903,25 @@ int create(Plan& p, const std::vector<uint32_t>& tspec, const std::vector<uint32
     }
     std::vector<uint32_t> desc4 = xdesc;
     desc4.resize((xdesc.size() + 3) / 4 * 4, kZeroRow);
+    const size_t ndesc4 = desc4.size();
+    desc4.insert(desc4.end(), tspec.begin(), tspec.end());
     // rows per scan CTA: what fits beside the table, in whole trips of the CTA
-    const int room = (int)((227 * 1024 - digits_smem(p)) / sizeof(double)) / kScanStep * kScanStep;
+    const int room = (int)((227 * 1024 - digits_smem(p) - 2 * sizeof(uint32_t)) / sizeof(double)) / kScanStep * kScanStep;
     p.scan_per = std::min(room, ((int)xdesc.size() + kScanStep - 1) / kScanStep * kScanStep);
     const size_t xbytes = (size_t)rows * chunk * kDigits;
     int rc;
     if ((rc = upload(&p.entries, entries.data(), entries.size())) || (rc = upload(&p.xdesc, desc4.data(), desc4.size())) ||
         (rc = upload(&p.tiles, tiles.data(), tiles.size())) || (rc = dalloc(&p.x, xbytes)) ||
-        (rc = dalloc(&p.rowmax, (size_t)rows)) || (rc = dalloc(&p.filled, (size_t)p.nsplit * p.ntiles + 1)) ||
+        (rc = dalloc(&p.rowmax, (size_t)rows + 2 * nm + 1 + chunk / kS + 1)) || (rc = dalloc(&p.filled, (size_t)p.nsplit * p.ntiles + 1)) ||
         (rc = dalloc(&p.partial, (size_t)p.nsplit * p.ntiles * kTile * kN)) ||
         (nsum && ((rc = dalloc(&p.spart, (size_t)scan_blocks(p, chunk) * nsum)) || (rc = dalloc(&p.sums, (size_t)nsum))))) {
         destroy(p);
         return rc;
     }
     p.err = p.filled + (size_t)p.nsplit * p.ntiles;
+    p.tspec = p.xdesc + ndesc4;
+    p.limits = p.rowmax + rows;
+    p.heavy = reinterpret_cast<uint32_t*>(p.limits + 2 * nm + 1);
     // padding rows are never written: zero the row blocks that hold any
     const size_t block = (size_t)p.nkb * kDigits * kBox;
     for (int rb = 0; rb < described(p) / kTile; rb++)
@@ -741,13 +955,18 @@ int prepare(const Plan& p, const double* q, const double* v, const double* vq, i
     if (k <= 0) return SCP3GPU_OK;
     if (k > p.chunk || k % kKB) return fail(SCP3GPU_ERR_ARG, "contract_i8: pass not in k-blocks");
     const int ndesc = described(p), nblk = (int)(k / kS), nx = scan_blocks(p, k);
-    SCP3_CUDA(cudaMemsetAsync(p.rowmax, 0, sizeof(int) * (size_t)p.rows, s));
+    uint32_t* any = p.heavy + p.chunk / kS;
+    const int lblocks = (1 + p.nm * (vq ? 2 : 1) + kLimitValues - 1) / kLimitValues;
+    limits_kernel<<<lblocks + (p.rows + kLimitThreads - 1) / kLimitThreads, kLimitThreads, 0, s>>>(
+        q, v, vq, p.nm, k, p.limits, any, lblocks, p.rowmax, p.rows);
+    SCP3_CUDA(cudaGetLastError());
     const auto digits = p.dual ? digits_kernel<true> : digits_kernel<false>;
     if (int rc = allow_smem(scan_kernel)) return rc;
     if (int rc = allow_smem(digits)) return rc;
     scan_kernel<<<dim3(nx, scan_chunks(p)), kScanThreads, scan_smem(p), s>>>(p.entries, p.v_entry, p.trows, p.xdesc,
                                                                             ndesc, p.dual, p.nsum, p.scan_per, p.nm, q,
-                                                                            v, vq, nblk, p.rowmax, p.spart);
+                                                                            v, vq, nblk, p.rowmax, p.spart,
+                                                                            p.limits, p.heavy, any);
     SCP3_CUDA(cudaGetLastError());
     if (p.nsum) add_sums_kernel<<<(p.nsum + 31) / 32, 256, 0, s>>>(p.spart, p.nsum, nx, p.sums);
     SCP3_CUDA(cudaGetLastError());
@@ -755,18 +974,19 @@ int prepare(const Plan& p, const double* q, const double* v, const double* vq, i
     const int want = std::max(1, 4 * p.sms / nblk);
     const int per = std::max(kDigitThreads, ((ndesc + want - 1) / want + 3) / 4 * 4);
     digits<<<dim3(nblk, (ndesc + per - 1) / per), kDigitThreads, digits_smem(p), s>>>(
-        p.entries, p.v_entry, p.xdesc, ndesc, p.dual, per, p.nm, q, v, vq, p.rowmax, p.nkb, p.x);
+        p.entries, p.v_entry, p.trows, p.xdesc, ndesc, p.dual, per, p.nm, q, v, vq, p.rowmax, p.heavy, p.nkb, p.x);
     SCP3_CUDA(cudaGetLastError());
     return SCP3GPU_OK;
 }
 
-int contract(const Plan& p, int64_t k, cudaStream_t s)
+int contract(const Plan& p, const double* q, const double* v, const double* vq, int64_t k, cudaStream_t s)
 {
     if (k <= 0) return SCP3GPU_OK;
     const int units = p.ntiles * p.nsplit;
     if (int rc = allow_smem(contract_i8_kernel)) return rc;
+    const HeavyArgs ha{p.heavy, p.heavy + p.chunk / kS, p.tspec, p.xdesc, p.dual, p.nm, q, v, vq};
     contract_i8_kernel<<<std::min(units, p.sms), kThreads, kSmem, s>>>(p.x, (long long)p.nkb, p.rowmax, p.tiles, p.ntiles,
-                                                                       p.nsplit, (int)(k / kKB), units, p.partial, p.filled, p.err);
+                                                                       p.nsplit, (int)(k / kKB), units, p.partial, p.filled, p.err, ha);
     SCP3_CUDA(cudaGetLastError());
     return SCP3GPU_OK;
 }

@@ -24,11 +24,15 @@ struct Plan {
     int ntiles = 0, nsplit = 1, sms = 148;
     int64_t chunk = 0, nkb = 0;    // samples and k-blocks of a whole pass
     uint8_t* x = nullptr;          // [row block][k-block][digit 1..7][128 x 64]
-    int* rowmax = nullptr;         // [rows] high word of the row's largest |value| of the pass
+    int* rowmax = nullptr;         // [rows] high word of the row's largest |value| of the pass, then limits, heavy
     int v_entry = -1;              // table entry of V, -1 = none
     int scan_per = 0;              // rows per CTA of the scan
     int16_t* entries = nullptr;    // [nm][12] table entry of each kind of each mode, -1 = none
-    uint32_t* xdesc = nullptr;
+    uint32_t *xdesc = nullptr, *tspec = nullptr;     // row descriptors, then table entries
+    // samples left out of the digits and added in FP64 (contract_i8.cu, "Range"): the
+    // pass's limits of V, q and dV/dq (high words), a bit per sample, whether there are any
+    int* limits = nullptr;         // [1 + 2 nm]
+    uint32_t* heavy = nullptr;     // [chunk / 32], then any
     int4* tiles = nullptr;         // (A row, B rows 0..127, 1 = that panel only, B rows 128..255)
     double* partial = nullptr;     // [nsplit][ntiles][128 x 256] tile-local column-major
     double* spart = nullptr;       // [blocks of the scan][nsum]
@@ -50,9 +54,10 @@ void destroy(Plan& p);
 int zero(const Plan& p, cudaStream_t s);
 // Samples of a pass holding nvalid samples (padding samples carry V = 0 and dV/dq = 0).
 inline int64_t pass_samples(int64_t nvalid) { return (nvalid + kKB - 1) / kKB * kKB; }
-// The digits of a pass of k samples (vq may be null), then its products into the partials.
+// The digits of a pass of k samples (vq may be null), then its products into the partials
+// (of the same arrays).
 int prepare(const Plan& p, const double* q, const double* v, const double* vq, int64_t k, cudaStream_t s);
-int contract(const Plan& p, int64_t k, cudaStream_t s);
+int contract(const Plan& p, const double* q, const double* v, const double* vq, int64_t k, cudaStream_t s);
 int plan_splits(int ntiles, int64_t chunk, int sms);   // sample ranges per tile of a pass
 int table_room();                                     // table entries that fit a CTA
 int check(const Plan& p, cudaStream_t s);   // synchronises; SCP3GPU_ERR_TIMEOUT after an expired wait

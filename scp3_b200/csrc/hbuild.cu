@@ -266,7 +266,7 @@ int launch_chunk(scp3gpu_hbuild* h, int64_t index0, int64_t nvalid, const double
     }
     if (rc) return rc;
     Timed t(h, 2);
-    return i8::contract(h->ip, a.n, h->stream);
+    return i8::contract(h->ip, h->q64, h->v, nullptr, a.n, h->stream);
 }
 
 }  // namespace
@@ -724,7 +724,7 @@ int scp3gpu_hbuild_add_epot(scp3gpu_hbuild* h, const double* q, const double* V,
             SCP3_CUDA(cudaMemsetAsync(h->q64, 0, sizeof(double) * kn * nm, h->stream));
             SCP3_CUDA(cudaMemcpyAsync(h->q64, q + off * nm, sizeof(double) * c * nm, cudaMemcpyHostToDevice, h->stream));
             rc = i8::prepare(h->ip, h->q64, h->v, nullptr, kn, h->stream);
-            if (!rc) rc = i8::contract(h->ip, kn, h->stream);
+            if (!rc) rc = i8::contract(h->ip, h->q64, h->v, nullptr, kn, h->stream);
             SCP3_CUDA(cudaStreamSynchronize(h->stream));
         }
         if (rc) return rc;

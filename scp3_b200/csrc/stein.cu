@@ -1056,7 +1056,7 @@ int stein_pass(const SteinPlan& p, const uint32_t* desc, const double* q, const 
                                  nflush * (tc::kSlotsPerFlush / tc::kKBlock2), p.nosign, false, p.P, p.err,
                                  std::min(units, sms), s);
     } else {
-        if (!(rc = i8::prepare(p.ip, q, v, vq, k, s))) rc = i8::contract(p.ip, k, s);
+        if (!(rc = i8::prepare(p.ip, q, v, vq, k, s))) rc = i8::contract(p.ip, q, v, vq, k, s);
     }
     if (rc) return rc;
     if (p.tcpairs) return SCP3GPU_OK;      // the pair sums were part of the products
