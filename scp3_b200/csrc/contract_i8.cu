@@ -867,7 +867,10 @@ constexpr int kScanStep = kScanThreads, kMinScanRows = 2048;     // rows a scan 
 int table_room() { return (int)((227 * 1024 - sizeof(double) * kMinScanRows) / (sizeof(double) * kS)); }
 
 // Clocks of a pass: waves of units, each 136 per sample (34 products of 128 clocks per
-// 32 samples) and four drains, and the 256 KB partials' clearing and read-out.
+// 32 samples) and four drains of 10,000; and 150 a unit for its partial, stored by the first
+// drain and summed at read-out.  With 75 (the read-out's traffic alone) bases of one
+// and two tiles get more splits and lose: 8192 samples of one tile 122 splits 143.4 us, 86
+// (as chosen) 141.0; 4096 of two tiles 61 splits 144.6 and 147.4 us, 43 143.4 and 145.9.
 int plan_splits(int ntiles, int64_t chunk, int sms)
 {
     int best_m = 1;
