@@ -105,8 +105,12 @@ int ensure_args(scp3gpu_batch* b, int64_t passes)
     b->args_pinned = nullptr;
     b->args_cap = 0;
     const int64_t cap = std::max<int64_t>(passes, 16);
-    SCP3_CUDA(cudaMalloc(&b->args_dev, sizeof(SampleArgs) * (size_t)cap * b->ncl));
-    SCP3_CUDA(cudaMallocHost(&b->args_pinned, sizeof(SampleArgs) * (size_t)cap * b->ncl));
+    SCP3_CUDA(device_malloc(&b->args_dev, sizeof(SampleArgs) * (size_t)cap * b->ncl));
+    if (cudaMallocHost(&b->args_pinned, sizeof(SampleArgs) * (size_t)cap * b->ncl) != cudaSuccess) {
+        (void)cudaGetLastError();
+        staging::trim();
+        SCP3_CUDA(cudaMallocHost(&b->args_pinned, sizeof(SampleArgs) * (size_t)cap * b->ncl));
+    }
     b->args_cap = cap;
     return SCP3GPU_OK;
 }

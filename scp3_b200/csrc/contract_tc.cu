@@ -880,22 +880,22 @@ int create(Plan& p, int nb, int nm, int n2_for_factors, int n3_for_factors, int 
     p.ntiles = (int)tiles.size();
     p.grid = (int)std::min<long long>((long long)p.ntiles * p.nsplit, sms);
     for (int b = 0; b < 2; b++) {
-        SCP3_CUDA(cudaMalloc(&p.x[b], sizeof(uint16_t) * 2 * (size_t)p.nb_pad * p.slots));
+        SCP3_CUDA(device_malloc(&p.x[b], sizeof(uint16_t) * 2 * (size_t)p.nb_pad * p.slots));
         // padding rows (nb..nb_pad) are never written by the expansion: zero once
         SCP3_CUDA(cudaMemset(p.x[b], 0, sizeof(uint16_t) * 2 * (size_t)p.nb_pad * p.slots));
-        SCP3_CUDA(cudaMalloc(&p.slot_of[b], sizeof(int) * (size_t)p.slots));
-        SCP3_CUDA(cudaMalloc(&p.group_meta[b], sizeof(int) * nflush));
+        SCP3_CUDA(device_malloc(&p.slot_of[b], sizeof(int) * (size_t)p.slots));
+        SCP3_CUDA(device_malloc(&p.group_meta[b], sizeof(int) * nflush));
     }
-    SCP3_CUDA(cudaMalloc(&p.tiles2, sizeof(int4) * tiles.size()));
+    SCP3_CUDA(device_malloc(&p.tiles2, sizeof(int4) * tiles.size()));
     SCP3_CUDA(cudaMemcpy(p.tiles2, tiles.data(), sizeof(int4) * tiles.size(), cudaMemcpyHostToDevice));
     const std::vector<uint32_t> fac = basis_factor_table(nm_for_factors, n2_for_factors, n3_for_factors);
-    SCP3_CUDA(cudaMalloc(&p.factors, sizeof(uint32_t) * fac.size()));
+    SCP3_CUDA(device_malloc(&p.factors, sizeof(uint32_t) * fac.size()));
     SCP3_CUDA(cudaMemcpy(p.factors, fac.data(), sizeof(uint32_t) * fac.size(), cudaMemcpyHostToDevice));
-    SCP3_CUDA(cudaMalloc(&p.desc_dev, sizeof(ExpandDesc) * 2));
-    SCP3_CUDA(cudaMalloc(&p.tile_index, sizeof(int) * owner.size()));
+    SCP3_CUDA(device_malloc(&p.desc_dev, sizeof(ExpandDesc) * 2));
+    SCP3_CUDA(device_malloc(&p.tile_index, sizeof(int) * owner.size()));
     SCP3_CUDA(cudaMemcpy(p.tile_index, owner.data(), sizeof(int) * owner.size(), cudaMemcpyHostToDevice));
-    SCP3_CUDA(cudaMalloc(&p.partial, sizeof(double) * (size_t)p.nsplit * p.ntiles * kTile * kN2));
-    SCP3_CUDA(cudaMalloc(&p.err_flag, sizeof(int)));
+    SCP3_CUDA(device_malloc(&p.partial, sizeof(double) * (size_t)p.nsplit * p.ntiles * kTile * kN2));
+    SCP3_CUDA(device_malloc(&p.err_flag, sizeof(int)));
     SCP3_CUDA(cudaMemset(p.err_flag, 0, sizeof(int)));
     return SCP3GPU_OK;
 }

@@ -402,15 +402,15 @@ static int host_pes(int pes, int nw, int64_t n, const double* crd, double* E, do
                  ib = sizeof(int) * (size_t)n, total = xb + gb + eb + ib;
     staging::Slot slot;
     char* d = nullptr;
-    const bool pooled = total <= staging::kScratchMax;
-    int rc = pooled ? slot.acquire() : SCP3GPU_OK;
-    if (!rc) rc = pooled ? slot.scratch(total, &d) : dalloc(&d, total);
+    // without pinned memory to be had as without the pool
+    const bool pooled = total <= staging::kScratchMax && slot.acquire() == SCP3GPU_OK;
+    int rc = pooled ? slot.scratch(total, &d) : dalloc(&d, total);
     if (rc) return rc;
     // geometries, then gradients, energies, sweeps
     double *dx = (double*)d, *dg = (double*)(d + xb), *de = (double*)(d + xb + gb);
     int* di = (int*)(d + xb + gb + eb);
     auto body = [&]() -> int {
-        const bool small = total <= staging::kPinned;
+        const bool small = pooled && total <= staging::kPinned;
         if (small) {
             std::memcpy(slot.pinned(), crd, xb);
             SCP3_CUDA(cudaMemcpyAsync(dx, slot.pinned(), xb, cudaMemcpyHostToDevice, 0));
@@ -875,12 +875,12 @@ int scp3gpu_hbuild_set_surrogate(scp3gpu_hbuild* h, scp3gpu_mlp* m, int mode)
         return fail(SCP3GPU_ERR_ARG, "surrogate: input width must equal nmodes, max_batch >= pass size, same device");
     DeviceGuard g(h->dev);
     if (int rc = drain_prep(h)) return rc;
-    if (!h->ybuf && cudaMalloc(&h->ybuf, sizeof(float) * (size_t)h->chunk) != cudaSuccess)
+    if (!h->ybuf && device_malloc(&h->ybuf, sizeof(float) * (size_t)h->chunk) != cudaSuccess)
         return fail(SCP3GPU_ERR_NOMEM, "surrogate output buffer");
     // a workspace per build, so builds sharing one network can run at once
     if (h->sur_ws) cudaFree(h->sur_ws);
     h->sur_ws = nullptr;
-    if (cudaMalloc(&h->sur_ws, sizeof(__nv_bfloat16) * net->infer_workspace((int)h->chunk)) != cudaSuccess)
+    if (device_malloc(&h->sur_ws, sizeof(__nv_bfloat16) * net->infer_workspace((int)h->chunk)) != cudaSuccess)
         return fail(SCP3GPU_ERR_NOMEM, "surrogate workspace");
     h->sur = m;
     h->sur_mode = mode;

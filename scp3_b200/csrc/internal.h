@@ -37,18 +37,26 @@ inline int allow_smem(K* kernel)
     return allow_smem_of(reinterpret_cast<const void*>(kernel));
 }
 
+// The library's device allocations: a failure gives up the transfer pool's idle memory first.
+template <typename T>
+inline cudaError_t device_malloc(T** p, size_t bytes)
+{
+    *p = nullptr;
+    cudaError_t e = cudaMalloc((void**)p, bytes);
+    if (e == cudaErrorMemoryAllocation) {
+        (void)cudaGetLastError();
+        staging::trim();
+        e = cudaMalloc((void**)p, bytes);
+    }
+    return e;
+}
+
 template <typename T>
 inline int dalloc(T** p, size_t count)
 {
     *p = nullptr;
     if (count == 0) return SCP3GPU_OK;
-    cudaError_t e = cudaMalloc((void**)p, count * sizeof(T));
-    if (e == cudaErrorMemoryAllocation) {       // the transfer pool's idle memory first
-        (void)cudaGetLastError();
-        staging::trim();
-        e = cudaMalloc((void**)p, count * sizeof(T));
-    }
-    SCP3_CUDA(e);
+    SCP3_CUDA(device_malloc(p, count * sizeof(T)));
     return SCP3GPU_OK;
 }
 

@@ -516,39 +516,39 @@ int Net::alloc(int n_in_, int hidden_, int max_batch_)
     const int ins[4] = {n_in, hid, hid, hid}, outs[4] = {hid, hid, hid, 1};
     size_t off = 0;
     for (int l = 0; l < 4; l++) off += (size_t)outs[l] * ins[l] + outs[l];
-    SCP3_CUDA(cudaMalloc(&gflat, sizeof(float) * off));
+    SCP3_CUDA(device_malloc(&gflat, sizeof(float) * off));
     off = 0;
     for (int l = 0; l < 4; l++) {
         in[l] = ins[l];
         out[l] = outs[l];
         inpad[l] = l == 0 ? kin : hid;
         const size_t nw = (size_t)out[l] * in[l];
-        SCP3_CUDA(cudaMalloc(&w[l], sizeof(float) * nw));
-        SCP3_CUDA(cudaMalloc(&b[l], sizeof(float) * out[l]));
+        SCP3_CUDA(device_malloc(&w[l], sizeof(float) * nw));
+        SCP3_CUDA(device_malloc(&b[l], sizeof(float) * out[l]));
         gw[l] = gflat + off;             // gradients in the flat parameter order, one copy out
         gb[l] = gw[l] + nw;
         off += nw + out[l];
-        SCP3_CUDA(cudaMalloc(&mw[l], sizeof(float) * nw * 2));
-        SCP3_CUDA(cudaMalloc(&mb[l], sizeof(float) * out[l] * 2));
+        SCP3_CUDA(device_malloc(&mw[l], sizeof(float) * nw * 2));
+        SCP3_CUDA(device_malloc(&mb[l], sizeof(float) * out[l] * 2));
         SCP3_CUDA(cudaMemset(mw[l], 0, sizeof(float) * nw * 2));
         SCP3_CUDA(cudaMemset(mb[l], 0, sizeof(float) * out[l] * 2));
-        SCP3_CUDA(cudaMalloc(&wb[l], sizeof(__nv_bfloat16) * (size_t)out[l] * inpad[l]));
+        SCP3_CUDA(device_malloc(&wb[l], sizeof(__nv_bfloat16) * (size_t)out[l] * inpad[l]));
         SCP3_CUDA(cudaMemset(wb[l], 0, sizeof(__nv_bfloat16) * (size_t)out[l] * inpad[l]));
     }
-    SCP3_CUDA(cudaMalloc(&X, sizeof(__nv_bfloat16) * (size_t)max_batch * kin));
+    SCP3_CUDA(device_malloc(&X, sizeof(__nv_bfloat16) * (size_t)max_batch * kin));
     for (int l = 0; l < 3; l++) {
-        SCP3_CUDA(cudaMalloc(&Z[l], sizeof(float) * (size_t)max_batch * hid));
-        SCP3_CUDA(cudaMalloc(&H[l], sizeof(__nv_bfloat16) * (size_t)max_batch * hid));
+        SCP3_CUDA(device_malloc(&Z[l], sizeof(float) * (size_t)max_batch * hid));
+        SCP3_CUDA(device_malloc(&H[l], sizeof(__nv_bfloat16) * (size_t)max_batch * hid));
     }
-    SCP3_CUDA(cudaMalloc(&dA, sizeof(float) * (size_t)max_batch * hid));
-    SCP3_CUDA(cudaMalloc(&dB, sizeof(float) * (size_t)max_batch * hid));
-    SCP3_CUDA(cudaMalloc(&ybuf, sizeof(float) * max_batch));
-    SCP3_CUDA(cudaMalloc(&dy, sizeof(float) * max_batch));
-    SCP3_CUDA(cudaMalloc(&loss, sizeof(float)));
+    SCP3_CUDA(device_malloc(&dA, sizeof(float) * (size_t)max_batch * hid));
+    SCP3_CUDA(device_malloc(&dB, sizeof(float) * (size_t)max_batch * hid));
+    SCP3_CUDA(device_malloc(&ybuf, sizeof(float) * max_batch));
+    SCP3_CUDA(device_malloc(&dy, sizeof(float) * max_batch));
+    SCP3_CUDA(device_malloc(&loss, sizeof(float)));
     const size_t rb = max_batch / 64, nsplit = std::max<size_t>(1, std::min<size_t>(kDwSplits, max_batch / kDwRows));
-    SCP3_CUDA(cudaMalloc(&part, sizeof(float) * nsplit * hid * std::max(hid, n_in)));
-    for (int k = 0; k < 2; k++) SCP3_CUDA(cudaMalloc(&rsum[k], sizeof(float) * rb * hid));
-    SCP3_CUDA(cudaMalloc(&ysum, sizeof(float) * rb));
+    SCP3_CUDA(device_malloc(&part, sizeof(float) * nsplit * hid * std::max(hid, n_in)));
+    for (int k = 0; k < 2; k++) SCP3_CUDA(device_malloc(&rsum[k], sizeof(float) * rb * hid));
+    SCP3_CUDA(device_malloc(&ysum, sizeof(float) * rb));
     return SCP3GPU_OK;
 }
 
@@ -786,8 +786,8 @@ int scp3gpu_mlp_create(int n_in, int hidden, int max_batch, uint64_t seed, int d
     int rc = m->net.alloc(n_in, hidden, max_batch);
     if (!rc && cudaStreamCreateWithFlags(&m->s, cudaStreamNonBlocking) != cudaSuccess)
         rc = fail(SCP3GPU_ERR_CUDA, "stream creation failed");
-    if (!rc && (cudaMalloc(&m->qbuf, sizeof(float) * (size_t)m->net.max_batch * n_in) != cudaSuccess ||
-                cudaMalloc(&m->tbuf, sizeof(float) * (size_t)m->net.max_batch) != cudaSuccess))
+    if (!rc && (device_malloc(&m->qbuf, sizeof(float) * (size_t)m->net.max_batch * n_in) != cudaSuccess ||
+                device_malloc(&m->tbuf, sizeof(float) * (size_t)m->net.max_batch) != cudaSuccess))
         rc = fail(SCP3GPU_ERR_NOMEM, "mlp staging allocation failed");
     if (rc) {
         scp3gpu_mlp_destroy(m);
@@ -903,8 +903,8 @@ int scp3gpu_mlp_train(scp3gpu_mlp* m, const float* q, const float* t, int64_t n,
     float *qd = nullptr, *td = nullptr;
     int* idx = nullptr;
     int rc = SCP3GPU_OK;
-    if (cudaMalloc(&qd, sizeof(float) * (size_t)n * nin) != cudaSuccess || cudaMalloc(&td, sizeof(float) * n) != cudaSuccess ||
-        cudaMalloc(&idx, sizeof(int) * n) != cudaSuccess) {
+    if (device_malloc(&qd, sizeof(float) * (size_t)n * nin) != cudaSuccess || device_malloc(&td, sizeof(float) * n) != cudaSuccess ||
+        device_malloc(&idx, sizeof(int) * n) != cudaSuccess) {
         cudaFree(qd), cudaFree(td), cudaFree(idx);
         return fail(SCP3GPU_ERR_NOMEM, "mlp_train: data allocation failed");
     }

@@ -72,15 +72,21 @@ int Slot::acquire()
 Slot::~Slot()
 {
     if (!pinned_) return;
-    const Idle s{pinned_, dev_, dev_bytes_, device_};
+    Idle mine{pinned_, dev_, dev_bytes_, device_}, spare[kMaxIdle + 1];
+    size_t n = 0;
     {
         std::lock_guard<std::mutex> lock(mu());
-        if (idle().size() < kMaxIdle) {
-            idle().push_back(s);
-            return;
-        }
+        size_t held = mine.dev_bytes;
+        for (Idle& s : idle())
+            if ((held += s.dev_bytes) > kScratchMax) {         // its device memory, not the buffer
+                held -= s.dev_bytes;
+                spare[n++] = Idle{nullptr, s.dev, s.dev_bytes, s.device};
+                s.dev = nullptr, s.dev_bytes = 0;
+            }
+        if (idle().size() < kMaxIdle) idle().push_back(mine);
+        else spare[n++] = mine;
     }
-    drop(s);
+    for (size_t k = 0; k < n; k++) drop(spare[k]);
 }
 
 int Slot::scratch(size_t bytes, char** p)
@@ -184,3 +190,14 @@ int copy_out(void* dst, size_t pitch, const void* src, size_t width, size_t rows
 
 }  // namespace staging
 }  // namespace scp3
+
+// For tests: idle slots of the pool and the device memory they hold.
+extern "C" int scp3gpu_internal_staging_idle(size_t* device_bytes)
+{
+    using namespace scp3::staging;
+    std::lock_guard<std::mutex> lock(mu());
+    size_t held = 0;
+    for (const Idle& s : idle()) held += s.dev_bytes;
+    if (device_bytes) *device_bytes = held;
+    return (int)idle().size();
+}

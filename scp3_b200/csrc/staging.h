@@ -7,11 +7,12 @@ namespace scp3 {
 namespace staging {
 
 constexpr size_t kPinned = 8u << 20;       // pinned bytes of a slot
-constexpr size_t kScratchMax = 32u << 20;  // device bytes a slot keeps
+constexpr size_t kScratchMax = 32u << 20;  // device bytes of a slot, and of all idle ones together
 
 // One call's exclusive buffers on the current device, from the pool and back to it.  At
-// most eight idle slots are kept (64 MB pinned, 256 MB of device memory), and all of them are
-// freed when an allocation of the library fails (trim).
+// most eight idle slots are kept (64 MB pinned) with kScratchMax of device memory between
+// them, and all of them are freed when an allocation of the library fails (trim; the
+// libraries it calls and others on the same GPU do not know of them).
 class Slot {
 public:
     Slot() = default;
