@@ -31,10 +31,10 @@ struct WarpSlot {
     T* q;           // [group][qs] normal coordinates (the form's precision)
     T* crd;         // [group][9nw] geometries
     T* ms;          // [group][3nw] M sites
-    uint64_t* xs;   // [group][nm0] Sobol states of the group (dead once the normals are formed)
-    uint16_t* tl;   // [group * nm0] items that take the inverse CDF's tail branch
-    double* g;      // [group][9nw] gradients (gradient path), over xs and tl
+    double* g;      // [group][9nw] gradients (gradient path)
     char* sc;       // TTM3-F scratch, after g
+    uint64_t* xs;   // [group][nm0] Sobol states of the group; with tl from crd on, dead once
+    uint16_t* tl;   // the normals are formed: [group * nm0] items of the inverse CDF's tail
     int qs;         // q stride: nm0 rounded up to even (16-byte aligned rows)
 };
 
@@ -43,11 +43,12 @@ constexpr size_t round16(size_t b) { return (b + 15) & ~(size_t)15; }
 template <typename T>
 __host__ __device__ inline size_t slot_bytes(int pes, int nm0, int nw, bool grad = false)
 {
-    const size_t fixed = round16(sizeof(T) * kGroup * (((nm0 + 1) & ~1) + (size_t)(12 * nw)));
+    const size_t q = round16(sizeof(T) * kGroup * ((nm0 + 1) & ~1));
     const size_t normals = round16((size_t)kGroup * nm0 * (sizeof(uint64_t) + sizeof(uint16_t)));
-    const size_t force = (grad ? round16(sizeof(double) * kGroup * 9 * (size_t)nw) : 0) +
-                         (pes == SCP3GPU_PES_TTM3F ? round16(ttm::scratch_bytes<T>(nw)) : 0);
-    return fixed + (normals > force ? normals : force);
+    const size_t geometry = round16(sizeof(T) * kGroup * 12 * (size_t)nw) +
+                            (grad ? round16(sizeof(double) * kGroup * 9 * (size_t)nw) : 0) +
+                            (pes == SCP3GPU_PES_TTM3F ? round16(ttm::scratch_bytes<T>(nw)) : 0);
+    return q + (normals > geometry ? normals : geometry);
 }
 
 template <typename T>
@@ -56,13 +57,14 @@ __device__ inline WarpSlot<T> warp_slot(char* base, int nm0, int nw, bool grad =
     WarpSlot<T> s;
     s.qs = (nm0 + 1) & ~1;
     s.q = reinterpret_cast<T*>(base);
-    s.crd = s.q + (size_t)kGroup * s.qs;
+    char* over = base + round16(sizeof(T) * kGroup * s.qs);
+    s.crd = reinterpret_cast<T*>(over);
     s.ms = s.crd + 9 * nw * kGroup;
-    char* over = base + round16(sizeof(T) * kGroup * (s.qs + (size_t)(12 * nw)));
+    char* force = over + round16(sizeof(T) * kGroup * 12 * (size_t)nw);
+    s.g = reinterpret_cast<double*>(force);
+    s.sc = force + (grad ? round16(sizeof(double) * kGroup * 9 * (size_t)nw) : 0);
     s.xs = reinterpret_cast<uint64_t*>(over);
     s.tl = reinterpret_cast<uint16_t*>(s.xs + (size_t)kGroup * nm0);
-    s.g = reinterpret_cast<double*>(over);
-    s.sc = over + (grad ? round16(sizeof(double) * kGroup * 9 * (size_t)nw) : 0);
     return s;
 }
 
@@ -412,8 +414,8 @@ __device__ __forceinline__ void samples_body(const SampleArgs& a, char* smem)
                 if (a.q64) a.q64[s * a.nm + m] = (double)qm;
                 if (a.q32) a.q32[s * a.nm + m] = (float)qm;
             }
-            __syncwarp();
         }
+        __syncwarp();               // the next group's normals go over its geometries
     }
 }
 
