@@ -53,13 +53,14 @@ namespace {
 constexpr int kRedThreads = 256, kRedRows = 32, kRedTile = 8, kRedLd = 80;   // dim + 1 <= 80
 constexpr int kRedStage = 2 * kRedRows * kRedLd;     // rows of [g, V], then of [dq, 1]
 constexpr size_t kRedSmem = sizeof(double) * 2 * kRedStage;
-static_assert(kRedLd * kRedLd <= 2 * kRedStage, "the sums go over the stages");
+static_assert(kRedLd * kRedLd <= 2 * kRedStage && kRedTile * kRedTile * kRedThreads / 2 <= 2 * kRedStage,
+              "the sums go over the stages");
 
 // P[block] += sum over the block's samples of [g, V] [dq, 1]^T, column-major
 // (dim+1) x (dim+1).  nt = ceil((dim+1) / 8): thread (ti, tj) of a group of nt^2 threads
 // owns the 64 elements (ti + nt a, tj + nt b), and the CTA's groups take the staged rows
 // in turn, so a row costs a thread 16 conflict-free reads for 64 FMAs; the groups' sums
-// are added in order.  It was 16 elements per thread on pairs of reads each, bound by
+// are added in pairs.  It was 16 elements per thread on pairs of reads each, bound by
 // shared memory: hexamer, 141 us per 2^16 samples.
 __global__ void __launch_bounds__(kRedThreads) scp1_reduce_kernel(int dim, int64_t n, const double* __restrict__ V,
                                                                   const double* __restrict__ G,
@@ -112,17 +113,27 @@ __global__ void __launch_bounds__(kRedThreads) scp1_reduce_kernel(int dim, int64
         __syncthreads();                           // the stage is free for the next fetch
     }
     asm volatile("cp.async.wait_all;\n" ::: "memory");
-    for (int q = 0; q < groups; q++) {
+    // the upper half of the groups hands its sums to the lower, until one is left
+    for (int left = groups; left > 1;) {
+        const int low = (left + 1) / 2;
         __syncthreads();
-        if (g == q)
+        if (g >= low && g < left)
 #pragma unroll
-            for (int i = 0; i < kRedTile; i++)
+            for (int e = 0; e < kRedTile * kRedTile; e++)
+                sm[e * (kRedThreads / 2) + t - low * nt * nt] = acc[e / kRedTile][e % kRedTile];
+        __syncthreads();
+        if (g < left - low)
 #pragma unroll
-                for (int j = 0; j < kRedTile; j++) {
-                    double* p = sm + (tj + nt * j) * kRedLd + ti + nt * i;
-                    *p = q ? *p + acc[i][j] : acc[i][j];
-                }
+            for (int e = 0; e < kRedTile * kRedTile; e++)
+                acc[e / kRedTile][e % kRedTile] += sm[e * (kRedThreads / 2) + t];
+        left = low;
     }
+    __syncthreads();
+    if (g == 0)
+#pragma unroll
+        for (int i = 0; i < kRedTile; i++)
+#pragma unroll
+            for (int j = 0; j < kRedTile; j++) sm[(tj + nt * j) * kRedLd + ti + nt * i] = acc[i][j];
     __syncthreads();
     double* Pb = P + (size_t)blockIdx.x * E;
     for (int e = t; e < E; e += kRedThreads) {
