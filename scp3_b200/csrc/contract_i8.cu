@@ -279,6 +279,96 @@ __device__ __forceinline__ void add_heavy(const HeavyArgs& a, int4 ti, int w0, i
     }
 }
 
+// Passes of few samples, in FP64 throughout.  CTA b < ntiles ranges: the unit of tile
+// b % ntiles and sample range b / ntiles of `ranges`; `batch` samples at a time (few_batch),
+// the table's entries, the rows' values and their products, 8 x 4 elements of a 128 x 128
+// block per thread.  The other CTAs: the summed rows (from row ndesc of xdesc on), one per
+// warp.
+constexpr int kFewThreads = 512;
+
+__global__ void __launch_bounds__(kFewThreads, 1)
+    few_samples_kernel(const int4* __restrict__ tiles, int ntiles, int ranges, int k, int trows, int batch, int ndesc,
+                       int nsum, double* __restrict__ sums, double* __restrict__ partial, int* __restrict__ filled,
+                       HeavyArgs a)
+{
+    extern __shared__ __align__(16) double few[];  // [batch][rows], [batch][columns], [batch][table]
+    const int u = blockIdx.x, t = threadIdx.x;
+    if (u >= ntiles * ranges) {
+        const int i = (u - ntiles * ranges) * (kFewThreads / 32) + (t >> 5);
+        if (i >= nsum) return;
+        const uint32_t d = a.xdesc[ndesc + i];
+        const uint32_t sp[3] = {a.tspec[d & 1023u], a.tspec[(d >> 10) & 1023u], a.tspec[d >> 20]};
+        double x = 0.0;
+        for (int s = t & 31; s < k; s += 32) {
+            const double V = a.v[s], *q = a.q + (int64_t)s * a.nm, *vq = a.vq + (int64_t)s * a.nm;
+            x += entry_value(sp[0], q, V, vq) * entry_value(sp[1], q, V, vq) * entry_value(sp[2], q, V, vq);
+        }
+#pragma unroll
+        for (int o = 16; o; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+        if ((t & 31) == 0) sums[i] += x;
+        return;
+    }
+    double *sa = few, *sb = sa + batch * kTile, *tab = sb + batch * kN;
+    const int split = u / ntiles, lo = (int)((long long)k * split / ranges), hi = (int)((long long)k * (split + 1) / ranges);
+    const int4 ti = tiles[u % ntiles];
+    double* P = partial + (size_t)u * (size_t)(kTile * kN);
+    bool store = filled[u] == 0;                   // the partial holds nothing yet
+    // thread t forms row t of the tile's 128 + 256 (entry 0 is the constant 1)
+    const int row = t < kTile ? ti.x + t : t < 2 * kTile ? ti.y + t - kTile : ti.w + t - 2 * kTile;
+    const bool on = t < (ti.z ? 2 * kTile : kTile + kN), timesV = a.dual && row >= a.dual;
+    const uint32_t d = on ? a.xdesc[timesV ? row - a.dual : row] : kZeroRow;
+    double* out = t < kTile ? sa + t : sb + t - kTile;
+    const int stride = t < kTile ? kTile : kN;
+    const int tx = t & 15, ty = (t >> 4) & 15, c0 = t >> 8 << 6;
+    for (int s = lo; s < hi; s += batch, store = false) {
+        const int nh = min(batch, hi - s);
+        for (int e = t; e < nh * trows; e += kFewThreads) {
+            const int h = e / trows, i = e - h * trows;
+            const int64_t o = (int64_t)(s + h) * a.nm;
+            tab[e] = entry_value(a.tspec[i], a.q + o, a.v[s + h], a.vq + o);
+        }
+        __syncthreads();
+        if (on)
+#pragma unroll 4
+            for (int h = 0; h < nh; h++) {
+                const double* th = tab + h * trows;
+                double val = 0.0;
+                if (d != kZeroRow) {
+                    val = th[d & 1023u] * th[(d >> 10) & 1023u] * th[d >> 20];
+                    if (timesV) val *= a.v[s + h];
+                }
+                out[h * stride] = val;
+            }
+        __syncthreads();
+#pragma unroll 1
+        for (int c = c0; c < (ti.z ? kTile : kN); c += 128) {
+            double acc[8][4] = {};
+#pragma unroll 2
+            for (int h = 0; h < nh; h++) {
+                double x[8], y[4];
+#pragma unroll
+                for (int i = 0; i < 8; i++) x[i] = sa[h * kTile + tx + 16 * i];
+#pragma unroll
+                for (int j = 0; j < 4; j++) y[j] = sb[h * kN + c + ty + 16 * j];
+#pragma unroll
+                for (int i = 0; i < 8; i++)
+#pragma unroll
+                    for (int j = 0; j < 4; j++) acc[i][j] = fma(x[i], y[j], acc[i][j]);
+            }
+#pragma unroll
+            for (int i = 0; i < 8; i++)
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    double* p = P + (size_t)(c + ty + 16 * j) * kTile + tx + 16 * i;
+                    if (store) *p = acc[i][j];
+                    else add_f64(p, acc[i][j]);
+                }
+        }
+        __syncthreads();
+    }
+    if (t == 0 && lo < hi) filled[u] = 1;          // read by all before the barriers above
+}
+
 __global__ void __launch_bounds__(kThreads, 1)
     contract_i8_kernel(const uint8_t* __restrict__ x, long long nkb_alloc, const int* __restrict__ rowmax,
                        const int4* __restrict__ tiles, int ntiles, int nsplit, int nkb_pass, int units,
@@ -922,6 +1012,7 @@ int create(Plan& p, const std::vector<uint32_t>& tspec, const std::vector<uint32
         return rc;
     }
     p.err = p.filled + (size_t)p.nsplit * p.ntiles;
+    for (const int4& t : tiles) p.half_tiles += t.z != 0;
     p.tspec = p.xdesc + ndesc4;
     p.limits = p.rowmax + rows;
     p.heavy = reinterpret_cast<uint32_t*>(p.limits + 2 * nm + 1);
@@ -953,10 +1044,36 @@ int zero(const Plan& p, cudaStream_t s)
     return SCP3GPU_OK;
 }
 
+// Samples that few_samples_kernel takes at a time, and its shared memory
+static size_t few_smem(const Plan& p, int batch) { return sizeof(double) * (size_t)batch * (kTile + kN + p.trows); }
+static int few_batch(const Plan& p) { return few_smem(p, 32) <= 227 * 1024 ? 32 : 16; }
+
+// Sample ranges (of at least 8) of a pass of k samples in FP64 (few_samples_kernel), 0 where
+// the digits are faster.  Both sides in clocks, fitted to passes of 64 to 8192 samples of 28
+// bases: an SM's units in turn, 1400 a sample and tile (910 in one of a single B panel),
+// beside the summed rows, 27 a sample; against limits, scan and digits, then waves of units
+// with four drains.  The choice was slower than the other by more than 6 % in four of 224.
+// Time of a whole pass with the digits always and as chosen: dimer, one tile, 256 samples
+// 73.0 and 35.2 us (with FP64 tiles, before the digits, 49.7), 4096 72.9 and 41.9 (70.7); a
+// trimer with triples, three tiles, 1024 90.3 and 48.2 (64.3); hexamer, 28 tiles, 256 105.3
+// and 78.9 (98.1), 512 111.7 and 116.3 (115.3) and so left to the digits.
+int few_ranges(int ntiles, int half_tiles, int nsplit, int nsum, int sms, int64_t k)
+{
+    const int64_t ranges = std::max<int64_t>(1, std::min<int64_t>(nsplit, k / 8));
+    auto per_sm = [&](int64_t units) { return (double)((units + sms - 1) / sms); };
+    const double tile = 1400.0 - 490.0 * half_tiles / ntiles;
+    const double few = 12000.0 + std::max(per_sm(ntiles * ranges) * (5000.0 + tile * k / ranges), nsum ? 27.0 * k : 0.0);
+    const double digits = (half_tiles == ntiles ? 35000.0 : 73000.0) +
+                          per_sm((int64_t)ntiles * nsplit) * (50000.0 + 136.0 * k / nsplit);
+    return few < digits ? (int)ranges : 0;
+}
+static int few_ranges(const Plan& p, int64_t k) { return few_ranges(p.ntiles, p.half_tiles, p.nsplit, p.nsum, p.sms, k); }
+
 int prepare(const Plan& p, const double* q, const double* v, const double* vq, int64_t k, cudaStream_t s)
 {
     if (k <= 0) return SCP3GPU_OK;
     if (k > p.chunk || k % kKB) return fail(SCP3GPU_ERR_ARG, "contract_i8: pass not in k-blocks");
+    if (few_ranges(p, k)) return SCP3GPU_OK;       // contract() forms the rows itself
     const int ndesc = described(p), nblk = (int)(k / kS), nx = scan_blocks(p, k);
     uint32_t* any = p.heavy + p.chunk / kS;
     const int lblocks = (1 + p.nm * (vq ? 2 : 1) + kLimitValues - 1) / kLimitValues;
@@ -986,8 +1103,17 @@ int contract(const Plan& p, const double* q, const double* v, const double* vq, 
 {
     if (k <= 0) return SCP3GPU_OK;
     const int units = p.ntiles * p.nsplit;
-    if (int rc = allow_smem(contract_i8_kernel)) return rc;
     const HeavyArgs ha{p.heavy, p.heavy + p.chunk / kS, p.tspec, p.xdesc, p.dual, p.nm, q, v, vq};
+    if (const int ranges = few_ranges(p, k)) {
+        if (int rc = allow_smem(few_samples_kernel)) return rc;
+        constexpr int kWarps = kFewThreads / 32;
+        const int batch = few_batch(p);
+        few_samples_kernel<<<p.ntiles * ranges + (p.nsum + kWarps - 1) / kWarps, kFewThreads, few_smem(p, batch), s>>>(
+            p.tiles, p.ntiles, ranges, (int)k, p.trows, batch, described(p), p.nsum, p.sums, p.partial, p.filled, ha);
+        SCP3_CUDA(cudaGetLastError());
+        return SCP3GPU_OK;
+    }
+    if (int rc = allow_smem(contract_i8_kernel)) return rc;
     contract_i8_kernel<<<std::min(units, p.sms), kThreads, kSmem, s>>>(p.x, (long long)p.nkb, p.rowmax, p.tiles, p.ntiles,
                                                                        p.nsplit, (int)(k / kKB), units, p.partial, p.filled, p.err, ha);
     SCP3_CUDA(cudaGetLastError());
@@ -1004,6 +1130,13 @@ int check(const Plan& p, cudaStream_t s)
 
 }  // namespace i8
 }  // namespace scp3
+
+// Host-only view of the rule for passes of few samples, for tests: the sample ranges of a
+// pass of k samples in FP64, 0 for the digits.
+extern "C" int scp3gpu_internal_few_ranges(int ntiles, int half_tiles, int nsplit, int nsum, int sms, int64_t k)
+{
+    return ntiles < 1 || nsplit < 1 || sms < 1 || k < 1 ? -1 : scp3::i8::few_ranges(ntiles, half_tiles, nsplit, nsum, sms, k);
+}
 
 // Host-only view of the contraction's digit sweeps, for tests: the digit of step e of
 // sweep t (0..3) and whether its sum with step e - 1 is the sweep's larger one; returns

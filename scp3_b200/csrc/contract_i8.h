@@ -22,6 +22,7 @@ constexpr int kKB = 64;                      // samples per k-block
 struct Plan {
     int rows = 0, dual = 0, nsum = 0, nm = 0, trows = 0;
     int ntiles = 0, nsplit = 1, sms = 148;
+    int half_tiles = 0;            // tiles of one B panel
     int64_t chunk = 0, nkb = 0;    // samples and k-blocks of a whole pass
     uint8_t* x = nullptr;          // [row block][k-block][digit 1..7][128 x 64]
     int* rowmax = nullptr;         // [rows] high word of the row's largest |value| of the pass, then limits, heavy
@@ -55,10 +56,11 @@ int zero(const Plan& p, cudaStream_t s);
 // Samples of a pass holding nvalid samples (padding samples carry V = 0 and dV/dq = 0).
 inline int64_t pass_samples(int64_t nvalid) { return (nvalid + kKB - 1) / kKB * kKB; }
 // The digits of a pass of k samples (vq may be null), then its products into the partials
-// (of the same arrays).
+// (of the same arrays).  Passes of few samples are added in FP64 by contract() alone.
 int prepare(const Plan& p, const double* q, const double* v, const double* vq, int64_t k, cudaStream_t s);
 int contract(const Plan& p, const double* q, const double* v, const double* vq, int64_t k, cudaStream_t s);
 int plan_splits(int ntiles, int64_t chunk, int sms);   // sample ranges per tile of a pass
+int few_ranges(int ntiles, int half_tiles, int nsplit, int nsum, int sms, int64_t k);
 int table_room();                                     // table entries that fit a CTA
 int check(const Plan& p, cudaStream_t s);   // synchronises; SCP3GPU_ERR_TIMEOUT after an expired wait
 
