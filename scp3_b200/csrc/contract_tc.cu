@@ -315,11 +315,12 @@ __global__ void __launch_bounds__(kThreads, 1)
 // a diagonal block that hold upper elements), read along the partials' rows and written to
 // both triangles, the mirror through shared memory (one thread per element of the full
 // matrix read half of them across the partials' columns: 3825 functions 392 us, now 136).
-// blockDim (32, 8 kGroups): group g of a CTA sums a contiguous share of the splits, the
-// shares then added in order; kY = 8 and four groups for bases of a few tiles, which have
-// up to one split per SM.
+// blockDim (32, min(kY, 8) kGroups): group g of a CTA sums a contiguous share of the splits,
+// the shares then added in order; kY = 8 and four groups for bases of a few tiles, which have
+// up to one split per SM, kY = 2 and sixteen for those of one
+// tile (13 functions, 148 splits: a read-out on the device 14.1 us with four, 8.0).
 template <int kGroups, int kY, bool kFilled>
-__global__ void __launch_bounds__(256 * kGroups) unpack_n256_kernel(const double* __restrict__ partial,
+__global__ void __launch_bounds__(32 * (kY < 8 ? kY : 8) * kGroups) unpack_n256_kernel(const double* __restrict__ partial,
                                                                     const int* __restrict__ block_owner, int nt,
                                                                     int nblk, int ntiles, int nsplit, int nb,
                                                                     double divisor, const double* __restrict__ diag,
@@ -327,7 +328,7 @@ __global__ void __launch_bounds__(256 * kGroups) unpack_n256_kernel(const double
                                                                     const int* __restrict__ err,
                                                                     const int* __restrict__ filled)
 {
-    constexpr int kParts = kTile / 32 * (kTile / kY);
+    constexpr int kParts = kTile / 32 * (kTile / kY), kR = kY < 8 ? kY : 8;
     __shared__ double v[kGroups][kY][33];
     // block (ti, tj), row-major over ti <= tj < nblk, and its part
     int p = blockIdx.x / kParts, ti = 0;
@@ -339,26 +340,26 @@ __global__ void __launch_bounds__(256 * kGroups) unpack_n256_kernel(const double
     const int x0 = (part & 3) * 32, y0 = (part >> 2) * kY;
     const int gx0 = (tr ? tj : ti) * kTile + x0, gy0 = (tr ? ti : tj) * kTile + y0;
     if (gx0 >= nb || gy0 >= nb || (diagonal && gx0 >= gy0 + kY)) return;
-    const int x = threadIdx.x, y8 = threadIdx.y & 7, g = threadIdx.y >> 3;
+    const int x = threadIdx.x, y8 = threadIdx.y % kR, g = threadIdx.y / kR;
     const size_t unit = (size_t)ntiles * (kTile * kN2);
     const double* P = partial + (size_t)t * (kTile * kN2) + (size_t)(h * kTile + y0) * kTile + x0 + x;
     const int s1 = nsplit * (g + 1) / kGroups;
-    double sum[kY / 8] = {};
+    double sum[kY / kR] = {};
 #pragma unroll 8
     for (int s = nsplit * g / kGroups; s < s1; s++) {
         const bool on = !kFilled || __ldg(filled + (size_t)s * ntiles + t) != 0;
 #pragma unroll
-        for (int k = 0; k < kY / 8; k++)
-            if (on) sum[k] += P[s * unit + (size_t)(y8 + 8 * k) * kTile];
+        for (int k = 0; k < kY / kR; k++)
+            if (on) sum[k] += P[s * unit + (size_t)(y8 + kR * k) * kTile];
     }
 #pragma unroll
-    for (int k = 0; k < kY / 8; k++) v[g][y8 + 8 * k][x] = sum[k];
+    for (int k = 0; k < kY / kR; k++) v[g][y8 + kR * k][x] = sum[k];
     __syncthreads();
     const bool bad = err && *err;
     if (g == 0) {
 #pragma unroll
-        for (int k = 0; k < kY / 8; k++) {
-            const int y = y8 + 8 * k;
+        for (int k = 0; k < kY / kR; k++) {
+            const int y = y8 + kR * k;
             double val = v[0][y][x];
 #pragma unroll
             for (int q = 1; q < kGroups; q++) val += v[q][y][x];
@@ -372,7 +373,7 @@ __global__ void __launch_bounds__(256 * kGroups) unpack_n256_kernel(const double
     }
     __syncthreads();
     if (g) return;
-    for (int e = threadIdx.y * 32 + x; e < 32 * kY; e += 256) {
+    for (int e = threadIdx.y * 32 + x; e < 32 * kY; e += 32 * kR) {
         const int gy = gy0 + e % kY, gx = gx0 + e / kY;
         if (gx < nb && gy < nb && !(diagonal && gx >= gy)) M[(size_t)gx * ld + gy] = v[0][e % kY][e / kY];
     }
@@ -845,10 +846,11 @@ int launch_unpack(const double* partial, const int* owner, int nt, int ntiles, i
     if (total <= 0) return SCP3GPU_OK;
     const int nblk = (nb + kTile - 1) / kTile;
     const unsigned grid = (unsigned)(nblk * (nblk + 1) / 2 * 16);
-    const bool few = nsplit < 16;
+    const bool few = nsplit < 16, one = !few && nblk == 1;
     const auto kern = few ? (filled ? unpack_n256_kernel<1, 32, true> : unpack_n256_kernel<1, 32, false>)
-                          : (filled ? unpack_n256_kernel<4, 8, true> : unpack_n256_kernel<4, 8, false>);
-    kern<<<few ? grid : 4 * grid, dim3(32, few ? 8 : 32), 0, s>>>(partial, owner, nt, nblk, ntiles, nsplit, nb, divisor,
+                      : one ? (filled ? unpack_n256_kernel<16, 2, true> : unpack_n256_kernel<16, 2, false>)
+                            : (filled ? unpack_n256_kernel<4, 8, true> : unpack_n256_kernel<4, 8, false>);
+    kern<<<few ? grid : one ? 16 * grid : 4 * grid, dim3(32, few ? 8 : 32), 0, s>>>(partial, owner, nt, nblk, ntiles, nsplit, nb, divisor,
                                                                   diag, zpe, M, ld, err, filled);
     SCP3_CUDA(cudaGetLastError());
     return SCP3GPU_OK;

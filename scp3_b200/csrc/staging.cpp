@@ -125,12 +125,14 @@ int copy_out(void* dst, size_t pitch, const void* src, size_t width, size_t rows
     // Memory the driver knows (pinned above all) takes one DMA; only pageable memory gains
     // from the pool (12 MB of Mout: pageable 2.04 ms plain, 1.51 staged; pinned, in a
     // build of 2^20 host normals, 6.3 ms a step plain, 6.9 staged).
-    cudaPointerAttributes at{};
-    const cudaError_t ea = cudaPointerGetAttributes(&at, dst);
-    if (ea != cudaSuccess) (void)cudaGetLastError();
-    const bool known = ea == cudaSuccess && at.type != cudaMemoryTypeUnregistered;
+    auto known = [&] {
+        cudaPointerAttributes at{};
+        const cudaError_t ea = cudaPointerGetAttributes(&at, dst);
+        if (ea != cudaSuccess) (void)cudaGetLastError();
+        return ea == cudaSuccess && at.type != cudaMemoryTypeUnregistered;
+    };
     // so do small copies, rows longer than a piece, or where there is no pinned memory
-    if (known || total < 2 * kPiece || per > kPiece || slot.acquire() != SCP3GPU_OK) {
+    if (total < 2 * kPiece || per > kPiece || known() || slot.acquire() != SCP3GPU_OK) {
         if (flat) SCP3_CUDA(cudaMemcpyAsync(dst, src, total, cudaMemcpyDeviceToHost, s));
         else SCP3_CUDA(cudaMemcpy2DAsync(dst, pitch, src, width, width, rows, cudaMemcpyDeviceToHost, s));
         SCP3_CUDA(cudaStreamSynchronize(s));

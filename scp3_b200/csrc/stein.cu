@@ -526,16 +526,20 @@ __global__ void __launch_bounds__(32 * kRowSumWarps) stein_rowsum_kernel(const f
 // Element (i, j) of the dense matrix from its terms: for each mode m that r =
 // min(i, j) or c = max(i, j) excites, C at virtual row (m, r) column c, or at
 // (m, c) column r, or the pair sum D^m when both excite m; the mean over those
-// modes; <0|V|0> from the ground row.  C: FP64 tiles of 128 x 128, row-major,
-// `ct` per tile row (N256 = false); or the split form's 128 x 256 unit partials
-// (N256 = true), tile (row panel r, column panel pair q) at tile_of[r * ct + q]
-// with `ct` = column panel pairs, tile-local column-major.  With wb_off (the
-// split form's pair sums as products) the term of a pair exciting m in both
-// functions is C at W_b row (m, rank of r, level of c in m), column
-// red3(c without its mode-m factor).  `filled` (kFilled, the FP64 form): units whose
-// flag is zero hold no sums; their values are read all the same, so that the loads do not
-// wait on the flags, and dropped.
-template <int kY, bool kFilled>
+// modes; <0|V|0> from the ground row.  C: the 128 x 256 unit partials of either form,
+// tile (row panel r, column panel pair q) at tile_of[r * ct + q] with `ct` = column
+// panel pairs, tile-local column-major.  With wb_off (the pair sums as products) the
+// term of a pair exciting m in both functions is C at W_b row (m, rank of r, level of
+// c in m), column red3(c without its mode-m factor).  `filled` (kFilled, the FP64
+// form): units whose flag is zero hold no sums; their values are read all the same, so
+// that the loads do not wait on the flags, and dropped.
+//
+// kLanes > 1: as many lanes per element instead, over the sample ranges, for bases of a few
+// tiles, which have up to one range per SM: one thread read these in turn (Mout to the host,
+// FP64 form: 13 functions 59 us, with 32 lanes 34; 34 functions 92 and 37; 91 functions 73
+// and 51.  On the device, BF16x3, 16 ranges: 253 functions 44 us, with 8 lanes 32; 288
+// functions 35 and 37, 496 functions 34 and 54).
+template <int kY, bool kFilled, int kLanes = 1>
 __global__ void __launch_bounds__(256) stein_unpack_kernel(const uint32_t* __restrict__ desc, const int* __restrict__ rank3,
                                     const int* __restrict__ voff, const int64_t* __restrict__ doff, int nb, int nv,
                                     int ct, int nsplit, int dsplit, const double* __restrict__ C,
@@ -556,6 +560,7 @@ __global__ void __launch_bounds__(256) stein_unpack_kernel(const uint32_t* __res
     while (p >= nblk - a0) p -= nblk - a0, a0++;
     const int r0 = 32 * a0, c0 = 32 * (a0 + p) + kY * (blockIdx.x % (32 / kY));
     const bool bad = *err != 0;
+    const int x = threadIdx.x & 31, y8 = threadIdx.x >> 5, s0 = x % kLanes;
     // a term whose tile the plan did not make reads NaN into the element (never,
     // by construction; a visible result rather than an out-of-range read)
     auto cidx = [&](int vr, int col) -> int64_t {
@@ -569,20 +574,18 @@ __global__ void __launch_bounds__(256) stein_unpack_kernel(const uint32_t* __res
         if (kFilled) {
             const int64_t nt = csize / (128 * 256);
             const int* fl = filled + x / (128 * 256);
-#pragma unroll 4
-            for (int s = 0; s < nsplit; s++) {
+#pragma unroll 8
+            for (int s = s0; s < nsplit; s += kLanes) {
                 const double c = C[s * csize + x];
                 t += __ldg(fl + s * nt) ? c : 0.0;
             }
         } else {
-            for (int s = 0; s < nsplit; s++) t += C[s * csize + x];
+            for (int s = s0; s < nsplit; s += kLanes) t += C[s * csize + x];
         }
         return t;
     };
-    const int x = threadIdx.x & 31, y8 = threadIdx.x >> 5;
-    for (int y = y8; y < kY; y += 8) {
-        const int r = r0 + x, c = c0 + y;
-        if (r >= nb || c >= nb || r > c) continue;
+    // the mean over the modes of the element's terms (kLanes: a lane's share of it)
+    auto element = [&](int r, int c) -> double {
         int mr[3], lr[3], mc[3], lc[3];
         const int nr = decode(desc[r], mr, lr), ncn = decode(desc[c], mc, lc);
         double val = 0.0;
@@ -602,7 +605,7 @@ __global__ void __launch_bounds__(256) stein_unpack_kernel(const uint32_t* __res
                     t += csum(x);
                 } else if (sum_off && sum_off[m * 4 + lc[b]] >= 0) {
                     // summed row (m, rank of r, level of c in m): c without m is the constant
-                    t = sums[sum_off[m * 4 + lc[b]] + rank3[3 * r + a]];
+                    if (s0 == 0) t = sums[sum_off[m * 4 + lc[b]] + rank3[3 * r + a]];
                 } else if (wb_off) {
                     // W_b row (m, rank of r, level of c in m) against Phi of c without m
                     const int64_t x = cidx(wb_off[m * 4 + lc[b]] + rank3[3 * r + a], red3[3 * c + b]);
@@ -612,7 +615,8 @@ __global__ void __launch_bounds__(256) stein_unpack_kernel(const uint32_t* __res
                     const int en = voff[m + 1] - voff[m];
                     const int ra = rank3[3 * r + a], rb = rank3[3 * c + b];
                     const int64_t x = doff[m] + (int64_t)min(ra, rb) * en + max(ra, rb);
-                    for (int s = 0; s < dsplit; s++) t += D[s * dsize + x];
+#pragma unroll 8
+                    for (int s = s0; s < dsplit; s += kLanes) t += D[s * dsize + x];
                 }
                 val += t;
                 ns++;
@@ -629,11 +633,32 @@ __global__ void __launch_bounds__(256) stein_unpack_kernel(const uint32_t* __res
             }
             val /= (double)ns;
         }
+        return val;
+    };
+    auto finish = [&](double val, int r, int c) {
         val = val / divisor;
         if (diag && r == c) val = (val + diag[r]) + zpe;
         if (bad) val = __longlong_as_double(0x7ff8000000000000ll);     // a pass did not finish
-        v[y][x] = val;
         M[(size_t)c * ld + r] = val;
+        return val;
+    };
+    if constexpr (kLanes > 1) {
+        // element e of the upper triangle, by columns: c (c + 1) / 2 <= e
+        const int e = (blockIdx.x * 256 + threadIdx.x) / kLanes;
+        int c = (int)((sqrtf(8.0f * e + 1.0f) - 1.0f) * 0.5f);
+        while (c * (c + 1) / 2 > e) c--;
+        while ((c + 1) * (c + 2) / 2 <= e) c++;
+        const int r = e - c * (c + 1) / 2;
+        double val = c < nb ? element(r, c) : 0.0;
+#pragma unroll
+        for (int o = kLanes / 2; o; o >>= 1) val += __shfl_xor_sync(0xffffffffu, val, o);
+        if (s0 == 0 && c < nb) M[(size_t)r * ld + c] = finish(val, r, c);
+        return;
+    }
+    for (int y = y8; y < kY; y += 8) {
+        const int r = r0 + x, c = c0 + y;
+        if (r >= nb || c >= nb || r > c) continue;
+        v[y][x] = finish(element(r, c), r, c);
     }
     __syncthreads();
     for (int e = threadIdx.x; e < 32 * kY; e += 256) {
@@ -1085,15 +1110,19 @@ int stein_unpack(const SteinPlan& p, const uint32_t* desc, double divisor, const
     const int nblk = (p.nb + 31) / 32;
     const unsigned grid = (unsigned)(nblk * (nblk + 1) / 2);
     const bool fine = grid < 600;       // fewer CTAs than a GPU holds: a quarter of the columns each
-    auto kern = p.split ? (fine ? stein_unpack_kernel<8, false> : stein_unpack_kernel<32, false>)
-                        : (fine ? stein_unpack_kernel<8, true> : stein_unpack_kernel<32, true>);
+    const bool many = std::max(p.nsplit, p.tcpairs ? 1 : p.dsplit) >= 16;
+    const int lanes = many && p.nb <= 128 ? 32 : many && p.nb <= 256 ? 8 : 1;
+    auto kern = lanes == 32 ? (p.split ? stein_unpack_kernel<8, false, 32> : stein_unpack_kernel<8, true, 32>)
+              : lanes == 8  ? (p.split ? stein_unpack_kernel<8, false, 8> : stein_unpack_kernel<8, true, 8>)
+              : fine        ? (p.split ? stein_unpack_kernel<8, false> : stein_unpack_kernel<8, true>)
+                            : (p.split ? stein_unpack_kernel<32, false> : stein_unpack_kernel<32, true>);
     if (p.split) {
         int err = 0;
         SCP3_CUDA(cudaMemcpyAsync(&err, p.err, sizeof(int), cudaMemcpyDeviceToHost, s));
         SCP3_CUDA(cudaStreamSynchronize(s));
         if (err) return fail(SCP3GPU_ERR_TIMEOUT, "tensor-core contraction: a bounded pipeline wait expired");
     }
-    kern<<<fine ? 4 * grid : grid, 256, 0, s>>>(desc, p.rank3, p.voff, p.doff, p.nb, p.nv, p.bpairs, p.nsplit, p.dsplit,
+    kern<<<lanes > 1 ? (p.nb * (p.nb + 1) / 2 * lanes + 255) / 256 : fine ? 4 * grid : grid, 256, 0, s>>>(desc, p.rank3, p.voff, p.doff, p.nb, p.nv, p.bpairs, p.nsplit, p.dsplit,
                                              p.split ? p.P : p.ip.partial, p.D, (int64_t)p.ntiles2 * 128 * 256, p.dsize,
                                              divisor, diag, zpe, M, ld, p.tile_of, p.red3,
                                              p.tcpairs ? p.wb_off : nullptr, p.nsum ? p.sum_off : nullptr,
