@@ -471,6 +471,9 @@ int scp3gpu_batch_create(const scp3gpu_config* cfgs, int ncl, int64_t chunk, int
         }
         if ((rc = upload(&b->desc_dev[i], d.data(), d.size()))) return bail(rc);
     }
+    // the tables' copies and the operand's clearing run on the default stream, for which the
+    // batch's streams do not wait
+    if (cudaStreamSynchronize(cudaStreamLegacy) != cudaSuccess) return bail(fail(SCP3GPU_ERR_CUDA, "batch create sync failed"));
     SCP3_CUDA(cudaEventRecord(b->args_copied, b->stream));
     if ((rc = zero_sums(b))) return bail(rc);
     if (!(flags & SCP3GPU_BATCH_NO_AUTOTUNE)) {

@@ -1024,8 +1024,6 @@ int create(Plan& p, const std::vector<uint32_t>& tspec, const std::vector<uint32
             if (dual) SCP3_CUDA(cudaMemset(p.x + (rb + dual / kTile) * block, 0, block));
         }
     SCP3_CUDA(cudaMemset(p.filled, 0, sizeof(int) * ((size_t)p.nsplit * p.ntiles + 1)));
-    // the handle's streams do not wait for the default stream, where these run
-    SCP3_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
     return SCP3GPU_OK;
 }
 

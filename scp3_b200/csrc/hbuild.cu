@@ -651,6 +651,9 @@ int scp3gpu_hbuild_create(const scp3gpu_config* c, scp3gpu_hbuild** out)
                 return bail(rc);
         }
     }
+    // the tables' copies and the clearing of buffers run on the default stream, for which the
+    // handle's streams do not wait
+    if (cudaStreamSynchronize(cudaStreamLegacy) != cudaSuccess) return bail(fail(SCP3GPU_ERR_CUDA, "create sync failed"));
     if ((rc = zero_sums(h))) return bail(rc);
     if (cudaStreamSynchronize(h->stream) != cudaSuccess) return bail(fail(SCP3GPU_ERR_CUDA, "create sync failed"));
     *out = h;
@@ -783,6 +786,7 @@ static int build_dense(scp3gpu_hbuild* h, int mode, double* dst = nullptr, int64
         if (!h->hodiag) {
             const std::vector<double> d = ho_diagonal(h->omega_sel, h->cfg.n2, h->cfg.n3);
             if ((rc = upload(&h->hodiag, d.data(), d.size()))) return rc;
+            SCP3_CUDA(cudaStreamSynchronize(cudaStreamLegacy));     // h->stream does not wait for the copy
         }
         diag = h->hodiag;
         divisor = (double)h->count;

@@ -806,7 +806,9 @@ int scp3gpu_mlp_create(int n_in, int hidden, int max_batch, uint64_t seed, int d
             return fail(SCP3GPU_ERR_CUDA, "mlp init copy failed");
         }
     }
-    if ((rc = m->net.sync_bf16(m->s)) || cudaStreamSynchronize(m->s) != cudaSuccess) {
+    // these copies and alloc()'s clearing run on the default stream, for which m->s does not wait
+    if (cudaStreamSynchronize(cudaStreamLegacy) != cudaSuccess) rc = fail(SCP3GPU_ERR_CUDA, "mlp init failed");
+    if (rc || (rc = m->net.sync_bf16(m->s)) || cudaStreamSynchronize(m->s) != cudaSuccess) {
         scp3gpu_mlp_destroy(m);
         return rc ? rc : fail(SCP3GPU_ERR_CUDA, "mlp init failed");
     }
@@ -850,6 +852,7 @@ int scp3gpu_mlp_set_params(scp3gpu_mlp* m, const float* p, int64_t n)
         SCP3_CUDA(cudaMemcpy(m->net.b[l], p, sizeof(float) * m->net.out[l], cudaMemcpyHostToDevice));
         p += m->net.out[l];
     }
+    SCP3_CUDA(cudaStreamSynchronize(cudaStreamLegacy));      // m->s does not wait for these copies
     int rc = m->net.sync_bf16(m->s);
     if (rc) return rc;
     SCP3_CUDA(cudaStreamSynchronize(m->s));

@@ -209,7 +209,8 @@ int scp3gpu_scp1_create(int pes, int nw, int64_t chunk, int device, scp3gpu_scp1
         return rc;
     }
     if (cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaMemsetAsync(h->capped, 0, sizeof(*h->capped), h->stream) != cudaSuccess) {
+        cudaMemsetAsync(h->capped, 0, sizeof(*h->capped), h->stream) != cudaSuccess ||
+        cudaStreamSynchronize(cudaStreamLegacy) != cudaSuccess) {     // the table's copy
         free_all(h);
         delete h;
         return fail(SCP3GPU_ERR_CUDA, "scp1: stream creation failed");

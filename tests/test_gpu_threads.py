@@ -99,3 +99,52 @@ def test_new_handle_beside_default_stream_work(api):
     finally:
         stop.set()
         t.join()
+
+
+@pytest.mark.parametrize("kind", ["bf16x3", "gradient_bf16x3", "gradient_fp64", "batch", "network", "scp1"])
+def test_new_handles_of_every_form_beside_default_stream_work(api, kind):
+    """As above for the handles whose tables or operands are cleared or copied to on the
+    default stream: their first result is an old handle's, bit for bit."""
+    import torch
+    from scp3_b200 import inputs, surrogate
+    rng = np.random.default_rng(0)
+    q, t = rng.normal(size=(512, 48)).astype(np.float32), rng.normal(size=512).astype(np.float32)
+    nw, x0, MUa, omega = inputs.load("cluster_6_100")
+
+    def first():
+        if kind == "batch":
+            b = api.Batch([dict(nw=nw, x0=x0, MUa=MUa, omega=omega)] * 2)
+            b.accumulate(100, 5000)
+            out = b.read(1)
+        elif kind == "network":
+            b = surrogate.MLP(48, 256, 512)
+            b.set_params(b.get_params()[::-1].copy())
+            out = np.append(b(q), b.loss_and_grad(q, t)[1])
+        elif kind == "scp1":
+            b = api.SCP1Average("qtip4pf", nw)
+            out = b.sums(x0, np.full(54, 0.5), np.eye(54) * 0.03, 5, 0, 500)[2]
+        else:
+            b = build(api, "cluster_6_100", kind.split("_")[-1], "gradient" if "_" in kind else "direct", 48, 10, 0)
+            b.accumulate(100, 5000)
+            out = b.read(1)
+        b.close()
+        return out
+
+    want = first()
+    stop = threading.Event()
+
+    def busy():
+        a = torch.randn(4096, 4096, device="cuda")
+        while not stop.is_set():
+            for _ in range(20):
+                torch.mm(a, a)
+            torch.cuda.current_stream().synchronize()
+
+    th = threading.Thread(target=busy)
+    th.start()
+    try:
+        for _ in range(6):
+            assert np.array_equal(first(), want)
+    finally:
+        stop.set()
+        th.join()
