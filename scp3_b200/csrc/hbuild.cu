@@ -817,7 +817,17 @@ int scp3gpu_hbuild_read_dev(scp3gpu_hbuild* h, double* M_dev, int64_t ld, int mo
     (void)cudaGetLastError();   // a pending error of an earlier, unrelated call is not this call's
     if (!h || !M_dev || ld < h->nb || (mode != 0 && mode != 1)) return fail(SCP3GPU_ERR_ARG, "read_dev: bad arguments");
     DeviceGuard g(h->dev);
-    return build_dense(h, mode, M_dev, ld);
+    // The kernels write to memory of this device; other memory that the driver knows (another
+    // device's, pinned) takes a copy, and a pointer that it does not know no kernel may follow.
+    cudaPointerAttributes at{};
+    SCP3_CUDA(cudaPointerGetAttributes(&at, M_dev));
+    if (at.type == cudaMemoryTypeUnregistered) return fail(SCP3GPU_ERR_ARG, "read_dev: not device memory");
+    if (at.type == cudaMemoryTypeManaged || (at.type == cudaMemoryTypeDevice && at.device == h->dev))
+        return build_dense(h, mode, M_dev, ld);
+    if (int rc = build_dense(h, mode)) return rc;
+    SCP3_CUDA(cudaMemcpy2DAsync(M_dev, sizeof(double) * ld, h->dense, sizeof(double) * h->nb, sizeof(double) * h->nb,
+                                h->nb, cudaMemcpyDefault, h->stream));
+    return SCP3GPU_OK;
 }
 
 int scp3gpu_hbuild_eigvals(scp3gpu_hbuild* h, int64_t nsub, int k, double* evals)
