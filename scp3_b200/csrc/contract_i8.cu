@@ -145,8 +145,19 @@ constexpr int kLimitThreads = kLimitSamples * kLimitValues;
 
 __device__ __forceinline__ int high_word(double x) { return __double2hiint(x) & 0x7fffffff; }
 
-// Limits of V, q and dV/dq, kLimitValues of these per block, from samples spread over the
-// pass; zeros (padding samples among them) and values that are not finite do not count,
+// Sample j of the ns that the limits are taken from: one at a scattered place in each of
+// ns parts of a pass of k.  Not every (k / ns)-th: Sobol points a power of two apart agree in
+// their first digits, so that a coordinate of all of them may lie next to zero (hexamer, 2^17
+// samples from some first points on: 9.1 ms instead of 4.1, most samples being over the limit).
+__host__ __device__ __forceinline__ long long limit_sample(int j, int ns, long long k)
+{
+    const long long lo = k * j / ns, hi = k * (j + 1) / ns;
+    uint32_t h = (uint32_t)(j + 1) * 2654435769u;
+    h = (h ^ (h >> 15)) * 2246822519u;
+    return lo + (long long)((h ^ (h >> 13)) % (uint32_t)(hi - lo));
+}
+
+// Limits of V, q and dV/dq, kLimitValues of these per block, from limit_sample()s; zeros (padding samples among them) and values that are not finite do not count,
 // and with nothing left any value but zero is over the limit.  The high word is the
 // logarithm's piecewise linear form, so the sums are integers.  The blocks from lblocks on
 // clear rowmax.
@@ -169,7 +180,7 @@ __global__ void __launch_bounds__(kLimitThreads) limits_kernel(const double* __r
     const int j = t / kLimitValues, i = (int)blockIdx.x * kLimitValues + t % kLimitValues;
     int h = 0;
     if (j < ns && i < nq) {
-        const long long s = k * j / ns;
+        const long long s = limit_sample(j, ns, k);
         h = high_word(i == 0 ? v[s] : i <= nm ? q[s * nm + i - 1] : vq[s * nm + i - 1 - nm]);
     }
     if (h > 0 && h < 0x7ff00000) {
@@ -1128,6 +1139,13 @@ int check(const Plan& p, cudaStream_t s)
 
 }  // namespace i8
 }  // namespace scp3
+
+// Host-only view of the limits' samples, for tests: sample j of a pass of k, -1 past the last.
+extern "C" int64_t scp3gpu_internal_limit_sample(int j, int64_t k)
+{
+    const int ns = (int)std::min<int64_t>(scp3::i8::kLimitSamples, k);
+    return j < 0 || j >= ns ? -1 : scp3::i8::limit_sample(j, ns, k);
+}
 
 // Host-only view of the rule for passes of few samples, for tests: the sample ranges of a
 // pass of k samples in FP64, 0 for the digits.
