@@ -118,14 +118,15 @@ struct TailTable {
 };
 __device__ TailTable kTail;
 
-// Interval of x, 0 .. kTailSpans - 1; -1 where the table has none: below 1.5, past the
-// last one, and for a NaN (coincident sites, coordinates that are not finite).  Two
-// intervals per octave: exponent and first bit of the fraction, from 1.5 on.
 template <typename T>
-__host__ __device__ __forceinline__ int tail_span(T x)
+__host__ __device__ __forceinline__ constexpr T tail_end() { return T(sizeof(T) == 4 ? 17.0 : 37.0); }
+
+// Interval of x, 0 .. kTailSpans - 1, for 1.5 <= x <= tail_end(): two per octave, exponent
+// and first bit of the fraction, from 1.5 on.
+template <typename T>
+__host__ __device__ __forceinline__ int tail_interval(T x)
 {
     constexpr bool F = sizeof(T) == 4;
-    if (!(x >= T(1.5) && x <= T(F ? 17.0 : 37.0))) return -1;
 #ifdef __CUDA_ARCH__
     if constexpr (F) return (__float_as_int(x) >> 22) - 255;
     else return (__double2hiint(x) >> 19) - 2047;
@@ -143,11 +144,22 @@ __host__ __device__ __forceinline__ int tail_span(T x)
 #endif
 }
 
+// Which form smear_tail takes: the interval, -1 the series below 1.5, -2 none.  Only -2 can
+// be a NaN (coincident sites, coordinates that are not finite).
+template <typename T>
+__host__ __device__ __forceinline__ int tail_span(T x)
+{
+    if (!(x <= tail_end<T>())) return -2;
+    return x < T(1.5) ? -1 : tail_interval(x);
+}
+
 template <typename T>
 __device__ __forceinline__ T smear_tail(T x, T e1, T x13)
 {
     constexpr bool F = sizeof(T) == 4;
-    if (x < T(1.5)) {
+    const int i = tail_span(x);
+    if (i == -2) return x > T(1.5) ? T(0) : x;     // past the table; a NaN stays one
+    if (i == -1) {
         T s = T(0);
 #pragma unroll
         for (int n = F ? 14 : 22; n >= 0; n--) {
@@ -156,8 +168,6 @@ __device__ __forceinline__ T smear_tail(T x, T e1, T x13)
         }
         return e1 * (T(1) + x * s) - x13 * T(kGamma23);
     }
-    const int i = tail_span(x);
-    if (i < 0) return x > T(1.5) ? T(0) : x;       // past the table; a NaN stays one
     T s;
     if constexpr (F) {
         const T t = x * __ldg(kTail.scalef + i) - __ldg(kTail.shiftf + i);

@@ -713,7 +713,7 @@ int launch_std_normal(int dims, int64_t index0, int64_t n, const int64_t* vdir, 
 // up in, -1 where the table is not read.
 extern "C" int scp3gpu_internal_tail_span(double x, int fp32)
 {
-    return fp32 ? scp3::ttm::tail_span((float)x) : scp3::ttm::tail_span(x);
+    return std::max(-1, fp32 ? scp3::ttm::tail_span((float)x) : scp3::ttm::tail_span(x));
 }
 
 // Host-only view of the water-pair items of the four-sample qTIP4P/f kernels, for
