@@ -23,10 +23,10 @@
 // small.  Samples whose |V|, |q_m| or |dV/dq_m| is more than 2^9, 2^4 and 2^9 times that
 // quantity's geometric mean over 128 samples of the pass, or not finite, are therefore left
 // out of the digits (zero) and of the scales, and their products added in FP64 at the end
-// of contract_i8_kernel (add_heavy).  2^4 lies above every point of the Sobol sequence
-// (|q| < 6.3), 2^9 above the largest |V| of 2^17 points of the clusters looked at (8 to 490
-// times the mean), so ordinary builds have such samples rarely or not at all: the limits
-// cost a launch of 4 us in place of a memset.  One V of 2^14 at 1, 10^2, 10^3, 10^6 and
+// of contract_i8_kernel (add_heavy).  2^4 times the mean of 128 coordinates (0.28 to 0.34)
+// is 4.5 or more, which one in 10^9 passes, 2^9 above the largest |V| of 2^17 points of the
+// clusters looked at (8 to 490 times the mean), so ordinary builds have such samples rarely
+// or not at all: the limits cost a launch of 4 us in place of a memset.  One V of 2^14 at 1, 10^2, 10^3, 10^6 and
 // 10^12 times the others' rms, elements in which it vanishes, largest error over the sum
 // of |terms|: 2.8e-17, 8.7e-17, 2.8e-17, 2.8e-17, 2.8e-17 (an FP64 product 5.7e-17 in each;
 // without the limits 4.9e-17, 2.1e-16, 2.2e-15, 1.5e-12, 1.9e-6).  Hexamer, 2^16 samples,

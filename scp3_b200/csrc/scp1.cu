@@ -12,8 +12,8 @@
 //
 // Two kernels per chunk of samples:
 //   scp1_samples_kernel   (sampling.cu, beside the potentials' constant tables)
-//                         one warp per sample (contiguous, balanced ranges per
-//                         warp, Gray-code Sobol walk), isqrtM_U staged in
+//                         four samples per warp (contiguous, balanced ranges
+//                         per warp, Gray-code Sobol walk), isqrtM_U staged in
 //                         shared memory, the potential's energy and gradient
 //                         (the same warp code as the gradient estimator); writes
 //                         V, g and dq per sample.

@@ -1,6 +1,7 @@
 // The gradient (default) estimator of SCP3: addEpot(q, V, Vq, M)
-// (ScaledMatrixElements.cpp:102-725 with the formulas of TripleExcitations.h),
-// FP64, as dense products on the FP64 pipe.
+// (ScaledMatrixElements.cpp:102-725 with the formulas of TripleExcitations.h), as dense
+// products on the tensor cores: of FP64 values by their digits (contract_i8.cu), or BF16x3
+// (contract_tc.cu).
 //
 // Every formula of the reference follows one rule.  For the pair (i, j) let S be
 // the modes either function excites and p_m(q_m) = h_a(q_m) h_b(q_m) the
@@ -21,10 +22,11 @@
 //     T^m_ij = sum_s [R_i^m K^m_a0](s) Phi_j(s)
 // is one row of a product W Phi^T, with one "virtual row" W_(m,i) = R_i^m K^m_a0
 // per (mode, function exciting it): 2352 rows against 1225 columns for the
-// hexamer doubles basis, an FP64 GEMM (contract_fp64.cu, rectangular form).
+// hexamer doubles basis.
 // When both excite m, T^m_ij = sum_s R_i^m R_j^m K^m_ab is a pair sum over the
-// functions exciting m, kept per mode (stein_pairs_kernel; 48 x 49^2 pairs for
-// the hexamer doubles basis against 48 x 49 x 1225 products in the GEMM).  The
+// functions exciting m: products of the same operand where that pays (rows
+// W_b(m, i) = R_i^m K^m_ab against R_j^m, itself a basis function), else summed in
+// FP64 per mode (stein_pairs_kernel).  The
 // read-out forms each element from its |S| <= 6 terms and divides by |S|;
 // <0|V|0> comes from one more virtual row, W = V, against Phi_0 = 1.
 //
