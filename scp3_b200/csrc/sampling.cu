@@ -33,37 +33,50 @@ struct WarpSlot {
     T* ms;          // [group][3nw] M sites
     double* g;      // [group][9nw] gradients (gradient path)
     char* sc;       // TTM3-F scratch, after g
-    uint64_t* xs;   // [group][nm0] Sobol states of the group; with tl from crd on, dead once
-    uint16_t* tl;   // the normals are formed: [group * nm0] items of the inverse CDF's tail
+    uint64_t* xs;   // [group][nm0] Sobol states of the group; with tl from crd on (slot_bytes), dead
+    uint16_t* tl;   // once the normals are formed: [group * nm0] items of the inverse CDF's tail
     int qs;         // q stride: nm0 rounded up to even (16-byte aligned rows)
 };
 
 constexpr size_t round16(size_t b) { return (b + 15) & ~(size_t)15; }
 
+// A group's Sobol states share the bytes of its geometries and of what follows: staged beside
+// them they took large clusters a block per SM and L1 (16 waters, 2^16 samples: FP64 1264 us and
+// 1933, FP32 with its states behind the geometries 1045 and, over them, 884).  `apart`: behind
+// the sites all the same, for the batch's FP32 qTIP4P/f kernel, which spills with the
+// overlap (4096 samples of two clusters 72.5 us and 74.5).
 template <typename T>
-__host__ __device__ inline size_t slot_bytes(int pes, int nm0, int nw, bool grad = false)
+__host__ __device__ inline size_t slot_bytes(int pes, int nm0, int nw, bool grad = false, bool apart = false)
 {
     const size_t q = round16(sizeof(T) * kGroup * ((nm0 + 1) & ~1));
     const size_t normals = round16((size_t)kGroup * nm0 * (sizeof(uint64_t) + sizeof(uint16_t)));
-    const size_t geometry = round16(sizeof(T) * kGroup * 12 * (size_t)nw) +
-                            (grad ? round16(sizeof(double) * kGroup * 9 * (size_t)nw) : 0) +
-                            (pes == SCP3GPU_PES_TTM3F ? round16(ttm::scratch_bytes<T>(nw)) : 0);
-    return q + (normals > geometry ? normals : geometry);
+    const size_t geometry = round16(sizeof(T) * kGroup * 12 * (size_t)nw);
+    const size_t force = (grad ? round16(sizeof(double) * kGroup * 9 * (size_t)nw) : 0) +
+                         (pes == SCP3GPU_PES_TTM3F ? round16(ttm::scratch_bytes<T>(nw)) : 0);
+    if (apart) return q + geometry + (normals > force ? normals : force);
+    return q + (normals > geometry + force ? normals : geometry + force);
 }
 
-template <typename T>
-__device__ inline WarpSlot<T> warp_slot(char* base, int nm0, int nw, bool grad = false)
+// kChain: the pointers are formed one from the other, else from the base; the registers of
+// the TTM3-F instances decide (2^16 samples, hexamer: gradients FP64 1621 us one from the
+// other, 1706 from the base, FP32 1274 and 1360; energies FP64 890 and 916, FP32 424 and 397;
+// dimer, FP64 energies 389 and 370).
+template <typename T, bool kChain, bool kApart = false>
+__device__ inline WarpSlot<T> warp_slot(char* base, int nm0, int nw, bool grad)
 {
     WarpSlot<T> s;
     s.qs = (nm0 + 1) & ~1;
     s.q = reinterpret_cast<T*>(base);
-    char* over = base + round16(sizeof(T) * kGroup * s.qs);
-    s.crd = reinterpret_cast<T*>(over);
+    s.crd = s.q + (size_t)kGroup * s.qs;         // whole multiples of 16 bytes each, as the next
     s.ms = s.crd + 9 * nw * kGroup;
-    char* force = over + round16(sizeof(T) * kGroup * 12 * (size_t)nw);
-    s.g = reinterpret_cast<double*>(force);
-    s.sc = force + (grad ? round16(sizeof(double) * kGroup * 9 * (size_t)nw) : 0);
-    s.xs = reinterpret_cast<uint64_t*>(over);
+    if (kChain) {
+        s.g = reinterpret_cast<double*>(s.ms + 3 * nw * kGroup);
+        s.sc = reinterpret_cast<char*>(s.g + (grad ? 9 * nw * kGroup : 0));
+    } else {
+        s.g = nullptr;                           // no gradients there
+        s.sc = base + round16(sizeof(T) * kGroup * (s.qs + (size_t)(12 * nw)));
+    }
+    s.xs = kApart ? reinterpret_cast<uint64_t*>(s.sc) : reinterpret_cast<uint64_t*>(s.crd);
     s.tl = reinterpret_cast<uint16_t*>(s.xs + (size_t)kGroup * nm0);
     return s;
 }
@@ -188,7 +201,7 @@ struct Pair<float> {
 
 // G: the gradient path (dV/dq) is compiled in; the energy-only instances keep
 // their registers for the energy path.
-template <int PES, typename T, bool G = false, int NW = 8>
+template <int PES, typename T, bool G = false, int NW = 8, bool kApart = false>
 __device__ __forceinline__ void samples_body(const SampleArgs& a, char* smem);
 
 // Blocks per SM the registers must allow: qTIP4P/f, 4 for the FP32 energies (64
@@ -211,6 +224,9 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, sample_blocks<PES, T, G, 
     samples_body<PES, T, G, NW>(a, smem);
 }
 
+template <int PES, typename T>
+constexpr bool kBatchApart = PES == SCP3GPU_PES_QTIP4PF && sizeof(T) == 4;
+
 // Several clusters of a batch: cluster blockIdx.y takes args[blockIdx.y].
 template <int PES, typename T>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32, sample_blocks<PES, T, false>())
@@ -222,10 +238,10 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, sample_blocks<PES, T, fal
     __shared__ SampleArgs a;
     if (threadIdx.x == 0) a = args[blockIdx.y];
     __syncthreads();
-    samples_body<PES, T>(a, smem);
+    samples_body<PES, T, false, 8, kBatchApart<PES, T>>(a, smem);
 }
 
-template <int PES, typename T, bool G, int NW>
+template <int PES, typename T, bool G, int NW, bool kApart>
 __device__ __forceinline__ void samples_body(const SampleArgs& a, char* smem)
 {
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
@@ -257,7 +273,7 @@ __device__ __forceinline__ void samples_body(const SampleArgs& a, char* smem)
         __syncthreads();
     }
     char* slots = smem + (mua_in_smem ? mua_b : 0) + (muat_in_smem ? muat_smem_bytes(nw, a.nm) : 0);
-    WarpSlot<T> w = warp_slot<T>(slots + wib * slot_bytes<T>(PES, nm0, nw, grad), nm0, nw, grad);
+    WarpSlot<T> w = warp_slot<T, G || (sizeof(T) == 8 && NW == 8), kApart>(slots + wib * slot_bytes<T>(PES, nm0, nw, grad, kApart), nm0, nw, grad);
     // Each warp takes one contiguous range of samples, the ranges balanced to
     // within one sample (the grid is sized to the SMs, so there is no tail wave):
     // the Sobol state of the first is formed from the Gray code of its index, the
@@ -429,7 +445,7 @@ __global__ void __launch_bounds__(32) pes_kernel(int nw, int64_t n, const double
 {
     extern __shared__ __align__(16) char smem[];
     const int lane = threadIdx.x, N3 = 9 * nw;
-    const WarpSlot<double> w = warp_slot<double>(smem, 0, nw, G);
+    const WarpSlot<double> w = warp_slot<double, G>(smem, 0, nw, G);
     for (int64_t g0 = (int64_t)blockIdx.x * NG; g0 < n; g0 += (int64_t)gridDim.x * NG) {
         const int gn = (int)(n - g0 < NG ? n - g0 : NG);
         for (int c = lane; c < gn * N3; c += 32) w.crd[c] = crd[g0 * N3 + c];
@@ -465,7 +481,7 @@ __global__ void __launch_bounds__(kS1Warps * 32, PES == SCP3GPU_PES_TTM3F ? 1 : 
     double* U = s1;
     for (int e = threadIdx.x; e < dim * dim; e += blockDim.x) U[e] = a.U[e];
     char* slot = reinterpret_cast<char*>(s1) + round16(sizeof(double) * dim * dim) + (size_t)wib * scp1_slot(PES, nw, dim);
-    const WarpSlot<double> w = warp_slot<double>(slot, dim, nw, true);      // w.q: y = std_normal % sqrt(d)
+    const WarpSlot<double> w = warp_slot<double, true>(slot, dim, nw, true);      // w.q: y = std_normal % sqrt(d)
     double* dq = reinterpret_cast<double*>(slot + slot_bytes<double>(PES, dim, nw, true));   // [group][dim]
     __syncthreads();
     const int64_t nwarps = (int64_t)gridDim.x * kS1Warps;
@@ -578,7 +594,7 @@ int launch_samples_batch_t(const SampleArgs* args_host, const SampleArgs* args_d
         const size_t b = mua_smem_bytes<T>(args_host[c].nw, args_host[c].nm0);
         if (b <= kMuaSmemMax) mua = std::max(mua, b);
     }
-    const size_t sm = kWarpsPerBlock * slot_bytes<T>(PES, nm0, nw, false) + mua;
+    const size_t sm = kWarpsPerBlock * slot_bytes<T>(PES, nm0, nw, false, kBatchApart<PES, T>) + mua;
     if (int rc = allow_smem(samples_batch_kernel<PES, T>)) return rc;
     const int per = grid_for((n + kRun - 1) / kRun);   // per cluster; the clusters share the SMs
     samples_batch_kernel<PES, T><<<dim3((unsigned)per, (unsigned)ncl), kWarpsPerBlock * 32, sm, s>>>(args_dev);
