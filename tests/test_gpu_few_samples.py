@@ -213,3 +213,27 @@ def test_digits_not_finite(api):
     hb.add_epot(q, V)
     assert not np.isfinite(hb.read(0)).any()
     hb.close()
+
+
+def test_digits_gradient_not_finite(api):
+    """A NaN in dV/dq_m, or V = inf at a sample of digits: as FP64 sums have it."""
+    n = 16100
+    hb = handle(api, "gradient", 6, 6, 0)
+    rng = np.random.default_rng(12)
+    q, V, Vq = rng.normal(scale=np.sqrt(0.5), size=(n, 6)), rng.normal(size=n), rng.normal(size=(n, 6))
+    hb.add_epot_grad(q, V, Vq)
+    good = hb.read(0)
+    Vq[17, 2] = np.nan
+    hb.reset()
+    hb.add_epot_grad(q, V, Vq)
+    M = hb.read(0)
+    has = np.array([False] + [m == 2 for m in range(6)] * 2 + [2 in (m, k) for m in range(6) for k in range(m + 1, 6)])
+    assert np.isnan(M[has]).all()
+    clean = M[np.ix_(~has, ~has)]
+    # the marked sample's terms, added in FP64 now: a rounding each of sums of 1e5 at most
+    assert np.isfinite(clean).all() and np.abs(clean - good[np.ix_(~has, ~has)]).max() <= 1e-9
+    V[18] = np.inf
+    hb.reset()
+    hb.add_epot_grad(q, V, Vq)
+    assert not np.isfinite(hb.read(0)).any()
+    hb.close()
